@@ -16,10 +16,10 @@
 //
 // Parallelism.  A node row of the factor and of the forward substitution depends on
 // the rows of its lower blocks, a row of the backward substitution on those of its
-// upper blocks: rows are grouped by level (longest dependency chain) on the host.  The
-// factorisation runs one launch per level with a warp per node row; each substitution
-// is one persistent launch in which warps take rows in level order and wait on per-row
-// ready flags (see ilu_lower_sweep_kernel).  The preconditioner application is
+// upper blocks: rows are ordered by level (longest dependency chain) on the host.  The
+// factorisation (a CTA per node row) and each substitution (a warp per node row) are one
+// persistent launch each, which takes rows in level order and waits for single rows (see
+// ilu_factor_rows_kernel, ilu_sweep_kernel).  The preconditioner application is
 // captured once into a CUDA graph whose kernels take the Krylov vector's index from
 // device memory.  The Arnoldi step (two classical
 // Gram-Schmidt passes) uses blocked dot products with fixed partial-sum order, so
@@ -284,209 +284,11 @@ __global__ void ilu_factor_level_kernel(T* __restrict__ F, const int64_t* __rest
   if (lane < ND && D[lane * ND + lane] == T(0)) atomicOr(status, (unsigned)GALES_ERR_SINGULAR);
 }
 
-// The same factorisation step with the block row I and, for each lower block K, row
-// K's diagonal and upper blocks staged in shared memory (one warp per CTA): the row's
-// column search, its updates and the diagonal step then run on shared memory, and each
-// K costs one coalesced copy.  Same operations in the same order as above.
-template <int ND, typename T>
-__global__ void ilu_factor_level_smem_kernel(T* __restrict__ F, const int64_t* __restrict__ f_rp,
-                                             const int32_t* __restrict__ f_col, const int64_t* __restrict__ f_diag,
-                                             const int32_t* __restrict__ rows, int64_t count,
-                                             unsigned int* __restrict__ status, int max_row, int max_u) {
-  constexpr int BB = ND * ND;
-  extern __shared__ __align__(16) unsigned char sm_raw[];
-  T* R = reinterpret_cast<T*>(sm_raw);             // [max_row][BB] the block row
-  T* UK = R + (size_t)max_row * BB;                // [1 + max_u][BB] row K from its diagonal on
-  int32_t* RC = (int32_t*)(UK + (size_t)(1 + max_u) * BB);  // [max_row] the row's columns
-  int32_t* UC = RC + max_row;                      // [max_u] row K's upper columns
-  const int64_t w = blockIdx.x;
-  if (w >= count) return;
-  const int lane = threadIdx.x & 31;
-  const int32_t I = rows[w];
-  const int64_t p0 = f_rp[I], p1 = f_rp[I + 1];
-  const int nb = (int)(p1 - p0), bd = (int)(f_diag[I] - p0);
-  for (int64_t e = lane; e < (int64_t)nb * BB; e += 32) R[e] = F[p0 * BB + e];
-  for (int e = lane; e < nb; e += 32) RC[e] = f_col[p0 + e];
-  __syncwarp();
-  for (int b = 0; b < bd; ++b) {
-    const int32_t K = RC[b];
-    const int64_t dK = f_diag[K];
-    const int nu = (int)(f_rp[K + 1] - dK - 1);
-    for (int64_t e = lane; e < (int64_t)(nu + 1) * BB; e += 32) UK[e] = F[dK * BB + e];
-    for (int e = lane; e < nu; e += 32) UC[e] = f_col[dK + 1 + e];
-    __syncwarp();
-    T* B = R + (size_t)b * BB;
-    if (lane < ND) {
-      T row[ND];
-#pragma unroll
-      for (int c = 0; c < ND; ++c) row[c] = B[lane * ND + c];
-#pragma unroll
-      for (int c = 0; c < ND; ++c) {
-        T s = row[c];
-#pragma unroll
-        for (int c2 = 0; c2 < c; ++c2) s -= row[c2] * UK[c2 * ND + c];
-        row[c] = s / UK[c * ND + c];
-      }
-#pragma unroll
-      for (int c = 0; c < ND; ++c) B[lane * ND + c] = row[c];
-    }
-    __syncwarp();
-    const int items = nu * ND;
-    for (int it = lane; it < items; it += 32) {
-      const int qi = it / ND, r = it - qi * ND;
-      const int64_t pos = find_col(RC, b + 1, nb, UC[qi]);
-      if (pos < 0) continue;
-      T l[ND];
-#pragma unroll
-      for (int m = 0; m < ND; ++m) l[m] = B[r * ND + m];
-      const T* U = UK + (size_t)(1 + qi) * BB;
-      T* tgt = R + pos * BB + r * ND;
-#pragma unroll
-      for (int c = 0; c < ND; ++c) {
-        T s = tgt[c];
-#pragma unroll
-        for (int m = 0; m < ND; ++m) s -= l[m] * U[m * ND + c];
-        tgt[c] = s;
-      }
-    }
-    __syncwarp();
-  }
-  T* D = R + (size_t)bd * BB;
-  const int ncols = (nb - bd) * ND;
-  for (int r = 1; r < ND; ++r) {
-    for (int c2 = 0; c2 < r; ++c2) {
-      const T l = D[r * ND + c2] / D[c2 * ND + c2];
-      __syncwarp();
-      if (lane == 0) D[r * ND + c2] = l;
-      for (int e = lane; e < ncols; e += 32) {
-        const int bb = e / ND;
-        const int c = e - bb * ND;
-        if (bb == 0 && c <= c2) continue;
-        T* Rb = D + (size_t)bb * BB;
-        Rb[r * ND + c] -= l * Rb[c2 * ND + c];
-      }
-      __syncwarp();
-    }
-  }
-  for (int64_t e = lane; e < (int64_t)nb * BB; e += 32) F[p0 * BB + e] = R[e];
-  if (lane < ND && D[lane * ND + lane] == T(0)) atomicOr(status, (unsigned)GALES_ERR_SINGULAR);
-}
-
-// Block sums of one node row's lower (upper) blocks: lanes form G = 32 / ND groups of
-// ND; lane (g, r) accumulates row r over the blocks g, g + G, ...  The column indices of
-// up to 8 blocks per lane are loaded first, so that every block's loads are in flight at
-// once (a row's substitution is one dependency level, bound by memory latency).  The
-// group partial sums are added in group order (deterministic).
-template <int ND, typename T, bool L2Z = false>
-__device__ __forceinline__ T block_row_sum(const T* __restrict__ F, const int32_t* __restrict__ f_col, int64_t pa,
-                                           int64_t pb, const T* z, T* red) {
-  constexpr int BB = ND * ND, G = 32 / ND;
-  const int lane = threadIdx.x & 31;
-  const int g = lane / ND, r = lane - g * ND;
-  T s = 0;
-  if (g < G) {
-    for (int64_t base = pa + g; base < pb; base += 8 * G) {
-      int32_t cidx[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const int64_t p = base + (int64_t)k * G;
-        cidx[k] = p < pb ? f_col[p] : -1;
-      }
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        if (cidx[k] < 0) continue;
-        const T* B = F + (base + (int64_t)k * G) * BB + r * ND;
-        const T* zc = z + (int64_t)cidx[k] * ND;
-#pragma unroll
-        for (int c = 0; c < ND; ++c) s += B[c] * (L2Z ? __ldcg(zc + c) : zc[c]);
-      }
-    }
-  }
-  red[lane] = s;
-  __syncwarp();
-  T t = 0;
-  if (lane < ND)
-#pragma unroll
-    for (int q = 0; q < G; ++q) t += red[q * ND + lane];
-  __syncwarp();
-  return t;
-}
-
-// y_I = L_II^-1 (v_I - sum_K L_IK y_K), L_II unit lower: warp per node row.  The
-// working vector zw is the output column itself for an FP64 factor (zw_follows = 1) or
-// a T scratch vector.
-template <int ND, typename T>
-__global__ void ilu_lower_level_kernel(const T* __restrict__ F, const int64_t* __restrict__ f_rp,
-                                       const int32_t* __restrict__ f_col, const int64_t* __restrict__ f_diag,
-                                       const int32_t* __restrict__ rows, int64_t count, const double* vbase,
-                                       T* zwbase, const int* __restrict__ jidx, int64_t ld, int zw_follows) {
-  constexpr int BB = ND * ND;
-  __shared__ T red[kWarpsPerBlock][32];
-  const int64_t w = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-  if (w >= count) return;
-  const int lane = threadIdx.x & 31;
-  const int64_t off = jidx ? (int64_t)(*jidx) * ld : 0;
-  const double* v = vbase + off;
-  T* zw = zwbase + (zw_follows ? off : 0);
-  const int32_t I = rows[w];
-  const int64_t p0 = f_rp[I], pd = f_diag[I];
-  const int r = lane < ND ? lane : 0;
-  const T vi = (T)v[(int64_t)I * ND + r];
-  T s = vi - block_row_sum<ND, T>(F, f_col, p0, pd, zw, red[threadIdx.x >> 5]);
-  const T* D = F + pd * BB + r * ND;
-#pragma unroll
-  for (int c = 0; c < ND - 1; ++c) {
-    const T zc = __shfl_sync(0xffffffffu, s, c);
-    if (lane > c) s -= D[c] * zc;
-  }
-  if (lane < ND) zw[(int64_t)I * ND + lane] = s;
-}
-
-// x_I = U_II^-1 (y_I - sum_J U_IJ x_J), in place on zw; with a scratch zw the row is
-// also written to the FP64 output column.
-template <int ND, typename T>
-__global__ void ilu_upper_level_kernel(const T* __restrict__ F, const int64_t* __restrict__ f_rp,
-                                       const int32_t* __restrict__ f_col, const int64_t* __restrict__ f_diag,
-                                       const int32_t* __restrict__ rows, int64_t count, T* zwbase,
-                                       double* zoutbase, const int* __restrict__ jidx, int64_t ld, int zw_follows) {
-  constexpr int BB = ND * ND;
-  __shared__ T red[kWarpsPerBlock][32];
-  const int64_t w = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-  if (w >= count) return;
-  const int lane = threadIdx.x & 31;
-  const int64_t off = jidx ? (int64_t)(*jidx) * ld : 0;
-  T* zw = zwbase + (zw_follows ? off : 0);
-  double* zout = zoutbase + off;
-  const int32_t I = rows[w];
-  const int64_t p1 = f_rp[I + 1], pd = f_diag[I];
-  const int r = lane < ND ? lane : 0;
-  const T yi = zw[(int64_t)I * ND + r];
-  T s = yi - block_row_sum<ND, T>(F, f_col, pd + 1, p1, zw, red[threadIdx.x >> 5]);
-  const T* D = F + pd * BB + r * ND;
-#pragma unroll
-  for (int c = ND - 1; c >= 0; --c) {
-    const T mine = s / D[c];  // meaningful on lane c only
-    const T xc = __shfl_sync(0xffffffffu, mine, c);
-    if (lane == c) s = xc;
-    else if (lane < c) s -= D[c] * xc;
-  }
-  if (lane < ND) {
-    zw[(int64_t)I * ND + lane] = s;
-    if (!zw_follows) zout[(int64_t)I * ND + lane] = (double)s;
-  }
-}
-
-// Sync-free substitutions: one persistent launch per triangle instead of one launch per
-// level.  A warp claims node rows from a ticket counter in level order (rows[] lists
-// them level by level), waits until the rows of its row's lower (upper) blocks are
-// marked ready, substitutes exactly as the level kernels do, and marks its row ready.
-// A warp only ever waits on rows of earlier levels, whose tickets were claimed before
-// its own by warps that are running, so the sweep always progresses; every wait is
-// still bounded (kSpinMax polls), after which GALES_ERR_TIMEOUT is set in the status
-// word and the row is left as it stands.  One lane writes a finished row and releases
-// its flag; waiting lanes acquire the flags and then read the rows from L2 (the
-// writer's L1 is not this SM's).  The row's factor blocks are prefetched into L1 before
-// it waits, so that only the dependent loads remain on the critical path.
+// Waits of the persistent kernels below.  A CTA or warp claims rows from a ticket counter
+// in level order (rows[] lists them level by level) and only ever waits on rows of earlier
+// levels, whose tickets were claimed before its own by CTAs or warps that are running, so
+// these kernels always progress; every wait is still bounded (kSpinMax polls), after which
+// GALES_ERR_TIMEOUT is set in the status word and the row goes on with what it has.
 constexpr long long kSpinMax = 1ll << 22;
 
 __device__ __forceinline__ int ld_acquire(const int* f) {
@@ -505,112 +307,309 @@ __device__ __forceinline__ bool wait_flag(const int* f) {
   return false;
 }
 
-// Prefetch into L1 the factor blocks rows [pa, pb) that lane (g, r) of block_row_sum
-// will read (and their column indices), before the row waits on its dependencies.
-template <int ND, typename T>
-__device__ __forceinline__ void prefetch_row(const T* __restrict__ F, const int32_t* __restrict__ f_col, int64_t pa,
-                                             int64_t pb) {
-  constexpr int BB = ND * ND, G = 32 / ND;
-  const int lane = threadIdx.x & 31;
-  const int g = lane / ND, r = lane - g * ND;
-  if (g < G)
-    for (int64_t p = pa + g; p < pb; p += G) {
-      const T* row = F + p * BB + r * ND;
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(row));
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(row + ND - 1));
-    }
-  for (int64_t p = pa + lane; p < pb; p += 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(f_col + p));
+template <typename T>
+__device__ __forceinline__ void cp_async_word(T* dst, const T* src) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  if constexpr (sizeof(T) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
 }
 
+// Shared memory of one factorisation CTA: the block row I, two buffers with a row K's
+// diagonal and upper blocks, the row's columns and, per buffer, the upper blocks of row K
+// that row I has (their index in row K and their position in row I).
 template <int ND, typename T>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock)
-    ilu_lower_sweep_kernel(const T* __restrict__ F, const int64_t* __restrict__ f_rp, const int32_t* __restrict__ f_col,
+struct FactorSmem {
+  static constexpr int BB = ND * ND;
+  static size_t bytes(int max_row, int max_u) {
+    return ((size_t)max_row + 2 * (1 + (size_t)max_u)) * BB * sizeof(T) +
+           ((size_t)max_row + 4 * (size_t)max_u) * sizeof(int32_t);
+  }
+};
+
+// The numeric factorisation in one persistent launch, a CTA per node row I.  For its lower
+// blocks K in ascending order: L_IK = A_IK U_KK^-1 (row-wise substitution, lane r < ND of
+// warp 0 owns row r), then A_IJ -= L_IK U_KJ for the upper blocks J of row K present in row
+// I (a thread per entry), then the Doolittle step of the diagonal block applied across the
+// whole block row, pivot by pivot.  Every entry sees the subtractions of the scalar ikj
+// order, unfused.
+// Bound: the FP64 pipe (2 lanes per SM and clock) by the ~49 ND multiply-subtract pairs of
+// each (K, J), and the chain of rows.  A row waits for row K only when it reaches K, so the
+// long part of its work runs while its last neighbours are still in progress, and the next
+// K's blocks are copied to shared memory (cp.async) during the current update when that row
+// is done already.  One warp per row and one launch per level (all of a row's inputs final
+// before it starts) took 725 ms on the 157k-node tet system; a level has ~210 rows, too few
+// warps for the FP64 pipes of 152 SMs.
+constexpr int kFactorThreads = 128;
+
+template <int ND, typename T>
+__global__ void __launch_bounds__(kFactorThreads)
+    ilu_factor_rows_kernel(T* __restrict__ F, const int64_t* __restrict__ f_rp, const int32_t* __restrict__ f_col,
                            const int64_t* __restrict__ f_diag, const int32_t* __restrict__ rows, int64_t n,
-                           const double* vbase, T* zwbase, const int* __restrict__ jidx, int64_t ld, int zw_follows,
-                           unsigned int* ticket, int* ready, unsigned int* status) {
+                           unsigned int* ticket, int* ready, unsigned int* __restrict__ status, int max_row,
+                           int max_u) {
   constexpr int BB = ND * ND;
-  __shared__ T red[kWarpsPerBlock][32];
-  const int lane = threadIdx.x & 31;
-  const int64_t off = jidx ? (int64_t)(*jidx) * ld : 0;
-  const double* v = vbase + off;
-  T* zw = zwbase + (zw_follows ? off : 0);
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  T* R = reinterpret_cast<T*>(sm_raw);                      // [max_row][BB] the block row
+  T* UB = R + (size_t)max_row * BB;                         // [2][1 + max_u][BB] row K from its diagonal on
+  int32_t* RC = (int32_t*)(UB + 2 * (size_t)(1 + max_u) * BB);  // [max_row] the row's columns
+  int32_t* MQ = RC + max_row;                               // [2][max_u] matching blocks: index in row K
+  int32_t* MP = MQ + 2 * max_u;                             // [2][max_u] and position in row I
+  __shared__ int nm[2], s_row, s_next;
+  __shared__ T ls[ND];
+  const int tid = threadIdx.x;
   for (;;) {
-    unsigned int t = 0;
-    if (lane == 0) t = atomicAdd(ticket, 1u);
-    t = __shfl_sync(0xffffffffu, t, 0);
-    if ((int64_t)t >= n) break;
-    const int32_t I = rows[t];
-    const int64_t p0 = f_rp[I], pd = f_diag[I];
-    prefetch_row<ND, T>(F, f_col, p0, pd + 1);
-    bool ok = true;
-    for (int64_t p = p0 + lane; p < pd && ok; p += 32) ok = wait_flag(ready + f_col[p]);
-    if (!ok) atomicOr(status, (unsigned)GALES_ERR_TIMEOUT);
-    __syncwarp();
-    const int r = lane < ND ? lane : 0;
-    const T vi = (T)v[(int64_t)I * ND + r];
-    T s = vi - block_row_sum<ND, T, true>(F, f_col, p0, pd, zw, red[threadIdx.x >> 5]);
-    const T* D = F + pd * BB + r * ND;
-#pragma unroll
-    for (int c = 0; c < ND - 1; ++c) {
-      const T zc = __shfl_sync(0xffffffffu, s, c);
-      if (lane > c) s -= D[c] * zc;
+    if (tid == 0) {
+      const unsigned int t = atomicAdd(ticket, 1u);
+      s_row = (int64_t)t < n ? rows[t] : -1;
+      nm[0] = nm[1] = 0;
     }
-    // lane 0 writes the row, then releases its ready flag
-    T row[ND];
+    __syncthreads();
+    const int32_t I = s_row;
+    if (I < 0) break;
+    const int64_t p0 = f_rp[I];
+    const int nb = (int)(f_rp[I + 1] - p0), bd = (int)(f_diag[I] - p0);
+    for (int e = tid; e < nb * BB; e += kFactorThreads) R[e] = F[p0 * BB + e];
+    for (int e = tid; e < nb; e += kFactorThreads) RC[e] = f_col[p0 + e];
+    __syncthreads();
+    // starts the copy of lower block b's row K into buffer b & 1 and lists its matches
+    auto load = [&](int b) {
+      const int64_t dK = f_diag[RC[b]];
+      const int nu = (int)(f_rp[RC[b] + 1] - dK - 1), buf = b & 1;
+      T* U = UB + (size_t)buf * (1 + max_u) * BB;
+      for (int e = tid; e < (nu + 1) * BB; e += kFactorThreads) cp_async_word(U + e, F + dK * BB + e);
+      for (int q = tid; q < nu; q += kFactorThreads) {
+        const int pos = (int)find_col(RC, b + 1, nb, f_col[dK + 1 + q]);
+        if (pos < 0) continue;
+        const int at = atomicAdd(&nm[buf], 1);
+        MQ[buf * max_u + at] = q;
+        MP[buf * max_u + at] = pos;
+      }
+    };
+    bool have = false;
+    for (int b = 0; b < bd; ++b) {
+      const int buf = b & 1;
+      if (!have) {
+        if (tid == 0 && !wait_flag(ready + RC[b])) atomicOr(status, (unsigned)GALES_ERR_TIMEOUT);
+        __syncthreads();
+        load(b);
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();
+      const T* UK = UB + (size_t)buf * (1 + max_u) * BB;
+      T* B = R + (size_t)b * BB;
+      if (tid < ND) {
+        T row[ND];
 #pragma unroll
-    for (int c = 0; c < ND; ++c) row[c] = __shfl_sync(0xffffffffu, s, c);
-    if (lane == 0) {
+        for (int c = 0; c < ND; ++c) row[c] = B[tid * ND + c];
 #pragma unroll
-      for (int c = 0; c < ND; ++c) zw[(int64_t)I * ND + c] = row[c];
+        for (int c = 0; c < ND; ++c) {
+          T s = row[c];
+#pragma unroll
+          for (int c2 = 0; c2 < c; ++c2) s -= row[c2] * UK[c2 * ND + c];
+          row[c] = s / UK[c * ND + c];
+        }
+#pragma unroll
+        for (int c = 0; c < ND; ++c) B[tid * ND + c] = row[c];
+      } else if (tid == 32) {
+        s_next = b + 1 < bd ? ld_acquire(ready + RC[b + 1]) : 0;
+        nm[buf ^ 1] = 0;
+      }
+      __syncthreads();
+      have = s_next != 0;
+      if (have) load(b + 1);
+      const int items = nm[buf] * BB;
+      for (int t = tid; t < items; t += kFactorThreads) {
+        const int i = t / BB, rc = t - i * BB, r = rc / ND, c = rc - r * ND;
+        const T* U = UK + (size_t)(1 + MQ[buf * max_u + i]) * BB + c;
+        T* tgt = R + (size_t)MP[buf * max_u + i] * BB + rc;
+        T s = *tgt;
+#pragma unroll
+        for (int m = 0; m < ND; ++m) s -= B[r * ND + m] * U[m * ND];
+        *tgt = s;
+      }
+      __syncthreads();
+    }
+    // Doolittle step of the diagonal block across the upper blocks: pivots c2 in order, all
+    // rows below a pivot at once
+    T* D = R + (size_t)bd * BB;
+    const int ncols = (nb - bd) * ND;
+    for (int c2 = 0; c2 < ND - 1; ++c2) {
+      const int nr = ND - 1 - c2;
+      if (tid < nr) {
+        const int r = c2 + 1 + tid;
+        const T l = D[r * ND + c2] / D[c2 * ND + c2];
+        D[r * ND + c2] = l;
+        ls[r] = l;
+      }
+      __syncthreads();
+      for (int t = tid; t < nr * ncols; t += kFactorThreads) {
+        const int rr = t / ncols, e = t - rr * ncols, r = c2 + 1 + rr;
+        const int bb = e / ND, c = e - bb * ND;
+        if (bb == 0 && c <= c2) continue;
+        T* Rb = D + (size_t)bb * BB;
+        Rb[r * ND + c] -= ls[r] * Rb[c2 * ND + c];
+      }
+      __syncthreads();
+    }
+    for (int e = tid; e < nb * BB; e += kFactorThreads) F[p0 * BB + e] = R[e];
+    if (tid < ND && D[tid * ND + tid] == T(0)) atomicOr(status, (unsigned)GALES_ERR_SINGULAR);
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();
       st_release(ready + I, 1);
     }
   }
 }
 
-template <int ND, typename T>
+// Triangular substitutions, one persistent launch per triangle, a warp per node row:
+//   lower  y_I = L_II^-1 (v_I - sum_K L_IK y_K), L_II unit lower
+//   upper  x_I = U_II^-1 (y_I - sum_J U_IJ x_J)
+// A sweep is a chain of levels (749 on the 157k-node tet system, ~210 rows each), so its
+// time is the latency of one level, not the bytes of the factor.  The words of the result
+// are their own ready flags: the result vector is filled with a bit pattern that no row
+// stores (kUnset, a NaN), lanes poll the words that they need with relaxed loads, which
+// leave L1 alone, and a finished row is stored without a fence.  A level is then one
+// store-to-load trip through L2 plus the row's own arithmetic; separate flags (release
+// store, acquire load, then the load of the values) cost three such trips, and an acquire
+// also empties the L1 that the factor had been prefetched into: 9.8 us a level with an FP32
+// factor, 14 us with FP64.  Before it polls, a row loads its factor blocks into registers:
+// lanes form G = 32 / ND groups of ND, lane (g, r) holds row r of the blocks g, g + G, ...
+// (KB at a time).  Blocks are taken in the order in which their rows finish (ascending for
+// the lower sweep, descending for the upper one), all first polls in flight together.  The
+// diagonal block's reciprocals and the scaling of its rows by them are formed before the
+// wait too, which leaves one multiply-add per unknown on the chain.
+template <typename T>
+struct SweepWord;
+template <>
+struct SweepWord<double> {
+  using Bits = unsigned long long;
+  static constexpr Bits kUnset = ~0ull, kNan = 0x7ff8000000000000ull;
+  static __device__ __forceinline__ Bits load(const double* p) {
+    Bits v;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+  }
+  static __device__ __forceinline__ void store(double* p, double x) {
+    Bits v = (Bits)__double_as_longlong(x);
+    if (v == kUnset) v = kNan;
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+  }
+  static __device__ __forceinline__ double value(Bits v) { return __longlong_as_double((long long)v); }
+};
+template <>
+struct SweepWord<float> {
+  using Bits = unsigned int;
+  static constexpr Bits kUnset = ~0u, kNan = 0x7fc00000u;
+  static __device__ __forceinline__ Bits load(const float* p) {
+    Bits v;
+    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+  }
+  static __device__ __forceinline__ void store(float* p, float x) {
+    Bits v = __float_as_uint(x);
+    if (v == kUnset) v = kNan;
+    asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+  }
+  static __device__ __forceinline__ float value(Bits v) { return __uint_as_float(v); }
+};
+
+__device__ __forceinline__ double sweep_fma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float sweep_fma(float a, float b, float c) { return fmaf(a, b, c); }
+
+// In (lower: the FP64 right-hand side vbase; upper: the lower sweep's result yin) and out
+// (zw, kUnset before the launch; upper: also the FP64 column zoutbase).  The ticket starts
+// at ~0u (it is cleared together with zw), so the first claim is row 0 of the order.
+template <int ND, typename T, bool LOWER>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock)
-    ilu_upper_sweep_kernel(const T* __restrict__ F, const int64_t* __restrict__ f_rp, const int32_t* __restrict__ f_col,
-                           const int64_t* __restrict__ f_diag, const int32_t* __restrict__ rows, int64_t n, T* zwbase,
-                           double* zoutbase, const int* __restrict__ jidx, int64_t ld, int zw_follows,
-                           unsigned int* ticket, int* ready, unsigned int* status) {
-  constexpr int BB = ND * ND;
-  __shared__ T red[kWarpsPerBlock][32];
+    ilu_sweep_kernel(const T* __restrict__ F, const int64_t* __restrict__ f_rp, const int32_t* __restrict__ f_col,
+                     const int64_t* __restrict__ f_diag, const int32_t* __restrict__ rows, int64_t n,
+                     const double* __restrict__ vbase, const T* __restrict__ yin, T* zw, double* zoutbase,
+                     const int* __restrict__ jidx, int64_t ld, unsigned int* ticket, unsigned int* status) {
+  using W = SweepWord<T>;
+  constexpr int BB = ND * ND, G = 32 / ND;
+  constexpr int KB = 56 / ND < 8 ? 56 / ND : 8;   // blocks per lane held in registers
   const int lane = threadIdx.x & 31;
+  const int g = lane / ND, r = lane < G * ND ? lane - g * ND : 0;
   const int64_t off = jidx ? (int64_t)(*jidx) * ld : 0;
-  T* zw = zwbase + (zw_follows ? off : 0);
-  double* zout = zoutbase + off;
   for (;;) {
     unsigned int t = 0;
-    if (lane == 0) t = atomicAdd(ticket, 1u);
+    if (lane == 0) t = atomicAdd(ticket, 1u) + 1u;
     t = __shfl_sync(0xffffffffu, t, 0);
     if ((int64_t)t >= n) break;
     const int32_t I = rows[t];
-    const int64_t p1 = f_rp[I + 1], pd = f_diag[I];
-    prefetch_row<ND, T>(F, f_col, pd, p1);
-    bool ok = true;
-    for (int64_t p = pd + 1 + lane; p < p1 && ok; p += 32) ok = wait_flag(ready + f_col[p]);
-    if (!ok) atomicOr(status, (unsigned)GALES_ERR_TIMEOUT);
-    __syncwarp();
-    const int r = lane < ND ? lane : 0;
-    const T yi = __ldcg(zw + (int64_t)I * ND + r);
-    T s = yi - block_row_sum<ND, T, true>(F, f_col, pd + 1, p1, zw, red[threadIdx.x >> 5]);
-    const T* D = F + pd * BB + r * ND;
+    const int64_t pd = f_diag[I];
+    const int64_t pa = LOWER ? f_rp[I] : pd + 1;
+    const int nblk = (int)((LOWER ? pd : f_rp[I + 1]) - pa);
+    // row r of the diagonal block and the right-hand side
+    T D[ND];
 #pragma unroll
-    for (int c = ND - 1; c >= 0; --c) {
-      const T mine = s / D[c];  // meaningful on lane c only
-      const T xc = __shfl_sync(0xffffffffu, mine, c);
-      if (lane == c) s = xc;
-      else if (lane < c) s -= D[c] * xc;
+    for (int c = 0; c < ND; ++c) D[c] = F[pd * BB + r * ND + c];
+    T s = LOWER ? (T)vbase[off + (int64_t)I * ND + r] : yin[(int64_t)I * ND + r];
+    T rd = T(1);
+    if constexpr (!LOWER) {
+      T dg = D[0];
+#pragma unroll
+      for (int c = 1; c < ND; ++c) dg = r == c ? D[c] : dg;
+      rd = T(1) / dg;
+#pragma unroll
+      for (int c = 0; c < ND; ++c) D[c] *= rd;
     }
-    if (!zw_follows && lane < ND) zout[(int64_t)I * ND + lane] = (double)s;
-    // lane 0 writes the row of the working vector, then releases its ready flag
-    T row[ND];
+    T sum = T(0);
+    bool late = false;
+    for (int k0 = 0; k0 < nblk; k0 += KB * G) {
+      int64_t zc[KB];
+      T B[KB][ND];
 #pragma unroll
-    for (int c = 0; c < ND; ++c) row[c] = __shfl_sync(0xffffffffu, s, c);
-    if (lane == 0) {
+      for (int k = 0; k < KB; ++k) {
+        const int i = k0 + k * G + g;
+        const bool on = g < G && i < nblk;
+        const int64_t p = pa + (LOWER ? i : nblk - 1 - i);
+        zc[k] = on ? (int64_t)f_col[p] * ND + r : -1;
 #pragma unroll
-      for (int c = 0; c < ND; ++c) zw[(int64_t)I * ND + c] = row[c];
-      st_release(ready + I, 1);
+        for (int c = 0; c < ND; ++c) B[k][c] = on ? F[p * BB + r * ND + c] : T(0);
+      }
+      typename W::Bits w[KB];
+#pragma unroll
+      for (int k = 0; k < KB; ++k) w[k] = zc[k] >= 0 ? W::load(zw + zc[k]) : typename W::Bits(0);
+#pragma unroll
+      for (int k = 0; k < KB; ++k) {
+        if (k0 + k * G >= nblk) break;   // the same for every lane
+        for (long long spin = 0; __any_sync(0xffffffffu, w[k] == W::kUnset); ++spin) {
+          if (spin >= kSpinMax) {
+            late = true;
+            break;
+          }
+          if (w[k] == W::kUnset) w[k] = W::load(zw + zc[k]);
+        }
+        const T zk = W::value(w[k]);
+#pragma unroll
+        for (int c = 0; c < ND; ++c)
+          sum = sweep_fma(B[k][c], __shfl_sync(0xffffffffu, zk, (g < G ? g : 0) * ND + c), sum);
+      }
+    }
+    if (late && lane == 0) atomicOr(status, (unsigned)GALES_ERR_TIMEOUT);
+    // the groups' sums in a fixed order
+    T tot = sum;
+#pragma unroll
+    for (int q = 1; q < G; ++q) tot += __shfl_sync(0xffffffffu, sum, q * ND + r);
+    s -= tot;
+    if constexpr (LOWER) {
+#pragma unroll
+      for (int c = 0; c < ND - 1; ++c) {
+        const T zcv = __shfl_sync(0xffffffffu, s, c);
+        if (lane > c) s = sweep_fma(-D[c], zcv, s);
+      }
+    } else {
+      s *= rd;
+#pragma unroll
+      for (int c = ND - 1; c > 0; --c) {
+        const T xc = __shfl_sync(0xffffffffu, s, c);
+        if (lane < c) s = sweep_fma(-D[c], xc, s);
+      }
+    }
+    if (lane < ND) {
+      W::store(zw + (int64_t)I * ND + lane, s);
+      if constexpr (!LOWER) zoutbase[off + (int64_t)I * ND + lane] = (double)s;
     }
   }
 }
@@ -750,15 +749,17 @@ struct gales_solver {
   Dev<int64_t> d_node_rp, d_f_rp, d_f_diag, d_a2f;
   Dev<int32_t> d_node_col, d_f_col, d_rows_f, d_rows_b;
   Dev<double> d_F, d_V, d_Z, d_w, d_r, d_x, d_part, d_h, d_h2, d_y, d_vals, d_b;
-  Dev<float> d_Ff, d_zf;     // FP32 factor and its substitution vector (GALES_PRECOND_ILU_FP32)
+  Dev<float> d_Ff;           // FP32 factor (GALES_PRECOND_ILU_FP32)
   Dev<int> d_j;
-  Dev<int> d_sync;           // sweep tickets [2] and ready flags [2][n_nodes] of the substitutions
+  Dev<int> d_ready;          // factorisation: ticket, then a ready flag per node row
+  Dev<unsigned char> d_sweep;  // substitutions: the two result vectors (factor's type), then two tickets
   Dev<unsigned int> d_status;
   double* h_buf = nullptr;   // pinned: Hessenberg column and the least-squares solution
   int m = 0;                 // Krylov vectors per cycle
   int max_row = 0, max_u = 0;  // longest factor row, longest upper part (blocks)
   int smem_optin = 0;          // opt-in shared memory per CTA
-  size_t factor_smem = 0;      // dynamic shared memory of the staged factor kernel (0: not used)
+  size_t factor_smem = 0;      // dynamic shared memory of the factorisation kernel (0: level launches)
+  int factor_ctas = 1;         // its resident CTAs per SM
   int dot_blocks = 1;
   cudaGraphExec_t prec_graph = nullptr;
   cudaStream_t cap = nullptr;
@@ -801,69 +802,66 @@ template <>
 float* factor_ptr<float>(gales_solver* s) { return s->d_Ff.p; }
 
 // Launch wrappers for nd = ND and a factor stored in T (double: the reference's FP64
-// arithmetic; float: FP32 factor and substitutions, scratch vector d_zf).
+// arithmetic; float: FP32 factor and substitutions).
 template <int ND, typename T>
 struct Kernels {
-  static constexpr bool kF64 = sizeof(T) == sizeof(double);
   static cudaError_t to_factor(gales_solver* s, const double* vals, cudaStream_t st) {
     matrix_to_factor_kernel<ND, T><<<grid_for(s->n_nodes), 32 * kWarpsPerBlock, 0, st>>>(
         vals, s->d_node_rp.p, s->d_a2f.p, s->n_nodes, factor_ptr<T>(s));
     return cudaGetLastError();
   }
-  static size_t factor_smem(int max_row, int max_u) {
-    return ((size_t)max_row + 1 + max_u) * ND * ND * sizeof(T) + ((size_t)max_row + max_u) * sizeof(int32_t);
-  }
+  // The persistent factorisation where a block row and two rows' upper parts fit the shared
+  // memory of an SM; rows too long for that take the level launches on global memory.
   static cudaError_t prepare(gales_solver* s) {
-    const size_t bytes = factor_smem(s->max_row, s->max_u);
+    const size_t bytes = FactorSmem<ND, T>::bytes(s->max_row, s->max_u);
     s->factor_smem = 0;
-    if (bytes > (size_t)s->smem_optin) return cudaSuccess;  // rows too long: the global-memory kernel
-    cudaError_t e = cudaFuncSetAttribute(ilu_factor_level_smem_kernel<ND, T>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) s->factor_smem = bytes;
+    if (bytes > (size_t)s->smem_optin) return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(ilu_factor_rows_kernel<ND, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)bytes);
+    int nb = 0;
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ilu_factor_rows_kernel<ND, T>, kFactorThreads, bytes);
+    if (e == cudaSuccess && nb > 0) {
+      s->factor_smem = bytes;
+      s->factor_ctas = nb;
+    }
     return e;
   }
-  static cudaError_t factor_level(gales_solver* s, int l, cudaStream_t st) {
-    const int64_t o = s->lev_off_f[l], c = s->lev_off_f[l + 1] - o;
-    if (s->factor_smem)
-      ilu_factor_level_smem_kernel<ND, T><<<(unsigned)c, 32, s->factor_smem, st>>>(
-          factor_ptr<T>(s), s->d_f_rp.p, s->d_f_col.p, s->d_f_diag.p, s->d_rows_f.p + o, c, s->d_status.p,
-          s->max_row, s->max_u);
-    else
+  static cudaError_t factor(gales_solver* s, cudaStream_t st) {
+    if (s->factor_smem) {
+      cudaError_t e = cudaMemsetAsync(s->d_ready.p, 0, s->d_ready.n * sizeof(int), st);
+      if (e != cudaSuccess) return e;
+      const unsigned g = (unsigned)std::min<int64_t>(s->n_nodes, (int64_t)s->sms * s->factor_ctas);
+      ilu_factor_rows_kernel<ND, T><<<g, kFactorThreads, s->factor_smem, st>>>(
+          factor_ptr<T>(s), s->d_f_rp.p, s->d_f_col.p, s->d_f_diag.p, s->d_rows_f.p, s->n_nodes,
+          reinterpret_cast<unsigned int*>(s->d_ready.p), s->d_ready.p + 1, s->d_status.p, s->max_row, s->max_u);
+      ++s->launches;
+      return cudaGetLastError();
+    }
+    for (size_t l = 0; l + 1 < s->lev_off_f.size(); ++l) {
+      const int64_t o = s->lev_off_f[l], c = s->lev_off_f[l + 1] - o;
       ilu_factor_level_kernel<ND, T><<<grid_for(c), 32 * kWarpsPerBlock, 0, st>>>(
           factor_ptr<T>(s), s->d_f_rp.p, s->d_f_col.p, s->d_f_diag.p, s->d_rows_f.p + o, c, s->d_status.p);
-    return cudaGetLastError();
+      ++s->launches;
+      const cudaError_t e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
   }
-  static cudaError_t lower_level(gales_solver* s, int l, const double* v, double* z, const int* j, int64_t ld,
-                                 cudaStream_t st) {
-    const int64_t o = s->lev_off_f[l], c = s->lev_off_f[l + 1] - o;
-    T* zw = kF64 ? reinterpret_cast<T*>(z) : reinterpret_cast<T*>(s->d_zf.p);
-    ilu_lower_level_kernel<ND, T><<<grid_for(c), 32 * kWarpsPerBlock, 0, st>>>(
-        factor_ptr<T>(s), s->d_f_rp.p, s->d_f_col.p, s->d_f_diag.p, s->d_rows_f.p + o, c, v, zw, j, ld,
-        kF64 ? 1 : 0);
-    return cudaGetLastError();
-  }
-  static cudaError_t upper_level(gales_solver* s, int l, double* z, const int* j, int64_t ld, cudaStream_t st) {
-    const int64_t o = s->lev_off_b[l], c = s->lev_off_b[l + 1] - o;
-    T* zw = kF64 ? reinterpret_cast<T*>(z) : reinterpret_cast<T*>(s->d_zf.p);
-    ilu_upper_level_kernel<ND, T><<<grid_for(c), 32 * kWarpsPerBlock, 0, st>>>(
-        factor_ptr<T>(s), s->d_f_rp.p, s->d_f_col.p, s->d_f_diag.p, s->d_rows_b.p + o, c, zw, z, j, ld,
-        kF64 ? 1 : 0);
-    return cudaGetLastError();
-  }
-  // both substitutions as sync-free sweeps (tickets and ready flags cleared by the caller)
+  // both substitutions (result vectors and tickets set to all ones by the caller)
   static cudaError_t sweeps(gales_solver* s, const double* v, double* z, const int* j, int64_t ld, cudaStream_t st) {
-    T* zw = kF64 ? reinterpret_cast<T*>(z) : reinterpret_cast<T*>(s->d_zf.p);
+    T* y = reinterpret_cast<T*>(s->d_sweep.p);
+    T* x = y + s->n_rows;
+    unsigned int* tk = reinterpret_cast<unsigned int*>(x + s->n_rows);
     const unsigned g = std::min<unsigned>(grid_for(s->n_nodes), (unsigned)s->sms);
-    unsigned int* tk = reinterpret_cast<unsigned int*>(s->d_sync.p);
-    int* ready = s->d_sync.p + 2;
-    ilu_lower_sweep_kernel<ND, T><<<g, 32 * kWarpsPerBlock, 0, st>>>(
-        factor_ptr<T>(s), s->d_f_rp.p, s->d_f_col.p, s->d_f_diag.p, s->d_rows_f.p, s->n_nodes, v, zw, j, ld,
-        kF64 ? 1 : 0, tk, ready, s->d_status.p);
+    ilu_sweep_kernel<ND, T, true><<<g, 32 * kWarpsPerBlock, 0, st>>>(
+        factor_ptr<T>(s), s->d_f_rp.p, s->d_f_col.p, s->d_f_diag.p, s->d_rows_f.p, s->n_nodes, v, nullptr, y, nullptr,
+        j, ld, tk, s->d_status.p);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    ilu_upper_sweep_kernel<ND, T><<<g, 32 * kWarpsPerBlock, 0, st>>>(
-        factor_ptr<T>(s), s->d_f_rp.p, s->d_f_col.p, s->d_f_diag.p, s->d_rows_b.p, s->n_nodes, zw, z, j, ld,
-        kF64 ? 1 : 0, tk + 1, ready + s->n_nodes, s->d_status.p);
+    ilu_sweep_kernel<ND, T, false><<<g, 32 * kWarpsPerBlock, 0, st>>>(
+        factor_ptr<T>(s), s->d_f_rp.p, s->d_f_col.p, s->d_f_diag.p, s->d_rows_b.p, s->n_nodes, nullptr, y, x, z, j, ld,
+        tk + 1, s->d_status.p);
     return cudaGetLastError();
   }
   static cudaError_t spmv(gales_solver* s, const double* vals, const double* x, const double* b, double* y,
@@ -877,9 +875,7 @@ struct Kernels {
 struct Ops {
   cudaError_t (*prepare)(gales_solver*);
   cudaError_t (*to_factor)(gales_solver*, const double*, cudaStream_t);
-  cudaError_t (*factor_level)(gales_solver*, int, cudaStream_t);
-  cudaError_t (*lower_level)(gales_solver*, int, const double*, double*, const int*, int64_t, cudaStream_t);
-  cudaError_t (*upper_level)(gales_solver*, int, double*, const int*, int64_t, cudaStream_t);
+  cudaError_t (*factor)(gales_solver*, cudaStream_t);
   cudaError_t (*sweeps)(gales_solver*, const double*, double*, const int*, int64_t, cudaStream_t);
   cudaError_t (*spmv)(gales_solver*, const double*, const double*, const double*, double*, cudaStream_t);
 };
@@ -887,7 +883,7 @@ struct Ops {
 template <int ND, typename T>
 Ops ops_for() {
   using K = Kernels<ND, T>;
-  return {K::prepare, K::to_factor, K::factor_level, K::lower_level, K::upper_level, K::sweeps, K::spmv};
+  return {K::prepare, K::to_factor, K::factor, K::sweeps, K::spmv};
 }
 
 template <typename T>
@@ -914,10 +910,10 @@ inline bool has_ilu(const gales_solver* s) {
   return s->prm.precond == GALES_PRECOND_ILU || s->prm.precond == GALES_PRECOND_ILU_FP32;
 }
 
-// z = M^-1 v for columns addressed by *j (graph) or plain pointers (j null): the two
-// sync-free sweeps after clearing their tickets and ready flags.
+// z = M^-1 v for columns addressed by *j (graph) or plain pointers (j null): the two sweeps
+// after setting their result vectors and tickets to all ones (SweepWord::kUnset).
 int apply_prec(gales_solver* s, const Ops& o, const double* v, double* z, const int* j, int64_t ld, cudaStream_t st) {
-  SCK(s, cudaMemsetAsync(s->d_sync.p, 0, s->d_sync.n * sizeof(int), st), "clear sweep flags");
+  SCK(s, cudaMemsetAsync(s->d_sweep.p, 0xff, s->d_sweep.n, st), "clear sweep vectors");
   SCK(s, o.sweeps(s, v, z, j, ld, st), "substitutions");
   s->launches += 2;
   return 0;
@@ -945,12 +941,12 @@ int factorize(gales_solver* s, const Ops& o, const double* vals, cudaStream_t st
     SCK(s, cudaMemsetAsync(s->d_F.p, 0, s->d_F.n * sizeof(double), st), "clear factor");
   SCK(s, cudaMemsetAsync(s->d_status.p, 0, sizeof(unsigned int), st), "clear status");
   SCK(s, o.to_factor(s, vals, st), "matrix to factor");
-  const int nf = (int)s->lev_off_f.size() - 1;
-  for (int l = 0; l < nf; ++l) SCK(s, o.factor_level(s, l, st), "factor level");
-  s->launches += 1 + nf;
+  ++s->launches;
+  SCK(s, o.factor(s, st), "factorisation");
   unsigned int stat = 0;
   SCK(s, cudaMemcpyAsync(&stat, s->d_status.p, sizeof(stat), cudaMemcpyDeviceToHost, st), "status");
   SCK(s, cudaStreamSynchronize(st), "factorisation");
+  if (stat & GALES_ERR_TIMEOUT) return sfail(s, GALES_ERR_TIMEOUT, "a factorisation wait ran out");
   if (stat) return sfail(s, GALES_ERR_SINGULAR, "zero pivot in the incomplete factorisation");
   return 0;
 }
@@ -1069,11 +1065,13 @@ int gales_solver_create(gales_asm* h, const gales_solver_params* prm, gales_solv
       s->d_f_col.upload(s->f_col) || s->d_f_diag.upload(s->f_diag) || s->d_a2f.upload(a2f) ||
       s->d_rows_f.upload(s->rows_f) || s->d_rows_b.upload(s->rows_b) || (p.precond == GALES_PRECOND_ILU ? s->d_F.alloc(s->f_col.size() * bb)
                                        : s->d_Ff.alloc(s->f_col.size() * bb)) ||
-      (p.precond == GALES_PRECOND_ILU_FP32 ? s->d_zf.alloc(n_rows) : cudaSuccess) ||
       s->d_V.alloc((size_t)(s->m + 1) * n_rows) || s->d_Z.alloc((size_t)s->m * n_rows) || s->d_w.alloc(n_rows) ||
       s->d_r.alloc(n_rows) || s->d_x.alloc(n_rows) || s->d_part.alloc((size_t)s->dot_blocks * (s->m + 2)) ||
       s->d_h.alloc(s->m + 2) || s->d_h2.alloc(s->m + 2) || s->d_y.alloc(s->m + 2) || s->d_j.alloc(1) ||
-      s->d_sync.alloc(2 + 2 * (size_t)n_nodes) || s->d_status.alloc(1)) {
+      (has_ilu(s) ? s->d_ready.alloc(1 + (size_t)n_nodes) : cudaSuccess) ||
+      (has_ilu(s) ? s->d_sweep.alloc(2 * (size_t)n_rows * (p.precond == GALES_PRECOND_ILU ? sizeof(double) : sizeof(float)) +
+                                     2 * sizeof(unsigned int))
+                  : cudaSuccess) || s->d_status.alloc(1)) {
     cudaGetLastError();
     return bail(GALES_ERR_NO_MEMORY);
   }
@@ -1334,11 +1332,12 @@ void gales_solver_destroy(gales_solver* s) {
   for (auto* b : {&s->d_node_rp, &s->d_f_rp, &s->d_f_diag, &s->d_a2f}) b->release();
   for (auto* b : {&s->d_node_col, &s->d_f_col, &s->d_rows_f, &s->d_rows_b}) b->release();
   s->d_Ff.release();
-  s->d_zf.release();
   for (auto* b : {&s->d_F, &s->d_V, &s->d_Z, &s->d_w, &s->d_r, &s->d_x, &s->d_part, &s->d_h, &s->d_h2, &s->d_y,
                   &s->d_vals, &s->d_b})
     b->release();
   s->d_j.release();
+  s->d_ready.release();
+  s->d_sweep.release();
   s->d_status.release();
   delete s;
 }
