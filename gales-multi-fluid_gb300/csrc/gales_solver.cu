@@ -38,6 +38,7 @@
 namespace {
 
 constexpr int kWarpsPerBlock = 8;   // node rows per CTA in the level kernels
+constexpr int kSweepWarps = 10;     // warps per CTA of the sweeps, one CTA per SM
 constexpr int kDotThreads = 256;
 
 template <typename T>
@@ -464,20 +465,23 @@ __global__ void __launch_bounds__(kFactorThreads)
 // Triangular substitutions, one persistent launch per triangle, a warp per node row:
 //   lower  y_I = L_II^-1 (v_I - sum_K L_IK y_K), L_II unit lower
 //   upper  x_I = U_II^-1 (y_I - sum_J U_IJ x_J)
-// A sweep is a chain of levels (749 on the 157k-node tet system, ~210 rows each), so its
+// A sweep is a chain of levels (204 on a 27k-node system of tets, ~130 rows each), so its
 // time is the latency of one level, not the bytes of the factor.  The words of the result
 // are their own ready flags: the result vector is filled with a bit pattern that no row
 // stores (kUnset, a NaN), lanes poll the words that they need with relaxed loads, which
 // leave L1 alone, and a finished row is stored without a fence.  A level is then one
 // store-to-load trip through L2 plus the row's own arithmetic; separate flags (release
 // store, acquire load, then the load of the values) cost three such trips, and an acquire
-// also empties the L1 that the factor had been prefetched into: 9.8 us a level with an FP32
-// factor, 14 us with FP64.  Before it polls, a row loads its factor blocks into registers:
-// lanes form G = 32 / ND groups of ND, lane (g, r) holds row r of the blocks g, g + G, ...
-// (KB at a time).  Blocks are taken in the order in which their rows finish (ascending for
-// the lower sweep, descending for the upper one), all first polls in flight together.  The
-// diagonal block's reciprocals and the scaling of its rows by them are formed before the
-// wait too, which leaves one multiply-add per unknown on the chain.
+// also empties the L1 that the factor had been prefetched into: 9.4 us a level with an FP32
+// factor, 15 us with FP64 (M^-1 3.86 and 6.14 ms there; now 0.41 and 0.75 ms, 1.0 and 1.8 us
+// a level).  Before it polls, a row loads its factor blocks into registers: lanes form G = 32 /
+// ND groups of ND, lane (g, r) holds row r of the blocks g, g + G, ... (KB at a time).
+// Blocks are taken in the order in which their rows finish (ascending for the lower sweep,
+// descending for the upper one), all first polls in flight together.  With the diagonal
+// blocks' rows scaled in advance (scale_diag_kernel) the chain has one multiply-add per
+// unknown.  Ten warps per SM keep the next levels' rows loaded (M^-1 on a 157k-node system of
+// 372 levels with 4, 8 and 10 warps: 2.57, 1.72, 1.62 ms); a block's columns spread over the groups instead of a
+// block per group, with fewer products after the last arrival, was no faster (1.67).
 template <typename T>
 struct SweepWord;
 template <>
@@ -516,14 +520,31 @@ struct SweepWord<float> {
 __device__ __forceinline__ double sweep_fma(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float sweep_fma(float a, float b, float c) { return fmaf(a, b, c); }
 
+// The upper sweep's diagonal blocks: row r of U_II divided by its pivot, and the pivot's
+// reciprocal on the diagonal (thread per block row, once per factorisation; a division and
+// ND products per row and sweep otherwise, a third of the sweep's FP64 work).
+template <int ND, typename T>
+__global__ void scale_diag_kernel(const T* __restrict__ F, const int64_t* __restrict__ f_diag, int64_t n_rows,
+                                  T* __restrict__ Us) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_rows) return;
+  const int64_t node = i / ND;
+  const int r = (int)(i - node * ND);
+  const T* D = F + f_diag[node] * (ND * ND) + r * ND;
+  T* o = Us + i * ND;
+  const T rd = T(1) / D[r];
+#pragma unroll
+  for (int c = 0; c < ND; ++c) o[c] = c == r ? rd : D[c] * rd;
+}
+
 // In (lower: the FP64 right-hand side vbase; upper: the lower sweep's result yin) and out
 // (zw, kUnset before the launch; upper: also the FP64 column zoutbase).  The ticket starts
 // at ~0u (it is cleared together with zw), so the first claim is row 0 of the order.
 template <int ND, typename T, bool LOWER>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock)
+__global__ void __launch_bounds__(32 * kSweepWarps)
     ilu_sweep_kernel(const T* __restrict__ F, const int64_t* __restrict__ f_rp, const int32_t* __restrict__ f_col,
-                     const int64_t* __restrict__ f_diag, const int32_t* __restrict__ rows, int64_t n,
-                     const double* __restrict__ vbase, const T* __restrict__ yin, T* zw, double* zoutbase,
+                     const int64_t* __restrict__ f_diag, const T* __restrict__ Us, const int32_t* __restrict__ rows,
+                     int64_t n, const double* __restrict__ vbase, const T* __restrict__ yin, T* zw, double* zoutbase,
                      const int* __restrict__ jidx, int64_t ld, unsigned int* ticket, unsigned int* status) {
   using W = SweepWord<T>;
   constexpr int BB = ND * ND, G = 32 / ND;
@@ -543,18 +564,9 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
     // row r of the diagonal block and the right-hand side
     T D[ND];
 #pragma unroll
-    for (int c = 0; c < ND; ++c) D[c] = F[pd * BB + r * ND + c];
-    T s = LOWER ? (T)vbase[off + (int64_t)I * ND + r] : yin[(int64_t)I * ND + r];
-    T rd = T(1);
-    if constexpr (!LOWER) {
-      T dg = D[0];
-#pragma unroll
-      for (int c = 1; c < ND; ++c) dg = r == c ? D[c] : dg;
-      rd = T(1) / dg;
-#pragma unroll
-      for (int c = 0; c < ND; ++c) D[c] *= rd;
-    }
-    T sum = T(0);
+    for (int c = 0; c < ND; ++c) D[c] = LOWER ? F[pd * BB + r * ND + c] : Us[((int64_t)I * ND + r) * ND + c];
+    const T rhs = LOWER ? (T)vbase[off + (int64_t)I * ND + r] : yin[(int64_t)I * ND + r];
+    T sum = g == 0 ? -rhs : T(0), sum2 = T(0);
     bool late = false;
     for (int k0 = 0; k0 < nblk; k0 += KB * G) {
       int64_t zc[KB];
@@ -583,28 +595,39 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
         }
         const T zk = W::value(w[k]);
 #pragma unroll
-        for (int c = 0; c < ND; ++c)
-          sum = sweep_fma(B[k][c], __shfl_sync(0xffffffffu, zk, (g < G ? g : 0) * ND + c), sum);
+        for (int c = 0; c < ND; ++c) {
+          const T x = __shfl_sync(0xffffffffu, zk, (g < G ? g : 0) * ND + c);
+          if (c & 1) sum2 = sweep_fma(B[k][c], x, sum2);
+          else sum = sweep_fma(B[k][c], x, sum);
+        }
       }
     }
     if (late && lane == 0) atomicOr(status, (unsigned)GALES_ERR_TIMEOUT);
-    // the groups' sums in a fixed order
-    T tot = sum;
+    // the groups' sums in a fixed order; s = rhs - sum of the blocks
+    sum += sum2;
+    T part[G];
 #pragma unroll
-    for (int q = 1; q < G; ++q) tot += __shfl_sync(0xffffffffu, sum, q * ND + r);
-    s -= tot;
+    for (int q = 0; q < G; ++q) part[q] = __shfl_sync(0xffffffffu, sum, q * ND + r);
+#pragma unroll
+    for (int h = 1; h < G; h *= 2)
+#pragma unroll
+      for (int q = 0; q + h < G; q += 2 * h) part[q] += part[q + h];
+    T s = -part[0];
     if constexpr (LOWER) {
 #pragma unroll
       for (int c = 0; c < ND - 1; ++c) {
-        const T zcv = __shfl_sync(0xffffffffu, s, c);
-        if (lane > c) s = sweep_fma(-D[c], zcv, s);
+        const T x = __shfl_sync(0xffffffffu, s, c);
+        if (lane > c) s = sweep_fma(-D[c], x, s);
       }
     } else {
+      T rd = D[0];
+#pragma unroll
+      for (int c = 1; c < ND; ++c) rd = r == c ? D[c] : rd;
       s *= rd;
 #pragma unroll
       for (int c = ND - 1; c > 0; --c) {
-        const T xc = __shfl_sync(0xffffffffu, s, c);
-        if (lane < c) s = sweep_fma(-D[c], xc, s);
+        const T x = __shfl_sync(0xffffffffu, s, c);
+        if (lane < c) s = sweep_fma(-D[c], x, s);
       }
     }
     if (lane < ND) {
@@ -614,82 +637,148 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
   }
 }
 
-// y = A x (or y = b - A x) on the assembly's CSR values: warp per scalar row.
+// y = A x (or y = b - A x) on the assembly's CSR values: warp per node row.  Lanes form
+// G = 32 / ND groups of ND, lane (g, r) takes scalar row r over the node row's blocks g,
+// g + G, ...: ND multiply-adds a block and G - 1 adds at the end.  Bound: the FP64 pipe
+// (0.18 ms for the 115M entries of a 157k-node tet system at 2 lanes per SM and clock, DRAM
+// 0.14 ms); a warp per scalar row spent more FP64 issue slots on its shuffle sums than on
+// products: 1.28 ms there, now 0.32.
 template <int ND>
-__global__ void spmv_kernel(const double* __restrict__ vals, const int64_t* __restrict__ node_rp,
-                            const int32_t* __restrict__ node_col, int64_t n_rows, const double* __restrict__ x,
-                            const double* __restrict__ b, double* __restrict__ y) {
-  const int64_t row = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-  if (row >= n_rows) return;
+__global__ void __launch_bounds__(32 * kWarpsPerBlock)
+    spmv_kernel(const double* __restrict__ vals, const int64_t* __restrict__ node_rp,
+                const int32_t* __restrict__ node_col, int64_t n_nodes, const double* __restrict__ x,
+                const double* __restrict__ b, double* __restrict__ y) {
+  constexpr int G = 32 / ND;
+  const int64_t i = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  if (i >= n_nodes) return;
   const int lane = threadIdx.x & 31;
-  const int64_t i = row / ND;
-  const int k = (int)(row % ND);
-  const int64_t t0 = node_rp[i], len = (node_rp[i + 1] - t0) * ND;
-  const double* a = vals + t0 * ND * ND + k * len;
+  const int g = lane / ND, r = lane < G * ND ? lane - g * ND : 0;
+  const int64_t t0 = node_rp[i];
+  const int deg = (int)(node_rp[i + 1] - t0);
+  const double* a = vals + t0 * (ND * ND) + (int64_t)r * deg * ND;
   double s = 0.0;
-  for (int64_t e = lane; e < len; e += 32) s += a[e] * x[(int64_t)node_col[t0 + e / ND] * ND + e % ND];
+  if (g < G)
+#pragma unroll 2
+    for (int k = g; k < deg; k += G) {
+      const double* xc = x + (int64_t)node_col[t0 + k] * ND;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) y[row] = b ? b[row] - s : s;
+      for (int c = 0; c < ND; ++c) s = fma(__ldcs(a + k * ND + c), xc[c], s);
+    }
+  double tot = s;
+#pragma unroll
+  for (int q = 1; q < G; ++q) tot += __shfl_sync(0xffffffffu, s, q * ND + r);
+  if (lane < ND) {
+    const int64_t row = i * ND + lane;
+    y[row] = b ? b[row] - tot : tot;
+  }
 }
 
-// Partial dot products of w with the columns V[0..nv) (column stride ld), four columns
-// at a time: part[block][c].
-__global__ void mdot_kernel(const double* __restrict__ V, int64_t ld, int nv, const double* __restrict__ w,
-                            int64_t n, double* __restrict__ part) {
-  __shared__ double sh[kDotThreads / 32][4];
-  const int64_t per = (n + gridDim.x - 1) / gridDim.x;
-  const int64_t lo = (int64_t)blockIdx.x * per, hi = lo + per < n ? lo + per : n;
+// One pass of the Arnoldi step, mode kDots: h = V^T w; kSubDots: w -= V h, then h2 = V^T w
+// and h += h2; kSubNorm: w -= V h2, then hn[0] = ||w||.  nv columns of V, stride ld.  A CTA takes
+// tiles of kTile rows: a thread subtracts its rows, then the warps share the columns of the
+// dot products (lane partials in shared memory, kCols columns at a time, carried over the
+// tiles).  The last CTA to finish adds the CTAs' partial sums in a fixed order, so repeated
+// solves are bit-identical.  Bound: DRAM (V once per pass; a tile's columns come from L2 the
+// second time) and, with fused multiply-adds, as much FP64: 44 us per pass over 25 columns of
+// 1.1M rows.  Separate launches for the dots, their final sums (one CTA adding 304 partials
+// serially, 24 us each) and the updates took 0.47 ms a step on 189k rows, mostly launches; now
+// 0.16 ms.  Tiles of 256 rows and four CTAs per SM, against 512 and two, keep enough loads in
+// flight and a tile's columns in L2: 164 against 339 us for kSubDots at 1.1M rows, 33 columns.
+constexpr int kDots = 0, kSubDots = 1, kSubNorm = 2;
+constexpr int kTile = 256, kCols = 96;
+constexpr int kHs = 512;   // coefficients held in shared memory; those of more columns are read from L2
+
+template <int MODE>
+__global__ void __launch_bounds__(kDotThreads, 4)
+    arnoldi_kernel(const double* __restrict__ V, int64_t ld, int nv, double* __restrict__ w, int64_t n,
+                   double* __restrict__ h, double* __restrict__ h2, double* __restrict__ hn,
+                   double* __restrict__ part, unsigned int* __restrict__ count) {
+  __shared__ double ws[kTile];
+  __shared__ double acc[MODE == kSubNorm ? 1 : kCols][32];
+  __shared__ double red[kDotThreads / 32];
+  __shared__ double hs[kHs];
+  __shared__ bool last;
+  constexpr int NW = kDotThreads / 32;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int c0 = 0; c0 < nv; c0 += 4) {
-    double a[4] = {0.0, 0.0, 0.0, 0.0};
-    const int m = nv - c0 < 4 ? nv - c0 : 4;
-    for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-      const double wi = w[i];
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (q < m) a[q] += V[(int64_t)(c0 + q) * ld + i] * wi;
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) a[q] += __shfl_xor_sync(0xffffffffu, a[q], o);
-    if (lane == 0)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) sh[wid][q] = a[q];
-    __syncthreads();
-    if (threadIdx.x < m) {
-      double s = 0.0;
-      for (int k = 0; k < kDotThreads / 32; ++k) s += sh[k][threadIdx.x];
-      part[(int64_t)blockIdx.x * nv + c0 + threadIdx.x] = s;
-    }
+  const double* __restrict__ hsub = MODE == kSubDots ? h : h2;
+  if (MODE != kDots) {
+    for (int c = threadIdx.x; c < nv && c < kHs; c += kDotThreads) hs[c] = __ldcg(hsub + c);
     __syncthreads();
   }
-}
-
-// out[c] (mode 0) = sum_b part[b][c]; mode 1: out[c] += sum; mode 2: out[0] = sqrt(sum).
-__global__ void mdot_final_kernel(const double* __restrict__ part, int nb, int nv, double* __restrict__ out,
-                                  int mode) {
-  for (int c = threadIdx.x; c < nv; c += blockDim.x) {
-    double s = 0.0;
-    for (int b = 0; b < nb; ++b) s += part[(int64_t)b * nv + c];
-    if (mode == 0) out[c] = s;
-    else if (mode == 1) out[c] += s;
-    else out[c] = sqrt(s);
+  double nrm = 0.0;
+  const int nout = MODE == kSubNorm ? 1 : nv;
+  for (int cb = 0; cb == 0 || cb < nv; cb += kCols) {
+    const int nc = nv - cb < kCols ? nv - cb : kCols;
+    if constexpr (MODE != kSubNorm)
+      for (int c = wid; c < nc; c += NW) acc[c][lane] = 0.0;
+    for (int64_t lo = (int64_t)blockIdx.x * kTile; lo < n; lo += (int64_t)gridDim.x * kTile) {
+      const int m = (int)(n - lo < kTile ? n - lo : kTile);
+      for (int i = threadIdx.x; i < m; i += kDotThreads) {
+        double x = w[lo + i];
+        if (MODE != kDots && cb == 0 && nv > 0) {
+          const double* __restrict__ v = V + lo + i;
+          const int nh = nv < kHs ? nv : kHs;
+          double s0 = 0.0, s1 = 0.0;
+          int c = 0;
+#pragma unroll 4
+          for (; c + 1 < nh; c += 2) {
+            s0 = fma(v[(int64_t)c * ld], hs[c], s0);
+            s1 = fma(v[(int64_t)(c + 1) * ld], hs[c + 1], s1);
+          }
+          for (; c < nh; ++c) s0 = fma(v[(int64_t)c * ld], hs[c], s0);
+          for (; c < nv; ++c) s0 = fma(v[(int64_t)c * ld], __ldcg(hsub + c), s0);
+          x -= s0 + s1;
+          w[lo + i] = x;
+        }
+        if constexpr (MODE == kSubNorm) nrm = fma(x, x, nrm);
+        else ws[i] = x;
+      }
+      if constexpr (MODE == kSubNorm) continue;
+      __syncthreads();
+      for (int c = wid; c < nc; c += NW) {
+        const double* __restrict__ v = V + (int64_t)(cb + c) * ld + lo;
+        double a = acc[MODE == kSubNorm ? 0 : c][lane];
+        for (int i = lane; i < m; i += 32) a = fma(v[i], ws[i], a);
+        acc[MODE == kSubNorm ? 0 : c][lane] = a;
+      }
+      __syncthreads();
+    }
+    if constexpr (MODE == kSubNorm) break;
+    for (int c = wid; c < nc; c += NW) {
+      double a = acc[MODE == kSubNorm ? 0 : c][lane];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      if (lane == 0) part[(int64_t)blockIdx.x * nout + cb + c] = a;
+    }
   }
-}
-
-// w -= sum_c V[c] h[c]
-__global__ void axpy_multi_kernel(const double* __restrict__ V, int64_t ld, int nv, const double* __restrict__ h,
-                                  double* __restrict__ w, int64_t n) {
-  extern __shared__ double hs[];
-  for (int c = threadIdx.x; c < nv; c += blockDim.x) hs[c] = h[c];
+  if constexpr (MODE == kSubNorm) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
+    if (lane == 0) red[wid] = nrm;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double a = 0.0;
+      for (int q = 0; q < NW; ++q) a += red[q];
+      part[blockIdx.x] = a;
+    }
+  }
+  __threadfence();
   __syncthreads();
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int c = 0; c < nv; ++c) s += V[(int64_t)c * ld + i] * hs[c];
-    w[i] -= s;
+  if (threadIdx.x == 0) last = atomicAdd(count, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int c = wid; c < nout; c += NW) {
+    double a = 0.0;
+    for (unsigned int q = lane; q < gridDim.x; q += 32) a += __ldcg(part + (int64_t)q * nout + c);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (lane != 0) continue;
+    if constexpr (MODE == kDots) h[c] = a;
+    else if constexpr (MODE == kSubDots) { h2[c] = a; h[c] += a; }
+    else hn[0] = sqrt(a);
   }
+  if (threadIdx.x == 0) *count = 0;
 }
 
 // x += sum_c Z[c] y[c]
@@ -700,7 +789,7 @@ __global__ void update_x_kernel(const double* __restrict__ Z, int64_t ld, int nv
   __syncthreads();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     double s = 0.0;
-    for (int c = 0; c < nv; ++c) s += Z[(int64_t)c * ld + i] * ys[c];
+    for (int c = 0; c < nv; ++c) s = fma(Z[(int64_t)c * ld + i], ys[c], s);
     x[i] += s;
   }
 }
@@ -752,8 +841,9 @@ struct gales_solver {
   Dev<float> d_Ff;           // FP32 factor (GALES_PRECOND_ILU_FP32)
   Dev<int> d_j;
   Dev<int> d_ready;          // factorisation: ticket, then a ready flag per node row
+  Dev<unsigned char> d_udiag;  // the upper sweep's scaled diagonal blocks (factor's type)
   Dev<unsigned char> d_sweep;  // substitutions: the two result vectors (factor's type), then two tickets
-  Dev<unsigned int> d_status;
+  Dev<unsigned int> d_status, d_count;  // error bits; CTAs of an Arnoldi pass that are done
   double* h_buf = nullptr;   // pinned: Hessenberg column and the least-squares solution
   int m = 0;                 // Krylov vectors per cycle
   int max_row = 0, max_u = 0;  // longest factor row, longest upper part (blocks)
@@ -848,26 +938,31 @@ struct Kernels {
     }
     return cudaSuccess;
   }
+  static cudaError_t scale_diag(gales_solver* s, cudaStream_t st) {
+    scale_diag_kernel<ND, T><<<(unsigned)((s->n_rows + 127) / 128), 128, 0, st>>>(
+        factor_ptr<T>(s), s->d_f_diag.p, s->n_rows, reinterpret_cast<T*>(s->d_udiag.p));
+    return cudaGetLastError();
+  }
   // both substitutions (result vectors and tickets set to all ones by the caller)
   static cudaError_t sweeps(gales_solver* s, const double* v, double* z, const int* j, int64_t ld, cudaStream_t st) {
     T* y = reinterpret_cast<T*>(s->d_sweep.p);
     T* x = y + s->n_rows;
     unsigned int* tk = reinterpret_cast<unsigned int*>(x + s->n_rows);
-    const unsigned g = std::min<unsigned>(grid_for(s->n_nodes), (unsigned)s->sms);
-    ilu_sweep_kernel<ND, T, true><<<g, 32 * kWarpsPerBlock, 0, st>>>(
-        factor_ptr<T>(s), s->d_f_rp.p, s->d_f_col.p, s->d_f_diag.p, s->d_rows_f.p, s->n_nodes, v, nullptr, y, nullptr,
-        j, ld, tk, s->d_status.p);
+    const unsigned g = (unsigned)std::min<int64_t>((s->n_nodes + kSweepWarps - 1) / kSweepWarps, s->sms);
+    ilu_sweep_kernel<ND, T, true><<<g, 32 * kSweepWarps, 0, st>>>(
+        factor_ptr<T>(s), s->d_f_rp.p, s->d_f_col.p, s->d_f_diag.p, nullptr, s->d_rows_f.p, s->n_nodes, v, nullptr, y,
+        nullptr, j, ld, tk, s->d_status.p);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    ilu_sweep_kernel<ND, T, false><<<g, 32 * kWarpsPerBlock, 0, st>>>(
-        factor_ptr<T>(s), s->d_f_rp.p, s->d_f_col.p, s->d_f_diag.p, s->d_rows_b.p, s->n_nodes, nullptr, y, x, z, j, ld,
-        tk + 1, s->d_status.p);
+    ilu_sweep_kernel<ND, T, false><<<g, 32 * kSweepWarps, 0, st>>>(
+        factor_ptr<T>(s), s->d_f_rp.p, s->d_f_col.p, s->d_f_diag.p, reinterpret_cast<const T*>(s->d_udiag.p),
+        s->d_rows_b.p, s->n_nodes, nullptr, y, x, z, j, ld, tk + 1, s->d_status.p);
     return cudaGetLastError();
   }
   static cudaError_t spmv(gales_solver* s, const double* vals, const double* x, const double* b, double* y,
                           cudaStream_t st) {
-    spmv_kernel<ND><<<grid_for(s->n_rows), 32 * kWarpsPerBlock, 0, st>>>(vals, s->d_node_rp.p, s->d_node_col.p,
-                                                                        s->n_rows, x, b, y);
+    spmv_kernel<ND><<<grid_for(s->n_nodes), 32 * kWarpsPerBlock, 0, st>>>(vals, s->d_node_rp.p, s->d_node_col.p,
+                                                                         s->n_nodes, x, b, y);
     return cudaGetLastError();
   }
 };
@@ -876,6 +971,7 @@ struct Ops {
   cudaError_t (*prepare)(gales_solver*);
   cudaError_t (*to_factor)(gales_solver*, const double*, cudaStream_t);
   cudaError_t (*factor)(gales_solver*, cudaStream_t);
+  cudaError_t (*scale_diag)(gales_solver*, cudaStream_t);
   cudaError_t (*sweeps)(gales_solver*, const double*, double*, const int*, int64_t, cudaStream_t);
   cudaError_t (*spmv)(gales_solver*, const double*, const double*, const double*, double*, cudaStream_t);
 };
@@ -883,7 +979,7 @@ struct Ops {
 template <int ND, typename T>
 Ops ops_for() {
   using K = Kernels<ND, T>;
-  return {K::prepare, K::to_factor, K::factor, K::sweeps, K::spmv};
+  return {K::prepare, K::to_factor, K::factor, K::scale_diag, K::sweeps, K::spmv};
 }
 
 template <typename T>
@@ -919,13 +1015,13 @@ int apply_prec(gales_solver* s, const Ops& o, const double* v, double* z, const 
   return 0;
 }
 
-// norm / dots on device: out[0..nv) = V[0..nv)^T w (mode 0/1) or out[0] = ||w|| (mode 2)
-int mdot(gales_solver* s, const double* V, int64_t ld, int nv, const double* w, double* out, int mode,
-         cudaStream_t st) {
-  mdot_kernel<<<s->dot_blocks, kDotThreads, 0, st>>>(V, ld, nv, w, s->n_rows, s->d_part.p);
-  mdot_final_kernel<<<1, 256, 0, st>>>(s->d_part.p, s->dot_blocks, nv, out, mode);
-  s->launches += 2;
-  SCK(s, cudaGetLastError(), "dot products");
+// One Arnoldi pass over w (see arnoldi_kernel); nv = 0 with kSubNorm is hn[0] = ||w||.
+template <int MODE>
+int arnoldi(gales_solver* s, const double* V, int nv, double* w, double* hn, cudaStream_t st) {
+  arnoldi_kernel<MODE><<<s->dot_blocks, kDotThreads, 0, st>>>(V, s->n_rows, nv, w, s->n_rows, s->d_h.p, s->d_h2.p, hn,
+                                                             s->d_part.p, s->d_count.p);
+  ++s->launches;
+  SCK(s, cudaGetLastError(), "Arnoldi step");
   return 0;
 }
 
@@ -943,6 +1039,8 @@ int factorize(gales_solver* s, const Ops& o, const double* vals, cudaStream_t st
   SCK(s, o.to_factor(s, vals, st), "matrix to factor");
   ++s->launches;
   SCK(s, o.factor(s, st), "factorisation");
+  SCK(s, o.scale_diag(s, st), "diagonal blocks");
+  ++s->launches;
   unsigned int stat = 0;
   SCK(s, cudaMemcpyAsync(&stat, s->d_status.p, sizeof(stat), cudaMemcpyDeviceToHost, st), "status");
   SCK(s, cudaStreamSynchronize(st), "factorisation");
@@ -1041,7 +1139,7 @@ int gales_solver_create(gales_asm* h, const gales_solver_params* prm, gales_solv
   };
   cudaGetDevice(&s->device);
   cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->device);
-  s->dot_blocks = std::max(1, 2 * s->sms);
+  s->dot_blocks = (int)std::max<int64_t>(1, std::min<int64_t>(4 * s->sms, (n_rows + kTile - 1) / kTile));
   std::vector<int64_t> a2f;
   if (has_ilu(s)) {
     iluk_symbolic(n_nodes, s->node_rp.data(), s->node_col.data(), p.fill, s->f_rp, s->f_col, s->f_diag);
@@ -1069,9 +1167,11 @@ int gales_solver_create(gales_asm* h, const gales_solver_params* prm, gales_solv
       s->d_r.alloc(n_rows) || s->d_x.alloc(n_rows) || s->d_part.alloc((size_t)s->dot_blocks * (s->m + 2)) ||
       s->d_h.alloc(s->m + 2) || s->d_h2.alloc(s->m + 2) || s->d_y.alloc(s->m + 2) || s->d_j.alloc(1) ||
       (has_ilu(s) ? s->d_ready.alloc(1 + (size_t)n_nodes) : cudaSuccess) ||
+      (has_ilu(s) ? s->d_udiag.alloc((size_t)n_nodes * bb * (p.precond == GALES_PRECOND_ILU ? sizeof(double) : sizeof(float)))
+                  : cudaSuccess) ||
       (has_ilu(s) ? s->d_sweep.alloc(2 * (size_t)n_rows * (p.precond == GALES_PRECOND_ILU ? sizeof(double) : sizeof(float)) +
                                      2 * sizeof(unsigned int))
-                  : cudaSuccess) || s->d_status.alloc(1)) {
+                  : cudaSuccess) || s->d_status.alloc(1) || s->d_count.upload(std::vector<unsigned int>(1, 0u))) {
     cudaGetLastError();
     return bail(GALES_ERR_NO_MEMORY);
   }
@@ -1193,7 +1293,7 @@ int gales_solver_solve(gales_solver* s, const double* vals, const double* rhs, d
   double* hb = s->h_buf;
   std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), y(m), h(m + 2);
   // ||b||; r = b (x0 = 0)
-  int rc = mdot(s, db, 0, 1, db, s->d_h.p + m + 1, 2, st);
+  int rc = arnoldi<kSubNorm>(s, nullptr, 0, const_cast<double*>(db), s->d_h.p + m + 1, st);  // db is only read
   if (rc) return rc;
   SCK(s, cudaMemcpyAsync(hb, s->d_h.p + m + 1, sizeof(double), cudaMemcpyDeviceToHost, st), "norm");
   SCK(s, cudaStreamSynchronize(st), "norm");
@@ -1231,17 +1331,14 @@ int gales_solver_solve(gales_solver* s, const double* vals, const double* rhs, d
       SCK(s, o.spmv(s, dA, zj, nullptr, s->d_w.p, st), "spmv");
       ++s->launches;
       // two classical Gram-Schmidt passes: h = V^T w, w -= V h (twice; h summed)
-      rc = mdot(s, V, n, j + 1, s->d_w.p, s->d_h.p, 0, st);
+      rc = arnoldi<kDots>(s, V, j + 1, s->d_w.p, nullptr, st);
       if (rc) return rc;
-      axpy_multi_kernel<<<sg, 256, (j + 1) * sizeof(double), st>>>(V, n, j + 1, s->d_h.p, s->d_w.p, n);
-      rc = mdot(s, V, n, j + 1, s->d_w.p, s->d_h2.p, 0, st);
+      rc = arnoldi<kSubDots>(s, V, j + 1, s->d_w.p, nullptr, st);
       if (rc) return rc;
-      axpy_multi_kernel<<<sg, 256, (j + 1) * sizeof(double), st>>>(V, n, j + 1, s->d_h2.p, s->d_w.p, n);
-      mdot_final_kernel<<<1, 256, 0, st>>>(s->d_h2.p, 1, j + 1, s->d_h.p, 1);  // h += h2
-      rc = mdot(s, s->d_w.p, 0, 1, s->d_w.p, s->d_h.p + j + 1, 2, st);
+      rc = arnoldi<kSubNorm>(s, V, j + 1, s->d_w.p, s->d_h.p + j + 1, st);
       if (rc) return rc;
       scale_kernel<<<sg, 256, 0, st>>>(s->d_w.p, s->d_h.p + j + 1, V + (int64_t)(j + 1) * n, n);
-      s->launches += 4;
+      ++s->launches;
       SCK(s, cudaGetLastError(), "Arnoldi step");
       SCK(s, cudaMemcpyAsync(hb, s->d_h.p, (j + 2) * sizeof(double), cudaMemcpyDeviceToHost, st), "Hessenberg");
       SCK(s, cudaStreamSynchronize(st), "Arnoldi step");
@@ -1278,7 +1375,7 @@ int gales_solver_solve(gales_solver* s, const double* vals, const double* rhs, d
     // r = b - A x, beta = ||r||
     SCK(s, o.spmv(s, dA, dx, db, s->d_r.p, st), "residual");
     s->launches += 2;
-    rc = mdot(s, s->d_r.p, 0, 1, s->d_r.p, s->d_h.p + m + 1, 2, st);
+    rc = arnoldi<kSubNorm>(s, nullptr, 0, s->d_r.p, s->d_h.p + m + 1, st);
     if (rc) return rc;
     SCK(s, cudaMemcpyAsync(hb, s->d_h.p + m + 1, sizeof(double), cudaMemcpyDeviceToHost, st), "residual norm");
     SCK(s, cudaStreamSynchronize(st), "residual");
@@ -1338,7 +1435,9 @@ void gales_solver_destroy(gales_solver* s) {
   s->d_j.release();
   s->d_ready.release();
   s->d_sweep.release();
+  s->d_udiag.release();
   s->d_status.release();
+  s->d_count.release();
   delete s;
 }
 
