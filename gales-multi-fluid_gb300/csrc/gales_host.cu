@@ -813,8 +813,8 @@ int gales_asm_create(const gales_mesh_desc* m, const gales_material_desc* mat,
     gales_asm_destroy(h);
     return GALES_ERR_UNSUPPORTED;
   }
-  {  // chunk size per form (kRecordBytes of point records, a multiple of four elements);
-     // one record buffer for the larger
+  {  // chunk size per form (kRecordBytes of point records, a multiple of the elements of a
+     // block of records); one record buffer for the larger
     int sms = 0;
     if ((ce = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess)
       return bail(ce, "device attribute");
@@ -823,11 +823,11 @@ int gales_asm_create(const gales_mesh_desc* m, const gales_material_desc* mat,
     for (int f = 0; f < 2; ++f) {
       const size_t rb = h->ops[f].rec_bytes(h->nc);
       if (rb == 0) continue;
-      const long long cap = std::max<long long>(4, (long long)(kRecordBytes / rb) / 4 * 4);
+      const long long blk = h->ops[f].rec_block(h->nc);
+      const long long cap = std::max<long long>(blk, (long long)(kRecordBytes / rb) / blk * blk);
       h->chunk_elems[f] = std::max<long long>(1, std::min<long long>(cap, std::max<int64_t>(h->n_el, 1)));
       h->chunk_default[f] = h->chunk_elems[f];
-      // records are written in blocks of (elements per matrix CTA, at most 4) elements
-      bytes = std::max(bytes, rb * (size_t)(h->chunk_elems[f] + 4));
+      bytes = std::max(bytes, rb * (size_t)(h->chunk_elems[f] + blk));
     }
     if ((ce = h->qpbuf.alloc(std::max<size_t>(bytes, 16))) != cudaSuccess) return bail(ce, "point-record buffer");
   }
@@ -1119,7 +1119,7 @@ int run_interior(gales_asm* h, const KParams& k, int form, bool want_m, long lon
       cnt = std::min(cnt, chunk);
     }
     cnt = std::min(cnt, n - first);
-    LaunchResult r = ops.point(*kp, h->nc, buf, first, cnt, st);
+    LaunchResult r = ops.point(*kp, h->nc, want_m, buf, first, cnt, st);
     if (r.err != cudaSuccess) return cuda_fail(h, r.err, "point kernel");
     h->launches += r.launches;
     if (c == 0) {
@@ -1803,7 +1803,8 @@ int gales_asm_set_magma(gales_asm* h, gales_magma* m) {
   MagmaOps mo = h->dim == 2 ? (h->nen == 3 ? magma_ops_tri3() : magma_ops_quad4())
                             : (h->nen == 4 ? magma_ops_tet4() : magma_ops_hex8());
   for (int f = 0; f < 2; ++f) {  // kernel attributes, once, outside any stream capture
-    if (mo.interior[f].rec_bytes(h->nc) != h->ops_ch[f].rec_bytes(h->nc))
+    if (mo.interior[f].rec_bytes(h->nc) != h->ops_ch[f].rec_bytes(h->nc) ||
+        mo.interior[f].rec_block(h->nc) != h->ops_ch[f].rec_block(h->nc))
       return fail(h, GALES_ERR_UNSUPPORTED, "magma point records differ from the chemicals'");
     CK(h, mo.interior[f].prepare(h->nc), "kernel attributes");
     KParams k0;
@@ -1998,11 +1999,12 @@ extern "C" int gales_asm_assemble_noalloc(gales_asm* h, const double* I, const d
   const InteriorOps& ops = h->ops[form];
   const size_t rb = ops.rec_bytes(h->nc);
   if (rb == 0) return fail(h, GALES_ERR_UNSUPPORTED, "no interior kernel for this element/component count");
-  // point records are written in blocks of a matrix CTA's elements (at most 4), so a
-  // chunk is a multiple of 4 elements and its blocks never pass the chunk's bytes
-  if (4 * rb > GALES_NOALLOC_SCRATCH_BYTES)
+  // point records are written in blocks of rec_block() elements, so a chunk is a multiple of
+  // that and its blocks never pass the chunk's bytes
+  const long long blk = ops.rec_block(h->nc);
+  if (blk * rb > GALES_NOALLOC_SCRATCH_BYTES)
     return fail(h, GALES_ERR_UNSUPPORTED,
-                "four elements' point records (" + std::to_string(4 * rb) + " bytes) exceed the " +
+                "a block of point records (" + std::to_string(blk * rb) + " bytes) exceeds the " +
                     std::to_string((long long)GALES_NOALLOC_SCRATCH_BYTES) + "-byte no-allocation scratch");
   void* scratch = nullptr;
   int rc = noalloc_scratch(h, &scratch);
@@ -2023,10 +2025,10 @@ extern "C" int gales_asm_assemble_noalloc(gales_asm* h, const double* I, const d
   CK(h, cudaMemsetAsync(rhs, 0, (size_t)h->n_rows * sizeof(double), st), "memset rhs");
   // The point records of a chunk are written in full by the point kernel before the
   // matrix kernel reads them, so nothing in the scratch has to start at zero.
-  const long long chunk = (long long)(GALES_NOALLOC_SCRATCH_BYTES / rb) / 4 * 4;
+  const long long chunk = (long long)(GALES_NOALLOC_SCRATCH_BYTES / rb) / blk * blk;
   for (long long first = 0; first < h->n_el; first += chunk) {
     const long long cnt = std::min(chunk, h->n_el - first);
-    LaunchResult r = ops.point(k, h->nc, scratch, first, cnt, st);
+    LaunchResult r = ops.point(k, h->nc, true, scratch, first, cnt, st);
     if (r.err != cudaSuccess) return cuda_fail(h, r.err, "point kernel");
     h->launches += r.launches;
     r = ops.matrix(k, h->nc, true, scratch, first, cnt, st);

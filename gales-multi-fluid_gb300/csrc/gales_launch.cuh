@@ -6,7 +6,7 @@
 
 #include <type_traits>
 
-#include "gales_kernels.cuh"
+#include "gales_fp64.cuh"
 
 namespace gales {
 
@@ -22,9 +22,10 @@ struct InteriorInst {
   using RB = RecBlock<DIM, NEN, NC, NQ, S>;
   using SM = MatSmem<DIM, NEN, NC, NQ, S>;
   using M = MatShape<DIM, NEN, NC>;
-  // record bytes per element, rounded up: (elements + 4) of them hold the blocks of a
-  // chunk of elements
+  // record bytes per element, rounded up, and elements per block of records: a chunk of n
+  // elements needs at most (n + rec_block()) rec_bytes()
   static size_t rec_bytes() { return (RB::BYTES + M::EPC - 1) / M::EPC; }
+  static int rec_block() { return 4; }
   // resident point-kernel CTAs (128 threads) per SM
   static int point_occupancy() {
     int nb = 0;
@@ -33,7 +34,7 @@ struct InteriorInst {
       return 1;
     return nb > 0 ? nb : 1;
   }
-  static LaunchResult point(const KParams& k, void* buf, long long first, long long n, cudaStream_t st) {
+  static LaunchResult point(const KParams& k, bool, void* buf, long long first, long long n, cudaStream_t st) {
     if (n <= 0) return {cudaSuccess, 0};
     const long long threads = n * NQ;
     point_kernel<DIM, NEN, NC, NQ, FORM, S, EOS><<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(
@@ -62,7 +63,7 @@ struct InteriorInst {
     return cudaSuccess;
   }
   // persistent: at most (SMs x resident CTAs) CTAs, each looping over element groups
-  static LaunchResult matrix(const KParams& k, bool want_m, const void* buf, long long first, long long n,
+  static LaunchResult matrix(const KParams& k, bool want_m, void* buf, long long first, long long n,
                              cudaStream_t st) {
     if (n <= 0) return {cudaSuccess, 0};
     const size_t smem = SM::BYTES;
@@ -73,6 +74,58 @@ struct InteriorInst {
     if (want_m) matrix_kernel<DIM, NEN, NC, NQ, S, true><<<blocks, M::CTA, smem, st>>>(k, in, first, n);
     else matrix_kernel<DIM, NEN, NC, NQ, S, false><<<blocks, M::CTA, smem, st>>>(k, in, first, n);
     return {cudaGetLastError(), 1};
+  }
+};
+
+// The blocked rows' diagonal after the FP64 matrix stage, where some flag blocks a dof and the
+// blocks are scattered or contracted; counts the matrix launch too.
+template <int DIM, int NEN, int NC>
+LaunchResult dirichlet64(const KParams& k, const double* in, long long n, cudaStream_t st) {
+  const cudaError_t e = cudaGetLastError();
+  uint32_t any = 0u;
+  for (int f = 0; f < GALES_MAX_FLAGS; ++f) any |= k.dirichlet_mask[f];
+  if (e != cudaSuccess || !any || k.local_r) return {e, 1};
+  dirichlet64_kernel<DIM, NEN, NC><<<(unsigned)((n + 127) / 128), 128, 0, st>>>(k, in, n);
+  return {cudaGetLastError(), 2};
+}
+
+// The FP64 form of a simplex (gales_fp64.cuh).
+template <int DIM, int NC, int EOS>
+struct Simplex64Inst {
+  static constexpr int NEN = DIM + 1;
+  using R = Rec64<DIM, NEN, NC>;
+  static constexpr size_t kSmem = sizeof(Rows64Smem<DIM, NC>);
+  static size_t rec_bytes() { return R::ELEM_BYTES; }
+  static int rec_block() { return R::EB; }
+  static int point_occupancy() {
+    int nb = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, point64_kernel<DIM, NEN, NC, EOS, true>, 128, 0) !=
+        cudaSuccess)
+      return 1;
+    return nb > 0 ? nb : 1;
+  }
+  static cudaError_t prepare() {
+    return cudaFuncSetAttribute(rows64_kernel<DIM, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+  }
+  static LaunchResult point(const KParams& k, bool want_m, void* buf, long long first, long long n, cudaStream_t st) {
+    if (n <= 0) return {cudaSuccess, 0};
+    const unsigned blocks = (unsigned)((n * NEN + 127) / 128);
+    double* out = reinterpret_cast<double*>(buf);
+    if (want_m) point64_kernel<DIM, NEN, NC, EOS, true><<<blocks, 128, 0, st>>>(k, out, first, n);
+    else point64_kernel<DIM, NEN, NC, EOS, false><<<blocks, 128, 0, st>>>(k, out, first, n);
+    return {cudaGetLastError(), 1};
+  }
+  static LaunchResult matrix(const KParams& k, bool want_m, void* buf, long long first, long long n, cudaStream_t st) {
+    if (n <= 0) return {cudaSuccess, 0};
+    double* in = reinterpret_cast<double*>(buf);
+    const long long tasks = (n + R::EB - 1) / R::EB * R::ND;   // a warp each
+    if (!want_m) {
+      residual64_kernel<DIM, NEN, NC><<<(unsigned)((tasks + 3) / 4), 128, 0, st>>>(k, in, first, n);
+      return {cudaGetLastError(), 1};
+    }
+    const long long nblk = (n + R::EB - 1) / R::EB, ncta = (nblk + kRows64Warps - 1) / kRows64Warps * R::ND;
+    rows64_kernel<DIM, NC><<<(unsigned)ncta, 32 * kRows64Warps, kSmem, st>>>(k, in, first, n);
+    return dirichlet64<DIM, NEN, NC>(k, in, n, st);
   }
 };
 
@@ -104,9 +157,9 @@ struct InteriorOps {
   cudaError_t (*prepare)(int nc);
   int (*point_occupancy)(int nc);
   size_t (*rec_bytes)(int nc);
-  LaunchResult (*point)(const KParams&, int nc, void* buf, long long first, long long n, cudaStream_t);
-  LaunchResult (*matrix)(const KParams&, int nc, bool want_m, const void* buf, long long first, long long n,
-                         cudaStream_t);
+  int (*rec_block)(int nc);
+  LaunchResult (*point)(const KParams&, int nc, bool want_m, void* buf, long long first, long long n, cudaStream_t);
+  LaunchResult (*matrix)(const KParams&, int nc, bool want_m, void* buf, long long first, long long n, cudaStream_t);
 };
 
 #define GALES_NC_SWITCH(expr_nc, CALL) \
@@ -118,40 +171,53 @@ struct InteriorOps {
     default: break;                    \
   }
 
+template <int DIM, int NEN, int NC, int NQ, int FORM, int EOS>
+using InteriorOf = typename std::conditional<FORM == GALES_FORM_FP64 && NEN == DIM + 1, Simplex64Inst<DIM, NC, EOS>,
+                                             InteriorInst<DIM, NEN, NC, NQ, FORM, EOS>>::type;
+
 template <int DIM, int NEN, int NQ, int FORM, int EOS = kEosChemicals>
 struct InteriorDispatch {
+  template <int NC>
+  using I = InteriorOf<DIM, NEN, NC, NQ, FORM, EOS>;
   static cudaError_t prepare(int nc) {
-#define GALES_C(NC) return InteriorInst<DIM, NEN, NC, NQ, FORM, EOS>::prepare()
+#define GALES_C(NC) return I<NC>::prepare()
     GALES_NC_SWITCH(nc, GALES_C)
 #undef GALES_C
     return cudaErrorInvalidValue;
   }
   static int point_occupancy(int nc) {
-#define GALES_C(NC) return InteriorInst<DIM, NEN, NC, NQ, FORM, EOS>::point_occupancy()
+#define GALES_C(NC) return I<NC>::point_occupancy()
     GALES_NC_SWITCH(nc, GALES_C)
 #undef GALES_C
     return 1;
   }
   static size_t rec_bytes(int nc) {
-#define GALES_C(NC) return InteriorInst<DIM, NEN, NC, NQ, FORM, EOS>::rec_bytes()
+#define GALES_C(NC) return I<NC>::rec_bytes()
     GALES_NC_SWITCH(nc, GALES_C)
 #undef GALES_C
     return 0;
   }
-  static LaunchResult point(const KParams& k, int nc, void* buf, long long first, long long n, cudaStream_t st) {
-#define GALES_C(NC) return InteriorInst<DIM, NEN, NC, NQ, FORM, EOS>::point(k, buf, first, n, st)
+  static int rec_block(int nc) {
+#define GALES_C(NC) return I<NC>::rec_block()
+    GALES_NC_SWITCH(nc, GALES_C)
+#undef GALES_C
+    return 4;
+  }
+  static LaunchResult point(const KParams& k, int nc, bool want_m, void* buf, long long first, long long n,
+                            cudaStream_t st) {
+#define GALES_C(NC) return I<NC>::point(k, want_m, buf, first, n, st)
     GALES_NC_SWITCH(nc, GALES_C)
 #undef GALES_C
     return {cudaErrorInvalidValue, 0};
   }
-  static LaunchResult matrix(const KParams& k, int nc, bool want_m, const void* buf, long long first, long long n,
+  static LaunchResult matrix(const KParams& k, int nc, bool want_m, void* buf, long long first, long long n,
                              cudaStream_t st) {
-#define GALES_C(NC) return InteriorInst<DIM, NEN, NC, NQ, FORM, EOS>::matrix(k, want_m, buf, first, n, st)
+#define GALES_C(NC) return I<NC>::matrix(k, want_m, buf, first, n, st)
     GALES_NC_SWITCH(nc, GALES_C)
 #undef GALES_C
     return {cudaErrorInvalidValue, 0};
   }
-  static InteriorOps ops() { return {&prepare, &point_occupancy, &rec_bytes, &point, &matrix}; }
+  static InteriorOps ops() { return {&prepare, &point_occupancy, &rec_bytes, &rec_block, &point, &matrix}; }
 };
 
 // Boundary pass of one element type; S is the matrix arithmetic type of the form.

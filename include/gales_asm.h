@@ -204,10 +204,9 @@ int gales_asm_assemble(gales_asm* h, const double* I, const double* P, double dt
  * GALES_ERR_BAD_INPUT since staging them would allocate), the work runs on the
  * caller's stream only, and the per-point records live in one library-wide
  * device array of GALES_NOALLOC_SCRATCH_BYTES, which every GPU that loads the
- * library keeps until exit.  Point records are laid out in blocks of up to four
- * elements: when four elements' records exceed that size the call is rejected with
- * GALES_ERR_UNSUPPORTED; larger meshes are processed in chunks of a multiple of four
- * elements.
+ * library keeps until exit.  Point records are laid out in blocks of up to 32
+ * elements: when a block's records exceed that size the call is rejected with
+ * GALES_ERR_UNSUPPORTED; larger meshes are processed in chunks of whole blocks.
  * The first call on a device looks up the array's device address (once per
  * device) and keeps it for the life of the process; make that first call before any
  * stream capture.  A reset of the device (cudaDeviceReset, or any reset of its
