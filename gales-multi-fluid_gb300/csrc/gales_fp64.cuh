@@ -8,6 +8,7 @@
 //                     rounding to binary32), the whole residual of the point and the vectors
 //                     from which the element block is built.
 //   rows64_kernel   - simplices: one thread per (element, dof row r), see below.
+//   tensor64_kernel - quadrilaterals and hexahedra, see below.
 //   residual64_kernel - the rhs alone.
 //   dirichlet64_kernel - the diagonal of blocked rows, which needs the block's whole trace.
 //
@@ -32,15 +33,22 @@
 
 namespace gales {
 
+// Place of the product of directions k <= l in a record.
+__host__ __device__ constexpr int gg_at(int dim, int k, int l) { return k * dim - k * (k - 1) / 2 + (l - k); }
+
 // Words of a point's record and of an element's, in doubles.  Words named J.., r0, DE, zeta,
 // Z, Theta and their scalars and entries (ZU .. THE, ZV .. THV) carry the point's weight JxW.  A block holds EB elements, word
 // major with the element innermost: word f of point q of element l at [(q RW + f) EB + l], so
-// a warp whose lanes are elements reads 256 contiguous bytes a word.
+// a warp whose lanes are elements reads 256 contiguous bytes a word (quadrilaterals and
+// hexahedra, whose matrix stage has a CTA per element, keep a sector of 4 together).
 template <int DIM, int NEN, int NC>
 struct Rec64 {
   using L = Layout<DIM, NC>;
   static constexpr int ND = L::ND, NQ = NEN, N = NEN * ND;
-  static constexpr int EB = 32;
+  static constexpr bool SIMPLEX = NEN == DIM + 1;
+  static constexpr int EB = SIMPLEX ? 32 : 4;
+  static constexpr int NGG = SIMPLEX ? 0 : DIM * (DIM + 1) / 2;   // products of two directions
+  static constexpr int NG = SIMPLEX ? 0 : DIM * DIM;              // the directions themselves
   static constexpr int NR = 1 + NC;    // columns p, T, Y_1.. of r0 and of the energy row of DUDY
   static constexpr int JX = 0, JR = 1, RHO = 2, PR = 3, NU = 4, JMU = 5, JKAP = 6, EG = 7, ZU = 8, T0U = 9, THU = 10;
   static constexpr int ZE = 11, T0E = 12, THE = 13, E = 14;
@@ -49,7 +57,8 @@ struct Rec64 {
   static constexpr int Y = THV + DIM, H = Y + L::NYA, JRN = H + L::NYA, JRD = JRN + L::NYA, JRDH = JRD + L::NYA;
   static constexpr int R0 = JRDH + L::NYA, DE = R0 + NR;
   static constexpr int ZETA = DE + NR, ZZ = ZETA + ND, THETA = ZZ + ND;
-  static constexpr int RV = THETA + ND, PHI = RV + ND;
+  static constexpr int GG = THETA + ND, G = GG + NGG;
+  static constexpr int RV = G + NG, PHI = RV + ND;
   static constexpr int RW = PHI + DIM * ND;
   // element words: the rows' shares of the trace, then the scatter descriptors as 32-bit
   // integers: node, CSR row length, Dirichlet mask of each node b, then per (b, a) the unit
@@ -239,14 +248,31 @@ __device__ __forceinline__ bool tau_params(const KParams& k, const ElemGeo<DIM, 
   return false;
 }
 
-// Directions the element block is built in: the gradients of the barycentric coordinates
-// 1..DIM of a simplex (its nodes' shape gradients).
+// Directions the element block is built in, the gradients of the reference coordinates: those
+// of the barycentric coordinates 1..DIM of a simplex (its nodes' shape gradients), of xi, eta,
+// zeta of a quadrilateral or hexahedron (xi = sum_i xi_i N_i with the nodes' xi_i = +-1).
 template <int DIM, int NEN>
 __device__ __forceinline__ void directions(const ElemGeo<DIM, NEN>& q, double (&g)[DIM][DIM]) {
+  if constexpr (NEN == DIM + 1) {
 #pragma unroll
-  for (int k = 0; k < DIM; ++k)
+    for (int k = 0; k < DIM; ++k)
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) g[k][d] = q.ds[d][k + 1];
+      for (int d = 0; d < DIM; ++d) g[k][d] = q.ds[d][k + 1];
+  } else {
+#pragma unroll
+    for (int k = 0; k < DIM; ++k)
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) {
+        double s = 0.0;
+#pragma unroll
+        for (int i = 0; i < NEN; ++i) {
+          // element.hpp node order: x+ at 1, 2 (mod 4), y+ at 2, 3 (mod 4), z+ at 4..7
+          const bool plus = k == 0 ? ((i & 3) == 1 || (i & 3) == 2) : (k == 1 ? (i & 3) >= 2 : i >= 4);
+          s = plus ? s + q.ds[d][i] : s - q.ds[d][i];
+        }
+        g[k][d] = s;
+      }
+  }
 }
 
 // The point stage of one (element, point): about 1,100 FP64 operations, the FP64 pipe 84% busy
@@ -639,6 +665,20 @@ __device__ __forceinline__ void point64(const KParams& k, long long e, int iq, d
       W(R::T0V + d) = t0[1 + d];
       W(R::THV + d) = theta(z[1 + d], y[1 + d], t0[1 + d]);
     }
+    if constexpr (!R::SIMPLEX) {
+#pragma unroll
+      for (int a = 0; a < DIM; ++a) {
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) W(R::G + a * DIM + d) = g[a][d];
+#pragma unroll
+        for (int b = a; b < DIM; ++b) {
+          double s = g[a][0] * g[b][0];
+#pragma unroll
+          for (int d = 1; d < DIM; ++d) s = fma(g[a][d], g[b][d], s);
+          W(R::GG + gg_at(DIM, a, b)) = s;
+        }
+      }
+    }
 #pragma unroll
     for (int kk = 0; kk < DIM; ++kk) {
       double s = g[kk][0] * v[0], ek = g[kk][0] * f[0];
@@ -690,30 +730,53 @@ __global__ void __launch_bounds__(128) point64_kernel(const KParams k, double* _
   if (k.clear_n[0] > 0 || k.clear_n[1] > 0) clear_arrays(k);
 }
 
-// rhs of row r of the element at place l: -(sum_q N_b rv + sum_d dN_b/dx_d sum_q phi_d)
+// rhs of row r of the element at place l: -(sum_q N_b rv + sum_d dN_b/dx_d phi_d); a simplex's
+// gradients do not depend on the point.
 template <int DIM, int NEN, int NC, typename Sink>
 __device__ __forceinline__ void row_residual64(const KParams& k, const double* __restrict__ blk, int l, int r,
-                                               const ElemGeo<DIM, NEN>& q, Sink sink) {
+                                               const ElemGeo<DIM, NEN>* __restrict__ geo, Sink sink) {
   using R = Rec64<DIM, NEN, NC>;
   constexpr int NQ = NEN, ND = R::ND;
-  static_assert(NEN == DIM + 1, "gradients that do not depend on the point");
-  double rv[NQ], ph[DIM];
+  auto W = [&](int p, int f) -> double { return blk[(size_t)(p * R::RW + f) * R::EB + l]; };
+  if constexpr (R::SIMPLEX) {
+    double rv[NQ], ph[DIM];
 #pragma unroll
-  for (int d = 0; d < DIM; ++d) ph[d] = 0.0;
+    for (int d = 0; d < DIM; ++d) ph[d] = W(0, R::PHI + d * ND + r);
 #pragma unroll
-  for (int p = 0; p < NQ; ++p) {
-    rv[p] = blk[(size_t)(p * R::RW + R::RV + r) * R::EB + l];
+    for (int p = 0; p < NQ; ++p) {
+      rv[p] = W(p, R::RV + r);
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) ph[d] += blk[(size_t)(p * R::RW + R::PHI + d * ND + r) * R::EB + l];
-  }
+      for (int d = 0; d < DIM; ++d)
+        if (p > 0) ph[d] += W(p, R::PHI + d * ND + r);
+    }
 #pragma unroll
-  for (int b = 0; b < NEN; ++b) {
-    double s = q.ds[0][b] * ph[0];
+    for (int b = 0; b < NEN; ++b) {
+      double s = geo->ds[0][b] * ph[0];
 #pragma unroll
-    for (int d = 1; d < DIM; ++d) s = fma(q.ds[d][b], ph[d], s);
+      for (int d = 1; d < DIM; ++d) s = fma(geo->ds[d][b], ph[d], s);
 #pragma unroll
-    for (int p = 0; p < NQ; ++p) s = fma(k.sh_tab[p][b], rv[p], s);
-    sink(b, -s);
+      for (int p = 0; p < NQ; ++p) s = fma(k.sh_tab[p][b], rv[p], s);
+      sink(b, -s);
+    }
+  } else {
+    double s[NEN];
+#pragma unroll
+    for (int b = 0; b < NEN; ++b) s[b] = 0.0;
+#pragma unroll 1
+    for (int p = 0; p < NQ; ++p) {
+      const double rv = W(p, R::RV + r);
+      double ph[DIM];
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) ph[d] = W(p, R::PHI + d * ND + r);
+#pragma unroll
+      for (int b = 0; b < NEN; ++b) {
+        s[b] = fma(k.sh_tab[p][b], rv, s[b]);
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) s[b] = fma(geo[p].ds[d][b], ph[d], s[b]);
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < NEN; ++b) sink(b, -s[b]);
   }
 }
 
@@ -722,7 +785,7 @@ template <int DIM, int NEN, int NC>
 __global__ void __launch_bounds__(128) residual64_kernel(const KParams k, const double* __restrict__ in, long long first,
                                                          long long n) {
   using R = Rec64<DIM, NEN, NC>;
-  constexpr int ND = R::ND, EB = R::EB;
+  constexpr int ND = R::ND, EB = R::EB, NGE = geo_per_element<DIM, NEN>(NEN);
   const long long t = (long long)blockIdx.x * 128 + threadIdx.x;
   const int l = (int)(t % EB);
   const long long task = t / EB;
@@ -732,7 +795,7 @@ __global__ void __launch_bounds__(128) residual64_kernel(const KParams k, const 
   const long long e = k.el_list ? (long long)k.el_list[first + li] : first + li;
   const double* blk = in + (size_t)b * R::EW * EB;
   const int32_t* di = reinterpret_cast<const int32_t*>(blk + (size_t)R::INTS * EB);
-  row_residual64<DIM, NEN, NC>(k, blk, l, r, reinterpret_cast<const ElemGeo<DIM, NEN>*>(k.geo)[e], [&](int nb, double v) {
+  row_residual64<DIM, NEN, NC>(k, blk, l, r, reinterpret_cast<const ElemGeo<DIM, NEN>*>(k.geo) + e * NGE, [&](int nb, double v) {
     if (k.local_r) {
       k.local_r[(first + li) * R::N + nb * ND + r] = v;
     } else if (!(((uint32_t)di[(R::I_BLOCKED + nb) * EB + l] >> r) & 1u)) {
@@ -1020,7 +1083,7 @@ __global__ void __launch_bounds__(32 * kRows64Warps)
   if (vjp) {
     for (int c = 0; c < N; ++c) st[lane * NS + c] = 0.0;
   } else {
-    row_residual64<DIM, NEN, NC>(k, blk, l, r, geo, [&](int nb, double v) {
+    row_residual64<DIM, NEN, NC>(k, blk, l, r, &geo, [&](int nb, double v) {
       if (lane >= cnt) return;
       if (local) k.local_r[(first + li) * N + nb * ND + r] = v;
       else if (!(((uint32_t)di[(R::I_BLOCKED + nb) * EB + l] >> r) & 1u))
@@ -1089,6 +1152,370 @@ __global__ void __launch_bounds__(32 * kRows64Warps)
       const double val = st[el * NS + cx];
       if (val != 0.0) atomicAdd(k.vjp_g + (long long)di[(R::I_NODE + a) * EB + el] * ND + (cx - a * ND), val);
     }
+  }
+}
+
+// Matrix stage of quadrilaterals and hexahedra, a CTA per element.  In the reference
+// directions the block is
+//   block(b, a) = sum_q sum_ij phi_b^i(q) H_ij(q) phi_a^j(q),  phi^0 = N, phi^k = dN/dxi_k,
+// with nd x nd matrices H_ij of the point that do not know the nodes:
+//   H_00 = JxW (DUDY/dt - S0) + source's least squares     H_k0 = JxW (FPT_k (DUDY/dt - S0) - A_k)
+//   H_0l = -JxW S0 tau A_l (energy row alone)               H_kl = JxW (FPT_k A_l + K'_kl),
+// FPT_k = A_k tau for the test function with gradient e_k (see the head of this file).  A
+// thread per (point, dof row) forms the H_ij in shared memory (about 540 FP64 operations with
+// 8 dofs), then a thread per (row, column) contracts one direction after the other with the
+// one-dimensional shape functions (sum factorisation): 1,600 operations for its 64 entries of
+// the hexahedron against 3,072 for a direct contraction.  With FPT_b and the block rows formed
+// per test function and point it was 481,000 operations per hexahedron; now 131,000.  Bound:
+// the FP64 pipe.
+template <int DIM, int NC>
+struct Tensor64 {
+  static constexpr int NEN = 1 << DIM;
+  using R = Rec64<DIM, NEN, NC>;
+  static constexpr int ND = R::ND, NQ = NEN, NF = DIM + 1;
+  static constexpr int RS = ND | 1;             // row stride of a matrix (conflict-free stores by row)
+  static constexpr int HS = ND * RS;            // words of one matrix
+  static constexpr int T1 = NQ * ND, T2 = ND * ND;
+  static constexpr int THREADS = ((T1 > T2 ? T1 : T2) + 31) / 32 * 32;
+  struct Smem {
+    double H[NF * NF][NQ][HS];
+    int32_t off[NEN][NEN], rowlen[NEN], node[NEN];
+    uint32_t blocked[NEN];
+  };
+  // node and point of the corner with the given signs (element.hpp order)
+  static __device__ __forceinline__ int corner(int x, int y, int z) { return (z << 2) | (y ? 3 - x : x); }
+};
+
+// H_ij of point q, row r.
+template <int DIM, int NC>
+__device__ __forceinline__ void tensor_point64(const KParams& k, const double* __restrict__ blk, int l, int q, int r,
+                                               double (*H)[Tensor64<DIM, NC>::NQ][Tensor64<DIM, NC>::HS]) {
+  using T = Tensor64<DIM, NC>;
+  using R = typename T::R;
+  using L = Layout<DIM, NC>;
+  constexpr int ND = T::ND, iT = L::iT, iY = L::iY, NF = T::NF;
+  const bool rE = r == iT, rV = r >= 1 && r < iT, rY = r >= iY;
+  auto W = [&](int f) -> double { return blk[(size_t)(q * R::RW + f) * R::EB + l]; };
+  auto out = [&](int i, int j, int c) -> double& { return H[i * NF + j][q][r * T::RS + c]; };
+  const double rho = W(R::RHO), jx = W(R::JX), jr = W(R::JR), nu = W(R::NU), jmu = W(R::JMU);
+  const double wr = r == 0 ? 1.0 : W(rV ? R::V + r - 1 : (rE ? R::E : R::Y + r - iY));
+  const double wz = rE ? 1.0 : wr;
+  const double ur = fma(rho, wr, rE ? W(R::PR) : 0.0);
+  const double rhf = rV ? rho * W(R::F + r - 1) : (rY ? rho * W(R::H + r - iY) : 0.0);
+  const int fz = rE ? R::THETA : R::ZETA;
+  double v[DIM], g[DIM][DIM], s[DIM];
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) {
+    v[d] = W(R::V + d);
+    s[d] = W(R::S + d);
+#pragma unroll
+    for (int a = 0; a < DIM; ++a) g[a][d] = W(R::G + a * DIM + d);
+  }
+  // FPT_k DUDY = s_k Q + gZ_k Z + u'_r e_k r0 (p, T, Y columns), rho (FPT_k + FPT_k[E] v) (velocities);
+  // Qv, Qe, Qu: the part of FPT_k's velocity and energy entries and of FPT_k.u' that goes with s_k
+  double Q[L::iT + NC], Qv[DIM], DR[ND], KD[ND];
+  const double Qe = wz * W(rE ? R::THE : R::ZE);
+  const double Qu = fma(rhf, jr, wz * W(rE ? R::THU : R::ZU));
+  const double t0e = W(R::T0E), t0u = W(R::T0U);
+  double t0v[DIM], jm[DIM];
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) {
+    t0v[d] = W(R::T0V + d);
+    jm[d] = W(R::JM + d);
+    Qv[d] = fma(rV && d == r - 1 ? rho : 0.0, jm[d], wz * W((rE ? R::THV : R::ZV) + d));
+  }
+  double r0[R::NR], Z[R::NR];
+#pragma unroll
+  for (int c = 0; c < ND; ++c) {
+    const int ci = R::col_r0(c);
+    if (ci >= 0) {
+      r0[ci < 0 ? 0 : ci] = W(R::R0 + (ci < 0 ? 0 : ci));
+      Z[ci < 0 ? 0 : ci] = W(R::ZZ + c);
+      double x = fma(rhf, r0[ci < 0 ? 0 : ci], wz * W(fz + c));
+      if (c >= iY) x = fma(rY && c == r ? rho : 0.0, W(R::JRN + (c - iY) % L::NYA), x);
+      Q[c] = x;
+      DR[c] = rE ? W(R::DE + (ci < 0 ? 0 : ci)) : wr * r0[ci < 0 ? 0 : ci];
+    } else {
+      Q[c] = 0.0;
+      DR[c] = rE ? jr * v[(c - 1) % DIM] : 0.0;
+    }
+    if (c >= 1 && c != iT) DR[c] += c == r ? jr : 0.0;
+    // what multiplies grad.grad: the diffusive entries of K and nu DUDY
+    double kd = 0.0;
+    if (c >= 1 && c < iT) kd = rE ? jmu * v[(c < 1 ? 0 : c - 1) % DIM] : (c == r ? jmu : 0.0);
+    if (c == iT) kd = rE ? W(R::JKAP) : 0.0;
+    if (c >= iY) kd = rE ? W(R::JRDH + (c - iY) % L::NYA) : (c == r ? W(R::JRD + (c - iY) % L::NYA) : 0.0);
+    KD[c] = fma(nu, DR[c], kd);
+  }
+  // the viscous entries on the velocity columns: jmu a_l g_k + jlam a_k g_l, a = g[., r] or s (energy row)
+  double av[DIM];
+#pragma unroll
+  for (int a = 0; a < DIM; ++a) {
+    double x = 0.0;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) x = (rV && d == r - 1) ? g[a][d] : x;
+    av[a] = rE ? s[a] : x;
+  }
+  const double jlam = (-2.0 / 3.0) * jmu;
+#pragma unroll
+  for (int kk = 0; kk < DIM; ++kk) {
+    const double sk = s[kk], gZ = rV ? av[kk] : 0.0, ue = ur * W(R::EK + kk);
+    const double fe = fma(gZ, t0e, sk * Qe);
+    double fu = fma(ue, jr, fma(gZ, t0u, sk * Qu));
+    double fv[DIM], FD[ND];
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      fv[d] = fma(ur * g[kk][d], jm[d], fma(gZ, t0v[d], sk * Qv[d]));
+      FD[1 + d] = rho * fma(fe, v[d], fv[d]);
+    }
+#pragma unroll
+    for (int c = 0; c < ND; ++c) {
+      const int ci = R::col_r0(c);
+      if (ci >= 0) FD[c] = fma(ue, r0[ci < 0 ? 0 : ci], fma(gZ, Z[ci < 0 ? 0 : ci], sk * Q[c]));
+    }
+    // H_k0
+    const double ug = jx * ur, fr = fe * rho;
+#pragma unroll
+    for (int c = 0; c < ND; ++c) {
+      double x = fma(k.inv_dt, FD[c], -sk * DR[c]);
+      if (c >= 1 && c < iT) {
+        x = fma(-ug, g[kk][(c < 1 ? 0 : c - 1) % DIM], x);
+        x = fma(-fr, k.gravity[(c < 1 ? 0 : c - 1) % DIM], x);
+      }
+      if (c == 0) x = fma(-jx, av[kk], x);
+      out(1 + kk, 0, c) = x;
+    }
+    // H_kl
+    fu = fma(jlam, av[kk], fu);
+#pragma unroll
+    for (int ll = 0; ll < DIM; ++ll) {
+      const double gg = W(R::GG + (kk <= ll ? gg_at(DIM, kk, ll) : gg_at(DIM, ll, kk)));
+      const double p1 = jmu * av[ll];
+      double xp = fe * s[ll];
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) xp = fma(fv[d], g[ll][d], xp);
+#pragma unroll
+      for (int c = 0; c < ND; ++c) {
+        double x = c == 0 ? fma(s[ll], FD[c], xp) : s[ll] * FD[c];
+        x = fma(gg, KD[c], x);
+        if (c >= 1 && c < iT) {
+          x = fma(fu, g[ll][(c < 1 ? 0 : c - 1) % DIM], x);
+          x = fma(p1, g[kk][(c < 1 ? 0 : c - 1) % DIM], x);
+        }
+        out(1 + kk, 1 + ll, c) = x;
+      }
+    }
+  }
+  // H_00, and the energy row's H_0l: FPT_0 = -rho t_g
+  double F0[ND];
+#pragma unroll
+  for (int c = 0; c < ND; ++c) F0[c] = 0.0;
+  if (rE) {
+    const double c0 = -rho * W(R::EG);
+    double fv[DIM];
+#pragma unroll
+    for (int c = 0; c < ND; ++c) {
+      const int ci = R::col_r0(c);
+      if (ci >= 0) F0[c] = c0 * r0[ci < 0 ? 0 : ci];
+    }
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      fv[d] = (-rho * k.gravity[d]) * jm[d];
+      F0[1 + d] = rho * fv[d];
+    }
+#pragma unroll
+    for (int ll = 0; ll < DIM; ++ll) {
+      double xp = fv[0] * g[ll][0];
+#pragma unroll
+      for (int d = 1; d < DIM; ++d) xp = fma(fv[d], g[ll][d], xp);
+#pragma unroll
+      for (int c = 0; c < ND; ++c) {
+        double x = c == 0 ? fma(s[ll], F0[c], xp) : s[ll] * F0[c];
+        if (c >= 1 && c < iT) x = fma(c0 * jr, g[ll][(c < 1 ? 0 : c - 1) % DIM], x);
+        out(0, 1 + ll, c) = x;
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < ND; ++c) {
+    double x = k.inv_dt * (DR[c] + F0[c]);
+    if (c >= 1 && c < iT && rE) x = fma(-jr, k.gravity[(c < 1 ? 0 : c - 1) % DIM], x);
+    out(0, 0, c) = x;
+  }
+}
+
+template <int DIM, int NC>
+__global__ void __launch_bounds__(Tensor64<DIM, NC>::THREADS)
+    tensor64_kernel(const KParams k, double* in, long long first, long long n) {
+  using T = Tensor64<DIM, NC>;
+  using R = typename T::R;
+  constexpr int NEN = T::NEN, NQ = T::NQ, ND = T::ND, N = R::N, EB = R::EB, iT = Layout<DIM, NC>::iT;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  typename T::Smem& S = *reinterpret_cast<typename T::Smem*>(smem_raw);
+  const int tid = threadIdx.x;
+  const long long li = blockIdx.x;
+  const long long e = k.el_list ? (long long)k.el_list[first + li] : first + li;
+  const int l = (int)(li % EB);
+  const double* blk = in + (size_t)(li / EB) * R::EW * EB;
+  const int32_t* di = reinterpret_cast<const int32_t*>(blk + (size_t)R::INTS * EB);
+  for (int t = tid; t < NEN * NEN; t += T::THREADS) S.off[t / NEN][t % NEN] = di[(R::I_OFF + t) * EB + l];
+  if (tid < NEN) {
+    S.rowlen[tid] = di[(R::I_ROWLEN + tid) * EB + l];
+    S.node[tid] = di[(R::I_NODE + tid) * EB + l];
+    S.blocked[tid] = (uint32_t)di[(R::I_BLOCKED + tid) * EB + l];
+  }
+  const bool local = k.local_r != nullptr, vjp = k.vjp_lam != nullptr;
+  const int mode = k.scatter_mode;
+  if (tid < T::T1) tensor_point64<DIM, NC>(k, blk, l, tid / ND, tid % ND, S.H);
+  __syncthreads();
+  // rhs: a thread per (node, row)
+  if (!vjp && tid < N) {
+    const int b = tid / ND, rr = tid - b * ND;
+    const ElemGeo<DIM, NEN>* geo = reinterpret_cast<const ElemGeo<DIM, NEN>*>(k.geo) + e * NQ;
+    double x = 0.0;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      auto W = [&](int f) -> double { return blk[(size_t)(q * R::RW + f) * EB + l]; };
+      x = fma(k.sh_tab[q][b], W(R::RV + rr), x);
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) x = fma(geo[q].ds[d][b], W(R::PHI + d * ND + rr), x);
+    }
+    if (local) k.local_r[(first + li) * N + tid] = -x;
+    else if (!((S.blocked[b] >> rr) & 1u)) add_to(k.rhs + (long long)S.node[b] * ND + rr, -x, mode);
+  }
+  if (local && !k.local_m) return;
+  const bool active = tid < T::T2;
+  const int r = active ? tid / ND : 0, c = active ? tid - r * ND : 0;
+  const int at = r * T::RS + c;
+  // the H_0l are there on the energy row alone
+  const bool src = r == iT;
+  const bool any_src = __any_sync(0xffffffffu, src);
+  // one-dimensional shape functions at the lower point: near and far node (the upper point's are
+  // mirrored); derivatives -1/2, 1/2
+  double nA, nB;
+  if constexpr (DIM == 2) {
+    nA = k.sh_tab[0][0] + k.sh_tab[0][3];
+    nB = k.sh_tab[0][1] + k.sh_tab[0][2];
+  } else {
+    nA = (k.sh_tab[0][0] + k.sh_tab[0][3]) + (k.sh_tab[0][4] + k.sh_tab[0][7]);
+    nB = (k.sh_tab[0][1] + k.sh_tab[0][2]) + (k.sh_tab[0][5] + k.sh_tab[0][6]);
+  }
+  auto n1 = [&](int a, int q) { return a == q ? nA : nB; };
+  double tr = 0.0, vacc[NEN];
+#pragma unroll
+  for (int a = 0; a < NEN; ++a) vacc[a] = 0.0;
+  auto sink = [&](int b, int a, double x) {
+    if (a == b && r == c) tr += x;
+    if (vjp) {
+      const bool off = (S.blocked[b] >> r) & 1u;
+      const double lam = off ? 0.0 : __ldg(k.vjp_lam + (long long)S.node[b] * ND + r);
+#pragma unroll
+      for (int q = 0; q < NEN; ++q) vacc[q] = q == a ? fma(lam, x, vacc[q]) : vacc[q];
+      return;
+    }
+    if (!active) return;
+    if (local) {
+      k.local_m[(first + li) * (long long)(N * N) + (b * ND + r) * N + a * ND + c] = x;
+      return;
+    }
+    if ((S.blocked[b] >> r) & 1u) return;
+    if (x != 0.0) add_to(k.vals + (int64_t)S.off[b][a] * ND + (int64_t)r * S.rowlen[b] + c, x, mode);
+  };
+  // V[qy][qx][i][j], i, j in {0, xi, eta}: the plane's matrices after the contraction over zeta
+  // for the pair (bz, az)
+  auto plane = [&](int bz, int az) {
+    double V[2][2][3][3];
+#pragma unroll
+    for (int qy = 0; qy < 2; ++qy)
+#pragma unroll
+      for (int qx = 0; qx < 2; ++qx) {
+        if constexpr (DIM == 2) {
+          const int q = T::corner(qx, qy, 0);
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) V[qy][qx][i][j] = (i > 0 || j == 0 || src) ? S.H[i * T::NF + j][q][at] : 0.0;
+        } else {
+          const int q0 = T::corner(qx, qy, 0), q1 = T::corner(qx, qy, 1);
+          const double b0 = n1(bz, 0), b1 = n1(bz, 1), a0 = n1(az, 0), a1 = n1(az, 1);
+          const double w0 = b0 * a0, w1 = b1 * a1;
+          const double db = bz ? 0.5 : -0.5, da = az ? 0.5 : -0.5;
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+              if (i == 0 && j > 0) continue;
+              V[qy][qx][i][j] = fma(w1, S.H[i * T::NF + j][q1][at], w0 * S.H[i * T::NF + j][q0][at]);
+            }
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {   // zeta derivative of the test function
+            const double x = fma(db * a1, S.H[3 * T::NF + j][q1][at], (db * a0) * S.H[3 * T::NF + j][q0][at]);
+            if (j == 0) V[qy][qx][0][0] += x;
+            else V[qy][qx][0][j] = x;
+          }
+#pragma unroll
+          for (int i = 1; i < 3; ++i)     // of the trial function
+            V[qy][qx][i][0] = fma(da * b1, S.H[i * T::NF + 3][q1][at],
+                                  fma(da * b0, S.H[i * T::NF + 3][q0][at], V[qy][qx][i][0]));
+          V[qy][qx][0][0] = fma(db * da, S.H[15][q0][at] + S.H[15][q1][at], V[qy][qx][0][0]);
+          if (any_src) {
+            // lanes of other rows read words that no thread writes: selected away
+#pragma unroll
+            for (int j = 1; j < 3; ++j) {
+              const double h0 = src ? S.H[j][q0][at] : 0.0, h1 = src ? S.H[j][q1][at] : 0.0;
+              V[qy][qx][0][j] = fma(w1, h1, fma(w0, h0, V[qy][qx][0][j]));
+            }
+            const double h0 = src ? S.H[3][q0][at] : 0.0, h1 = src ? S.H[3][q1][at] : 0.0;
+            V[qy][qx][0][0] = fma(da * b1, h1, fma(da * b0, h0, V[qy][qx][0][0]));
+          }
+        }
+      }
+#pragma unroll 1
+    for (int yp = 0; yp < 4; ++yp) {
+      const int by = yp >> 1, ay = yp & 1;
+      const double b0 = n1(by, 0), b1 = n1(by, 1), a0 = n1(ay, 0), a1 = n1(ay, 1);
+      const double w0 = b0 * a0, w1 = b1 * a1;
+      const double db = by ? 0.5 : -0.5, da = ay ? 0.5 : -0.5, dd = db * da;
+      double U[2][4];   // per qx: 00, x0, 0x, xx
+#pragma unroll
+      for (int qx = 0; qx < 2; ++qx) {
+        const double (&A)[3][3] = V[0][qx], (&B)[3][3] = V[1][qx];
+        double x = fma(w1, B[0][0], w0 * A[0][0]);
+        x = fma(db * a1, B[2][0], fma(db * a0, A[2][0], x));
+        x = fma(da * b1, B[0][2], fma(da * b0, A[0][2], x));
+        U[qx][0] = fma(dd, A[2][2] + B[2][2], x);
+        x = fma(w1, B[1][0], w0 * A[1][0]);
+        U[qx][1] = fma(da * b1, B[1][2], fma(da * b0, A[1][2], x));
+        x = fma(w1, B[0][1], w0 * A[0][1]);
+        U[qx][2] = fma(db * a1, B[2][1], fma(db * a0, A[2][1], x));
+        U[qx][3] = fma(w1, B[1][1], w0 * A[1][1]);
+      }
+      const double xx = 0.25 * (U[0][3] + U[1][3]);
+#pragma unroll
+      for (int bx = 0; bx < 2; ++bx)
+#pragma unroll
+        for (int ax = 0; ax < 2; ++ax) {
+          const double hb = bx ? 0.5 : -0.5, ha = ax ? 0.5 : -0.5;
+          double x = bx == ax ? xx : -xx;
+          x = fma(n1(bx, 1) * n1(ax, 1), U[1][0], fma(n1(bx, 0) * n1(ax, 0), U[0][0], x));
+          x = fma(hb * n1(ax, 1), U[1][1], fma(hb * n1(ax, 0), U[0][1], x));
+          x = fma(ha * n1(bx, 1), U[1][2], fma(ha * n1(bx, 0), U[0][2], x));
+          sink(T::corner(bx, by, bz), T::corner(ax, ay, az), x);
+        }
+    }
+  };
+  if constexpr (DIM == 2) {
+    plane(0, 0);
+  } else {
+#pragma unroll 1
+    for (int zp = 0; zp < 4; ++zp) plane(zp >> 1, zp & 1);
+  }
+  if (local) return;
+  if (active && r == c) in[((size_t)(li / EB) * R::EW + R::TR + r) * EB + l] = tr;
+  if (vjp && active) {
+#pragma unroll
+    for (int a = 0; a < NEN; ++a)
+      if (vacc[a] != 0.0) atomicAdd(k.vjp_g + (long long)S.node[a] * ND + c, vacc[a]);
   }
 }
 

@@ -1,11 +1,12 @@
 // Element assembly kernels for fluid_mc (interior and boundary passes).
 //
-// Interior pass, two kernels per chunk of elements:
+// Interior pass of the mixed form (the FP64 form's is in gales_fp64.cuh), two kernels per
+// chunk of elements:
 //   point_kernel  - one thread per (element, quadrature point): interpolation
 //                   (quad.hpp:817-885), mixture EOS at P and I (fluid_2d.hpp:179-195),
 //                   flux scalars (fluid_2d.hpp:391-603), tau (fluid_2d.hpp:877-1022)
 //                   and the dc viscosity (fluid_2d.hpp:1027-1065), written as a point
-//                   record in the form's arithmetic type S.
+//                   record in the matrix stage's arithmetic type S.
 //   matrix_kernel - one warp per element (more for hexahedra), one lane per row of
 //                   the element block: Galerkin, least-squares and dc terms of RM_i
 //                   (fluid_2d.hpp:251-333) accumulated in registers over the points,
@@ -458,18 +459,15 @@ __device__ __noinline__ double compute_h_reference(const double* __restrict__ I,
 }
 
 // Point phase for one (element, quadrature point).
-//   GALES_FORM_FP64 : every step in FP64 with the reference's operations; tau uses
-//                     the uBLAS-faithful LU inverse.
-//   GALES_FORM_MIXED: FP64 for the mixture EOS and its derivatives, U - U_P, the
-//                     element size h and tau with the closed-form DUDY inverse; the
-//                     fluxes, least-squares residual and dc viscosity in FP32.
-template <int DIM, int NEN, int NC, int NQ, int FORM, typename S, int BPS, int EOS = kEosChemicals>
+// FP64 for the mixture EOS and its derivatives, U - U_P, the element size h and tau with the
+// closed-form DUDY inverse; the fluxes, least-squares residual and dc viscosity in FP32.
+template <int DIM, int NEN, int NC, int NQ, typename S, int BPS, int EOS = kEosChemicals>
 __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<QP<DIM, NEN, NC, S>, BPS>& out) {
   using L = Layout<DIM, NC>;
   using QPT = QP<DIM, NEN, NC, S>;
   constexpr int ND = L::ND;
   constexpr int NG = geo_per_element<DIM, NEN>(NQ);
-  using R = typename std::conditional<FORM == GALES_FORM_FP64, double, float>::type;
+  using R = float;
   static_assert(NQ == NEN, "point q carries the scatter descriptor of node q");
   int nodes[NEN];
 #pragma unroll
@@ -510,37 +508,21 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
     const double* pi = k.P + (long long)nodes[i] * ND;
 #pragma unroll
     for (int j = 0; j < ND; ++j) {
-      if constexpr (FORM == GALES_FORM_FP64) {
-        Pq[j] += sh[i] * __ldg(pi + j);
-        Iq[j] += sh[i] * Ie[i][j];
-      } else {
-        // P and I are interpolated alike so that P == I gives U == U_P exactly
-        Pq[j] = fma(sh[i], __ldg(pi + j), Pq[j]);
-        Iq[j] = fma(sh[i], Ie[i][j], Iq[j]);
-      }
+      // P and I are interpolated alike so that P == I gives U == U_P exactly
+      Pq[j] = fma(sh[i], __ldg(pi + j), Pq[j]);
+      Iq[j] = fma(sh[i], Ie[i][j], Iq[j]);
     }
   }
   // (I - P)/dt at the point, in the form's type (the least-squares mass term)
   R dd[ND];
 #pragma unroll
   for (int j = 0; j < ND; ++j) {
-    if constexpr (FORM == GALES_FORM_FP64) dd[j] = (Iq[j] - Pq[j]) / k.dt;
-    else dd[j] = narrow_rn(Iq[j] - Pq[j]) * k.inv_dt_f;
+    dd[j] = narrow_rn(Iq[j] - Pq[j]) * k.inv_dt_f;
   }
   // gradients: FP64 in the FP64 form; FP32 of nodal differences in the mixed form
   // (sum_i dN_i/dx = 0, so sum_i dN_i (I_i - I_0) is the same gradient)
   R dI[DIM][ND];
-  if constexpr (FORM == GALES_FORM_FP64) {
-#pragma unroll
-    for (int d = 0; d < DIM; ++d)
-#pragma unroll
-      for (int j = 0; j < ND; ++j) {
-        double b = 0.0;
-#pragma unroll
-        for (int i = 0; i < NEN; ++i) b += q.ds[d][i] * Ie[i][j];
-        dI[d][j] = b;
-      }
-  } else if constexpr (NEN == DIM + 1 && NQ >= 2 && NQ <= 32 && (32 % NQ) == 0) {
+  if constexpr (NEN == DIM + 1 && NQ >= 2 && NQ <= 32 && (32 % NQ) == 0) {
     // A simplex's gradient is the same at its NQ points, whose lanes are consecutive in
     // the warp: lane iq forms the columns j = iq, iq + NQ, ... of dI (its FP64 nodal
     // differences picked from its registers) and the lanes of the element exchange
@@ -593,7 +575,7 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
   // velocity gradient in FP64 (input of compute_h; fused in the mixed form, whose
   // compute_h falls back to the reference's operations where they matter)
   double dv[DIM][DIM];
-  constexpr bool kShareDv = FORM == GALES_FORM_MIXED && NEN == DIM + 1 && NQ >= DIM && NQ <= 32 && (32 % NQ) == 0;
+  constexpr bool kShareDv = NEN == DIM + 1 && NQ >= DIM && NQ <= 32 && (32 % NQ) == 0;
   if constexpr (kShareDv) {
     // A simplex's velocity gradient is the same at its NQ points, whose lanes are
     // consecutive in the warp (NQ divides 32): lane iq forms row a = min(iq, DIM - 1)
@@ -629,14 +611,10 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
     for (int a = 0; a < DIM; ++a)
 #pragma unroll
       for (int d = 0; d < DIM; ++d) {
-        if constexpr (FORM == GALES_FORM_FP64) {
-          dv[a][d] = dI[d][1 + a];
-        } else {
-          double b = q.ds[d][0] * Ie[0][1 + a];
+        double b = q.ds[d][0] * Ie[0][1 + a];
 #pragma unroll
-          for (int i = 1; i < NEN; ++i) b = fma(q.ds[d][i], Ie[i][1 + a], b);
-          dv[a][d] = b;
-        }
+        for (int i = 1; i < NEN; ++i) b = fma(q.ds[d][i], Ie[i][1 + a], b);
+        dv[a][d] = b;
       }
   }
   // previous-level conservative vector U_P (props at P with shear rate 0) and the
@@ -646,99 +624,57 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
   Props<NC> pr;
   Coef<DIM, NC> c;
   double v_nrm, iv = 0.0;
-  if constexpr (FORM == GALES_FORM_FP64) {
-    assign<DIM, NC>(Pq, p, v, T, Y);
-    if constexpr (EOS == kEosMagma) {
-      // props at P with shear rate 0 (fluid_2d.hpp:186), at I with the point's shear
-      // rate (fluid_2d.hpp:193-194)
-      Props<NC> prP;
-      unsigned st = magma_mixture<NC>(k.mg, p, T, Y, 0.0, prP);
-      conservative<DIM, NC>(prP.rho, prP.cv, v, T, Y, UP);
-      assign<DIM, NC>(Iq, p, v, T, Y);
-      st |= magma_mixture<NC>(k.mg, p, T, Y, shear_rate<DIM>(dv), pr);
-      if (st) flag_error(k, GALES_ERR_MAGMA, e);
-    } else {
-      double rhoP, cvP;
-      mixture_rho_cv<NC>(k.ch, p, T, Y, rhoP, cvP);
-      conservative<DIM, NC>(rhoP, cvP, v, T, Y, UP);
-      assign<DIM, NC>(Iq, p, v, T, Y);
-      mixture<NC>(k.ch, p, T, Y, pr);
-    }
-    make_coef<DIM, NC>(pr, p, v, T, Y, c);
-    conservative<DIM, NC>(pr.rho, pr.cv, v, T, Y, U);
-    v_nrm = sqrt(vsq<DIM>(v));
+  double pP, vP[DIM], TP, YP[NC];
+  assign<DIM, NC>(Pq, pP, vP, TP, YP);
+  assign<DIM, NC>(Iq, p, v, T, Y);
+  double rhoP, cvP;
+  if constexpr (EOS == kEosMagma) {
+    Props<NC> prP;
+    unsigned st = magma_mixture<NC>(k.mg, pP, TP, YP, 0.0, prP);
+    st |= magma_mixture<NC>(k.mg, p, T, Y, shear_rate<DIM>(dv), pr);
+    if (st) flag_error(k, GALES_ERR_MAGMA, e);
+    rhoP = prP.rho;
+    cvP = prP.cv;
+    pr.irho = 1.0 / pr.rho;
+#pragma unroll
+    for (int i = 0; i < NC; ++i) pr.irho_c[i] = 1.0 / pr.rho_c[i];
   } else {
-    double pP, vP[DIM], TP, YP[NC];
-    assign<DIM, NC>(Pq, pP, vP, TP, YP);
-    assign<DIM, NC>(Iq, p, v, T, Y);
-    double rhoP, cvP;
-    if constexpr (EOS == kEosMagma) {
-      Props<NC> prP;
-      unsigned st = magma_mixture<NC>(k.mg, pP, TP, YP, 0.0, prP);
-      st |= magma_mixture<NC>(k.mg, p, T, Y, shear_rate<DIM>(dv), pr);
-      if (st) flag_error(k, GALES_ERR_MAGMA, e);
-      rhoP = prP.rho;
-      cvP = prP.cv;
-      pr.irho = 1.0 / pr.rho;
-#pragma unroll
-      for (int i = 0; i < NC; ++i) pr.irho_c[i] = 1.0 / pr.rho_c[i];
-    } else {
-      mixture_pair_fast<NC>(k.ch, k.has_gas != 0, pP, TP, YP, p, T, Y, rhoP, cvP, pr);
-    }
-    conservative<DIM, NC>(rhoP, cvP, vP, TP, YP, UP);
-    double vv = v[0] * v[0];
-#pragma unroll
-    for (int d = 1; d < DIM; ++d) vv = fma(v[d], v[d], vv);
-    make_coef_fast<DIM, NC>(pr, p, v, vv, T, Y, c);
-    U[0] = pr.rho;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) U[1 + d] = pr.rho * v[d];
-    U[L::iT] = pr.rho * c.E;
-#pragma unroll
-    for (int i = 0; i < NC - 1; ++i) U[L::iY + i] = pr.rho * Y[i];
-    iv = rsqrt(vv);
-    v_nrm = vv > 0.0 ? vv * iv : 0.0;
+    mixture_pair_fast<NC>(k.ch, k.has_gas != 0, pP, TP, YP, p, T, Y, rhoP, cvP, pr);
   }
+  conservative<DIM, NC>(rhoP, cvP, vP, TP, YP, UP);
+  double vv = v[0] * v[0];
+#pragma unroll
+  for (int d = 1; d < DIM; ++d) vv = fma(v[d], v[d], vv);
+  make_coef_fast<DIM, NC>(pr, p, v, vv, T, Y, c);
+  U[0] = pr.rho;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) U[1 + d] = pr.rho * v[d];
+  U[L::iT] = pr.rho * c.E;
+#pragma unroll
+  for (int i = 0; i < NC - 1; ++i) U[L::iY + i] = pr.rho * Y[i];
+  iv = rsqrt(vv);
+  v_nrm = vv > 0.0 ? vv * iv : 0.0;
   const double dt = k.dt;
   // source S (gravity; fluid_2d.hpp:597-599) and the mass-term coefficient (U - U_P)/dt - S
   // the coefficients in the form's type R
   using CR = Coef<DIM, NC, R>;
   CR cr;
-  if constexpr (FORM == GALES_FORM_FP64) cr = c;
-  else cr = narrow<DIM, NC>(c);
+  cr = narrow<DIM, NC>(c);
   R SvR[ND];
 #pragma unroll
   for (int r = 0; r < ND; ++r) SvR[r] = R(0);
-  if constexpr (FORM == GALES_FORM_FP64) {
-    double Sv[ND];
+  const float rf = cr.rho;
+  float gv = 0.f;
 #pragma unroll
-    for (int r = 0; r < ND; ++r) Sv[r] = 0.0;
-    double gv = 0.0;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) {
-      Sv[1 + d] = pr.rho * k.gravity[d];
-      gv += k.gravity[d] * v[d];
-    }
-    Sv[L::iT] = pr.rho * (gv);
-#pragma unroll
-    for (int j = 0; j < ND; ++j) {
-      SvR[j] = Sv[j];
-      GALES_RECA(rv, j) = (U[j] - UP[j]) / dt - Sv[j];
-    }
-  } else {
-    const float rf = cr.rho;
-    float gv = 0.f;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) {
-      const float gd = k.gravity_f[d];
-      SvR[1 + d] = rf * gd;
-      gv = fmaf(gd, cr.v[d], gv);
-    }
-    SvR[L::iT] = rf * gv;
-    const float idt = k.inv_dt_f;
-#pragma unroll
-    for (int j = 0; j < ND; ++j) GALES_RECA(rv, j) = fmaf(narrow_rn(U[j] - UP[j]), idt, -SvR[j]);
+  for (int d = 0; d < DIM; ++d) {
+    const float gd = k.gravity_f[d];
+    SvR[1 + d] = rf * gd;
+    gv = fmaf(gd, cr.v[d], gv);
   }
+  SvR[L::iT] = rf * gv;
+  const float idt = k.inv_dt_f;
+#pragma unroll
+  for (int j = 0; j < ND; ++j) GALES_RECA(rv, j) = fmaf(narrow_rn(U[j] - UP[j]), idt, -SvR[j]);
   R Ur[ND];  // U in the form's type (discontinuity capturing); U[0] = rho
 #pragma unroll
   for (int j = 0; j < ND; ++j) Ur[j] = j == 0 ? cr.rho : to_s<R>(U[j]);
@@ -756,13 +692,9 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
     double trG = 0.0;
 #pragma unroll
     for (int d = 0; d < DIM; ++d) trG += q.G[d][d];
-    if constexpr (FORM == GALES_FORM_FP64) {
-      h = compute_h<DIM>(q.G, v, dv);
-    } else {
-      bool decided;
-      h = compute_h_fast<DIM>(q.G, trG, v, iv, dv, decided);
-      if (!decided) h = compute_h_reference<DIM, NEN, ND>(k.I, nodes, sh, q);
-    }
+    bool decided;
+    h = compute_h_fast<DIM>(q.G, trG, v, iv, dv, decided);
+    if (!decided) h = compute_h_reference<DIM, NEN, ND>(k.I, nodes, sh, q);
     const double cs = pr.c, rho = pr.rho, mu = pr.mu, cv = pr.cv, kappa = pr.kappa;
     double td[ND];
 #pragma unroll
@@ -781,7 +713,7 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
 #pragma unroll
       for (int i = 0; i < NC - 1; ++i) td[L::iY + i] = fmin(use, h * h / (pr.D_c[i] * 12));
       nondiag = true;
-    } else if (FORM == GALES_FORM_MIXED && k.tau == GALES_TAU_NON_DIAG_COMP_2019) {
+    } else if (k.tau == GALES_TAU_NON_DIAG_COMP_2019) {
       // the same parameters with one division for 1/(|v|(|v|+c)), 1/(mu kappa) and
       // tau_closed's 1/det (mixed form): r = 1/(a b d) gives 1/a = b d r, ...
       const double a = v_nrm * (v_nrm + cs), bmk = mu * kappa, det = tau_det<DIM, NC>(c);
@@ -800,18 +732,6 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
 #pragma unroll
       for (int i = 0; i < NC - 1; ++i)
         td[L::iY + i] = fmin(use, hh12 * (EOS == kEosMagma ? 1.0 / pr.D_c[i] : k.ch[i].inv_D));
-      nondiag = true;
-    } else if (k.tau == GALES_TAU_NON_DIAG_COMP_2019) {
-      double use;
-      if (k.steady) use = h / (2.0 * (v_nrm + cs)) + h / (2.0 * v_nrm);
-      else use = fmin(dt * 0.5, h / (2.0 * (v_nrm + cs)) + h / (2.0 * v_nrm));
-      td[0] = use;
-      const double tm = fmin(use, h * h * rho / (12.0 * mu));
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) td[1 + d] = tm;
-      td[L::iT] = fmin(use, h * h * rho * cv / (12.0 * kappa));
-#pragma unroll
-      for (int i = 0; i < NC - 1; ++i) td[L::iY + i] = fmin(use, h * h / (12.0 * pr.D_c[i]));
       nondiag = true;
     } else if (k.tau == GALES_TAU_DIAG_INCOMP_2007) {
       double use = 0.0;
@@ -868,22 +788,6 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
     if (!nondiag) {
 #pragma unroll
       for (int i = 0; i < ND; ++i) tau[i][i] = to_s<R>(td[i]);
-    } else if constexpr (FORM == GALES_FORM_FP64) {
-      double A0[ND][ND], Xinv[ND][ND];
-#pragma unroll
-      for (int r = 0; r < ND; ++r)
-#pragma unroll
-        for (int cc = 0; cc < ND; ++cc) A0[r][cc] = dudy_entry<DIM, NC, double>(c, r, cc);
-      if (lu_inverse<ND>(A0, Xinv)) flag_error(k, GALES_ERR_SINGULAR, e);
-#pragma unroll
-      for (int r = 0; r < ND; ++r)
-#pragma unroll
-        for (int cc = 0; cc < ND; ++cc) tau[r][cc] = Xinv[r][cc] * td[cc];
-      if (v_nrm / cs < 0.1) {
-        tau[0][0] = 1.0 / (1.0 / tau[0][0] + 1.0 / (rho * tau[1][1] * (trG)));
-#pragma unroll
-        for (int cc = 1; cc < ND; ++cc) tau[0][cc] = 0.0;
-      }
     } else {
       tau_closed<DIM, NC, R>(c, pr.irho, have_idet ? idet : 1.0 / tau_det<DIM, NC>(c), td,
                              v_nrm < 0.1 * cs, rho * trG, tau);
@@ -894,7 +798,7 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
     // matrix stage multiplies with), and w
     R zz[ND], yy[ND], gg[ND], gR[DIM];
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) gR[d] = FORM == GALES_FORM_FP64 ? R(k.gravity[d]) : R(k.gravity_f[d]);
+    for (int d = 0; d < DIM; ++d) gR[d] = R(k.gravity_f[d]);
 #pragma unroll
     for (int cc = 0; cc < ND; ++cc) zz[cc] = yy[cc] = gg[cc] = R(0);
 #pragma unroll
@@ -906,7 +810,7 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
       else { r0r = cr.drho_dY[r - L::iY]; mEr = cr.dE_dY[r - L::iY]; gr = R(0); }
 #pragma unroll
       for (int cc = 0; cc < ND; ++cc) {
-        if (FORM == GALES_FORM_MIXED && !tau_nz<DIM, NC>(r, cc)) {
+        if (!tau_nz<DIM, NC>(r, cc)) {
           GALES_RECA(tau, (r) * ND + (cc)) = S(0);
           continue;
         }
@@ -968,7 +872,7 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
         R Zn = R(0), Un = R(0), use1 = R(0);
 #pragma unroll
         for (int j = 0; j < ND; ++j) {
-          const R ui = FORM == GALES_FORM_FP64 ? R(k.u_ref_inv[j]) : R(k.u_ref_inv_f[j]);
+          const R ui = R(k.u_ref_inv_f[j]);
           const R z = ui * (AdI[j] - SvR[j]);
           const R u = ui * Ur[j];
           Zn += z * z;
@@ -983,7 +887,7 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
             R n2 = R(0);
 #pragma unroll
             for (int j = 0; j < ND; ++j) {
-              const R u = (FORM == GALES_FORM_FP64 ? R(k.u_ref_inv[j]) : R(k.u_ref_inv_f[j])) * dU[d][j];
+              const R u = R(k.u_ref_inv_f[j]) * dU[d][j];
               n2 += u * u;
             }
             const R n = sqrt(n2);
@@ -993,7 +897,7 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
         if (a == 1.0) nu = Zn * h * (R(1) / sqrt(use1));
         else if (a == 2.0) nu = Zn * h * h / Un;
         else if (a == 1.5) nu = Zn * h * ((R(1) / sqrt(use1)) + h / Un) / R(2);
-        nu = (FORM == GALES_FORM_FP64 ? R(k.dc_scale) : R(k.dc_scale_f)) * nu;
+        nu = R(k.dc_scale_f) * nu;
       }
     }
   }
@@ -1023,20 +927,11 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
   }
   // write the record (the mixed form takes the coefficients already rounded in cr and
   // the shape data rounded once per mesh)
-  if constexpr (FORM == GALES_FORM_MIXED) {
+  #pragma unroll
+  for (int i = 0; i < NEN; ++i) {
+    GALES_RECA(sh, i) = S(k.sh_tab_f[iq][i]);
 #pragma unroll
-    for (int i = 0; i < NEN; ++i) {
-      GALES_RECA(sh, i) = S(k.sh_tab_f[iq][i]);
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) GALES_RECA(ds, (d) * NEN + (i)) = S(q.ds_f[d][i]);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < NEN; ++i) {
-      GALES_RECA(sh, i) = to_s<S>(sh[i]);
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) GALES_RECA(ds, (d) * NEN + (i)) = to_s<S>(q.ds[d][i]);
-    }
+    for (int d = 0; d < DIM; ++d) GALES_RECA(ds, (d) * NEN + (i)) = S(q.ds_f[d][i]);
   }
   GALES_REC(JxW) = to_s<S>(JxW);
   GALES_REC(p) = S(cr.p);
@@ -1132,7 +1027,7 @@ __device__ __forceinline__ double widen(double d) { return d; }
 // point record of that point to a chunk buffer (L2-resident).  The mixed form is
 // held to 128 registers (4 CTAs per SM): more warps hide the FP64 latency better
 // than the spilled values cost.
-template <int DIM, int NEN, int NC, int NQ, int FORM, typename S, int EOS = kEosChemicals>
+template <int DIM, int NEN, int NC, int NQ, typename S, int EOS = kEosChemicals>
 __device__ __forceinline__ void point_block(const KParams& k, QP<DIM, NEN, NC, S>* __restrict__ out, long long first,
                                             long long n, int bid) {
   // chunk-local indices fit 32 bits (the host keeps a chunk's points below 2^31); 64-bit
@@ -1147,14 +1042,14 @@ __device__ __forceinline__ void point_block(const KParams& k, QP<DIM, NEN, NC, S
   using RB = RecBlock<DIM, NEN, NC, NQ, S>;
   const int blk = t / RB::BP;
   const RecOut<QPT, RB::BPS> o{reinterpret_cast<S*>(out) + (size_t)blk * (size_t)RB::WORDS, t - blk * RB::BP};
-  point_phase<DIM, NEN, NC, NQ, FORM, S, RB::BPS, EOS>(k, e, iq, o);
+  point_phase<DIM, NEN, NC, NQ, S, RB::BPS, EOS>(k, e, iq, o);
 }
 
-// Resident point-stage CTAs the register budget is set for: 4 for the mixed form with
-// the chemicals' EOS, 2 with the (out-of-line, register-hungry) magma EOS, 1 for FP64.
-template <int FORM, int EOS>
+// Resident point-stage CTAs the register budget is set for: 4 with the chemicals' EOS, 2
+// with the (out-of-line, register-hungry) magma EOS.
+template <int EOS>
 constexpr int point_min_ctas() {
-  return FORM == GALES_FORM_MIXED ? (EOS == kEosMagma ? 2 : 4) : 1;
+  return EOS == kEosMagma ? 2 : 4;
 }
 
 // Zeroes k.clear_p[a][0 .. k.clear_n[a]) with every thread of the launch (grid-stride;
@@ -1179,10 +1074,10 @@ __device__ __forceinline__ void clear_arrays(const KParams& k) {
   }
 }
 
-template <int DIM, int NEN, int NC, int NQ, int FORM, typename S, int EOS = kEosChemicals>
-__global__ void __launch_bounds__(128, point_min_ctas<FORM, EOS>()) point_kernel(const KParams k, QP<DIM, NEN, NC, S>* __restrict__ out,
+template <int DIM, int NEN, int NC, int NQ, typename S, int EOS = kEosChemicals>
+__global__ void __launch_bounds__(128, point_min_ctas<EOS>()) point_kernel(const KParams k, QP<DIM, NEN, NC, S>* __restrict__ out,
                                                      long long first, long long n) {
-  point_block<DIM, NEN, NC, NQ, FORM, S, EOS>(k, out, first, n, (int)blockIdx.x);
+  point_block<DIM, NEN, NC, NQ, S, EOS>(k, out, first, n, (int)blockIdx.x);
   if (k.clear_n[0] > 0 || k.clear_n[1] > 0) clear_arrays(k);
 }
 

@@ -15,9 +15,10 @@ struct LaunchResult {
   int launches;
 };
 
-template <int DIM, int NEN, int NC, int NQ, int FORM, int EOS = kEosChemicals>
+// The mixed form (gales_kernels.cuh).
+template <int DIM, int NEN, int NC, int NQ, int EOS = kEosChemicals>
 struct InteriorInst {
-  using S = typename std::conditional<FORM == GALES_FORM_FP64, double, float>::type;
+  using S = float;
   using Rec = QP<DIM, NEN, NC, S>;
   using RB = RecBlock<DIM, NEN, NC, NQ, S>;
   using SM = MatSmem<DIM, NEN, NC, NQ, S>;
@@ -29,7 +30,7 @@ struct InteriorInst {
   // resident point-kernel CTAs (128 threads) per SM
   static int point_occupancy() {
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, point_kernel<DIM, NEN, NC, NQ, FORM, S, EOS>, 128, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, point_kernel<DIM, NEN, NC, NQ, S, EOS>, 128, 0) !=
         cudaSuccess)
       return 1;
     return nb > 0 ? nb : 1;
@@ -37,7 +38,7 @@ struct InteriorInst {
   static LaunchResult point(const KParams& k, bool, void* buf, long long first, long long n, cudaStream_t st) {
     if (n <= 0) return {cudaSuccess, 0};
     const long long threads = n * NQ;
-    point_kernel<DIM, NEN, NC, NQ, FORM, S, EOS><<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(
+    point_kernel<DIM, NEN, NC, NQ, S, EOS><<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(
         k, reinterpret_cast<Rec*>(buf), first, n);
     return {cudaGetLastError(), 1};
   }
@@ -129,6 +130,46 @@ struct Simplex64Inst {
   }
 };
 
+// The FP64 form of a quadrilateral or hexahedron (gales_fp64.cuh).
+template <int DIM, int NC, int EOS>
+struct Tensor64Inst {
+  using T = Tensor64<DIM, NC>;
+  using R = typename T::R;
+  static constexpr int NEN = T::NEN;
+  static constexpr size_t kSmem = sizeof(typename T::Smem);
+  static size_t rec_bytes() { return R::ELEM_BYTES; }
+  static int rec_block() { return R::EB; }
+  static int point_occupancy() {
+    int nb = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, point64_kernel<DIM, NEN, NC, EOS, true>, 128, 0) !=
+        cudaSuccess)
+      return 1;
+    return nb > 0 ? nb : 1;
+  }
+  static cudaError_t prepare() {
+    return cudaFuncSetAttribute(tensor64_kernel<DIM, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+  }
+  static LaunchResult point(const KParams& k, bool want_m, void* buf, long long first, long long n, cudaStream_t st) {
+    if (n <= 0) return {cudaSuccess, 0};
+    const unsigned blocks = (unsigned)((n * NEN + 127) / 128);
+    double* out = reinterpret_cast<double*>(buf);
+    if (want_m) point64_kernel<DIM, NEN, NC, EOS, true><<<blocks, 128, 0, st>>>(k, out, first, n);
+    else point64_kernel<DIM, NEN, NC, EOS, false><<<blocks, 128, 0, st>>>(k, out, first, n);
+    return {cudaGetLastError(), 1};
+  }
+  static LaunchResult matrix(const KParams& k, bool want_m, void* buf, long long first, long long n, cudaStream_t st) {
+    if (n <= 0) return {cudaSuccess, 0};
+    double* in = reinterpret_cast<double*>(buf);
+    if (!want_m) {
+      const long long threads = (n + R::EB - 1) / R::EB * R::ND * R::EB;
+      residual64_kernel<DIM, NEN, NC><<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(k, in, first, n);
+      return {cudaGetLastError(), 1};
+    }
+    tensor64_kernel<DIM, NC><<<(unsigned)n, T::THREADS, kSmem, st>>>(k, in, first, n);
+    return dirichlet64<DIM, NEN, NC>(k, in, n, st);
+  }
+};
+
 template <int DIM, int NEN, int NC, int NS, int NSQ, typename S, int EOS = kEosChemicals>
 cudaError_t prepare_boundary_nc() {
   return cudaFuncSetAttribute(boundary_kernel<DIM, NEN, NC, NS, NSQ, S, EOS>,
@@ -172,8 +213,9 @@ struct InteriorOps {
   }
 
 template <int DIM, int NEN, int NC, int NQ, int FORM, int EOS>
-using InteriorOf = typename std::conditional<FORM == GALES_FORM_FP64 && NEN == DIM + 1, Simplex64Inst<DIM, NC, EOS>,
-                                             InteriorInst<DIM, NEN, NC, NQ, FORM, EOS>>::type;
+using InteriorOf = typename std::conditional<
+    FORM == GALES_FORM_MIXED, InteriorInst<DIM, NEN, NC, NQ, EOS>,
+    typename std::conditional<NEN == DIM + 1, Simplex64Inst<DIM, NC, EOS>, Tensor64Inst<DIM, NC, EOS>>::type>::type;
 
 template <int DIM, int NEN, int NQ, int FORM, int EOS = kEosChemicals>
 struct InteriorDispatch {

@@ -145,7 +145,7 @@ __host__ __device__ __forceinline__ void mixture(const DevChem* ch, double p, do
   o.alpha = alpha; o.beta = beta;
 }
 
-// The mixture in FP64 for the mixed form: state I in full (Props) and state P's rho
+// The mixture for both forms' point stages: state I in full (Props) and state P's rho
 // and cv (what U(P) needs), from per-chemical ratios precomputed on the host and one
 // division for both states.  A gas has 1/rho_c = R_c T/p, so
 //   1/rho = (T G + p C)/p = D/p,   G = sum_gas Y_c R_c,  C = sum_custom Y_c/rho_c,
@@ -261,29 +261,6 @@ __host__ __device__ __forceinline__ double shear_rate(const double (&dv)[DIM][DI
   }
 }
 
-// Only rho and cv (what U(P) needs); same operations as mixture().
-template <int NC>
-__device__ __forceinline__ void mixture_rho_cv(const DevChem* ch, double p, double T,
-                                               const double* Y, double& rho_out, double& cv_out) {
-  double rho = 0.0, cv = 0.0;
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    const DevChem& q = ch[c];
-    double r, v;
-    if (q.kind == GALES_CH_CUSTOM) {
-      r = q.rho;
-      v = (q.beta == 0.0) ? q.cp : q.cp - T * q.alpha * q.alpha / (r * q.beta);
-    } else {
-      r = p / (q.R * T);
-      v = q.cv;
-    }
-    rho += Y[c] / r;
-    cv += Y[c] * v;
-  }
-  rho_out = 1. / rho;
-  cv_out = cv;
-}
-
 // Scalars from which every frozen-coefficient matrix of the point is built
 // (fluid_2d.hpp:393-404, 531-533).
 template <int DIM, int NC, typename T = double>
@@ -383,7 +360,7 @@ __device__ __forceinline__ void make_coef(const Props<NC>& pr, double p, const d
   }
 }
 
-// make_coef for the mixed form, from mixture_pair_fast's reciprocals; vv = |v|^2.
+// make_coef from mixture_pair_fast's reciprocals; vv = |v|^2.
 template <int DIM, int NC>
 __device__ __forceinline__ void make_coef_fast(const Props<NC>& pr, double p, const double* v, double vv,
                                                double T, const double* Y, Coef<DIM, NC>& c) {
@@ -608,78 +585,7 @@ __device__ __forceinline__ void k_mv(const C& c, int k, int l, const T* x, T* y)
   }
 }
 
-// GALES::inverse (algorithm.hpp:399-416): uBLAS lu_factorize (partial pivoting on
-// the first max |.| of the column, reciprocal column scaling) + lu_substitute
-// against the identity.  Returns nonzero if a zero pivot was met.
-template <int N>
-__device__ __forceinline__ int lu_inverse(double (&A)[N][N], double (&X)[N][N]) {
-  int pm[N];
-#pragma unroll
-  for (int i = 0; i < N; ++i) pm[i] = i;
-  int singular = 0;
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    int imax = i;
-    double t = 0.0;
-#pragma unroll
-    for (int r = i; r < N; ++r) {
-      const double u = fabs(A[r][i]);
-      if (u > t) { imax = r; t = u; }
-    }
-    if (t == 0.0) imax = i;
-    if (A[imax][i] != 0.0) {
-      if (imax != i) {
-        pm[i] = imax;
-#pragma unroll
-        for (int r = i + 1; r < N; ++r)
-          if (r == imax)
-#pragma unroll
-            for (int c = 0; c < N; ++c) { const double s = A[i][c]; A[i][c] = A[r][c]; A[r][c] = s; }
-      }
-      const double rcp = 1.0 / A[i][i];
-#pragma unroll
-      for (int r = i + 1; r < N; ++r) A[r][i] *= rcp;
-    } else if (singular == 0) {
-      singular = i + 1;
-    }
-#pragma unroll
-    for (int r = i + 1; r < N; ++r)
-#pragma unroll
-      for (int c = i + 1; c < N; ++c) A[r][c] -= A[r][i] * A[i][c];
-  }
-#pragma unroll
-  for (int i = 0; i < N; ++i)
-#pragma unroll
-    for (int j = 0; j < N; ++j) X[i][j] = (i == j) ? 1.0 : 0.0;
-#pragma unroll
-  for (int i = 0; i < N; ++i)
-#pragma unroll
-    for (int r = i + 1; r < N; ++r)
-      if (pm[i] == r)
-#pragma unroll
-        for (int c = 0; c < N; ++c) { const double s = X[i][c]; X[i][c] = X[r][c]; X[r][c] = s; }
-#pragma unroll
-  for (int l = 0; l < N; ++l)
-#pragma unroll
-    for (int r = 0; r < N; ++r) {
-      const double t = X[r][l];
-      if (t != 0.0)
-#pragma unroll
-        for (int m = r + 1; m < N; ++m) X[m][l] -= A[m][r] * t;
-    }
-#pragma unroll
-  for (int l = N - 1; l >= 0; --l)
-#pragma unroll
-    for (int r = N - 1; r >= 0; --r) {
-      const double t = X[r][l] /= A[r][r];
-      if (t != 0.0)
-#pragma unroll
-        for (int m = r - 1; m >= 0; --m) X[m][l] -= A[m][r] * t;
-    }
-  return singular;
-}
-
-// tau = DUDY^{-1} diag(td) for the mixed form (fluid_2d.hpp:946-947), from the
+// tau = DUDY^{-1} diag(td) (fluid_2d.hpp:946-947), from the
 // structure of DUDY = w r0^T + rho M.  The velocity and mass-fraction rows of
 // DUDY^{-1} are (e_j - w_j e_p^T)/rho; the p and T rows come from the 2x2 system
 // [drho_dp drho_dT; de_dp de_dT] per column.  Every other entry is zero (tau_nz).
