@@ -1819,18 +1819,11 @@ struct alignas(16) BPointRec {
   S BK[DIM][ND][ND];
 };
 
+// Point records of one boundary element in shared memory (calls without a boundary point
+// stage: the element blocks of a list).
 template <int DIM, int NEN, int NC, int NS, int NSQ, typename S>
 struct BoundarySmem {
-  static constexpr int ND = Layout<DIM, NC>::ND, N = NEN * ND;
-  static constexpr int MS = N + 1;   // row stride of m: rows and columns bank-conflict free
   BPointRec<DIM, NEN, NC, S> pt[NS * NSQ];
-  S m[N * MS];           // element block accumulator
-  double r[N];
-  double wsum;
-  int64_t rowbase[NEN];
-  int32_t rowlen[NEN];
-  uint32_t blocked[NEN];
-  uint16_t slot[NEN][NEN];
 };
 
 // Boundary point physics (fluid_2d.hpp:341-349, 610-817) at one side point with
@@ -2036,196 +2029,191 @@ __global__ void __launch_bounds__(128) bpoint_kernel(const KParams k) {
   bpoint_phase<DIM, NEN, NC, S, EOS>(k, nodes, flag, sh, ds, JN, P, e);
   BPointRec<DIM, NEN, NC, S>& O = reinterpret_cast<BPointRec<DIM, NEN, NC, S>*>(k.bpt_rec)[t];
   O.pt = P;
-  bpoint_blocks<DIM, NC, S>(P.c, P.JNxW, k.side_bc[flag < GALES_MAX_FLAGS ? flag : 0], O.BA, O.BK);
+  if (k.vals || k.vjp_lam)
+    bpoint_blocks<DIM, NC, S>(P.c, P.JNxW, k.side_bc[flag < GALES_MAX_FLAGS ? flag : 0], O.BA, O.BK);
 }
 
-// Boundary pass, one warp per listed boundary element.  Lanes first evaluate one
-// side quadrature point each (thread per point, FP64: geometry, EOS, fluxes and the
-// boundary residual), then build BA and BK entry-parallel per point in the form's
-// matrix type S and accumulate
+// Boundary pass, stage 2: a CTA per listed boundary element, a thread per entry (jb, ja) of
+// the dof blocks.  From the point records, per flagged side point,
 //   m_ba += N_b (N_a BA - sum_l dN_a/dx_l BK_l)                 (fluid_2d.hpp:351-363)
-// before the element's own Dirichlet pass and scatter (fluid_assembly.hpp:57-63).
+// where the bracket is formed once per trial node and added into the blocks of the test nodes
+// on the side (N_b = 0 on the others), all nodes' entries (jb, ja) in registers; then the
+// element's own Dirichlet pass and scatter (fluid_assembly.hpp:57-63), consecutive threads on
+// consecutive columns.  A lane per block row, which formed the bracket again for every test
+, took 2.2 ms for the 4,900 boundary
+XX
+// Without matrix (k.vals and k.vjp_lam null) only the residual is formed.
+template <int NC, int DIM>
+__host__ __device__ constexpr int boundary_threads() {
+  return (Layout<DIM, NC>::ND * Layout<DIM, NC>::ND + 31) / 32 * 32;
+}
+
 template <int DIM, int NEN, int NC, int NS, int NSQ, typename S, int EOS = kEosChemicals>
-__global__ void __launch_bounds__(32) boundary_kernel(const KParams k) {
+__global__ void __launch_bounds__(boundary_threads<NC, DIM>()) boundary_kernel(const KParams k) {
   using L = Layout<DIM, NC>;
-  constexpr int ND = L::ND;
-  constexpr int N = NEN * ND;
-  constexpr int NT = N * N;
+  constexpr int ND = L::ND, N = NEN * ND, THREADS = boundary_threads<NC, DIM>();
   using BS = BoundarySmem<DIM, NEN, NC, NS, NSQ, S>;
-  constexpr int MS = BS::MS;
   using BR = BPointRec<DIM, NEN, NC, S>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  BS& B = *reinterpret_cast<BS*>(smem_raw);
-  const int lane = threadIdx.x;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ int64_t rowbase[NEN];
+  __shared__ int32_t rowlen[NEN], nodes[NEN];
+  __shared__ uint32_t blocked[NEN];
+  __shared__ uint16_t slot[NEN][NEN];
+  __shared__ double wsum[THREADS / 32];
+  const int tid = threadIdx.x;
   const long long li = blockIdx.x;
-  if (li >= k.n_list) return;
   const long long e = k.el_list[li];
-  int nodes[NEN];
-#pragma unroll
-  for (int a = 0; a < NEN; ++a) nodes[a] = __ldg(k.conn + e * NEN + a);
-  for (int t = lane; t < N * MS; t += 32) B.m[t] = S(0);
-  for (int t = lane; t < N; t += 32) B.r[t] = 0.0;
+  const bool want_m = k.vals || k.vjp_lam;
   // rows of the element's nodes and the element's slot table, for the scatter
-  if (lane < NEN) {
-    const int fl = k.node_flag ? __ldg(k.node_flag + nodes[lane]) : 0;
-    B.blocked[lane] = (fl >= 0 && fl < GALES_MAX_FLAGS) ? k.dirichlet_mask[fl] : 0u;
-    const int64_t r0 = __ldg(k.node_rp + nodes[lane]), r1 = __ldg(k.node_rp + nodes[lane] + 1);
-    B.rowbase[lane] = r0 * (int64_t)(ND * ND);
-    B.rowlen[lane] = (int32_t)((r1 - r0) * ND);
+  if (tid < NEN) {
+    const int nb = __ldg(k.conn + e * NEN + tid);
+    const int fl = k.node_flag ? __ldg(k.node_flag + nb) : 0;
+    nodes[tid] = nb;
+    blocked[tid] = (fl >= 0 && fl < GALES_MAX_FLAGS) ? k.dirichlet_mask[fl] : 0u;
+    const int64_t r0 = __ldg(k.node_rp + nb), r1 = __ldg(k.node_rp + nb + 1);
+    rowbase[tid] = r0 * (int64_t)(ND * ND);
+    rowlen[tid] = (int32_t)((r1 - r0) * ND);
   }
-  for (int t = lane; t < NEN * NEN; t += 32) B.slot[t / NEN][t % NEN] = __ldg(k.slot + e * NEN * NEN + t);
-  // (1) point physics and matrices: from the boundary point records of this element
-  // when the boundary point stage ran (k.bpt_rec), otherwise one lane per (side, point)
+  for (int t = tid; t < NEN * NEN; t += THREADS) slot[t / NEN][t % NEN] = __ldg(k.slot + e * NEN * NEN + t);
+  // (1) the points: the records of the boundary point stage, else one thread per (side, point)
+  const BR* rec;
+  int p0 = 0, p1 = NS * NSQ;
   if (k.bpt_rec) {
-    for (int t = lane; t < NS * NSQ; t += 32) B.pt[t].pt.flag = 0;
-    __syncwarp();
-    const int p0 = k.bpt_off[li], p1 = k.bpt_off[li + 1];
-    static_assert(sizeof(BR) % 16 == 0, "point record must be int4-aligned");
-    constexpr int W4 = sizeof(BR) / 16;
-    for (int t = lane; t < (p1 - p0) * W4; t += 32) {
-      const int pt = p0 + t / W4, w = t % W4;
-      reinterpret_cast<int4*>(&B.pt[k.bpt_ip[pt]])[w] =
-          reinterpret_cast<const int4*>(reinterpret_cast<const BR*>(k.bpt_rec) + pt)[w];
-    }
-  } else if (lane < NS * NSQ) {
-    const int s = lane / NSQ, iq = lane % NSQ;
-    const int flag = k.bd_sides[li * NS + s];
-    BPoint<DIM, NEN, NC, S>& P = B.pt[lane].pt;
-    P.flag = flag;
-    if (flag > 0) {
-      double X[NEN][DIM];
-#pragma unroll
-      for (int a = 0; a < NEN; ++a)
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) X[a][d] = __ldg(k.coords + (long long)nodes[a] * DIM + d);
-      Geo<DIM, NEN> q;
-      geometry<DIM, NEN>(X, k.sgp[s][iq], false, q);
-      if (!(q.J > 0.0)) flag_error(k, GALES_ERR_NEG_JACOBIAN, e);
-      double JNxW[DIM];
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) JNxW[d] = q.JN[d] * k.W_bd;
-      bpoint_phase<DIM, NEN, NC, S, EOS>(k, nodes, flag, q.sh, q.ds, JNxW, P, e);
-      bpoint_blocks<DIM, NC, S>(P.c, P.JNxW, k.side_bc[flag < GALES_MAX_FLAGS ? flag : 0], B.pt[lane].BA,
-                                B.pt[lane].BK);
-    }
-  }
-  __syncwarp();
-  // (2) per flagged point, the block m_ba += N_b (N_a BA - sum_l dN_a/dx_l BK_l) and the
-  // residual.  Lane l owns block rows l, l + 32, ...: its row's BA and BK rows are read
-  // once per point, the columns run at compile time; a block of at most 32 rows is
-  // accumulated in registers, a larger one in shared memory.
-  constexpr int RPL = (N + 31) / 32;
-  constexpr bool kRegs = N <= 32;
-  S acc[kRegs ? N : 1];
-#pragma unroll
-  for (int c = 0; c < (kRegs ? N : 1); ++c) acc[c] = S(0);
-  for (int ip = 0; ip < NS * NSQ; ++ip) {
-    const BR& R = B.pt[ip];
-    const BPoint<DIM, NEN, NC, S>& P = R.pt;
-    if (P.flag <= 0) continue;
-#pragma unroll
-    for (int rr = 0; rr < RPL; ++rr) {
-      const int row = lane + 32 * rr;
-      if (row < N) {
-        const int b = row / ND, jb = row - (row / ND) * ND;
-        const S shb = P.sh[b];
-        S ba[ND], bk[DIM][ND];
-#pragma unroll
-        for (int ja = 0; ja < ND; ++ja) {
-          ba[ja] = R.BA[jb][ja];
-#pragma unroll
-          for (int l = 0; l < DIM; ++l) bk[l][ja] = R.BK[l][jb][ja];
-        }
+    rec = reinterpret_cast<const BR*>(k.bpt_rec);
+    p0 = k.bpt_off[li];
+    p1 = k.bpt_off[li + 1];
+  } else {
+    BS& B = *reinterpret_cast<BS*>(smem_raw);
+    rec = B.pt;
+    if (tid < NS * NSQ) {
+      const int s = tid / NSQ, iq = tid % NSQ;
+      const int flag = k.bd_sides[li * NS + s];
+      BPoint<DIM, NEN, NC, S>& P = B.pt[tid].pt;
+      P.flag = flag;
+      if (flag > 0) {
+        int nd_[NEN];
+        double X[NEN][DIM];
 #pragma unroll
         for (int a = 0; a < NEN; ++a) {
-          const S sha = P.sh[a];
-          S dsa[DIM];
+          nd_[a] = __ldg(k.conn + e * NEN + a);
 #pragma unroll
-          for (int l = 0; l < DIM; ++l) dsa[l] = P.ds[l][a];
-#pragma unroll
-          for (int ja = 0; ja < ND; ++ja) {
-            S x = sha * ba[ja];
-#pragma unroll
-            for (int l = 0; l < DIM; ++l) x = madd(-dsa[l], bk[l][ja], x);
-            if constexpr (kRegs) acc[a * ND + ja] = madd(shb, x, acc[a * ND + ja]);
-            else B.m[row * MS + a * ND + ja] = madd(shb, x, B.m[row * MS + a * ND + ja]);
-          }
+          for (int d = 0; d < DIM; ++d) X[a][d] = __ldg(k.coords + (long long)nd_[a] * DIM + d);
         }
+        Geo<DIM, NEN> q;
+        geometry<DIM, NEN>(X, k.sgp[s][iq], false, q);
+        if (!(q.J > 0.0)) flag_error(k, GALES_ERR_NEG_JACOBIAN, e);
+        double JNxW[DIM];
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) JNxW[d] = q.JN[d] * k.W_bd;
+        bpoint_phase<DIM, NEN, NC, S, EOS>(k, nd_, flag, q.sh, q.ds, JNxW, P, e);
+        if (want_m)
+          bpoint_blocks<DIM, NC, S>(P.c, P.JNxW, k.side_bc[flag < GALES_MAX_FLAGS ? flag : 0], B.pt[tid].BA,
+                                    B.pt[tid].BK);
       }
     }
-    for (int t = lane; t < N; t += 32) B.r[t] = madd(P.shr[t / ND], P.rb[t % ND], B.r[t]);
-    __syncwarp();
   }
-  if constexpr (kRegs) {
-    if (lane < N)
+  __syncthreads();
+  // (2) residual, a thread per row
+  for (int t = tid; t < N; t += THREADS) {
+    const int b = t / ND, jb = t - b * ND;
+    double r = 0.0;
+    for (int ip = p0; ip < p1; ++ip)
+      if (rec[ip].pt.flag > 0) r = madd(rec[ip].pt.shr[b], rec[ip].pt.rb[jb], r);
+    if (k.local_r) k.local_r[li * N + t] = -r;
+    else if (!k.vjp_lam && !((blocked[b] >> jb) & 1u)) add_to(k.rhs + (long long)nodes[b] * ND + jb, -r, k.scatter_mode);
+  }
+  if (!want_m || (k.local_r && !k.local_m)) return;
+  // (3) the blocks' entries (jb, ja)
+  const bool active = tid < ND * ND;
+  const int jb = active ? tid / ND : 0, ja = active ? tid - jb * ND : 0;
+  S acc[NEN][NEN];
 #pragma unroll
-      for (int c = 0; c < N; ++c) B.m[lane * MS + c] = acc[c];
-    __syncwarp();
+  for (int b = 0; b < NEN; ++b)
+#pragma unroll
+    for (int a = 0; a < NEN; ++a) acc[b][a] = S(0);
+#pragma unroll 1
+  for (int ip = p0; ip < p1; ++ip) {
+    const BR& R = rec[ip];
+    if (R.pt.flag <= 0) continue;
+    const S ba = R.BA[jb][ja];
+    S bk[DIM], x[NEN];
+#pragma unroll
+    for (int l = 0; l < DIM; ++l) bk[l] = R.BK[l][jb][ja];
+#pragma unroll
+    for (int a = 0; a < NEN; ++a) {
+      x[a] = R.pt.sh[a] * ba;
+#pragma unroll
+      for (int l = 0; l < DIM; ++l) x[a] = madd(-R.pt.ds[l][a], bk[l], x[a]);
+    }
+#pragma unroll
+    for (int b = 0; b < NEN; ++b) {
+      const S shb = R.pt.sh[b];
+      if (shb == S(0)) continue;   // a node off the side
+#pragma unroll
+      for (int a = 0; a < NEN; ++a) acc[b][a] = madd(shb, x[a], acc[b][a]);
+    }
   }
-  if (k.local_r) {  // element-level output of execute_b: m = m_, r = -r_
-    for (int t = lane; t < N; t += 32) k.local_r[li * N + t] = -B.r[t];
-    if (k.local_m)
-      for (int t = lane; t < NT; t += 32) k.local_m[li * NT + t] = widen(B.m[(t / N) * MS + t % N]);
+  if (k.local_m) {  // element-level output of execute_b: m = m_, r = -r_
+    if (active)
+#pragma unroll
+      for (int b = 0; b < NEN; ++b)
+#pragma unroll
+        for (int a = 0; a < NEN; ++a) k.local_m[li * (long long)(N * N) + (b * ND + jb) * N + a * ND + ja] = widen(acc[b][a]);
     return;
   }
-  // second scatter pass with its own Dirichlet average avg = (1 + trace)/n
-  // (scatter.hpp:62-78), formed only where the element has a blocked row
+  // second scatter pass with its own Dirichlet average avg = (1 + trace)/n (scatter.hpp:62-78),
+  // formed only where the element has a blocked row
   uint32_t any_blocked = 0u;
 #pragma unroll
-  for (int a = 0; a < NEN; ++a) any_blocked |= B.blocked[a];
+  for (int a = 0; a < NEN; ++a) any_blocked |= blocked[a];
   double avg = 0.0;
-  if (any_blocked != 0u || k.vjp_lam) {
+  if (any_blocked != 0u) {
     double tr = 0.0;
-    for (int i = lane; i < N; i += 32) tr += widen(B.m[i * MS + i]);
+    if (active && jb == ja)
+#pragma unroll
+      for (int b = 0; b < NEN; ++b) tr += widen(acc[b][b]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) tr += __shfl_xor_sync(0xffffffffu, tr, o);
+    if ((tid & 31) == 0) wsum[tid >> 5] = tr;
+    __syncthreads();
+    tr = 0.0;
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; ++w) tr += wsum[w];
     avg = (1.0 + tr) * (1.0 / N);
   }
+  if (!active) return;
+  const int mode = k.scatter_mode;
   if (k.vjp_lam) {
     // frozen-tangent VJP: g += K^T lambda for this element's boundary block
-    for (int cx = lane; cx < N; cx += 32) {
-      double sum = 0.0;
-      for (int rw = 0; rw < N; ++rw) {
-        const int b = rw / ND, jb = rw % ND;
-        const double val = ((B.blocked[b] >> jb) & 1u) ? (rw == cx ? avg : 0.0) : widen(B.m[rw * MS + cx]);
-        sum += __ldg(k.vjp_lam + (long long)nodes[b] * ND + jb) * val;
+    double g[NEN];
+#pragma unroll
+    for (int a = 0; a < NEN; ++a) g[a] = 0.0;
+#pragma unroll
+    for (int b = 0; b < NEN; ++b) {
+      const bool off = (blocked[b] >> jb) & 1u;
+      const double lam = __ldg(k.vjp_lam + (long long)nodes[b] * ND + jb);
+#pragma unroll
+      for (int a = 0; a < NEN; ++a) {
+        const double val = off ? (a == b && ja == jb ? avg : 0.0) : widen(acc[b][a]);
+        g[a] = fma(lam, val, g[a]);
       }
-      if (sum != 0.0) atomicAdd(k.vjp_g + (long long)nodes[cx / ND] * ND + cx % ND, sum);
     }
+#pragma unroll
+    for (int a = 0; a < NEN; ++a)
+      if (g[a] != 0.0) atomicAdd(k.vjp_g + (long long)nodes[a] * ND + ja, g[a]);
     return;
   }
-  const int mode = k.scatter_mode;
-  for (int t = lane; t < N; t += 32) {
-    const int b = t / ND, jb = t % ND;
-    if (!((B.blocked[b] >> jb) & 1u)) add_to(k.rhs + (long long)nodes[b] * ND + jb, -B.r[t], mode);
-  }
-  if (k.vals) {
-    // lane = column (a, ja): one block row per step, consecutive lanes on consecutive
-    // columns of node a's run in the row
-    constexpr int CH = (N + 31) / 32;
 #pragma unroll
-    for (int h = 0; h < CH; ++h) {
-      const int cx = lane + 32 * h;
-      if (cx >= N) break;
-      const int a = cx / ND, ja = cx - (cx / ND) * ND;
+  for (int b = 0; b < NEN; ++b) {
+    double* row = k.vals + rowbase[b] + (int64_t)jb * rowlen[b] + ja;
+    if ((blocked[b] >> jb) & 1u) {
+      if (ja == jb) add_to(row + (int64_t)slot[b][b] * ND, avg, mode);
+      continue;
+    }
 #pragma unroll
-      for (int bq = 0; bq < NEN; ++bq) {
-        const uint32_t bl = B.blocked[bq];
-        const int64_t rl = B.rowlen[bq];
-        double* rowp = k.vals + B.rowbase[bq] + (int64_t)B.slot[bq][a] * ND + ja;
-#pragma unroll
-        for (int jb = 0; jb < ND; ++jb, rowp += rl) {
-          const int row = bq * ND + jb;
-          double val;
-          if ((bl >> jb) & 1u) {
-            if (row != cx) continue;
-            val = avg;
-          } else {
-            val = widen(B.m[row * MS + cx]);
-          }
-          if ((__double2hiint(val) & 0x7fffffff) | __double2loint(val)) add_to(rowp, val, mode);
-        }
-      }
+    for (int a = 0; a < NEN; ++a) {
+      const double val = widen(acc[b][a]);
+      if ((__double2hiint(val) & 0x7fffffff) | __double2loint(val)) add_to(row + (int64_t)slot[b][a] * ND, val, mode);
     }
   }
 }

@@ -187,8 +187,8 @@ LaunchResult launch_boundary_nc(const KParams& k, long long n_items, cudaStream_
     bpoint_kernel<DIM, NEN, NC, NS, NSQ, S, EOS><<<(unsigned)((k.n_bpt + 127) / 128), 128, 0, st>>>(k);
     ++launches;
   }
-  const size_t smem = sizeof(BoundarySmem<DIM, NEN, NC, NS, NSQ, S>);
-  boundary_kernel<DIM, NEN, NC, NS, NSQ, S, EOS><<<(unsigned)n_items, 32, smem, st>>>(k);
+  const size_t smem = k.bpt_rec ? 0 : sizeof(BoundarySmem<DIM, NEN, NC, NS, NSQ, S>);
+  boundary_kernel<DIM, NEN, NC, NS, NSQ, S, EOS><<<(unsigned)n_items, boundary_threads<NC, DIM>(), smem, st>>>(k);
   return {cudaGetLastError(), launches + 1};
 }
 
