@@ -22,9 +22,10 @@ SOURCES = (["gales_host.cu", "gales_mesh_io.cu", "gales_solver.cu", "gales_magma
            + [f"gales_vjp_{t}.cu" for t in ("hex8", "tet4", "tri3", "quad4")]
            + [f"gales_{t}_magma_{f}.cu" for t in ("hex8", "tet4", "tri3", "quad4") for f in ("fp64", "mixed")])
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-# -fmad=false: no implicit contraction in the FP64 form's units, which perform the
-# reference's IEEE operations (see gales_physics.cuh); the mixed form's units contract
-# freely (the few steps whose rounding must match use unfused intrinsics).
+# -fmad=false: no implicit contraction in the FP64 form's units, whose boundary fluxes, time
+# step and secondary variables perform the reference's IEEE operations (see
+# gales_physics.cuh); the mixed form's and the adjoint's units contract freely (the few steps
+# whose rounding must match use unfused intrinsics).
 FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-fmad=false", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
          "-Xcompiler", "-ffp-contract=off"]
 
@@ -53,7 +54,8 @@ def build(verbose: bool = False, force: bool = False) -> Path:
         src = CSRC / s
         obj = BUILD / (Path(s).stem + ".o")
         if force or _stale(obj, src):
-            flags = [("-fmad=true" if (f == "-fmad=false" and "_mixed" in src.name) else f) for f in FLAGS]
+            fused = "_mixed" in src.name or "_vjp_" in src.name
+            flags = [("-fmad=true" if (f == "-fmad=false" and fused) else f) for f in FLAGS]
             cmd = [nvcc, *ARCH, *flags, "-I", str(HERE.parent / "include"), "-c", str(src), "-o", str(obj)]
             jobs.append((s, cmd))
     pr_src = CSRC / "pipe_rates.cu"

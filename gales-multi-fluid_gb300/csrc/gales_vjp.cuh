@@ -60,99 +60,71 @@ GV_HD double dot(const double* a, const double* b) {
 }
 
 // ---------------------------------------------------------------------------
-// Mixture EOS (fluid_properties.hpp:199-227) with its tape.
+// Mixture EOS (fluid_properties.hpp:199-227) with its tape, in reciprocals: ir_c = 1/rho_c
+// (a gas has R T/p), A_c = alpha_c/rho_c and B_c = beta_c/rho_c, so that a state takes 1/p,
+// 1/rho and 1/sqrt(c2) and no division per component; the component constants of a point's two
+// states are formed once (CompK).
+struct CompK {
+  double ir, cvs, ig;   // custom: 1/rho, alpha^2/(rho beta); gas: 1/gamma = (cp - R)/cp
+};
+
 template <int NC>
 struct Mix {
   double Y[NC];
-  double r[NC], cvc[NC], c2t[NC];   // rho_c, cv_c, Y-free sound-speed term 1/(rho_c^2 s_c^2)
-  double ac[NC], bc[NC];            // alpha_c, beta_c
-  double irho, rho, mu, cp, cv, kappa, c2, c, alpha, beta;
+  double ir[NC], cvc[NC], c2t[NC];   // 1/rho_c, cv_c, Y-free sound-speed term 1/(rho_c^2 s_c^2)
+  double A[NC], B[NC];
+  double ip, irho, rho, mu, cp, cv, kappa, c2, isc, c, alpha, beta;
 };
 
-// Component values at (p, T): rho_c, cv_c, 1/(rho_c^2 s_c^2), alpha_c, beta_c.
-GV_HD void comp_eval(const DevChem& q, double p, double T, double& r, double& cvc, double& c2t, double& a,
-                     double& b) {
+GV_HD void comp_const(const DevChem& q, CompK& k) {
   if (q.kind == GALES_CH_CUSTOM) {
-    r = q.rho; a = q.alpha; b = q.beta;
-    if (b == 0.0) {
-      cvc = q.cp;
-      c2t = 1.e-40 / (r * r);
-    } else {
-      cvc = q.cp - T * a * a / (r * b);
-      c2t = b / r;                       // 1/(r^2 s^2) with s^2 = 1/(r b)
-    }
+    k.ir = 1.0 / q.rho;
+    k.cvs = q.beta == 0.0 ? 0.0 : q.alpha * q.alpha / (q.rho * q.beta);
+    k.ig = 0.0;
   } else {
-    const double R = q.R, g = q.cp / (q.cp - R);
-    r = p / (R * T);
-    a = 1.0 / T;
-    b = 1.0 / p;
-    cvc = q.cp - R;
-    c2t = 1.0 / (r * r * g * R * T);
-  }
-}
-
-// Adjoint of comp_eval: cotangents of (r, cvc, c2t, a, b) -> p, T and theta_c.
-GV_HD void comp_rev(const DevChem& q, double p, double T, double rb, double cvb, double c2b, double ab, double bb,
-                    double& pb, double& Tb, double* th) {
-  if (q.kind == GALES_CH_CUSTOM) {
-    const double r = q.rho, a = q.alpha, b = q.beta;
-    th[2] += cvb;                                          // d cv/d cp
-    if (b == 0.0) {
-      th[0] += c2b * (-2.e-40 / (r * r * r));
-    } else {
-      Tb += cvb * (-a * a / (r * b));
-      th[0] += cvb * (T * a * a / (r * r * b)) + c2b * (-b / (r * r));
-    }
-    th[0] += rb;
-  } else {
-    const double R = q.R, cp = q.cp, cv = cp - R, g = cp / cv;
-    const double r = p / (R * T);
-    // r = p/(R T)
-    pb += rb / (R * T);
-    Tb += rb * (-r / T);
-    double Rb = rb * (-r / R);
-    Tb += ab * (-1.0 / (T * T));
-    pb += bb * (-1.0 / (p * p));
-    // cv = cp - R
-    th[2] += cvb;
-    Rb -= cvb;
-    // c2t = 1/(r^2 g R T) = R T/(g p^2) = R T cv/(cp p^2)
-    const double c2t = R * T * cv / (cp * p * p);
-    pb += c2b * (-2.0 * c2t / p);
-    Tb += c2b * (c2t / T);
-    // d/dR of R (cp - R) = cp - 2R ; d/dcp of cv/cp = R/cp^2
-    Rb += c2b * (T * (cp - 2.0 * R) / (cp * p * p));
-    th[2] += c2b * (R * T * R / (cp * cp * p * p));
-    (void)g;
-    // theta_0 = M, R = R_u/M: dR/dM = -R^2/R_u
-    th[0] += Rb * (-R * R / kRu);
+    k.ir = k.cvs = 0.0;
+    k.ig = (q.cp - q.R) / q.cp;
   }
 }
 
 template <int NC>
-GV_HD void mix_forward(const DevChem* ch, double p, double T, const double* Y, Mix<NC>& m) {
-  double irho = 0.0, mu = 0.0, cp = 0.0, cv = 0.0, kappa = 0.0, c2 = 0.0;
+GV_HD void mix_forward(const DevChem* ch, const CompK* kc, double p, double T, const double* Y, Mix<NC>& m) {
+  double irho = 0.0, mu = 0.0, cp = 0.0, cv = 0.0, kappa = 0.0, c2 = 0.0, al = 0.0, be = 0.0;
+  bool gas = false;   // a material without a gas never divides by p
+#pragma unroll
+  for (int c = 0; c < NC; ++c) gas |= ch[c].kind != GALES_CH_CUSTOM;
+  m.ip = gas ? 1.0 / p : 0.0;
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
+    const DevChem& q = ch[c];
     m.Y[c] = Y[c];
-    comp_eval(ch[c], p, T, m.r[c], m.cvc[c], m.c2t[c], m.ac[c], m.bc[c]);
-    irho += Y[c] / m.r[c];
-    mu += Y[c] * ch[c].mu;
-    cp += Y[c] * ch[c].cp;
+    if (q.kind == GALES_CH_CUSTOM) {
+      m.ir[c] = kc[c].ir;
+      m.cvc[c] = q.cp - T * kc[c].cvs;
+      m.A[c] = q.alpha * kc[c].ir;
+      m.B[c] = q.beta * kc[c].ir;
+      m.c2t[c] = q.beta == 0.0 ? 1.e-40 * kc[c].ir * kc[c].ir : m.B[c];   // s^2 = 1/(rho beta)
+    } else {
+      m.A[c] = q.R * m.ip;
+      m.ir[c] = m.A[c] * T;
+      m.B[c] = m.ir[c] * m.ip;
+      m.cvc[c] = q.cp - q.R;
+      m.c2t[c] = m.B[c] * kc[c].ig;
+    }
+    irho += Y[c] * m.ir[c];
+    mu += Y[c] * q.mu;
+    cp += Y[c] * q.cp;
     cv += Y[c] * m.cvc[c];
-    kappa += Y[c] * ch[c].kappa;
+    kappa += Y[c] * q.kappa;
     c2 += Y[c] * m.c2t[c];
+    al += Y[c] * m.A[c];
+    be += Y[c] * m.B[c];
   }
   m.irho = irho;
   m.rho = 1.0 / irho;
   m.mu = mu; m.cp = cp; m.cv = cv; m.kappa = kappa; m.c2 = c2;
-  m.c = irho / sqrt(c2);
-  double al = 0.0, be = 0.0;
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    al += Y[c] * m.ac[c] / m.r[c];
-    be += Y[c] * m.bc[c] / m.r[c];
-  }
+  m.isc = 1.0 / sqrt(c2);
+  m.c = irho * m.isc;
   m.alpha = m.rho * al;
   m.beta = m.rho * be;
 }
@@ -162,29 +134,87 @@ struct MixBar {
   double rho, mu, cp, cv, kappa, c, alpha, beta;
 };
 
+// irb, cvcb: the components' 1/rho_c and cv_c cotangents from the coefficient layer.
 template <int NC>
-GV_HD void mix_reverse(const DevChem* ch, double p, double T, const Mix<NC>& m, const MixBar& o, const double* rcb,
-                       const double* cvcb, double& pb, double& Tb, double* Yb, double* th) {
-  // outputs: rho = 1/irho, c = irho/sqrt(c2), alpha = rho*al, beta = rho*be (+ per-component
-  // rho_c and cv_c cotangents rcb, cvcb from the coefficient layer)
-  double al = m.alpha / m.rho, be = m.beta / m.rho;
-  double rhob = o.rho + o.alpha * al + o.beta * be;
+GV_HD void mix_reverse(const DevChem* ch, const CompK* kc, double T, const Mix<NC>& m, const MixBar& o,
+                       const double* irb_in, const double* cvcb, double& pb, double& Tb, double* Yb, double* th) {
+  // outputs: rho = 1/irho, c = irho/sqrt(c2), alpha = rho sum Y A, beta = rho sum Y B
+  const double rhob = o.rho + (o.alpha * m.alpha + o.beta * m.beta) * m.irho;
   const double alb = o.alpha * m.rho, beb = o.beta * m.rho;
-  double irhob = -rhob * m.rho * m.rho + o.c / sqrt(m.c2);
-  const double c2b = o.c * (-0.5 * m.irho / (m.c2 * sqrt(m.c2)));
+  const double irhob = o.c * m.isc - rhob * m.rho * m.rho;
+  const double c2b = o.c * (-0.5 * m.irho * m.isc * m.isc * m.isc);
+  double ipb = 0.0;
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
-    const double Yc = m.Y[c], r = m.r[c];
-    double rb = rcb ? rcb[c] : 0.0;
-    double cvb = (cvcb ? cvcb[c] : 0.0) + o.cv * Yc;
-    double c2tb = c2b * Yc;
-    double ab = alb * Yc / r, bb = beb * Yc / r;
-    rb += -irhob * Yc / (r * r) - alb * Yc * m.ac[c] / (r * r) - beb * Yc * m.bc[c] / (r * r);
-    Yb[c] += irhob / r + o.mu * ch[c].mu + o.cp * ch[c].cp + o.cv * m.cvc[c] + o.kappa * ch[c].kappa +
-             c2b * m.c2t[c] + alb * m.ac[c] / r + beb * m.bc[c] / r;
+    const DevChem& q = ch[c];
+    const double Yc = m.Y[c];
+    const double irb = irb_in[c] + irhob * Yc, cvb = cvcb[c] + o.cv * Yc;
+    const double c2tb = c2b * Yc, Ab = alb * Yc, Bb = beb * Yc;
+    Yb[c] += irhob * m.ir[c] + o.mu * q.mu + o.cp * q.cp + o.cv * m.cvc[c] + o.kappa * q.kappa + c2b * m.c2t[c] +
+             alb * m.A[c] + beb * m.B[c];
     th[3 * c + 1] += o.mu * Yc;
-    th[3 * c + 2] += o.cp * Yc;
-    comp_rev(ch[c], p, T, rb, cvb, c2tb, ab, bb, pb, Tb, th + 3 * c);
+    th[3 * c + 2] += o.cp * Yc + cvb;
+    if (q.kind == GALES_CH_CUSTOM) {
+      const double ir = kc[c].ir;
+      const double it = irb + Ab * q.alpha + Bb * q.beta + c2tb * (q.beta == 0.0 ? 2.e-40 * ir : q.beta);
+      th[3 * c] += cvb * T * kc[c].cvs * ir - it * ir * ir;   // cv = cp - T alpha^2/(rho beta)
+      Tb -= cvb * kc[c].cvs;
+    } else {
+      // A = R/p, ir = A T, B = ir/p, c2t = B (cp - R)/cp
+      const double Bt = Bb + c2tb * kc[c].ig;
+      const double it = irb + Bt * m.ip, At = Ab + it * T;
+      ipb += Bt * m.ir[c] + At * q.R;
+      Tb += it * m.A[c];
+      const double x = c2tb * m.B[c] / q.cp;     // (cp - R)/cp: -1/cp in R, R/cp^2 in cp
+      const double Rb = At * m.ip - x - cvb;
+      th[3 * c + 2] += x * (1.0 - kc[c].ig);
+      th[3 * c] += Rb * (-q.R * q.R / kRu);      // theta_0 = M, R = R_u/M
+    }
+  }
+  pb -= ipb * m.ip * m.ip;
+}
+
+// The previous level: rho and cv alone (what U_P needs), and their parameter cotangents.
+template <int NC>
+struct MixP {
+  double Y[NC], ir[NC], ip, rho, cv;
+};
+
+template <int NC>
+GV_HD void mixp_forward(const DevChem* ch, const CompK* kc, double p, double T, const double* Y, MixP<NC>& m) {
+  double irho = 0.0, cv = 0.0;
+  bool gas = false;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) gas |= ch[c].kind != GALES_CH_CUSTOM;
+  m.ip = gas ? 1.0 / p : 0.0;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const DevChem& q = ch[c];
+    const bool custom = q.kind == GALES_CH_CUSTOM;
+    m.Y[c] = Y[c];
+    m.ir[c] = custom ? kc[c].ir : q.R * m.ip * T;
+    irho += Y[c] * m.ir[c];
+    cv += Y[c] * (custom ? q.cp - T * kc[c].cvs : q.cp - q.R);
+  }
+  m.rho = 1.0 / irho;
+  m.cv = cv;
+}
+
+template <int NC>
+GV_HD void mixp_reverse(const DevChem* ch, const CompK* kc, double T, const MixP<NC>& m, double rhob, double cvb_mix,
+                        double* th) {
+  const double irhob = -rhob * m.rho * m.rho;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const DevChem& q = ch[c];
+    const double irb = irhob * m.Y[c], cvb = cvb_mix * m.Y[c];
+    th[3 * c + 2] += cvb;
+    if (q.kind == GALES_CH_CUSTOM) {
+      const double ir = kc[c].ir;
+      th[3 * c] += cvb * T * kc[c].cvs * ir - irb * ir * ir;
+    } else {
+      th[3 * c] += (irb * T * m.ip - cvb) * (-q.R * q.R / kRu);
+    }
   }
 }
 
@@ -225,16 +255,16 @@ GV_HD void coef_forward(const Mix<NC>& m, const DevChem* ch, double p, const dou
   c.E = m.cv * T + 0.5 * dot<DIM>(v, v);
   c.drho_dp = rho * m.beta;
   c.drho_dT = -rho * m.alpha;
-  c.de_dp = (m.beta * p - m.alpha * T) / rho;
-  c.de_dT = m.cp - p * m.alpha / rho;
+  c.de_dp = (m.beta * p - m.alpha * T) * m.irho;
+  c.de_dT = m.cp - p * m.alpha * m.irho;
   c.mu = m.mu;
-  c.lam = -2.0 * m.mu / 3.0;
+  c.lam = (-2.0 / 3.0) * m.mu;
   c.kappa = m.kappa;
 #pragma unroll
   for (int i = 0; i < NC - 1; ++i) {
-    c.drho_dY[i] = -rho * rho * (1.0 / m.r[i] - 1.0 / m.r[NC - 1]);
+    c.drho_dY[i] = -rho * rho * (m.ir[i] - m.ir[NC - 1]);
     c.dE_dY[i] = m.cvc[i] * T - m.cvc[NC - 1] * T;
-    c.H[i] = m.cvc[i] * T + p / m.r[i];
+    c.H[i] = m.cvc[i] * T + p * m.ir[i];
     c.rhoD[i] = rho * ch[i].D;
     c.rhoDH[i] = c.rhoD[i] * c.H[i];
   }
@@ -269,14 +299,14 @@ GV_HD void cfbar_fold(CfBar<DIM, NC>& b) {
 }
 
 // Coefficient layer reverse: scalar cotangents -> mixture cotangents, per-component
-// rho_c / cv_c cotangents, and direct state cotangents (p, v, T).
+// 1/rho_c / cv_c cotangents, and direct state cotangents (p, v, T).
 template <int DIM, int NC>
 GV_HD void coef_reverse(const Mix<NC>& m, const DevChem* ch, const Cf<DIM, NC>& c, const CfBar<DIM, NC>& b,
-                        MixBar& o, double* rcb, double* cvcb, double& pb, double* vb, double& Tb, double* Yb) {
-  const double rho = m.rho, p = c.p, T = c.T;
+                        MixBar& o, double* irb, double* cvcb, double& pb, double* vb, double& Tb, double* Yb) {
+  const double rho = m.rho, irho = m.irho, p = c.p, T = c.T;
   o = MixBar{0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
-  for (int i = 0; i < NC; ++i) { rcb[i] = 0.0; cvcb[i] = 0.0; }
+  for (int i = 0; i < NC; ++i) { irb[i] = 0.0; cvcb[i] = 0.0; }
   // E = cv T + |v|^2/2
   o.cv += b.E * T; Tb += b.E * m.cv;
 #pragma unroll
@@ -289,85 +319,77 @@ GV_HD void coef_reverse(const Mix<NC>& m, const DevChem* ch, const Cf<DIM, NC>& 
   o.rho += b.drho_dp * m.beta - b.drho_dT * m.alpha;
   o.beta += b.drho_dp * rho;
   o.alpha -= b.drho_dT * rho;
-  // de_dp = (beta p - alpha T)/rho
-  o.beta += b.de_dp * p / rho;
-  o.alpha -= b.de_dp * T / rho;
-  pb += b.de_dp * m.beta / rho;
-  Tb -= b.de_dp * m.alpha / rho;
-  o.rho -= b.de_dp * (m.beta * p - m.alpha * T) / (rho * rho);
-  // de_dT = cp - p alpha/rho
+  // de_dp = (beta p - alpha T)/rho, de_dT = cp - p alpha/rho
+  const double g = b.de_dp * irho, f = b.de_dT * irho;
+  o.beta += g * p;
+  o.alpha -= g * T + f * p;
+  pb += g * m.beta - f * m.alpha;
+  Tb -= g * m.alpha;
+  o.rho += (f * p * m.alpha) * irho - g * c.de_dp;
   o.cp += b.de_dT;
-  pb -= b.de_dT * m.alpha / rho;
-  o.alpha -= b.de_dT * p / rho;
-  o.rho += b.de_dT * p * m.alpha / (rho * rho);
-  o.mu += b.mu - 2.0 * b.lam / 3.0;
+  o.mu += b.mu - (2.0 / 3.0) * b.lam;
   o.kappa += b.kappa;
 #pragma unroll
   for (int i = 0; i < NC - 1; ++i) {
     const int n = NC - 1;
-    // drho_dY = -rho^2 (1/r_i - 1/r_n)
-    o.rho += b.drho_dY[i] * (-2.0 * rho * (1.0 / m.r[i] - 1.0 / m.r[n]));
-    rcb[i] += b.drho_dY[i] * (rho * rho / (m.r[i] * m.r[i]));
-    rcb[n] -= b.drho_dY[i] * (rho * rho / (m.r[n] * m.r[n]));
+    // drho_dY = -rho^2 (1/rho_i - 1/rho_n)
+    o.rho += b.drho_dY[i] * (-2.0 * rho * (m.ir[i] - m.ir[n]));
+    irb[i] -= b.drho_dY[i] * (rho * rho);
+    irb[n] += b.drho_dY[i] * (rho * rho);
     // dE_dY = (cv_i - cv_n) T
     cvcb[i] += b.dE_dY[i] * T;
     cvcb[n] -= b.dE_dY[i] * T;
     Tb += b.dE_dY[i] * (m.cvc[i] - m.cvc[n]);
-    // rhoD = rho D, rhoDH = rho D H with H = cv_i T + p/r_i
+    // rhoD = rho D, rhoDH = rho D H with H = cv_i T + p/rho_i
     o.rho += b.rhoD[i] * ch[i].D + b.rhoDH[i] * ch[i].D * c.H[i];
     const double Hb = b.rhoDH[i] * c.rhoD[i];
     cvcb[i] += Hb * T;
     Tb += Hb * m.cvc[i];
-    pb += Hb / m.r[i];
-    rcb[i] -= Hb * p / (m.r[i] * m.r[i]);
+    pb += Hb * m.ir[i];
+    irb[i] += Hb * p;
   }
 }
 
 // ---------------------------------------------------------------------------
-// Bilinear forms with DUDY and A_d and their adjoints (weight s):
+// Products with DUDY and the adjoint of the bilinear form x^T DUDY y (weight s):
 //   x^T DUDY y = (x.w)(r0.y) + rho (sum_{r in v,Y} x_r y_r + x_E mE.y)
 //   x^T A_d y  = v_d x^T DUDY y + (x.u') y_{v_d} + (x_{v_d} + v_d x_E) y_p
-template <int DIM, int NC>
-GV_HD double xDy(const Cf<DIM, NC>& c, const double* x, const double* y) {
-  using L = Layout<DIM, NC>;
-  constexpr int ND = L::ND;
-  double xw = 0.0, ry = 0.0, my = 0.0, d = 0.0;
-#pragma unroll
-  for (int j = 0; j < ND; ++j) {
-    xw += x[j] * c.w[j];
-    ry += c.r0[j] * y[j];
-    my += c.mE[j] * y[j];
-    if (j >= 1 && j != L::iT) d += x[j] * y[j];
-  }
-  return xw * ry + c.rho * (d + x[L::iT] * my);
-}
-
 template <int DIM, int NC>
 GV_HD void Dy(const Cf<DIM, NC>& c, const double* y, double* out) {  // DUDY y
   using L = Layout<DIM, NC>;
   constexpr int ND = L::ND;
   double ry = 0.0, my = 0.0;
 #pragma unroll
-  for (int j = 0; j < ND; ++j) { ry += c.r0[j] * y[j]; my += c.mE[j] * y[j]; }
+  for (int j = 0; j < ND; ++j) {
+    if (j < 1 || j >= L::iT) ry += c.r0[j] * y[j];
+    my += c.mE[j] * y[j];
+  }
 #pragma unroll
   for (int r = 0; r < ND; ++r) {
-    double m = (r >= 1 && r != L::iT) ? y[r] : 0.0;
-    if (r == L::iT) m = my;
-    out[r] = c.w[r] * ry + c.rho * m;
+    const double m = r == L::iT ? my : y[r];
+    out[r] = r == 0 ? ry : c.w[r] * ry + c.rho * m;
   }
+}
+
+template <int DIM, int NC>
+GV_HD double xw_of(const Cf<DIM, NC>& c, const double* x) {  // x.w
+  double xw = x[0];
+#pragma unroll
+  for (int j = 1; j < Layout<DIM, NC>::ND; ++j) xw += x[j] * c.w[j];
+  return xw;
 }
 
 template <int DIM, int NC>
 GV_HD void DTx(const Cf<DIM, NC>& c, const double* x, double* out) {  // DUDY^T x
   using L = Layout<DIM, NC>;
   constexpr int ND = L::ND;
-  double xw = 0.0;
-#pragma unroll
-  for (int j = 0; j < ND; ++j) xw += x[j] * c.w[j];
+  const double xw = xw_of<DIM, NC>(c, x), re = c.rho * x[L::iT];
 #pragma unroll
   for (int j = 0; j < ND; ++j) {
-    double m = (j >= 1 && j != L::iT) ? x[j] : 0.0;
-    out[j] = c.r0[j] * xw + c.rho * (m + x[L::iT] * c.mE[j]);
+    double o = re * c.mE[j];
+    if (j >= 1 && j != L::iT) o += c.rho * x[j];
+    if (j < 1 || j >= L::iT) o += c.r0[j] * xw;
+    out[j] = o;
   }
 }
 
@@ -375,68 +397,21 @@ template <int DIM, int NC>
 GV_HD void xDy_rev(const Cf<DIM, NC>& c, const double* x, const double* y, double s, CfBar<DIM, NC>& b) {
   using L = Layout<DIM, NC>;
   constexpr int ND = L::ND;
-  double xw = 0.0, ry = 0.0, my = 0.0, d = 0.0;
+  double ry = 0.0, my = 0.0, d = 0.0;
 #pragma unroll
   for (int j = 0; j < ND; ++j) {
-    xw += x[j] * c.w[j];
-    ry += c.r0[j] * y[j];
+    if (j < 1 || j >= L::iT) ry += c.r0[j] * y[j];
     my += c.mE[j] * y[j];
     if (j >= 1 && j != L::iT) d += x[j] * y[j];
   }
+  const double sw = s * xw_of<DIM, NC>(c, x), sr = s * ry, sm = s * c.rho * x[L::iT];
 #pragma unroll
   for (int j = 0; j < ND; ++j) {
-    b.w[j] += s * ry * x[j];
-    b.r0[j] += s * xw * y[j];
-    b.mE[j] += s * c.rho * x[L::iT] * y[j];
+    if (j > 0) b.w[j] += sr * x[j];
+    if (j < 1 || j >= L::iT) b.r0[j] += sw * y[j];
+    b.mE[j] += sm * y[j];
   }
   b.rho += s * (d + x[L::iT] * my);
-}
-
-template <int DIM, int NC>
-GV_HD void Ay(const Cf<DIM, NC>& c, int d, const double* y, double* out) {  // A_d y
-  using L = Layout<DIM, NC>;
-  constexpr int ND = L::ND;
-  Dy<DIM, NC>(c, y, out);
-  const double vd = c.v[d];
-#pragma unroll
-  for (int r = 0; r < ND; ++r) {
-    const double up = c.rho * c.w[r] + (r == L::iT ? c.p : 0.0);
-    out[r] = vd * out[r] + up * y[1 + d];
-  }
-  out[1 + d] += y[0];
-  out[L::iT] += vd * y[0];
-}
-
-template <int DIM, int NC>
-GV_HD void ATx(const Cf<DIM, NC>& c, int d, const double* x, double* out) {  // A_d^T x
-  using L = Layout<DIM, NC>;
-  constexpr int ND = L::ND;
-  DTx<DIM, NC>(c, x, out);
-  const double vd = c.v[d];
-  double xu = 0.0;
-#pragma unroll
-  for (int r = 0; r < ND; ++r) xu += x[r] * (c.rho * c.w[r] + (r == L::iT ? c.p : 0.0));
-#pragma unroll
-  for (int j = 0; j < ND; ++j) out[j] *= vd;
-  out[1 + d] += xu;
-  out[0] += x[1 + d] + vd * x[L::iT];
-}
-
-template <int DIM, int NC>
-GV_HD void xAy_rev(const Cf<DIM, NC>& c, int d, const double* x, const double* y, double s, CfBar<DIM, NC>& b) {
-  using L = Layout<DIM, NC>;
-  constexpr int ND = L::ND;
-  const double vd = c.v[d];
-  b.v[d] += s * (xDy<DIM, NC>(c, x, y) + x[L::iT] * y[0]);
-  xDy_rev<DIM, NC>(c, x, y, s * vd, b);
-  double xw = 0.0;
-#pragma unroll
-  for (int r = 0; r < ND; ++r) xw += x[r] * c.w[r];
-  const double t = s * y[1 + d];
-  b.rho += t * xw;
-#pragma unroll
-  for (int r = 0; r < ND; ++r) b.w[r] += t * c.rho * x[r];
-  b.p += t * x[L::iT];
 }
 
 // ---------------------------------------------------------------------------
@@ -446,6 +421,26 @@ struct HTape {
   double nv, s0[DIM], acc[DIM], ip, s1[DIM], n1, s1n[DIM], s2[3], n2, s2n[3], alpha[3], Q;
   bool norm1, norm2;
 };
+
+// The steps that decide compute_h's branches are never fused into multiply-adds, whatever the
+// translation unit's setting (on the host the unit is compiled without contraction).
+#ifdef __CUDA_ARCH__
+GV_HD double hmul(double a, double b) { return __dmul_rn(a, b); }
+GV_HD double hadd(double a, double b) { return __dadd_rn(a, b); }
+GV_HD double hsub(double a, double b) { return __dsub_rn(a, b); }
+#else
+GV_HD double hmul(double a, double b) { return a * b; }
+GV_HD double hadd(double a, double b) { return a + b; }
+GV_HD double hsub(double a, double b) { return a - b; }
+#endif
+
+template <int DIM>
+GV_HD double hdot(const double* a, const double* b) {
+  double s = 0.0;
+#pragma unroll
+  for (int i = 0; i < DIM; ++i) s = hadd(s, hmul(a[i], b[i]));
+  return s;
+}
 
 template <int DIM>
 GV_HD double quadform(const double (&G)[DIM][DIM], const double* s) {
@@ -474,35 +469,32 @@ GV_HD void quadform_rev(const double (&G)[DIM][DIM], const double* s, double ab,
 template <int DIM>
 GV_HD double compute_h_fwd(const double (&G)[DIM][DIM], const double* v, const double (&dv)[DIM][DIM],
                            HTape<DIM>& t) {
-  t.nv = sqrt(dot<DIM>(v, v));
+  t.nv = sqrt(hdot<DIM>(v, v));
 #pragma unroll
   for (int i = 0; i < DIM; ++i) t.s0[i] = v[i] / t.nv;
   t.alpha[0] = quadform<DIM>(G, t.s0);
 #pragma unroll
-  for (int i = 0; i < DIM; ++i) {
-    double a = 0.0;
+  for (int i = 0; i < DIM; ++i) t.acc[i] = hdot<DIM>(dv[i], v);
+  t.ip = hdot<DIM>(t.acc, t.s0);
 #pragma unroll
-    for (int j = 0; j < DIM; ++j) a += dv[i][j] * v[j];
-    t.acc[i] = a;
-  }
-  t.ip = dot<DIM>(t.acc, t.s0);
-#pragma unroll
-  for (int i = 0; i < DIM; ++i) t.s1[i] = t.acc[i] - t.ip * t.s0[i];
-  t.n1 = sqrt(dot<DIM>(t.s1, t.s1));
+  for (int i = 0; i < DIM; ++i) t.s1[i] = hsub(t.acc[i], hmul(t.ip, t.s0[i]));
+  t.n1 = sqrt(hdot<DIM>(t.s1, t.s1));
   t.norm1 = t.n1 > kEps;
+  const double in1 = t.norm1 ? 1.0 / t.n1 : 1.0;
 #pragma unroll
-  for (int i = 0; i < DIM; ++i) t.s1n[i] = t.norm1 ? t.s1[i] / t.n1 : t.s1[i];
+  for (int i = 0; i < DIM; ++i) t.s1n[i] = t.s1[i] * in1;
   t.alpha[1] = quadform<DIM>(G, t.s1n);
   t.alpha[2] = 0.0;
   t.norm2 = false;
   if constexpr (DIM == 3) {
-    t.s2[0] = t.s0[1] * t.s1n[2] - t.s0[2] * t.s1n[1];
-    t.s2[1] = t.s1n[0] * t.s0[2] - t.s1n[2] * t.s0[0];
-    t.s2[2] = t.s0[0] * t.s1n[1] - t.s0[1] * t.s1n[0];
-    t.n2 = sqrt(dot<3>(t.s2, t.s2));
+    t.s2[0] = hsub(hmul(t.s0[1], t.s1n[2]), hmul(t.s0[2], t.s1n[1]));
+    t.s2[1] = hsub(hmul(t.s1n[0], t.s0[2]), hmul(t.s1n[2], t.s0[0]));
+    t.s2[2] = hsub(hmul(t.s0[0], t.s1n[1]), hmul(t.s0[1], t.s1n[0]));
+    t.n2 = sqrt(hdot<3>(t.s2, t.s2));
     t.norm2 = t.n2 > kEps;
+    const double in2 = t.norm2 ? 1.0 / t.n2 : 1.0;
 #pragma unroll
-    for (int i = 0; i < 3; ++i) t.s2n[i] = t.norm2 ? t.s2[i] / t.n2 : t.s2[i];
+    for (int i = 0; i < 3; ++i) t.s2n[i] = t.s2[i] * in2;
     t.alpha[2] = quadform<DIM>(G, t.s2n);
   }
   double Q = 0.0;
@@ -520,9 +512,9 @@ GV_HD void normalise_rev(const double* sn, double n, bool norm, const double* sn
     for (int i = 0; i < DIM; ++i) sb[i] += snb[i];
     return;
   }
-  const double pr = dot<DIM>(snb, sn);
+  const double pr = dot<DIM>(snb, sn), in = 1.0 / n;
 #pragma unroll
-  for (int i = 0; i < DIM; ++i) sb[i] += (snb[i] - pr * sn[i]) / n;
+  for (int i = 0; i < DIM; ++i) sb[i] += (snb[i] - pr * sn[i]) * in;
 }
 
 template <int DIM>
@@ -577,36 +569,72 @@ GV_HD void compute_h_rev(const double (&G)[DIM][DIM], const double* v, const dou
 }
 
 // ---------------------------------------------------------------------------
-// DUDY^{-1} in closed form (dense), the 2x2 solve per column of DUDY = w r0^T + rho M.
+// X = DUDY^{-1} in closed form (see tau_closed): dense rows p and T (x0, xT), the velocity and
+// mass-fraction rows are (e_j - w_j e_p)/rho.
 template <int DIM, int NC>
-GV_HD void dudy_inverse(const Cf<DIM, NC>& c, double (&X)[Layout<DIM, NC>::ND][Layout<DIM, NC>::ND]) {
+struct Inv {
+  double x0[Layout<DIM, NC>::ND], xT[Layout<DIM, NC>::ND], irho;
+};
+
+template <int DIM, int NC>
+GV_HD void dudy_inverse(const Cf<DIM, NC>& c, double irho, Inv<DIM, NC>& X) {
   using L = Layout<DIM, NC>;
-  constexpr int ND = L::ND;
-  const double irho = 1.0 / c.rho;
-  const double det = c.drho_dp * c.de_dT - c.drho_dT * c.de_dp;
+  const double idet = 1.0 / (c.drho_dp * c.de_dT - c.drho_dT * c.de_dp), q = irho * idet;
+  double sY = 0.0, sE = -c.E;
 #pragma unroll
-  for (int col = 0; col < ND; ++col) {
-    const double s = (col == 0) ? 1.0 : 0.0;
-    double xv[DIM], xy[L::NYA];
+  for (int j = 0; j < DIM; ++j) sE += c.v[j] * c.v[j];
 #pragma unroll
-    for (int j = 0; j < DIM; ++j) xv[j] = (((col == 1 + j) ? 1.0 : 0.0) - c.v[j] * s) * irho;
-#pragma unroll
-    for (int i = 0; i < NC - 1; ++i) xy[i] = (((col == L::iY + i) ? 1.0 : 0.0) - c.Y[i] * s) * irho;
-    double R1 = s, R2 = (((col == L::iT) ? 1.0 : 0.0) - c.E * s) * irho;
-#pragma unroll
-    for (int j = 0; j < DIM; ++j) R2 -= c.v[j] * xv[j];
-#pragma unroll
-    for (int i = 0; i < NC - 1; ++i) {
-      R1 -= c.drho_dY[i] * xy[i];
-      R2 -= c.dE_dY[i] * xy[i];
-    }
-    X[0][col] = (R1 * c.de_dT - c.drho_dT * R2) / det;
-    X[L::iT][col] = (c.drho_dp * R2 - c.de_dp * R1) / det;
-#pragma unroll
-    for (int j = 0; j < DIM; ++j) X[1 + j][col] = xv[j];
-#pragma unroll
-    for (int i = 0; i < NC - 1; ++i) X[L::iY + i][col] = xy[i];
+  for (int i = 0; i < NC - 1; ++i) {
+    sY += c.drho_dY[i] * c.Y[i];
+    sE += c.dE_dY[i] * c.Y[i];
   }
+  const double R1 = 1.0 + irho * sY, R2 = irho * sE;
+  X.irho = irho;
+  X.x0[0] = (R1 * c.de_dT - c.drho_dT * R2) * idet;
+  X.xT[0] = (c.drho_dp * R2 - c.de_dp * R1) * idet;
+#pragma unroll
+  for (int j = 0; j < DIM; ++j) {
+    X.x0[1 + j] = c.drho_dT * q * c.v[j];
+    X.xT[1 + j] = -c.drho_dp * q * c.v[j];
+  }
+  X.x0[L::iT] = -c.drho_dT * q;
+  X.xT[L::iT] = c.drho_dp * q;
+#pragma unroll
+  for (int i = 0; i < NC - 1; ++i) {
+    X.x0[L::iY + i] = (c.drho_dT * c.dE_dY[i] - c.drho_dY[i] * c.de_dT) * q;
+    X.xT[L::iY + i] = (c.de_dp * c.drho_dY[i] - c.drho_dp * c.dE_dY[i]) * q;
+  }
+}
+
+template <int DIM, int NC>
+GV_HD void inv_mul(const Cf<DIM, NC>& c, const Inv<DIM, NC>& X, const double* y, double* out) {  // X y
+  using L = Layout<DIM, NC>;
+  double a = 0.0, b = 0.0;
+#pragma unroll
+  for (int j = 0; j < L::ND; ++j) {
+    a += X.x0[j] * y[j];
+    b += X.xT[j] * y[j];
+  }
+#pragma unroll
+  for (int j = 1; j < L::ND; ++j) out[j] = X.irho * (y[j] - c.w[j] * y[0]);
+  out[0] = a;
+  out[L::iT] = b;
+}
+
+template <int DIM, int NC>
+GV_HD void inv_tmul(const Cf<DIM, NC>& c, const Inv<DIM, NC>& X, const double* y, double* out) {  // X^T y
+  using L = Layout<DIM, NC>;
+  double s = 0.0;
+#pragma unroll
+  for (int j = 0; j < L::ND; ++j) {
+    double o = X.x0[j] * y[0] + X.xT[j] * y[L::iT];
+    if (j >= 1 && j != L::iT) {
+      o += X.irho * y[j];
+      s += c.w[j] * y[j];
+    }
+    out[j] = o;
+  }
+  out[0] -= X.irho * s;
 }
 
 // ---------------------------------------------------------------------------
@@ -615,7 +643,9 @@ template <int DIM, int NEN, int NC>
 struct PTape {
   using L = Layout<DIM, NC>;
   static constexpr int ND = L::ND;
-  Mix<NC> m, mP;
+  CompK kc[NC];
+  Mix<NC> m;
+  MixP<NC> mP;
   Cf<DIM, NC> c;
   double vP[DIM], TP, EP;
   double U[ND], UP[ND], S[ND];
@@ -623,12 +653,14 @@ struct PTape {
   // tau
   bool tau_on, lowm;
   HTape<DIM> ht;
-  double vn, h, use, hv, td[ND], X[ND][ND], tau[ND][ND], tpre00, tpre11, Bm;
+  Inv<DIM, NC> X;
+  double vn, h, use, hv, td[ND], tpre00, tpre11, Bm, t00;
+  double wv[ND], xy0;          // tau Res; row p of DUDY^{-1} diag(td) Res
   int use_branch;            // 0: dt/2, 1: h/(2(v+c)) + h/(2v)
   int td_branch[ND];         // 0: use, 1: the capped term
   // dc
   bool dc_on;
-  double dU[DIM][ND], grho[DIM], gn, Jv[DIM], sJ, hdc, AdI[ND], Z[ND], Zn, Un, use1, nrm[DIM], nu0, nu;
+  double dU[DIM][ND], grho[DIM], gn, Jv[DIM], sJ, hdc, AdI[ND], Z[ND], Zn, Un, use1, nu0, nu;
   double sg[NEN];
 };
 
@@ -652,8 +684,10 @@ GV_HD void point_forward(const Ctx<DIM, NC>& x, const PGeo<DIM, NEN>& q, const d
   Y[NC - 1] = 1.0 - sY;
   YP[NC - 1] = 1.0 - sYP;
   t.TP = Pq[L::iT];
-  mix_forward<NC>(x.ch, Pq[0], t.TP, YP, t.mP);
-  mix_forward<NC>(x.ch, p, T, Y, t.m);
+#pragma unroll
+  for (int i = 0; i < NC; ++i) comp_const(x.ch[i], t.kc[i]);
+  mixp_forward<NC>(x.ch, t.kc, Pq[0], t.TP, YP, t.mP);
+  mix_forward<NC>(x.ch, t.kc, p, T, Y, t.m);
   coef_forward<DIM, NC>(t.m, x.ch, p, v, T, t.c);
   const Cf<DIM, NC>& c = t.c;
   // U, U_P, S and the mass term (fluid_2d.hpp:372-385, 597-599)
@@ -674,25 +708,32 @@ GV_HD void point_forward(const Ctx<DIM, NC>& x, const PGeo<DIM, NEN>& q, const d
   t.S[L::iT] = t.m.rho * gv;
   // least-squares residual Res = DUDY (I - P)/dt + sum_d A_d dI_d - S  (fluid_2d.hpp:282)
 #pragma unroll
-  for (int j = 0; j < ND; ++j) t.dd[j] = (Iq[j] - Pq[j]) / dt;
+  for (int j = 0; j < ND; ++j) t.dd[j] = (Iq[j] - Pq[j]) * x.inv_dt;
   Dy<DIM, NC>(c, t.dd, t.Res);
 #pragma unroll
-  for (int j = 0; j < ND; ++j) t.AdI[j] = 0.0;
+  for (int d = 0; d < DIM; ++d) Dy<DIM, NC>(c, dI[d], t.dU[d]);
+  double div = 0.0;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) div += dI[d][1 + d];
+  // sum_d A_d dI_d, A_d = v_d DUDY + u' e_vd^T + (e_vd + v_d e_E) e_p^T
+#pragma unroll
+  for (int j = 0; j < ND; ++j) {
+    double a = (t.U[j] + (j == L::iT ? p : 0.0)) * div;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) a += v[d] * t.dU[d][j];
+    t.AdI[j] = a;
+  }
 #pragma unroll
   for (int d = 0; d < DIM; ++d) {
-    double a[ND];
-    Ay<DIM, NC>(c, d, dI[d], a);
-#pragma unroll
-    for (int j = 0; j < ND; ++j) t.AdI[j] += a[j];
+    t.AdI[1 + d] += dI[d][0];
+    t.AdI[L::iT] += v[d] * dI[d][0];
   }
 #pragma unroll
   for (int j = 0; j < ND; ++j) t.Res[j] += t.AdI[j] - t.S[j];
   // tau (fluid_2d.hpp:877-960), 2019 or none
 #pragma unroll
-  for (int r = 0; r < ND; ++r)
-#pragma unroll
-    for (int cc = 0; cc < ND; ++cc) t.tau[r][cc] = 0.0;
-  t.vn = sqrt(dot<DIM>(v, v));
+  for (int r = 0; r < ND; ++r) t.wv[r] = 0.0;
+  t.vn = sqrt(hdot<DIM>(v, v));
   t.tau_on = t.vn >= kEps && x.tau == GALES_TAU_NON_DIAG_COMP_2019;
   t.lowm = false;
   if (t.tau_on) {
@@ -703,17 +744,19 @@ GV_HD void point_forward(const Ctx<DIM, NC>& x, const PGeo<DIM, NEN>& q, const d
       for (int d = 0; d < DIM; ++d) dv[a][d] = dI[d][1 + a];
     t.h = compute_h_fwd<DIM>(q.G, v, dv, t.ht);
     const double cs = t.m.c, h = t.h, vn = t.vn;
-    t.hv = h / (2.0 * (vn + cs)) + h / (2.0 * vn);
+    t.hv = (0.5 * h) * (2.0 * vn + cs) / (vn * (vn + cs));   // h/(2(|v| + c)) + h/(2|v|)
     t.use_branch = (x.steady || t.hv <= dt * 0.5) ? 1 : 0;
     t.use = t.use_branch ? t.hv : dt * 0.5;
     const double use = t.use, rho = t.m.rho;
+    const double hh = h * h * (1.0 / 12.0);
     double cap[ND];
     cap[0] = use;
+    const double capv = hh * rho / t.m.mu;
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) cap[1 + d] = h * h * rho / (12.0 * t.m.mu);
-    cap[L::iT] = h * h * rho * t.m.cv / (12.0 * t.m.kappa);
+    for (int d = 0; d < DIM; ++d) cap[1 + d] = capv;
+    cap[L::iT] = hh * rho * t.m.cv / t.m.kappa;
 #pragma unroll
-    for (int i = 0; i < NC - 1; ++i) cap[L::iY + i] = h * h / (12.0 * x.ch[i].D);
+    for (int i = 0; i < NC - 1; ++i) cap[L::iY + i] = hh / x.ch[i].D;
     t.td_branch[0] = 0;
     t.td[0] = use;
 #pragma unroll
@@ -721,24 +764,23 @@ GV_HD void point_forward(const Ctx<DIM, NC>& x, const PGeo<DIM, NEN>& q, const d
       t.td_branch[j] = cap[j] < use ? 1 : 0;
       t.td[j] = t.td_branch[j] ? cap[j] : use;
     }
-    dudy_inverse<DIM, NC>(c, t.X);
+    dudy_inverse<DIM, NC>(c, t.m.irho, t.X);
+    double y[ND];
 #pragma unroll
-    for (int r = 0; r < ND; ++r)
-#pragma unroll
-      for (int cc = 0; cc < ND; ++cc) t.tau[r][cc] = t.X[r][cc] * t.td[cc];
-    t.tpre00 = t.tau[0][0];
-    t.tpre11 = t.tau[1][1];
-    if (vn / cs < 0.1) {
+    for (int j = 0; j < ND; ++j) y[j] = t.td[j] * t.Res[j];
+    inv_mul<DIM, NC>(c, t.X, y, t.wv);
+    t.xy0 = t.wv[0];
+    if (vn < 0.1 * cs) {
+      // row p: tau00 = 1/(1/a + 1/B), zero elsewhere
       t.lowm = true;
+      t.tpre00 = t.X.x0[0] * t.td[0];
+      t.tpre11 = t.m.irho * t.td[1];
       t.Bm = rho * t.tpre11 * q.trG;
-      t.tau[0][0] = 1.0 / (1.0 / t.tpre00 + 1.0 / t.Bm);
-#pragma unroll
-      for (int cc = 1; cc < ND; ++cc) t.tau[0][cc] = 0.0;
+      t.t00 = t.tpre00 * t.Bm / (t.tpre00 + t.Bm);
+      t.wv[0] = t.t00 * t.Res[0];
     }
   }
   // dc viscosity (fluid_2d.hpp:1027-1065)
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) Dy<DIM, NC>(c, dI[d], t.dU[d]);
   t.nu = 0.0;
   t.dc_on = false;
   if (x.dc_2006) {
@@ -747,8 +789,9 @@ GV_HD void point_forward(const Ctx<DIM, NC>& x, const PGeo<DIM, NEN>& q, const d
     for (int d = 0; d < DIM; ++d) { t.grho[d] = t.dU[d][0]; s += t.grho[d] * t.grho[d]; }
     t.gn = sqrt(s);
     if (!(t.gn < kEps)) {
+      const double ign = 1.0 / t.gn;
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) t.Jv[d] = t.grho[d] / t.gn;
+      for (int d = 0; d < DIM; ++d) t.Jv[d] = t.grho[d] * ign;
       double hs = 0.0;
 #pragma unroll
       for (int i = 0; i < NEN; ++i) {
@@ -772,20 +815,17 @@ GV_HD void point_forward(const Ctx<DIM, NC>& x, const PGeo<DIM, NEN>& q, const d
         }
         t.Zn = sqrt(Zn);
         t.Un = sqrt(Un);
-        double use1 = 0.0;
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) {
-          double n2 = 0.0;
-#pragma unroll
-          for (int j = 0; j < ND; ++j) {
-            const double u = x.u_ref_inv[j] * t.dU[d][j];
-            n2 += u * u;
-          }
-          t.nrm[d] = sqrt(n2);
-          use1 += t.nrm[d] * t.nrm[d];
-        }
-        t.use1 = use1;
         const double a = x.dc_sharp, hd = t.hdc;
+        double use1 = 0.0;
+        if (a != 2.0)
+#pragma unroll
+          for (int d = 0; d < DIM; ++d)
+#pragma unroll
+            for (int j = 0; j < ND; ++j) {
+              const double u = x.u_ref_inv[j] * t.dU[d][j];
+              use1 += u * u;
+            }
+        t.use1 = use1;
         double nu = 0.0;
         if (a == 1.0) nu = t.Zn * hd * (1.0 / sqrt(use1));
         else if (a == 2.0) nu = t.Zn * hd * hd / t.Un;
@@ -796,31 +836,20 @@ GV_HD void point_forward(const Ctx<DIM, NC>& x, const PGeo<DIM, NEN>& q, const d
     }
   }
   // phi0 = rv - S0 tau Res,  phi_d = F_dif,d - F_adv,d + nu dU_d + A_d tau Res
-  double wv[ND];
+  const double* wv = t.wv;
+  double Dw[ND];
+  Dy<DIM, NC>(c, wv, Dw);
 #pragma unroll
-  for (int r = 0; r < ND; ++r) {
-    double s = 0.0;
-#pragma unroll
-    for (int cc = 0; cc < ND; ++cc) s += t.tau[r][cc] * t.Res[cc];
-    wv[r] = s;
-  }
-#pragma unroll
-  for (int j = 0; j < ND; ++j) phi0[j] = (t.U[j] - t.UP[j]) / dt - t.S[j];
+  for (int j = 0; j < ND; ++j) phi0[j] = (t.U[j] - t.UP[j]) * x.inv_dt - t.S[j];
   {
     double s0w = 0.0;
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) s0w += t.m.rho * x.gravity[d] * wv[1 + d];
-    phi0[L::iT] -= s0w;
+    for (int d = 0; d < DIM; ++d) s0w += x.gravity[d] * wv[1 + d];
+    phi0[L::iT] -= t.m.rho * s0w;
   }
-  const double rho = t.m.rho, pp = c.p, E = c.E;
 #pragma unroll
   for (int d = 0; d < DIM; ++d) {
-    double aw[ND];
-    Ay<DIM, NC>(c, d, wv, aw);
     // viscous stress row d
-    double div = 0.0;
-#pragma unroll
-    for (int k = 0; k < DIM; ++k) div += dI[k][1 + k];
     double tsd[DIM];
 #pragma unroll
     for (int j = 0; j < DIM; ++j) tsd[j] = c.mu * (dI[d][1 + j] + dI[j][1 + d]) + (j == d ? c.lam * div : 0.0);
@@ -837,15 +866,14 @@ GV_HD void point_forward(const Ctx<DIM, NC>& x, const PGeo<DIM, NEN>& q, const d
       fd[L::iY + i] = c.rhoD[i] * dI[d][L::iY + i];
     }
     fd[L::iT] = en;
-    double fa[ND];
-    fa[0] = rho * v[d];
+    // A_d tau Res - F_adv,d = v_d (DUDY tau Res) + u' (wv_vd - v_d) + (wv_p - p) e_vd + v_d wv_p e_E
 #pragma unroll
-    for (int j = 0; j < DIM; ++j) fa[1 + j] = rho * v[d] * v[j] + (j == d ? pp : 0.0);
-    fa[L::iT] = v[d] * (rho * E + pp);
-#pragma unroll
-    for (int i = 0; i < NC - 1; ++i) fa[L::iY + i] = rho * v[d] * Y[i];
-#pragma unroll
-    for (int j = 0; j < ND; ++j) phi[d][j] = fd[j] - fa[j] + t.nu * t.dU[d][j] + aw[j];
+    for (int j = 0; j < ND; ++j) {
+      const double up = t.U[j] + (j == L::iT ? p : 0.0);
+      phi[d][j] = fd[j] + t.nu * t.dU[d][j] + v[d] * Dw[j] + up * (wv[1 + d] - v[d]);
+    }
+    phi[d][1 + d] += wv[0] - p;
+    phi[d][L::iT] += v[d] * wv[0];
   }
 }
 
@@ -870,60 +898,37 @@ GV_HD void point_reverse(const Ctx<DIM, NC>& x, const PGeo<DIM, NEN>& q, const d
   for (int d = 0; d < DIM; ++d)
 #pragma unroll
     for (int j = 0; j < ND; ++j) dUb[d][j] = 0.0;
-  // tau Res again
-  double wv[ND];
-#pragma unroll
-  for (int r = 0; r < ND; ++r) {
-    double s = 0.0;
-#pragma unroll
-    for (int cc = 0; cc < ND; ++cc) s += t.tau[r][cc] * t.Res[cc];
-    wv[r] = s;
-  }
+  const double* wv = t.wv;
+  double Dw[ND];
+  Dy<DIM, NC>(c, wv, Dw);
   // ---- phi_d
   double div = 0.0;
 #pragma unroll
   for (int k = 0; k < DIM; ++k) div += dI[k][1 + k];
-  double divb = 0.0;
+  double divb = 0.0, xs[ND], wu[ND];
+#pragma unroll
+  for (int j = 0; j < ND; ++j) xs[j] = wu[j] = 0.0;
 #pragma unroll
   for (int d = 0; d < DIM; ++d) {
     const double* pb = phib[d];
-    // A_d wv
-    double at[ND];
-    ATx<DIM, NC>(c, d, pb, at);
-#pragma unroll
-    for (int j = 0; j < ND; ++j) wvb[j] += at[j];
-    xAy_rev<DIM, NC>(c, d, pb, wv, 1.0, b);
-    // nu dU_d
-    double du = 0.0;
+    // A_d wv - F_adv,d = v_d DUDY wv + u' (wv_vd - v_d) + (wv_p - p) e_vd + v_d wv_p e_E
+    const double vd = c.v[d], tt = wv[1 + d] - vd;
+    const double pw = xw_of<DIM, NC>(c, pb), pu = rho * pw + c.p * pb[L::iT];
+    double pDw = 0.0, du = 0.0;
 #pragma unroll
     for (int j = 0; j < ND; ++j) {
+      pDw += pb[j] * Dw[j];
+      xs[j] += vd * pb[j];
+      wu[j] += tt * pb[j];
       du += pb[j] * t.dU[d][j];
-      dUb[d][j] += t.nu * pb[j];
+      dUb[d][j] = t.nu * pb[j];
     }
     nub += du;
-    // - F_adv,d
-    const double vd = c.v[d];
-    b.rho -= pb[0] * vd;
-    b.v[d] -= pb[0] * rho;
-#pragma unroll
-    for (int j = 0; j < DIM; ++j) {
-      // rho v_d v_j + p d_jd
-      b.rho -= pb[1 + j] * vd * c.v[j];
-      b.v[d] -= pb[1 + j] * rho * c.v[j];
-      b.v[j] -= pb[1 + j] * rho * vd;
-      if (j == d) b.p -= pb[1 + j];
-    }
-    // v_d (rho E + p)
-    b.v[d] -= pb[L::iT] * (rho * c.E + c.p);
-    b.rho -= pb[L::iT] * vd * c.E;
-    b.E -= pb[L::iT] * vd * rho;
-    b.p -= pb[L::iT] * vd;
-#pragma unroll
-    for (int i = 0; i < NC - 1; ++i) {
-      b.rho -= pb[L::iY + i] * vd * c.Y[i];
-      b.v[d] -= pb[L::iY + i] * rho * c.Y[i];
-      b.Y[i] -= pb[L::iY + i] * rho * vd;
-    }
+    wvb[1 + d] += pu;
+    wvb[0] += pb[1 + d] + vd * pb[L::iT];
+    b.v[d] += pDw + pb[L::iT] * wv[0] - pu;
+    b.rho += tt * pw;
+    b.p += tt * pb[L::iT] - pb[1 + d];
     // F_dif,d: momentum rows tau_dj, energy row v.tau_d + kappa dT + sum rhoDH dY, species rhoD dY
     double tsd[DIM];
 #pragma unroll
@@ -952,12 +957,22 @@ GV_HD void point_reverse(const Ctx<DIM, NC>& x, const PGeo<DIM, NEN>& q, const d
   }
 #pragma unroll
   for (int k = 0; k < DIM; ++k) dIb[k][1 + k] += divb;
+  {
+    double at[ND];
+    DTx<DIM, NC>(c, xs, at);
+#pragma unroll
+    for (int j = 0; j < ND; ++j) {
+      wvb[j] += at[j];
+      if (j > 0) b.w[j] += rho * wu[j];
+    }
+    xDy_rev<DIM, NC>(c, xs, wv, 1.0, b);
+  }
   // ---- phi0 = (U - U_P)/dt - S - S0 wv
   double UPb[ND];
 #pragma unroll
   for (int j = 0; j < ND; ++j) {
-    Ub[j] += phi0b[j] / dt;
-    UPb[j] = -phi0b[j] / dt;
+    Ub[j] += phi0b[j] * x.inv_dt;
+    UPb[j] = -phi0b[j] * x.inv_dt;
     Sb[j] -= phi0b[j];
   }
 #pragma unroll
@@ -992,23 +1007,27 @@ GV_HD void point_reverse(const Ctx<DIM, NC>& x, const PGeo<DIM, NEN>& q, const d
     }
     // Zn = |Z|, Z = u_ref_inv (AdI - S)
     if (t.Zn > 0.0) {
+      const double zf = Znb / t.Zn;
 #pragma unroll
       for (int j = 0; j < ND; ++j) {
-        const double g = Znb * t.Z[j] / t.Zn * x.u_ref_inv[j];
+        const double zj = zf * t.Z[j], g = zj * x.u_ref_inv[j];
         AdIb[j] += g;
         Sb[j] -= g;
-        if (urib) urib[j] += Znb * t.Z[j] / t.Zn * (t.AdI[j] - t.S[j]);
+        if (urib) urib[j] += zj * (t.AdI[j] - t.S[j]);
       }
     }
     // Un = |u_ref_inv U|
     if (t.Un > 0.0) {
+      const double uf = Unb / t.Un;
 #pragma unroll
       for (int j = 0; j < ND; ++j) {
-        Ub[j] += Unb * x.u_ref_inv[j] * x.u_ref_inv[j] * t.U[j] / t.Un;
-        if (urib) urib[j] += Unb * x.u_ref_inv[j] * t.U[j] * t.U[j] / t.Un;
+        const double uj = uf * x.u_ref_inv[j] * t.U[j];
+        Ub[j] += uj * x.u_ref_inv[j];
+        if (urib) urib[j] += uj * t.U[j];
       }
     }
     // use1 = sum_d |u_ref_inv dU_d|^2
+    if (use1b != 0.0)
 #pragma unroll
     for (int d = 0; d < DIM; ++d)
 #pragma unroll
@@ -1026,18 +1045,12 @@ GV_HD void point_reverse(const Ctx<DIM, NC>& x, const PGeo<DIM, NEN>& q, const d
       for (int i = 0; i < NEN; ++i) sum += t.sg[i] * q.ds[d][i];
       Jb[d] = sJb * sum;
     }
-    const double pr = dot<DIM>(Jb, t.Jv);
+    const double pr = dot<DIM>(Jb, t.Jv), ign = 1.0 / t.gn;
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) dUb[d][0] += (Jb[d] - pr * t.Jv[d]) / t.gn;
+    for (int d = 0; d < DIM; ++d) dUb[d][0] += (Jb[d] - pr * t.Jv[d]) * ign;
   }
-  // ---- tau: the loss term wv . wvb with wv = tau Res
-#pragma unroll
-  for (int cc = 0; cc < ND; ++cc) {
-    double sum = 0.0;
-#pragma unroll
-    for (int r = 0; r < ND; ++r) sum += t.tau[r][cc] * wvb[r];
-    Resb[cc] += sum;
-  }
+  // ---- tau: the loss term wv . wvb with wv = tau Res, tau = DUDY^{-1} diag(td) but for row p
+  // at low Mach numbers
   double vb_h[DIM], dvb[DIM][DIM];
 #pragma unroll
   for (int a = 0; a < DIM; ++a) {
@@ -1047,91 +1060,69 @@ GV_HD void point_reverse(const Ctx<DIM, NC>& x, const PGeo<DIM, NEN>& q, const d
   }
   double cvb_tau = 0.0, csb_tau = 0.0;
   if (t.tau_on) {
-    double taub[ND][ND];
+    // With X = DUDY^{-1}, y = diag(td) Res and pX = X^T wvb, the loss pX . (DUDY dX y) has the
+    // cotangents diag(td) pX of Res, diag(Res) pX of td and -pX (X y)^T of DUDY
+    double wl[ND], pX[ND], tdb[ND], qX[ND];
 #pragma unroll
-    for (int r = 0; r < ND; ++r)
+    for (int j = 0; j < ND; ++j) {
+      wl[j] = (j == 0 && t.lowm) ? 0.0 : wvb[j];
+      qX[j] = j == 0 ? t.xy0 : wv[j];
+    }
+    inv_tmul<DIM, NC>(c, t.X, wl, pX);
 #pragma unroll
-      for (int cc = 0; cc < ND; ++cc) taub[r][cc] = wvb[r] * t.Res[cc];
+    for (int j = 0; j < ND; ++j) {
+      tdb[j] = t.Res[j] * pX[j];
+      Resb[j] += t.td[j] * pX[j];
+    }
+    xDy_rev<DIM, NC>(c, pX, qX, -1.0, b);
     if (t.lowm) {
-      // tau00 = 1/(1/a + 1/B) with B = rho tau11 trG; row 0 off-diagonals set to zero
-      const double t00 = t.tau[0][0];
-      const double ab = taub[0][0] * (t00 / t.tpre00) * (t00 / t.tpre00);
-      const double Bb = taub[0][0] * (t00 / t.Bm) * (t00 / t.Bm);
-      taub[0][0] = ab;
+      // tau00 = 1/(1/a + 1/B), a = X00 td_0, B = rho (td_1/rho) trG
+      Resb[0] += t.t00 * wvb[0];
+      const double tb = wvb[0] * t.Res[0], fa = t.t00 / t.tpre00, fB = t.t00 / t.Bm;
+      const double ab = tb * fa * fa, Bb = tb * fB * fB;
+      tdb[0] += ab * t.X.x0[0];
+      tdb[1] += Bb * q.trG;
+      const double al = ab * t.td[0];
+      double px[ND], qx[ND];
 #pragma unroll
-      for (int cc = 1; cc < ND; ++cc) taub[0][cc] = 0.0;
-      taub[1][1] += Bb * rho * q.trG;
-      b.rho += Bb * t.tpre11 * q.trG;
-    }
-    // tau = X diag(td)
-    double Xb[ND][ND], tdb[ND];
-#pragma unroll
-    for (int cc = 0; cc < ND; ++cc) {
-      tdb[cc] = 0.0;
-#pragma unroll
-      for (int r = 0; r < ND; ++r) {
-        Xb[r][cc] = taub[r][cc] * t.td[cc];
-        tdb[cc] += taub[r][cc] * t.X[r][cc];
+      for (int j = 0; j < ND; ++j) {
+        px[j] = al * t.X.x0[j];
+        qx[j] = j == 0 ? t.X.x0[0] : (j == L::iT ? t.X.xT[0] : -c.w[j] * t.m.irho);
       }
-    }
-    // X = DUDY^{-1}: DUDY-bar = -X^T Xb X^T, folded into the coefficient cotangents
-    // entry by entry through e_r^T DUDY e_c
-    double T1[ND][ND];
-#pragma unroll
-    for (int r = 0; r < ND; ++r)
-#pragma unroll
-      for (int cc = 0; cc < ND; ++cc) {
-        double sum = 0.0;
-#pragma unroll
-        for (int k = 0; k < ND; ++k) sum += t.X[k][r] * Xb[k][cc];
-        T1[r][cc] = sum;
-      }
-#pragma unroll
-    for (int r = 0; r < ND; ++r) {
-      double Dbr[ND];
-#pragma unroll
-      for (int cc = 0; cc < ND; ++cc) {
-        double sum = 0.0;
-#pragma unroll
-        for (int k = 0; k < ND; ++k) sum += T1[r][k] * t.X[cc][k];
-        Dbr[cc] = -sum;
-      }
-      double er[ND];
-#pragma unroll
-      for (int k = 0; k < ND; ++k) er[k] = (k == r) ? 1.0 : 0.0;
-      xDy_rev<DIM, NC>(c, er, Dbr, 1.0, b);
+      xDy_rev<DIM, NC>(c, px, qx, -1.0, b);
     }
     // td_0 = use, td_j = min(use, cap_j)
     const double h = t.h, vn = t.vn, cs = t.m.c;
-    double useb = tdb[0], hb = 0.0;
+    double useb = tdb[0], hb = 0.0, hs = 0.0, gv_ = 0.0, gT = 0.0;
 #pragma unroll
     for (int j = 1; j < ND; ++j) {
       if (!t.td_branch[j]) {
         useb += tdb[j];
         continue;
       }
+      // td_j is its cap: h^2 rho/(12 mu), h^2 rho cv/(12 kappa), h^2/(12 D)
+      const double g = tdb[j] * t.td[j];
+      hs += g;
       if (j < L::iT) {
-        const double cap = h * h * rho / (12.0 * t.m.mu);   // h^2 rho/(12 mu)
-        hb += tdb[j] * 2.0 * cap / h;
-        b.rho += tdb[j] * cap / rho;
-        b.mu -= tdb[j] * cap / t.m.mu;
+        gv_ += g;
       } else if (j == L::iT) {
-        const double cap = h * h * rho * t.m.cv / (12.0 * t.m.kappa);
-        hb += tdb[j] * 2.0 * cap / h;
-        b.rho += tdb[j] * cap / rho;
-        cvb_tau += tdb[j] * cap / t.m.cv;
-        b.kappa -= tdb[j] * cap / t.m.kappa;
-      } else {
-        const double cap = h * h / (12.0 * x.ch[j - L::iY].D);
-        hb += tdb[j] * 2.0 * cap / h;
+        gT += g;
       }
     }
+    if (hs != 0.0) hb += 2.0 * hs / h;
+    if (gv_ != 0.0) b.mu -= gv_ / t.m.mu;
+    if (gT != 0.0) {
+      cvb_tau += gT / t.m.cv;
+      b.kappa -= gT / t.m.kappa;
+    }
+    b.rho += (gv_ + gT) * t.m.irho;
     double vnb = 0.0;
     if (t.use_branch) {
       // use = h/(2(vn + c)) + h/(2 vn)
-      hb += useb * (1.0 / (2.0 * (vn + cs)) + 1.0 / (2.0 * vn));
-      vnb += useb * (-h / (2.0 * (vn + cs) * (vn + cs)) - h / (2.0 * vn * vn));
-      csb_tau += useb * (-h / (2.0 * (vn + cs) * (vn + cs)));
+      const double i1 = 0.5 / (vn + cs), i2 = 0.5 / vn;
+      hb += useb * (i1 + i2);
+      csb_tau -= useb * h * 2.0 * i1 * i1;
+      vnb -= useb * h * 2.0 * (i1 * i1 + i2 * i2);
     }
     double dv[DIM][DIM];
 #pragma unroll
@@ -1139,8 +1130,9 @@ GV_HD void point_reverse(const Ctx<DIM, NC>& x, const PGeo<DIM, NEN>& q, const d
 #pragma unroll
       for (int d = 0; d < DIM; ++d) dv[a][d] = dI[d][1 + a];
     compute_h_rev<DIM>(q.G, c.v, dv, t.ht, hb, vb_h, dvb);
+    vnb /= vn;
 #pragma unroll
-    for (int k = 0; k < DIM; ++k) vb_h[k] += vnb * c.v[k] / vn;
+    for (int k = 0; k < DIM; ++k) vb_h[k] += vnb * c.v[k];
 #pragma unroll
     for (int a = 0; a < DIM; ++a)
 #pragma unroll
@@ -1157,24 +1149,29 @@ GV_HD void point_reverse(const Ctx<DIM, NC>& x, const PGeo<DIM, NEN>& q, const d
     double ddb[ND];
     DTx<DIM, NC>(c, Resb, ddb);
 #pragma unroll
-    for (int j = 0; j < ND; ++j) Ib[j] += ddb[j] / dt;
+    for (int j = 0; j < ND; ++j) Ib[j] += ddb[j] * x.inv_dt;
   }
+  // sum_d A_d dI_d and dU_d = DUDY dI_d: the cotangent of DUDY dI_d is dUb_d + v_d AdIb
+  const double aw = xw_of<DIM, NC>(c, AdIb), au = rho * aw + c.p * AdIb[L::iT];
+  b.rho += div * aw;
+  b.p += div * AdIb[L::iT];
+#pragma unroll
+  for (int j = 1; j < ND; ++j) b.w[j] += div * rho * AdIb[j];
 #pragma unroll
   for (int d = 0; d < DIM; ++d) {
-    xAy_rev<DIM, NC>(c, d, AdIb, dI[d], 1.0, b);
-    double at[ND];
-    ATx<DIM, NC>(c, d, AdIb, at);
+    double xd[ND], at[ND], s = AdIb[L::iT] * dI[d][0];
+#pragma unroll
+    for (int j = 0; j < ND; ++j) {
+      xd[j] = dUb[d][j] + c.v[d] * AdIb[j];
+      s += AdIb[j] * t.dU[d][j];
+    }
+    b.v[d] += s;
+    xDy_rev<DIM, NC>(c, xd, dI[d], 1.0, b);
+    DTx<DIM, NC>(c, xd, at);
 #pragma unroll
     for (int j = 0; j < ND; ++j) dIb[d][j] += at[j];
-  }
-  // dU_d = DUDY dI_d
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) {
-    xDy_rev<DIM, NC>(c, dUb[d], dI[d], 1.0, b);
-    double at[ND];
-    DTx<DIM, NC>(c, dUb[d], at);
-#pragma unroll
-    for (int j = 0; j < ND; ++j) dIb[d][j] += at[j];
+    dIb[d][1 + d] += au;
+    dIb[d][0] += AdIb[1 + d] + c.v[d] * AdIb[L::iT];
   }
   // S = (0, rho g, rho g.v, 0)
   {
@@ -1196,29 +1193,22 @@ GV_HD void point_reverse(const Ctx<DIM, NC>& x, const PGeo<DIM, NEN>& q, const d
   cfbar_fold<DIM, NC>(b);
   // ---- coefficients -> mixture -> state and parameters
   MixBar o;
-  double rcb[NC], cvcb[NC], pb = 0.0, Tb = 0.0, vb[DIM], Yb[NC];
+  double irb[NC], cvcb[NC], pb = 0.0, Tb = 0.0, vb[DIM], Yb[NC];
 #pragma unroll
   for (int k = 0; k < DIM; ++k) vb[k] = vb_h[k];
 #pragma unroll
   for (int i = 0; i < NC; ++i) Yb[i] = 0.0;
-  coef_reverse<DIM, NC>(t.m, x.ch, c, b, o, rcb, cvcb, pb, vb, Tb, Yb);
+  coef_reverse<DIM, NC>(t.m, x.ch, c, b, o, irb, cvcb, pb, vb, Tb, Yb);
   o.cv += cvb_tau;
   o.c += csb_tau;
-  mix_reverse<NC>(x.ch, c.p, c.T, t.m, o, rcb, cvcb, pb, Tb, Yb, th);
+  mix_reverse<NC>(x.ch, t.kc, c.T, t.m, o, irb, cvcb, pb, Tb, Yb, th);
   // U_P = rho_P (1, v_P, E_P, Y_P): parameters only
   {
-    MixBar oP{0, 0, 0, 0, 0, 0, 0, 0};
-    double wP[ND];
+    double rPb = 0.0;
 #pragma unroll
     for (int j = 0; j < ND; ++j)
-      wP[j] = (j == 0) ? 1.0 : (j < L::iT ? t.vP[j - 1] : (j == L::iT ? t.EP : t.mP.Y[j - L::iY]));
-#pragma unroll
-    for (int j = 0; j < ND; ++j) oP.rho += UPb[j] * wP[j];
-    oP.cv += UPb[L::iT] * t.mP.rho * t.TP;
-    double pPb = 0.0, TPb = 0.0, YPb[NC];
-#pragma unroll
-    for (int i = 0; i < NC; ++i) YPb[i] = 0.0;
-    mix_reverse<NC>(x.ch, Pq[0], t.TP, t.mP, oP, nullptr, nullptr, pPb, TPb, YPb, th);
+      rPb += UPb[j] * (j == 0 ? 1.0 : (j < L::iT ? t.vP[j - 1] : (j == L::iT ? t.EP : t.mP.Y[j - L::iY])));
+    mixp_reverse<NC>(x.ch, t.kc, t.TP, t.mP, rPb, UPb[L::iT] * t.mP.rho * t.TP, th);
   }
   // state cotangents: p, v, T, Y_i (Y_nc = 1 - sum Y_i)
   Ib[0] += pb;
@@ -1235,6 +1225,7 @@ GV_HD void point_reverse(const Ctx<DIM, NC>& x, const PGeo<DIM, NEN>& q, const d
 template <int DIM, int NC>
 struct BTape {
   using L = Layout<DIM, NC>;
+  CompK kc[NC];
   Mix<NC> m;
   Cf<DIM, NC> c;
   double ts[DIM][DIM], qf[DIM], Jf[DIM][L::NYA], div;
@@ -1253,7 +1244,9 @@ GV_HD void bpoint_forward(const Ctx<DIM, NC>& x, const gales_side_bc& bc, const 
 #pragma unroll
   for (int i = 0; i < NC - 1; ++i) { Y[i] = Iq[L::iY + i]; sY += Y[i]; }
   Y[NC - 1] = 1.0 - sY;
-  mix_forward<NC>(x.ch, p, T, Y, t.m);
+#pragma unroll
+  for (int i = 0; i < NC; ++i) comp_const(x.ch[i], t.kc[i]);
+  mix_forward<NC>(x.ch, t.kc, p, T, Y, t.m);
   coef_forward<DIM, NC>(t.m, x.ch, p, v, T, t.c);
   const Cf<DIM, NC>& c = t.c;
   const double rho = t.m.rho;
@@ -1422,21 +1415,21 @@ GV_HD void bpoint_reverse(const Ctx<DIM, NC>& x, const gales_side_bc& bc, const 
     }
   cfbar_fold<DIM, NC>(b);
   MixBar o;
-  double rcb[NC], cvcb[NC], pb = 0.0, Tb = 0.0, vb[DIM], Yb[NC];
+  double irb[NC], cvcb[NC], pb = 0.0, Tb = 0.0, vb[DIM], Yb[NC];
 #pragma unroll
   for (int k = 0; k < DIM; ++k) vb[k] = 0.0;
 #pragma unroll
   for (int i = 0; i < NC; ++i) Yb[i] = 0.0;
-  coef_reverse<DIM, NC>(t.m, x.ch, c, b, o, rcb, cvcb, pb, vb, Tb, Yb);
+  coef_reverse<DIM, NC>(t.m, x.ch, c, b, o, irb, cvcb, pb, vb, Tb, Yb);
   // H_i = cv_i T + p/rho_i
 #pragma unroll
   for (int i = 0; i < NC - 1; ++i) {
     cvcb[i] += Hb[i] * c.T;
     Tb += Hb[i] * t.m.cvc[i];
-    pb += Hb[i] / t.m.r[i];
-    rcb[i] -= Hb[i] * c.p / (t.m.r[i] * t.m.r[i]);
+    pb += Hb[i] * t.m.ir[i];
+    irb[i] += Hb[i] * c.p;
   }
-  mix_reverse<NC>(x.ch, c.p, c.T, t.m, o, rcb, cvcb, pb, Tb, Yb, th);
+  mix_reverse<NC>(x.ch, t.kc, c.T, t.m, o, irb, cvcb, pb, Tb, Yb, th);
   Ib[0] += pb;
 #pragma unroll
   for (int k = 0; k < DIM; ++k) Ib[1 + k] += vb[k];

@@ -11,6 +11,11 @@
 // Rows under a Dirichlet constraint are zero in the rhs whatever the state
 // (scatter.hpp:70-78), so their lambda entries are masked out.  k.vjp_th receives the
 // parameter cotangents [3 nc] followed by the u_ref_inv cotangents [nd].
+//
+// Bound: the FP64 pipe (87% busy).  A point takes about 3,100 FP64 operations with 7 dofs (5.3
+// ms for 215,622 tets); with dense nd x nd products for the reverse of DUDY^{-1}, one product
+// per direction for the A_d, a division per component and term of the mixture and no fused
+// multiply-adds it took 11,800 (16.3 ms).
 #pragma once
 
 #include "gales_kernels.cuh"
@@ -47,17 +52,37 @@ __device__ __forceinline__ bool masked_lambda(const KParams& k, int nd_, double*
   return any;
 }
 
-// Warp sums of per-thread cotangents added to k.vjp_th[off + i].
+// Warp sums of NP per-thread cotangents added to k.vjp_th[i].  The lanes halve the values
+// among them step by step (16 values: 16 additions a lane, against 80 for sixteen butterflies).
 template <int NP>
-__device__ __forceinline__ void reduce_params(const KParams& k, const double (&th)[NP], int off) {
+__device__ __forceinline__ void reduce_params(const KParams& k, const double (&th)[NP]) {
   if (!k.vjp_th) return;
+  constexpr int P = NP <= 4 ? 4 : (NP <= 8 ? 8 : (NP <= 16 ? 16 : 32));
+  static_assert(NP <= 32, "one value per lane at most");
+  const int lane = threadIdx.x & 31;
+  double x[P];
 #pragma unroll
-  for (int i = 0; i < NP; ++i) {
-    double x = th[i];
+  for (int i = 0; i < P; ++i) x[i] = i < NP ? th[i < NP ? i : 0] : 0.0;
+  int at = 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if ((threadIdx.x & 31) == 0 && x != 0.0) atomicAdd(k.vjp_th + off + i, x);
+  for (int s = 0; s < 5; ++s) {
+    const int o = 16 >> s, half = P >> (s + 1);
+    if (half > 0) {
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < P / 2; ++i) {
+        if (i >= half) break;
+        const double send = up ? x[i] : x[i + half], keep = up ? x[i + half] : x[i];
+        x[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+      if (up) at += half;
+    } else {
+      x[0] += __shfl_xor_sync(0xffffffffu, x[0], o);
+    }
   }
+  // lanes that differ in the low bits alone hold the same sum
+  const bool first = (lane & (32 / P - 1)) == 0;
+  if (first && at < NP && x[0] != 0.0) atomicAdd(k.vjp_th + at, x[0]);
 }
 
 template <int DIM, int NEN, int NC, int NQ>
@@ -68,11 +93,9 @@ __global__ void __launch_bounds__(128) vjp_interior_kernel(const KParams k, long
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long li = t / NQ;
   const int iq = (int)(t % NQ);
-  double th[3 * NC], urib[ND];
+  double th[3 * NC + ND];   // parameters, then u_ref_inv
 #pragma unroll
-  for (int i = 0; i < 3 * NC; ++i) th[i] = 0.0;
-#pragma unroll
-  for (int j = 0; j < ND; ++j) urib[j] = 0.0;
+  for (int i = 0; i < 3 * NC + ND; ++i) th[i] = 0.0;
   if (li < n) {
     const long long e = k.el_list ? (long long)k.el_list[li] : li;
     int nodes[NEN];
@@ -109,13 +132,16 @@ __global__ void __launch_bounds__(128) vjp_interior_kernel(const KParams k, long
 #pragma unroll
         for (int j = 0; j < ND; ++j) {
           const double Ia = __ldg(k.I + (long long)nodes[a] * ND + j);
-          Iq[j] += sh * Ia;
-          Pq[j] += sh * __ldg(k.P + (long long)nodes[a] * ND + j);
-          L0[j] += sh * lam[a][j];
+          // the velocity and its gradient with the residual's unfused operations (compute_h's
+          // branches hang on their rounding where a velocity field is rank one)
+          const bool vel = j >= 1 && j <= DIM;
+          Iq[j] = vel ? add_rn(Iq[j], mul_rn(sh, Ia)) : fma(sh, Ia, Iq[j]);
+          Pq[j] = fma(sh, __ldg(k.P + (long long)nodes[a] * ND + j), Pq[j]);
+          L0[j] = fma(sh, lam[a][j], L0[j]);
 #pragma unroll
           for (int d = 0; d < DIM; ++d) {
-            dI[d][j] += g.ds[d][a] * Ia;
-            Ld[d][j] += g.ds[d][a] * lam[a][j];
+            dI[d][j] = vel ? add_rn(dI[d][j], mul_rn(g.ds[d][a], Ia)) : fma(g.ds[d][a], Ia, dI[d][j]);
+            Ld[d][j] = fma(g.ds[d][a], lam[a][j], Ld[d][j]);
           }
         }
       }
@@ -137,7 +163,7 @@ __global__ void __launch_bounds__(128) vjp_interior_kernel(const KParams k, long
 #pragma unroll
         for (int d = 0; d < DIM; ++d) dIb[d][j] = 0.0;
       }
-      vjp::point_reverse<DIM, NEN, NC>(x, pg, Iq, dI, Pq, tp, L0, Ld, Ib, dIb, th, urib);
+      vjp::point_reverse<DIM, NEN, NC>(x, pg, Iq, dI, Pq, tp, L0, Ld, Ib, dIb, th, th + 3 * NC);
 #pragma unroll
       for (int a = 0; a < NEN; ++a) {
         const double sh = k.sh_tab[iq][a];
@@ -151,8 +177,7 @@ __global__ void __launch_bounds__(128) vjp_interior_kernel(const KParams k, long
       }
     }
   }
-  reduce_params<3 * NC>(k, th, 0);
-  reduce_params<ND>(k, urib, 3 * NC);
+  reduce_params<3 * NC + ND>(k, th);
 }
 
 template <int DIM, int NEN, int NC, int NS, int NSQ>
@@ -228,7 +253,7 @@ __global__ void __launch_bounds__(128) vjp_boundary_kernel(const KParams k) {
         }
     }
   }
-  reduce_params<3 * NC>(k, th, 0);
+  reduce_params<3 * NC>(k, th);
 }
 
 // Launchers for one element type.
