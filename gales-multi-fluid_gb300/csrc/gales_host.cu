@@ -149,7 +149,7 @@ constexpr int kVjpAux = 3 * GALES_MAX_COMP + GALES_MAX_ND;
 // Chunks of the interior pass.  On this GPU an FP64 instruction occupies the FMA
 // pipe that the FP32 instructions issue to, so the FP64-bound point stage and the
 // FP32 matrix stage gain nothing from sharing an SM: each chunk runs the point kernel
-// over all its elements, then the persistent matrix kernel, on the caller's stream.
+// over all its elements, then the matrix kernel, on the caller's stream.
 // Chunks are as large as kRecordBytes of point records allow (the whole mesh for the
 // 1.0M-tet workload), so that few launch tails remain; the records go through DRAM,
 // which the compute-bound stages leave mostly idle.  A host-buffer call cuts the pass

@@ -303,23 +303,37 @@ __device__ __forceinline__ void geometry(const double (&X)[NEN][DIM], const doub
 // offset u = node_rp(b) nd + slot(b, a), so that dof row jb of node b holds node a's
 // columns from nd u + jb rowlen on.  The matrix stage then reads everything it needs
 // from the record block.  Integers are stored as the bit patterns of S words.
+//
+// The words lie in the order in which the matrix stage needs them, so that what a dof row r
+// reads of a point is two contiguous pieces: a range from mu (from rho when only the residual
+// is formed) to the last member listed for its kind of row, and row[r].
 template <int DIM, int NEN, int NC, typename S>
 struct QP {
   using L = Layout<DIM, NC>;
   using Scalar = S;
   static constexpr int ND = L::ND;
-  S sh[NEN], ds[DIM][NEN], JxW;
-  S p, v[DIM], Y[NC], rho, E, drho_dp, drho_dT, de_dp, de_dT, mu, lambda, kappa;
-  S drho_dY[L::NYA], dE_dY[L::NYA], rhoD[L::NYA], rhoDH[L::NYA];
-  S tau[ND][ND];
-  // structure vectors of DUDY = w r0^T + rho M and their products with tau:
-  // w = (1, v, E, Y), z = r0^T tau, y = mE^T tau (mE: energy row of M), tg = g^T tau_v
-  S w[ND], z[ND], y[ND], tg[ND];
+  static constexpr bool AFF = NEN == DIM + 1;
+  static constexpr int RP = DIM + 3;
+  // every row of the matrix
+  S mu, lambda, kappa, rhoD[L::NYA], rhoDH[L::NYA];
+  S drho_dp, drho_dT, de_dp, de_dT, drho_dY[L::NYA], dE_dY[L::NYA];
   S nu;             // dc_scale_fact * nu_shoc (0 when dc is off or inactive)
-  S rv[ND];         // coefficient of N_b:    (U - U_P)/dt - S
-  S rf[DIM][ND];    // coefficient of dN_b/dx_k:  F_dif,k - F_adv,k + shock dI/dx_k
+  // every row.  DUDY = w r0^T + rho M with w = (1, v, E, Y); z = r0^T tau; tau rows v_d have
+  // entries in column p and on the diagonal
+  S rho, p, JxW, v[DIM], E, Y[L::NYA], z[ND], tvp[DIM], tvd[DIM];
   S res[ND];        // least-squares residual Res (fluid_2d.hpp:282)
-  S d_node, d_rowlen, d_blocked, d_off[NEN];  // scatter descriptor of node b = q (see above)
+  S ds[AFF ? 1 : DIM * NEN];
+  // velocity rows
+  S tau0[ND];       // tau row p
+  // energy row: y = mE^T tau (mE: energy row of M), tg = g^T tau_v
+  S y[ND], tg[L::iT];
+  // row r: coefficient of N_b, (U - U_P)/dt - S; of dN_b/dx_k, F_dif,k - F_adv,k + shock
+  // dI/dx_k; mass fractions: tau's column p and diagonal
+  S row[ND * RP];
+  // not staged: shape gradients of a simplex (point 0), scatter descriptor of node b = q (see
+  // above)
+  S dse[AFF ? DIM * NEN : 1];
+  S d_node, d_rowlen, d_blocked, d_off[NEN];
 };
 
 __device__ __forceinline__ float int_word(float, int32_t v) { return __int_as_float(v); }
@@ -327,55 +341,28 @@ __device__ __forceinline__ double int_word(double, int32_t v) { return __longlon
 __device__ __forceinline__ int32_t word_int(float w) { return __float_as_int(w); }
 __device__ __forceinline__ int32_t word_int(double w) { return (int32_t)__double_as_longlong(w); }
 
-// Lane layout of the matrix stage (see matrix_kernel); the point stage lays its
-// records out in the matrix CTAs' blocks.
+// Point records are stored in blocks of EB = 32 elements, word-major with the element
+// innermost: word f of point q of element l is at [(q RW + f) EB + l], so that a point's words
+// are one piece of memory (the matrix stage's bulk copies) and a word of a matrix warp, a lane
+// per element, is 128 contiguous bytes; a warp of the point stage stores each word as runs of
+// 32 / NQ elements.  After the points a block holds the element rows' shares of the trace
+// (doubles [ND NEN][EB]).
 template <int DIM, int NEN, int NC>
-struct MatShape {
-  static constexpr int ND = Layout<DIM, NC>::ND;
-  static constexpr int N = NEN * ND;                  // rows (and columns) of the block
-  static constexpr int AG = NEN >= 8 ? 2 : 1;          // trial-node groups per row
-  static constexpr int NA = NEN / AG;                  // trial nodes per lane
-  static constexpr int LANES = N * AG;
-  static constexpr int WPE = (LANES + 31) / 32;        // warps per element
-  static constexpr int EPC = WPE == 1 ? 4 : (WPE == 2 ? 2 : 1);  // elements per CTA
-  static constexpr int ET = WPE * 32;                  // threads per element
-  static constexpr int CTA = EPC * ET;
-  static constexpr int NS = N + 1;                     // stage row stride (doubles)
-  static constexpr bool AFFINE = NEN == DIM + 1;
-};
-
-// Point records are stored in blocks of BP = (elements per matrix CTA) x NQ points, the
-// points one matrix CTA group reads, word-major inside a block: word f of point p is at
-// [f * BPS + p] with the odd stride BPS = BP + 1, so that the lanes of a matrix warp
-// reading word f + i * nd of one point (the rows of tau) hit distinct banks.  A block
-// is padded to a whole number of 16-byte units and is copied to shared memory as it
-// lies (one bulk copy).  A warp of the point stage stores each word for its 32
-// consecutive points as runs of BP contiguous words.
-template <int DIM, int NEN, int NC, int NQ, typename S>
 struct RecBlock {
-  using QPT = QP<DIM, NEN, NC, S>;
-  static constexpr int EPC = MatShape<DIM, NEN, NC>::EPC;
-  static constexpr int BP = EPC * NQ;
-  static constexpr int BPS = BP + 1;
-  static constexpr int RW = (int)(sizeof(QPT) / sizeof(S));   // words per record
-  static constexpr int V = (int)(16 / sizeof(S));
-  static constexpr int WORDS = (RW * BPS + V - 1) / V * V;    // words per block
-  static constexpr size_t BYTES = (size_t)WORDS * sizeof(S);
-  static_assert(sizeof(QPT) % sizeof(S) == 0, "a record is a whole number of words");
+  using QPT = QP<DIM, NEN, NC, float>;
+  static constexpr int EB = 32, NQ = NEN, ND = Layout<DIM, NC>::ND;
+  static constexpr int RW = (int)(sizeof(QPT) / sizeof(float));   // words per record
+  static constexpr size_t TR_OFF = (size_t)NQ * RW * EB * sizeof(float);
+  static constexpr size_t BYTES = TR_OFF + (size_t)ND * NEN * EB * sizeof(double);
+  static_assert(sizeof(QPT) % sizeof(float) == 0, "a record is a whole number of words");
 };
 
-// One point's words in a block being written (point stage) or read (matrix stage).
-template <typename QPT, int BPS>
+// One point's words in a block being written (point stage); p: word 0 of the point.
+template <typename QPT, int EB>
 struct RecOut {
   using S = typename QPT::Scalar;
-  S* __restrict__ blk;
-  int p;
-  __device__ __forceinline__ S& at(size_t off) const { return blk[(off / sizeof(S)) * BPS + p]; }
-};
-template <typename S, int BPS>
-struct RecIn {
-  const S* b;  // word 0 of the point
-  __device__ __forceinline__ S operator[](int f) const { return b[f * BPS]; }
+  S* __restrict__ p;
+  __device__ __forceinline__ S& at(size_t off) const { return p[(off / sizeof(S)) * EB]; }
 };
 #define GALES_REC(m) out.at(offsetof(QPT, m))
 #define GALES_RECA(m, i) out.at(offsetof(QPT, m) + (size_t)(i) * sizeof(S))
@@ -461,8 +448,8 @@ __device__ __noinline__ double compute_h_reference(const double* __restrict__ I,
 // Point phase for one (element, quadrature point).
 // FP64 for the mixture EOS and its derivatives, U - U_P, the element size h and tau with the
 // closed-form DUDY inverse; the fluxes, least-squares residual and dc viscosity in FP32.
-template <int DIM, int NEN, int NC, int NQ, typename S, int BPS, int EOS = kEosChemicals>
-__device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<QP<DIM, NEN, NC, S>, BPS>& out) {
+template <int DIM, int NEN, int NC, int NQ, typename S, int EB, int EOS = kEosChemicals>
+__device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<QP<DIM, NEN, NC, S>, EB>& out) {
   using L = Layout<DIM, NC>;
   using QPT = QP<DIM, NEN, NC, S>;
   constexpr int ND = L::ND;
@@ -674,7 +661,7 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
   SvR[L::iT] = rf * gv;
   const float idt = k.inv_dt_f;
 #pragma unroll
-  for (int j = 0; j < ND; ++j) GALES_RECA(rv, j) = fmaf(narrow_rn(U[j] - UP[j]), idt, -SvR[j]);
+  for (int j = 0; j < ND; ++j) GALES_RECA(row, j * QPT::RP) = fmaf(narrow_rn(U[j] - UP[j]), idt, -SvR[j]);
   R Ur[ND];  // U in the form's type (discontinuity capturing); U[0] = rho
 #pragma unroll
   for (int j = 0; j < ND; ++j) Ur[j] = j == 0 ? cr.rho : to_s<R>(U[j]);
@@ -795,7 +782,7 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
   }
   {
     // z = r0^T tau, y = mE^T tau, tg = sum_d g_d tau[v_d] from the rounded tau (what the
-    // matrix stage multiplies with), and w
+    // matrix stage multiplies with)
     R zz[ND], yy[ND], gg[ND], gR[DIM];
 #pragma unroll
     for (int d = 0; d < DIM; ++d) gR[d] = R(k.gravity_f[d]);
@@ -810,12 +797,13 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
       else { r0r = cr.drho_dY[r - L::iY]; mEr = cr.dE_dY[r - L::iY]; gr = R(0); }
 #pragma unroll
       for (int cc = 0; cc < ND; ++cc) {
-        if (!tau_nz<DIM, NC>(r, cc)) {
-          GALES_RECA(tau, (r) * ND + (cc)) = S(0);
-          continue;
-        }
+        if (!tau_nz<DIM, NC>(r, cc)) continue;
         const R t = tau[r][cc];
-        GALES_RECA(tau, (r) * ND + (cc)) = S(t);
+        if (r == 0) GALES_RECA(tau0, cc) = S(t);
+        else if (r < L::iT && cc == 0) GALES_RECA(tvp, r - 1) = S(t);
+        else if (r < L::iT && cc == r) GALES_RECA(tvd, r - 1) = S(t);
+        else if (r >= L::iY && cc == 0) GALES_RECA(row, r * QPT::RP + DIM + 1) = S(t);
+        else if (r >= L::iY && cc == r) GALES_RECA(row, r * QPT::RP + DIM + 2) = S(t);
         if (r < 1 || r >= L::iT) zz[cc] = madd(r0r, t, zz[cc]);
         yy[cc] = madd(mEr, t, yy[cc]);
         if (r >= 1 && r < L::iT) gg[cc] = madd(gr, t, gg[cc]);
@@ -825,8 +813,7 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
     for (int cc = 0; cc < ND; ++cc) {
       GALES_RECA(z, cc) = S(zz[cc]);
       GALES_RECA(y, cc) = S(yy[cc]);
-      GALES_RECA(tg, cc) = S(gg[cc]);
-      GALES_RECA(w, cc) = S(cc == 0 ? R(1) : (cc < L::iT ? cr.v[cc - 1] : (cc == L::iT ? cr.E : cr.Y[cc - L::iY])));
+      if (cc < L::iT) GALES_RECA(tg, cc) = S(gg[cc]);
     }
   }
   // fluxes, least-squares residual and dc in the form's type R
@@ -923,22 +910,27 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
 #pragma unroll
     for (int i = 0; i < NC - 1; ++i) fa[L::iY + i] = rhoR * vk * cr.Y[i];
 #pragma unroll
-    for (int j = 0; j < ND; ++j) GALES_RECA(rf, (d) * ND + (j)) = S(fd[j] - fa[j] + nu * dU[d][j]);
+    for (int j = 0; j < ND; ++j) GALES_RECA(row, j * QPT::RP + 1 + d) = S(fd[j] - fa[j] + nu * dU[d][j]);
   }
   // write the record (the mixed form takes the coefficients already rounded in cr and
   // the shape data rounded once per mesh)
-  #pragma unroll
-  for (int i = 0; i < NEN; ++i) {
-    GALES_RECA(sh, i) = S(k.sh_tab_f[iq][i]);
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) GALES_RECA(ds, (d) * NEN + (i)) = S(q.ds_f[d][i]);
+  for (int i = 0; i < NEN; ++i) {
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      if constexpr (QPT::AFF) {
+        if (iq == 0) GALES_RECA(dse, d * NEN + i) = S(q.ds_f[d][i]);
+      } else {
+        GALES_RECA(ds, d * NEN + i) = S(q.ds_f[d][i]);
+      }
+    }
   }
   GALES_REC(JxW) = to_s<S>(JxW);
   GALES_REC(p) = S(cr.p);
 #pragma unroll
   for (int d = 0; d < DIM; ++d) GALES_RECA(v, d) = S(cr.v[d]);
 #pragma unroll
-  for (int i = 0; i < NC; ++i) GALES_RECA(Y, i) = S(cr.Y[i]);
+  for (int i = 0; i < NC - 1; ++i) GALES_RECA(Y, i) = S(cr.Y[i]);
   GALES_REC(rho) = S(cr.rho); GALES_REC(E) = S(cr.E);
   GALES_REC(drho_dp) = S(cr.drho_dp); GALES_REC(drho_dT) = S(cr.drho_dT);
   GALES_REC(de_dp) = S(cr.de_dp); GALES_REC(de_dT) = S(cr.de_dT);
@@ -1039,10 +1031,11 @@ __device__ __forceinline__ void point_block(const KParams& k, QP<DIM, NEN, NC, S
   const long long g = first + li;
   const long long e = k.el_list ? (long long)k.el_list[g] : g;
   using QPT = QP<DIM, NEN, NC, S>;
-  using RB = RecBlock<DIM, NEN, NC, NQ, S>;
-  const int blk = t / RB::BP;
-  const RecOut<QPT, RB::BPS> o{reinterpret_cast<S*>(out) + (size_t)blk * (size_t)RB::WORDS, t - blk * RB::BP};
-  point_phase<DIM, NEN, NC, NQ, S, RB::BPS, EOS>(k, e, iq, o);
+  using RB = RecBlock<DIM, NEN, NC>;
+  const int blk = li / RB::EB;
+  S* base = reinterpret_cast<S*>(reinterpret_cast<unsigned char*>(out) + (size_t)blk * RB::BYTES);
+  const RecOut<QPT, RB::EB> o{base + (size_t)iq * RB::RW * RB::EB + (li - blk * RB::EB)};
+  point_phase<DIM, NEN, NC, NQ, S, RB::EB, EOS>(k, e, iq, o);
 }
 
 // Resident point-stage CTAs the register budget is set for: 4 with the chemicals' EOS, 2
@@ -1079,509 +1072,6 @@ __global__ void __launch_bounds__(128, point_min_ctas<EOS>()) point_kernel(const
                                                      long long first, long long n) {
   point_block<DIM, NEN, NC, NQ, S, EOS>(k, out, first, n, (int)blockIdx.x);
   if (k.clear_n[0] > 0 || k.clear_n[1] > 0) clear_arrays(k);
-}
-
-// Interior pass, stage 2: element matrices.  Lane (b, r, g) owns row (b, r) of the
-// element block (test node b, dof r) for the trial nodes of group g, and builds it
-// per quadrature point (fluid_2d.hpp:264-331) from
-//   JxW [ FPT_b RM_a + N_a X_b ]   with
-//   WA_b  = sum_k dN_b/dx_k A_k
-//   FPT_b = (WA_b - N_b S0) tau                       least-squares weight
-//   RM_a  = N_a DUDY/dt + WA_a - N_a S0               least-squares operator
-//   X_b   = N_b (DUDY/dt - S0) - WA_b                 Galerkin mass, source, advection
-// plus the viscous/diffusive and dc terms sum_kl dN_b/dx_k K'_kl dN_a/dx_l with
-// K'_kl = K_kl + nu d_kl DUDY.
-// None of the nd x nd matrices is formed.  DUDY = w r0^T + rho M (w = (1, v, E, Y),
-// r0 its first row, M zero but for the velocity and mass-fraction diagonal and the
-// energy row mE), A_k = v_k DUDY + u' e_{v_k}^T + (e_{v_k} + v_k e_E) e_p^T with
-// u' = U + p e_E, and S0 = e_E sigma^T with sigma = rho g on the velocity columns
-// (fluid_2d.hpp:407-575).  With s_b = dN_b/dx . v these give, row r of the lane,
-//   FPT_b[r]   = s_b (w_r z + rho Mtau[r]) + u'_r t_b + kappa_br tau[0] - N_b [r=E] rho t_g
-//   (FPT_b RM_a)[r] = alpha_a (FPT_b DUDY)[r] + (FPT_b[r].u') gamma_a
-//                     + (FPT_b[r].kappa_a) e_p - N_a FPT_b[r][E] sigma
-//   X_b[r]     = beta_b DUDY[r] - u'_r gamma_b - kappa_br e_p - N_b [r=E] sigma
-// where z = r0^T tau, Mtau = M tau, t_b = sum_k dN_b/dx_k tau[v_k], t_g = sum_k g_k
-// tau[v_k], gamma_a = dN_a/dx on the velocity columns, kappa_a = dN_a/dx on the
-// velocity rows + s_a e_E, alpha_a = N_a/dt + s_a, beta_b = N_b/dt - s_b.  K'_kl is
-// applied in closed form from a few point scalars (mu, lambda, mu v, lambda v, kappa,
-// rho D_i, rho D_i H_i) and nu DUDY: per point for non-affine elements, once from
-// JxW-weighted sums for simplices (their shape gradients do not depend on the point).
-
-// Per-point vectors t_b = sum_k dN_b/dx_k tau[v_k] shared by the lanes of an element
-// (w, z, y and t_g come with the point record).
-template <int DIM, int NEN, int NC, int NQ, typename S>
-struct PointVecs {
-  static constexpr int ND = Layout<DIM, NC>::ND;
-  S tb[NQ][NEN][ND];
-};
-
-// Shared memory of one element slot of a matrix CTA: the per-point vectors t_b, the
-// element block staged for the scatter (in the form's type; widened to FP64 as it is
-// scattered), and the per-warp partial traces.
-template <int DIM, int NEN, int NC, int NQ, typename S>
-struct ElemSmem {
-  using M = MatShape<DIM, NEN, NC>;
-  PointVecs<DIM, NEN, NC, NQ, S> pv;
-  S stage[M::N * M::NS];
-  double wsum[M::WPE];
-};
-
-// Shared memory of a matrix CTA: two record blocks (the group being assembled and the
-// next one, in flight), the element slots and the two transaction barriers of the
-// blocks.  Offsets in bytes; every part 16-byte aligned.
-template <int DIM, int NEN, int NC, int NQ, typename S>
-struct MatSmem {
-  using RB = RecBlock<DIM, NEN, NC, NQ, S>;
-  using ES = ElemSmem<DIM, NEN, NC, NQ, S>;
-  static constexpr size_t ES_BYTES = (sizeof(ES) + 15) / 16 * 16;
-  static constexpr size_t OFF_ES = 2 * RB::BYTES;
-  static constexpr size_t OFF_BAR = OFF_ES + (size_t)MatShape<DIM, NEN, NC>::EPC * ES_BYTES;
-  static constexpr size_t BYTES = OFF_BAR + 16;
-};
-
-template <int WPE>
-__device__ __forceinline__ void elem_sync(int el_in_cta) {
-  if constexpr (WPE == 1) {
-    __syncwarp();
-  } else {
-    asm volatile("bar.sync %0, %1;" ::"r"(el_in_cta + 1), "r"(WPE * 32) : "memory");
-  }
-}
-
-// Point scalars entering K'_kl (JxW-weighted, summed over the points of a simplex).
-template <int DIM, int NC, typename S>
-struct KSums {
-  using L = Layout<DIM, NC>;
-  S mu, lambda, kappa, muv[DIM], lamv[DIM], rhoD[L::NYA], rhoDH[L::NYA];
-};
-
-// Adds sum_kl gb_k K_kl(r, :) ga_l to row r of one (b, a) block (the closed form of
-// the contraction; fluid_2d.hpp:531-571), branch-free in r:
-//   velocity row v_j: mu gb_m ga_j + lambda gb_j ga_m + mu (gb.ga) d_mj  on column v_m
-//   energy row      : mu v_m (gb.ga) + gb_m (ga.mu v) + ga_m (gb.lambda v) on v_m,
-//                     kappa (gb.ga) on T, rho D_i H_i (gb.ga) on Y_i
-//   mass-fraction row Y_i: rho D_i (gb.ga) on Y_i.
-template <int DIM, int NC, typename S>
-__device__ __forceinline__ void add_viscous_row(S (&acc)[Layout<DIM, NC>::ND], int r, const KSums<DIM, NC, S>& ks,
-                                                const S* gb, const S* ga) {
-  using L = Layout<DIM, NC>;
-  const bool cV = r >= 1 && r < L::iT, cE = r == L::iT;
-  S gg = gb[0] * ga[0], gamv = ga[0] * ks.muv[0], gblv = gb[0] * ks.lamv[0];
-  S gbj = S(0), gaj = S(0);
-#pragma unroll
-  for (int d = 1; d < DIM; ++d) {
-    gg = madd(gb[d], ga[d], gg);
-    gamv = madd(ga[d], ks.muv[d], gamv);
-    gblv = madd(gb[d], ks.lamv[d], gblv);
-  }
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) {
-    gbj = (r == 1 + d) ? gb[d] : gbj;
-    gaj = (r == 1 + d) ? ga[d] : gaj;
-  }
-  const S p1 = cV ? ks.mu * gaj : (cE ? gamv : S(0));
-  const S p2 = cV ? ks.lambda * gbj : (cE ? gblv : S(0));
-  const S p3 = cV ? ks.mu * gg : S(0);
-#pragma unroll
-  for (int m = 0; m < DIM; ++m) {
-    S x = madd(gb[m], p1, ga[m] * p2);
-    if (cE) x = madd(ks.muv[m], gg, x);
-    if (r == 1 + m) x += p3;
-    acc[1 + m] += x;
-  }
-  acc[L::iT] = madd(cE ? ks.kappa : S(0), gg, acc[L::iT]);
-#pragma unroll
-  for (int y = 0; y < NC - 1; ++y) {
-    const S q = cE ? ks.rhoDH[y] : ((r == L::iY + y) ? ks.rhoD[y] : S(0));
-    acc[L::iY + y] = madd(q, gg, acc[L::iY + y]);
-  }
-}
-
-// Element stage of one group of EPC elements (list positions first + li, li = grp EPC
-// + ec) from their record block blk in shared memory; the lanes of slot ec build its
-// rows.  Elements past n are skipped.
-template <int DIM, int NEN, int NC, int NQ, typename S, bool WANT_M>
-__device__ __forceinline__ void matrix_group(const KParams& k, const S* __restrict__ blk,
-                                             ElemSmem<DIM, NEN, NC, NQ, S>& E, long long first, long long n,
-                                             long long grp) {
-  using L = Layout<DIM, NC>;
-  using M = MatShape<DIM, NEN, NC>;
-  using QPT = QP<DIM, NEN, NC, S>;
-  using RB = RecBlock<DIM, NEN, NC, NQ, S>;
-  constexpr int ND = M::ND, N = M::N, NA = M::NA, NT = N * N, WPE = M::WPE, ET = M::ET, NS = M::NS;
-  constexpr int BPS = RB::BPS;
-  constexpr int iT = L::iT, iY = L::iY;
-  constexpr bool AFF = M::AFFINE;
-  const int tid = threadIdx.x;
-  const int ec = tid / ET;      // element slot in the CTA
-  const int gl = tid % ET;      // thread index within the element
-  const long long li = grp * M::EPC + ec;
-  if (li >= n) return;          // whole element groups skip together
-  const long long g = first + li;
-  const S* el = blk + ec * NQ;  // word f of point q of this element: el[f * BPS + q]
-  auto rec = [&](int q) { return RecIn<S, BPS>{el + q}; };
-  // scatter descriptor words of node b (carried by point b)
-  auto d_int = [&](int b, int f) { return word_int(el[f * BPS + b]); };
-  S grav[DIM];
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) grav[d] = S(k.gravity[d]);
-  auto& pv = E.pv;
-  // t_b per point
-  for (int t = gl; t < NQ * NEN * ND; t += ET) {
-    const int q = t / (NEN * ND), u = t % (NEN * ND), b = u / ND, col = u % ND;
-    const RecIn<S, BPS> c = rec(q);
-    S x = c[GALES_W(ds) + b] * c[GALES_W(tau) + ND + col];
-#pragma unroll
-    for (int d = 1; d < DIM; ++d) x = madd(c[GALES_W(ds) + d * NEN + b], c[GALES_W(tau) + (1 + d) * ND + col], x);
-    pv.tb[q][b][col] = x;
-  }
-  elem_sync<WPE>(ec);
-  const bool active = gl < M::LANES;
-  const int row = active ? gl % N : 0;
-  const int grp_a = active ? gl / N : 0;
-  const int b = row / ND, r = row % ND;
-  const int a0 = grp_a * NA;
-  const bool cV = r >= 1 && r < iT, cE = r == iT, cvy = r >= 1 && r != iT;
-  S acc[NA][ND];
-#pragma unroll
-  for (int i = 0; i < NA; ++i)
-#pragma unroll
-    for (int j = 0; j < ND; ++j) acc[i][j] = S(0);
-  S racc = S(0);
-  S Dnu[ND];
-  KSums<DIM, NC, S> ksum;
-  if constexpr (AFF) {
-#pragma unroll
-    for (int j = 0; j < ND; ++j) Dnu[j] = S(0);
-    ksum.mu = ksum.lambda = ksum.kappa = S(0);
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) ksum.muv[d] = ksum.lamv[d] = S(0);
-#pragma unroll
-    for (int y = 0; y < L::NYA; ++y) ksum.rhoD[y] = ksum.rhoDH[y] = S(0);
-  }
-  const S idt = S(k.inv_dt);
-  const int mrow_f = cvy ? GALES_W(tau) + r * ND : GALES_W(y);
-  for (int q = 0; q < NQ; ++q) {
-    const RecIn<S, BPS> c = rec(q);
-    const S rho = c[GALES_W(rho)], p = c[GALES_W(p)], jx = c[GALES_W(JxW)];
-    S gb[DIM], vq[DIM];
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) {
-      gb[d] = c[GALES_W(ds) + d * NEN + b];
-      vq[d] = c[GALES_W(v) + d];
-    }
-    const S Nb = c[GALES_W(sh) + b];
-    S sb = gb[0] * vq[0];
-#pragma unroll
-    for (int d = 1; d < DIM; ++d) sb = madd(gb[d], vq[d], sb);
-    const S wr = c[GALES_W(w) + r];
-    const S ur = madd(rho, wr, cE ? p : S(0));
-    S gsel = S(0);
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) gsel = (r == 1 + d) ? gb[d] : gsel;
-    const S kap = (cE ? sb : S(0)) + gsel;
-    // row r of FPT_b
-    const S cz = sb * wr, cm = (r == 0) ? S(0) : sb * rho, cg = cE ? -Nb * rho : S(0);
-    const S* tb = &pv.tb[q][b][0];
-    S F[ND];
-#pragma unroll
-    for (int j = 0; j < ND; ++j) {
-      S x = cz * c[GALES_W(z) + j];
-      x = madd(cm, c[mrow_f + j], x);
-      x = madd(ur, tb[j], x);
-      x = madd(kap, c[GALES_W(tau) + j], x);
-      F[j] = madd(cg, c[GALES_W(tg) + j], x);
-    }
-    // residual row: N_b rv + sum_k dN_b/dx_k rf_k + FPT_b Res (fluid_2d.hpp:253-262, 280-290)
-    {
-      S x = Nb * c[GALES_W(rv) + r];
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) x = madd(gb[d], c[GALES_W(rf) + d * ND + r], x);
-#pragma unroll
-      for (int j = 0; j < ND; ++j) x = madd(F[j], c[GALES_W(res) + j], x);
-      racc = madd(jx, x, racc);
-    }
-    if constexpr (WANT_M) {
-      // FPT_b DUDY, DUDY row r, and the a-independent velocity-column terms
-      S fw = F[0];
-#pragma unroll
-      for (int j = 1; j < ND; ++j) fw = madd(F[j], c[GALES_W(w) + j], fw);
-      const S fu = madd(rho, fw, p * F[iT]);
-      const S rF = rho * F[iT];
-      S FD[ND], Dr[ND];
-#pragma unroll
-      for (int j = 0; j < ND; ++j) {
-        S r0j, mEj;
-        if (j == 0) { r0j = c[GALES_W(drho_dp)]; mEj = c[GALES_W(de_dp)]; }
-        else if (j < iT) { r0j = S(0); mEj = vq[j - 1]; }
-        else if (j == iT) { r0j = c[GALES_W(drho_dT)]; mEj = c[GALES_W(de_dT)]; }
-        else { r0j = c[GALES_W(drho_dY) + j - iY]; mEj = c[GALES_W(dE_dY) + j - iY]; }
-        S x = madd(rF, mEj, (j >= 1 && j != iT) ? rho * F[j] : S(0));
-        FD[j] = (j >= 1 && j < iT) ? x : madd(fw, r0j, x);
-        S dd = madd(cE ? rho : S(0), mEj, (cvy && r == j) ? rho : S(0));
-        Dr[j] = (j >= 1 && j < iT) ? dd : madd(wr, r0j, dd);
-      }
-      S hv[DIM];
-      const S fe = rho * (F[iT] + (cE ? Nb : S(0)));
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) hv[d] = -madd(ur, gb[d], fe * grav[d]);
-      const S beta = madd(Nb, idt, -sb);
-      KSums<DIM, NC, S> ks;
-      S nu_j = S(0);
-      if constexpr (!AFF) {
-        ks.mu = jx * c[GALES_W(mu)]; ks.lambda = jx * c[GALES_W(lambda)]; ks.kappa = jx * c[GALES_W(kappa)];
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) { ks.muv[d] = ks.mu * vq[d]; ks.lamv[d] = ks.lambda * vq[d]; }
-#pragma unroll
-        for (int y = 0; y < L::NYA; ++y) {
-          ks.rhoD[y] = jx * c[GALES_W(rhoD) + y];
-          ks.rhoDH[y] = jx * c[GALES_W(rhoDH) + y];
-        }
-        nu_j = jx * c[GALES_W(nu)];
-      }
-#pragma unroll
-      for (int ai = 0; ai < NA; ++ai) {
-        const int a = a0 + ai;
-        S ga[DIM];
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) ga[d] = c[GALES_W(ds) + d * NEN + a];
-        const S Na = c[GALES_W(sh) + a];
-        S sa = ga[0] * vq[0];
-#pragma unroll
-        for (int d = 1; d < DIM; ++d) sa = madd(ga[d], vq[d], sa);
-        S fk = sa * F[iT];
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) fk = madd(ga[d], F[1 + d], fk);
-        const S A1 = jx * madd(Na, idt, sa), A4 = jx * Na, A2 = A4 * beta, A3 = jx * fu;
-        acc[ai][0] = madd(A1, FD[0], madd(A2, Dr[0], madd(jx, madd(-Na, kap, fk), acc[ai][0])));
-#pragma unroll
-        for (int d = 0; d < DIM; ++d)
-          acc[ai][1 + d] = madd(A1, FD[1 + d], madd(A2, Dr[1 + d], madd(A3, ga[d], madd(A4, hv[d], acc[ai][1 + d]))));
-#pragma unroll
-        for (int j = iT; j < ND; ++j) acc[ai][j] = madd(A1, FD[j], madd(A2, Dr[j], acc[ai][j]));
-        if constexpr (!AFF) {
-          add_viscous_row<DIM, NC, S>(acc[ai], r, ks, gb, ga);
-          S gg = gb[0] * ga[0];
-#pragma unroll
-          for (int d = 1; d < DIM; ++d) gg = madd(gb[d], ga[d], gg);
-          const S gn = gg * nu_j;
-#pragma unroll
-          for (int j = 0; j < ND; ++j) acc[ai][j] = madd(gn, Dr[j], acc[ai][j]);
-        }
-      }
-      if constexpr (AFF) {
-        const S mu = c[GALES_W(mu)], lam = c[GALES_W(lambda)];
-        const S jn = jx * c[GALES_W(nu)];
-#pragma unroll
-        for (int j = 0; j < ND; ++j) Dnu[j] = madd(jn, Dr[j], Dnu[j]);
-        ksum.mu = madd(jx, mu, ksum.mu);
-        ksum.lambda = madd(jx, lam, ksum.lambda);
-        ksum.kappa = madd(jx, c[GALES_W(kappa)], ksum.kappa);
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) {
-          ksum.muv[d] = madd(jx * mu, vq[d], ksum.muv[d]);
-          ksum.lamv[d] = madd(jx * lam, vq[d], ksum.lamv[d]);
-        }
-#pragma unroll
-        for (int y = 0; y < L::NYA; ++y) {
-          ksum.rhoD[y] = madd(jx, c[GALES_W(rhoD) + y], ksum.rhoD[y]);
-          ksum.rhoDH[y] = madd(jx, c[GALES_W(rhoDH) + y], ksum.rhoDH[y]);
-        }
-      }
-    }
-  }
-  if constexpr (WANT_M && AFF) {
-    // viscous/diffusive and dc terms of a simplex, from the point sums
-    const RecIn<S, BPS> c = rec(0);
-    S gb[DIM];
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) gb[d] = c[GALES_W(ds) + d * NEN + b];
-#pragma unroll
-    for (int ai = 0; ai < NA; ++ai) {
-      S ga[DIM];
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) ga[d] = c[GALES_W(ds) + d * NEN + a0 + ai];
-      add_viscous_row<DIM, NC, S>(acc[ai], r, ksum, gb, ga);
-      S gg = gb[0] * ga[0];
-#pragma unroll
-      for (int d = 1; d < DIM; ++d) gg = madd(gb[d], ga[d], gg);
-#pragma unroll
-      for (int j = 0; j < ND; ++j) acc[ai][j] = madd(gg, Dnu[j], acc[ai][j]);
-    }
-  }
-  // Dirichlet rows (scatter.hpp:62-78) and scatter (scatter.hpp:96-97)
-  const bool local = k.local_r != nullptr;
-  const bool blk_row = !local && (((uint32_t)d_int(b, GALES_W(d_blocked)) >> r) & 1u);
-  double avg = 0.0;
-  if constexpr (WANT_M) {
-    // avg_val = (1 + trace)/n (scatter.hpp:65-68), only where the element has a blocked
-    // row (the same for every lane of the element)
-    uint32_t any_blocked = 0u;
-#pragma unroll
-    for (int i = 0; i < NEN; ++i) any_blocked |= (uint32_t)d_int(i, GALES_W(d_blocked));
-    const bool need_avg = !local && any_blocked != 0u;
-    double tr = 0.0;
-    if (need_avg) {
-      S dg = S(0);
-#pragma unroll
-      for (int ai = 0; ai < NA; ++ai)
-#pragma unroll
-        for (int j = 0; j < ND; ++j) dg = (a0 + ai == b && j == r) ? acc[ai][j] : dg;
-      tr = active ? widen(dg) : 0.0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) tr += __shfl_xor_sync(0xffffffffu, tr, o);
-      if constexpr (WPE > 1) {
-        if ((gl & 31) == 0) E.wsum[gl >> 5] = tr;
-      }
-    }
-    elem_sync<WPE>(ec);
-    if (need_avg) {
-      if constexpr (WPE > 1) {
-        tr = E.wsum[0];
-#pragma unroll
-        for (int w = 1; w < WPE; ++w) tr += E.wsum[w];
-      }
-      avg = (1.0 + tr) * (1.0 / N);
-    }
-    if (active) {
-      S* srow = E.stage + row * NS + a0 * ND;
-#pragma unroll
-      for (int ai = 0; ai < NA; ++ai)
-#pragma unroll
-        for (int j = 0; j < ND; ++j) srow[ai * ND + j] = acc[ai][j];
-    }
-    elem_sync<WPE>(ec);
-  }
-  // staged entry (row rw, column cx) as scattered: a blocked row (Dirichlet) is avg on
-  // the diagonal and zero elsewhere (scatter.hpp:62-78)
-  auto staged = [&](int rw, int cx) -> double {
-    const int bn = rw / ND, jr = rw - bn * ND;
-    if (!local && ((((uint32_t)d_int(bn, GALES_W(d_blocked))) >> jr) & 1u)) return rw == cx ? avg : 0.0;
-    return widen(E.stage[rw * NS + cx]);
-  };
-  if (WANT_M && k.vjp_lam) {
-    // frozen-tangent VJP: g += K^T lambda for this element's block (Dirichlet rows included)
-    for (int cx = gl; cx < N; cx += ET) {
-      double sum = 0.0;
-      for (int rw = 0; rw < N; ++rw)
-        sum += __ldg(k.vjp_lam + (long long)d_int(rw / ND, GALES_W(d_node)) * ND + rw % ND) * staged(rw, cx);
-      if (sum != 0.0) atomicAdd(k.vjp_g + (long long)d_int(cx / ND, GALES_W(d_node)) * ND + cx % ND, sum);
-    }
-    return;
-  }
-  if (local) {  // element-level output of execute_i (fluid_2d.hpp:200-201): m = m_, r = -r_
-    if (active && grp_a == 0) k.local_r[g * N + row] = widen(-racc);
-    if (WANT_M && k.local_m)
-      for (int t = gl; t < NT; t += ET) k.local_m[g * NT + t] = widen(E.stage[(t / N) * NS + t % N]);
-    return;
-  }
-  const int mode = k.scatter_mode;
-  if (active && grp_a == 0 && !blk_row)
-    add_to(k.rhs + (long long)d_int(b, GALES_W(d_node)) * ND + r, widen(-racc), mode);
-  if constexpr (WANT_M) {
-    // One block row per warp step: lane l covers columns l, l+32, ... of the row; node
-    // sb_'s dof row jb holds node a's columns from nd off(sb_, a) + jb rowlen on, so
-    // consecutive lanes write the contiguous nd-runs.
-    constexpr int CH = (N + 31) / 32;   // column passes per row
-    const int lane = gl & 31, warp = gl >> 5;
-#pragma unroll
-    for (int h = 0; h < CH; ++h) {
-      const int cx = lane + 32 * h;
-      if (cx >= N) break;
-      const int a = cx / ND, ja = cx - a * ND;
-      for (int sb_ = 0; sb_ < NEN; ++sb_) {
-        const int64_t rl = d_int(sb_, GALES_W(d_rowlen));
-        const uint32_t bl = (uint32_t)d_int(sb_, GALES_W(d_blocked));
-        double* rowp = k.vals + (int64_t)d_int(sb_, GALES_W(d_off) + a) * ND + (int64_t)warp * rl + ja;
-        const int64_t step = (int64_t)WPE * rl;
-        for (int jb = warp; jb < ND; jb += WPE, rowp += step) {
-          if ((bl >> jb) & 1u) {  // blocked row: avg on its diagonal only
-            if (cx == sb_ * ND + jb) add_to(rowp, avg, mode);
-            continue;
-          }
-          const double val = widen(E.stage[(sb_ * ND + jb) * NS + cx]);
-          if ((__double2hiint(val) & 0x7fffffff) | __double2loint(val)) add_to(rowp, val, mode);
-        }
-      }
-    }
-  }
-}
-
-// Bulk copies of record blocks into shared memory with transaction barriers
-// (cp.async.bulk and mbarrier, sm_90+).  Every wait is bounded.
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_fence_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0u;
-}
-// Bounded wait on phase `parity` of a transaction barrier: false after kMbarTries
-// polls (each poll may suspend the thread for a while), far beyond any bulk copy.
-constexpr long long kMbarTries = 1ll << 24;
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  for (long long i = 0; i < kMbarTries; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
-}
-
-// Interior pass, stage 2 (persistent): CTA c assembles the element groups c, c + grid,
-// ... of the n listed elements whose records start at `in`.  One thread issues the bulk
-// copy of the next group's record block into the second buffer before the CTA works
-// on the current one, so the copy overlaps the element arithmetic.  A barrier wait
-// that runs out (it cannot on a working device) sets GALES_ERR_TIMEOUT, waits (again
-// bounded) for the other buffer's copy and ends the CTA.
-template <int DIM, int NEN, int NC, int NQ, typename S, bool WANT_M>
-__global__ void __launch_bounds__(MatShape<DIM, NEN, NC>::CTA)
-    matrix_kernel(const KParams k, const S* __restrict__ in, long long first, long long n) {
-  using RB = RecBlock<DIM, NEN, NC, NQ, S>;
-  using SM = MatSmem<DIM, NEN, NC, NQ, S>;
-  using ES = ElemSmem<DIM, NEN, NC, NQ, S>;
-  constexpr int EPC = MatShape<DIM, NEN, NC>::EPC, ET = MatShape<DIM, NEN, NC>::ET;
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  S* buf[2] = {reinterpret_cast<S*>(smem_raw), reinterpret_cast<S*>(smem_raw + RB::BYTES)};
-  ES& E = *reinterpret_cast<ES*>(smem_raw + SM::OFF_ES + (size_t)(threadIdx.x / ET) * SM::ES_BYTES);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + SM::OFF_BAR);
-  const long long ngroups = (n + EPC - 1) / EPC;
-  if (threadIdx.x == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    mbar_fence_init();
-  }
-  __syncthreads();
-  long long grp = blockIdx.x;
-  if (threadIdx.x == 0 && grp < ngroups) bulk_load(buf[0], in + grp * RB::WORDS, (uint32_t)RB::BYTES, &bar[0]);
-  for (int it = 0; grp < ngroups; ++it, grp += gridDim.x) {
-    const int cur = it & 1;
-    const long long nxt = grp + gridDim.x;
-    if (threadIdx.x == 0 && nxt < ngroups)
-      bulk_load(buf[cur ^ 1], in + nxt * RB::WORDS, (uint32_t)RB::BYTES, &bar[cur ^ 1]);
-    const bool ok = mbar_wait(&bar[cur], (uint32_t)((it >> 1) & 1));
-    if (__syncthreads_or(!ok)) {
-      if (threadIdx.x == 0) {
-        flag_error(k, GALES_ERR_TIMEOUT, first + grp * EPC);
-        if (nxt < ngroups) mbar_wait(&bar[cur ^ 1], (uint32_t)(((it + 1) >> 1) & 1));
-      }
-      return;
-    }
-    matrix_group<DIM, NEN, NC, NQ, S, WANT_M>(k, buf[cur], E, first, n, grp);
-    __syncthreads();  // the buffer and the element slots are free again
-  }
 }
 
 // ---------------------------------------------------------------------------

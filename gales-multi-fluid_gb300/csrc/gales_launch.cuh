@@ -7,6 +7,7 @@
 #include <type_traits>
 
 #include "gales_fp64.cuh"
+#include "gales_rows32.cuh"
 
 namespace gales {
 
@@ -15,18 +16,24 @@ struct LaunchResult {
   int launches;
 };
 
-// The mixed form (gales_kernels.cuh).
+// Whether some node flag blocks a dof.
+inline bool any_dirichlet(const KParams& k) {
+  uint32_t any = 0u;
+  for (int f = 0; f < GALES_MAX_FLAGS; ++f) any |= k.dirichlet_mask[f];
+  return any != 0u;
+}
+
+// The mixed form (gales_kernels.cuh, gales_rows32.cuh).
 template <int DIM, int NEN, int NC, int NQ, int EOS = kEosChemicals>
 struct InteriorInst {
   using S = float;
   using Rec = QP<DIM, NEN, NC, S>;
-  using RB = RecBlock<DIM, NEN, NC, NQ, S>;
-  using SM = MatSmem<DIM, NEN, NC, NQ, S>;
-  using M = MatShape<DIM, NEN, NC>;
-  // record bytes per element, rounded up, and elements per block of records: a chunk of n
-  // elements needs at most (n + rec_block()) rec_bytes()
-  static size_t rec_bytes() { return (RB::BYTES + M::EPC - 1) / M::EPC; }
-  static int rec_block() { return 4; }
+  using RB = RecBlock<DIM, NEN, NC>;
+  using T = Rows32<DIM, NEN, NC>;
+  // record bytes per element and elements per block of records: a chunk of n elements needs
+  // at most (n + rec_block()) rec_bytes()
+  static size_t rec_bytes() { return RB::BYTES / RB::EB; }
+  static int rec_block() { return RB::EB; }
   // resident point-kernel CTAs (128 threads) per SM
   static int point_occupancy() {
     int nb = 0;
@@ -42,39 +49,21 @@ struct InteriorInst {
         k, reinterpret_cast<Rec*>(buf), first, n);
     return {cudaGetLastError(), 1};
   }
-  // resident matrix CTAs per SM (set by prepare)
-  static int& matrix_occupancy() {
-    static int occ = 1;
-    return occ;
-  }
-  // dynamic shared memory limits, set once per device before any launch (also before
-  // a stream capture), and the matrix kernel's occupancy
-  static cudaError_t prepare() {
-    const int smem = (int)SM::BYTES;
-    cudaError_t e = cudaFuncSetAttribute(matrix_kernel<DIM, NEN, NC, NQ, S, true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(matrix_kernel<DIM, NEN, NC, NQ, S, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem);
-    if (e != cudaSuccess) return e;
-    int nb = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, matrix_kernel<DIM, NEN, NC, NQ, S, true>, M::CTA, smem);
-    if (e != cudaSuccess) return e;
-    matrix_occupancy() = nb > 0 ? nb : 1;
-    return cudaSuccess;
-  }
-  // persistent: at most (SMs x resident CTAs) CTAs, each looping over element groups
+  static cudaError_t prepare() { return cudaSuccess; }
   static LaunchResult matrix(const KParams& k, bool want_m, void* buf, long long first, long long n,
                              cudaStream_t st) {
     if (n <= 0) return {cudaSuccess, 0};
-    const size_t smem = SM::BYTES;
-    const long long groups = (n + M::EPC - 1) / M::EPC;
-    const long long cap = (long long)(k.sms > 0 ? k.sms : 1) * matrix_occupancy();
-    const unsigned blocks = (unsigned)(groups < cap ? groups : cap);
-    const S* in = reinterpret_cast<const S*>(buf);
-    if (want_m) matrix_kernel<DIM, NEN, NC, NQ, S, true><<<blocks, M::CTA, smem, st>>>(k, in, first, n);
-    else matrix_kernel<DIM, NEN, NC, NQ, S, false><<<blocks, M::CTA, smem, st>>>(k, in, first, n);
-    return {cudaGetLastError(), 1};
+    const unsigned ctas = (unsigned)((n + RB::EB - 1) / RB::EB * T::ND);
+    unsigned char* in = reinterpret_cast<unsigned char*>(buf);
+    if (!want_m) {
+      rows32_kernel<DIM, NEN, NC, false><<<ctas, T::THREADS, 0, st>>>(k, in, first, n);
+      return {cudaGetLastError(), 1};
+    }
+    rows32_kernel<DIM, NEN, NC, true><<<ctas, T::THREADS, 0, st>>>(k, in, first, n);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess || !any_dirichlet(k) || k.local_r) return {e, 1};
+    dirichlet32_kernel<DIM, NEN, NC><<<(unsigned)((n + 127) / 128), 128, 0, st>>>(k, in, n);
+    return {cudaGetLastError(), 2};
   }
 };
 
@@ -83,9 +72,7 @@ struct InteriorInst {
 template <int DIM, int NEN, int NC>
 LaunchResult dirichlet64(const KParams& k, const double* in, long long n, cudaStream_t st) {
   const cudaError_t e = cudaGetLastError();
-  uint32_t any = 0u;
-  for (int f = 0; f < GALES_MAX_FLAGS; ++f) any |= k.dirichlet_mask[f];
-  if (e != cudaSuccess || !any || k.local_r) return {e, 1};
+  if (e != cudaSuccess || !any_dirichlet(k) || k.local_r) return {e, 1};
   dirichlet64_kernel<DIM, NEN, NC><<<(unsigned)((n + 127) / 128), 128, 0, st>>>(k, in, n);
   return {cudaGetLastError(), 2};
 }
