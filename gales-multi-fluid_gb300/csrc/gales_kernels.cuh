@@ -85,6 +85,7 @@ struct KParams {
   const void* bgeo;
   void* bpt_rec;
   int64_t n_bpt;
+  int32_t bd_stage;            // launches of the boundary pass: 0 both stages, 1 the points, 2 the elements
   // arrays the point stage zeroes beside its own work (the first chunk's launch clears
   // A and b, whose first writers are the matrix and boundary stages after it)
   double* clear_p[2];

@@ -165,15 +165,17 @@ cudaError_t prepare_boundary_nc() {
 }
 
 // Boundary pass: with point records (k.bpt_rec) the point stage runs first, one thread
-// per flagged side point; the element stage then reads the records.
+// per flagged side point; the element stage then reads the records.  k.bd_stage 1 launches the
+// point stage alone, 2 the element stage alone.
 template <int DIM, int NEN, int NC, int NS, int NSQ, typename S, int EOS = kEosChemicals>
 LaunchResult launch_boundary_nc(const KParams& k, long long n_items, cudaStream_t st) {
   if (n_items == 0) return {cudaSuccess, 0};
   int launches = 0;
-  if (k.bpt_rec && k.n_bpt > 0) {
+  if (k.bpt_rec && k.n_bpt > 0 && k.bd_stage != 2) {
     bpoint_kernel<DIM, NEN, NC, NS, NSQ, S, EOS><<<(unsigned)((k.n_bpt + 127) / 128), 128, 0, st>>>(k);
     ++launches;
   }
+  if (k.bd_stage == 1) return {cudaGetLastError(), launches};
   const size_t smem = k.bpt_rec ? 0 : sizeof(BoundarySmem<DIM, NEN, NC, NS, NSQ, S>);
   boundary_kernel<DIM, NEN, NC, NS, NSQ, S, EOS><<<(unsigned)n_items, boundary_threads<NC, DIM>(), smem, st>>>(k);
   return {cudaGetLastError(), launches + 1};
