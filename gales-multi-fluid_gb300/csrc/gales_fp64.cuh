@@ -380,12 +380,12 @@ __device__ __forceinline__ void point64(const KParams& k, long long e, int iq, d
     assign<DIM, NC>(Pq, pP, vP, TP, YP);
     assign<DIM, NC>(Iq, p, v, T, Y);
     if constexpr (EOS == kEosMagma) {
-      Props<NC> prP;
-      unsigned st = magma_mixture<NC>(k.mg, pP, TP, YP, 0.0, prP);
+      double oP[2];
+      unsigned st = magma_rho_cv(k.mg, NC, pP, TP, YP, oP);
       st |= magma_mixture<NC>(k.mg, p, T, Y, shear_rate<DIM>(dv), pr);
       if (st) flag_error(k, GALES_ERR_MAGMA, e);
-      rhoP = prP.rho;
-      cvP = prP.cv;
+      rhoP = oP[0];
+      cvP = oP[1];
       pr.irho = 1.0 / pr.rho;
 #pragma unroll
       for (int i = 0; i < NC; ++i) pr.irho_c[i] = 1.0 / pr.rho_c[i];

@@ -29,6 +29,9 @@ struct DevMagma {
   double visc_M, visc_P[7];                               // Giordano composition terms
   double wf_comp[3];                                      // melt, H2O, CO2 of the magma
   double crystal_vf, crystal_rho;
+  // constants of the assembly's form (gales_magma_fast.cuh): wf/M; dVdT^2/(-M dVdp), with which
+  // the melt's cv = cp - T q; 1/M and 1/gamma; (1 - vf)^-2.5; Pal's bubble radius
+  double melt_m0, melt_q, vol_iM[2], gas_ig[2], crystal_er, bubble_r;
   int gas_on_mu, crystal_on_mu;
   int n_p, n_T;
   // custom_mix / ch_as_mix (kind != GALES_SUBMIX_MAGMA): the chemical's constants
@@ -128,6 +131,14 @@ inline void build_constants(const gales_magma_desc& d, DevMagma& g) {
   g.visc_P[6] = 0.3 * (m[2] + m[4] + m[5] + m[6] + m[7]);
   g.crystal_vf = d.crystal_fraction;
   g.crystal_rho = d.crystal_rho;
+  g.melt_m0 = g.wf_comp[0] / g.melt_M;
+  g.melt_q = g.melt_dVdT * g.melt_dVdT / (-g.melt_dVdp * g.melt_M);
+  for (int k = 0; k < 2; ++k) {
+    g.vol_iM[k] = 1.0 / g.vol_M[k];
+    g.gas_ig[k] = 1.0 / g.gas_gamma[k];
+  }
+  g.crystal_er = std::pow(1.0 - 1.0 * g.crystal_vf, -2.5);
+  g.bubble_r = std::cbrt(3.0 / (4 * 3.142 * 1.e11));
   g.gas_on_mu = d.gas_on_mu;
   g.crystal_on_mu = d.crystal_on_mu;
   g.n_p = d.n_p;

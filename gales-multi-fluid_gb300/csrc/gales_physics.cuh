@@ -13,7 +13,7 @@
 #include <cstdint>
 
 #include "../../include/gales_asm.h"
-#include "gales_magma.cuh"
+#include "gales_magma_fast.cuh"
 
 namespace gales {
 
@@ -227,7 +227,12 @@ constexpr int kEosMagma = 1;
 // GALES_MAGMA_* bits.
 static __device__ __noinline__ unsigned magma_point(const magma_mix::DevMagma* mg, int nc, double p, double T,
                                                     const double* Y, double sr, double* f, double (*comp)[4]) {
-  return magma_mix::mix_point(mg, nc, p, T, Y, sr, f, comp);
+  return magma_mix::fast::mix_point(mg, nc, p, T, Y, sr, f, comp);
+}
+
+static __device__ __noinline__ unsigned magma_rho_cv(const magma_mix::DevMagma* mg, int nc, double p, double T,
+                                                     const double* Y, double* o) {
+  return magma_mix::fast::mix_rho_cv(mg, nc, p, T, Y, o[0], o[1]);
 }
 
 // Props of the magma mixture; the mixture's own chemical diffusivity is not formed by
