@@ -19,7 +19,8 @@
 // upper blocks: rows are ordered by level (longest dependency chain) on the host.  The
 // factorisation (a CTA per node row) and each substitution (a warp per node row) are one
 // persistent launch each, which takes rows in level order and waits for single rows (see
-// ilu_factor_rows_kernel, ilu_sweep_kernel).  The preconditioner application is
+// ilu_factor_rows_kernel, ilu_sweep_kernel; ilu_sweep_cluster_kernel where the vector fits in
+// shared memory).  The preconditioner application is
 // captured once into a CUDA graph whose kernels take the Krylov vector's index from
 // device memory.  The Arnoldi step (two classical
 // Gram-Schmidt passes) uses blocked dot products with fixed partial-sum order, so
@@ -637,6 +638,202 @@ __global__ void __launch_bounds__(32 * kSweepWarps)
   }
 }
 
+// Small systems: each sweep by one thread-block cluster, whose CTAs hold the whole result vector
+// in shared memory (n ND words <= kClusterSmem).  A finished row is stored into every CTA's copy
+// and polled locally, so a level pays a trip to a neighbour's shared memory in place of one
+// through L2.  With an FP64 factor the off-diagonal blocks are multiplied by the inverse of their
+// row's diagonal block in advance (scale_rows_kernel), which leaves no solve, ND dependent FP64
+// operations, after the last arrival:
+//   lower  y_I = L_II^-1 v_I - sum_K (L_II^-1 L_IK) y_K, upper alike with U_II.
+// An FP32 factor keeps its blocks: rounding them once more would double the sweeps' error.
+// Rows go to the cluster's warps in turn, in level order; all warps are resident, so every wait
+// ends (and is bounded, see kSpinMax).  Bound: the FP64 latency of the products and sums after a
+// row's last arrival.  M^-1 of a 2,145-node channel (161 levels, 5 dofs): 0.23 ms with an FP64
+// factor and 0.13 with FP32, against 0.41 and 0.24 through L2.  4 or 12 warps per CTA: 0.23,
+// 0.24; a block's columns spread over the lanes, each polling its own word: 0.22 and 0.15.
+constexpr int kClusterWarps = 8;
+constexpr size_t kClusterSmem = 200 * 1024;
+template <typename T>
+constexpr bool kClusterScaled = sizeof(T) == 8;
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+template <typename T>
+__device__ __forceinline__ typename SweepWord<T>::Bits cluster_poll(uint32_t at) {
+  typename SweepWord<T>::Bits v;
+  if constexpr (sizeof(T) == 8) asm volatile("ld.relaxed.cluster.shared::cta.b64 %0, [%1];" : "=l"(v) : "r"(at) : "memory");
+  else asm volatile("ld.relaxed.cluster.shared::cta.b32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+  return v;
+}
+// stores x into CTA rank's copy of the word at shared address at
+template <typename T>
+__device__ __forceinline__ void cluster_store(uint32_t at, uint32_t rank, T x) {
+  using W = SweepWord<T>;
+  uint32_t to;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(at), "r"(rank));
+  if constexpr (sizeof(T) == 8) {
+    typename W::Bits v = (typename W::Bits)__double_as_longlong(x);
+    if (v == W::kUnset) v = W::kNan;
+    asm volatile("st.relaxed.cluster.shared::cluster.b64 [%0], %1;" ::"r"(to), "l"(v) : "memory");
+  } else {
+    typename W::Bits v = __float_as_uint(x);
+    if (v == W::kUnset) v = W::kNan;
+    asm volatile("st.relaxed.cluster.shared::cluster.b32 [%0], %1;" ::"r"(to), "r"(v) : "memory");
+  }
+}
+
+// S = the off-diagonal factor blocks times the inverse of their row's diagonal block (warp per
+// node row, a lane per block column; the diagonal of U scaled as in Us).
+template <int ND, typename T>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock)
+    scale_rows_kernel(const T* __restrict__ F, const int64_t* __restrict__ f_rp, const int64_t* __restrict__ f_diag,
+                      const T* __restrict__ Us, int64_t n, T* __restrict__ S) {
+  constexpr int BB = ND * ND;
+  const int64_t I = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  if (I >= n) return;
+  const int lane = threadIdx.x & 31;
+  const int64_t p0 = f_rp[I], p1 = f_rp[I + 1], pd = f_diag[I];
+  for (int64_t it = lane; it < (p1 - p0) * ND; it += 32) {
+    const int64_t p = p0 + it / ND;
+    const int c = (int)(it % ND);
+    if (p == pd) continue;
+    T x[ND];
+#pragma unroll
+    for (int r = 0; r < ND; ++r) x[r] = F[p * BB + r * ND + c];
+    if (p < pd) {
+      const T* D = F + pd * BB;
+#pragma unroll
+      for (int q = 0; q < ND - 1; ++q)
+#pragma unroll
+        for (int r = q + 1; r < ND; ++r) x[r] = sweep_fma(-D[r * ND + q], x[q], x[r]);
+    } else {
+      const T* D = Us + I * BB;
+#pragma unroll
+      for (int r = 0; r < ND; ++r) x[r] *= D[r * ND + r];
+#pragma unroll
+      for (int q = ND - 1; q > 0; --q)
+#pragma unroll
+        for (int r = 0; r < q; ++r) x[r] = sweep_fma(-D[r * ND + q], x[q], x[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < ND; ++r) S[p * BB + r * ND + c] = x[r];
+  }
+}
+
+// In (lower: the FP64 right-hand side vbase; upper: the lower sweep's result y) and out (lower:
+// y; upper: the FP64 column zoutbase).  D: the factor (lower) or the scaled diagonal blocks.
+template <int ND, typename T, bool LOWER>
+__global__ void __launch_bounds__(32 * kClusterWarps)
+    ilu_sweep_cluster_kernel(const T* __restrict__ S, const int64_t* __restrict__ f_rp,
+                             const int32_t* __restrict__ f_col, const int64_t* __restrict__ f_diag,
+                             const T* __restrict__ Dg, const int32_t* __restrict__ rows, int64_t n,
+                             const double* __restrict__ vbase, T* __restrict__ y, double* __restrict__ zoutbase,
+                             const int* __restrict__ jidx, int64_t ld, unsigned int* status) {
+  using W = SweepWord<T>;
+  constexpr int BB = ND * ND, G = 32 / ND;
+  constexpr int KB = 56 / ND < 8 ? 56 / ND : 8;   // blocks per lane held in registers
+  extern __shared__ __align__(16) unsigned char sweep_smem[];
+  T* z = reinterpret_cast<T*>(sweep_smem);
+  const uint32_t z0 = (uint32_t)__cvta_generic_to_shared(z);
+  const int lane = threadIdx.x & 31;
+  const int g = lane / ND, r = lane < G * ND ? lane - g * ND : 0;
+  const uint32_t nc = gridDim.x;   // one cluster
+  const int64_t off = jidx ? (int64_t)(*jidx) * ld : 0;
+  for (int64_t i = threadIdx.x; i < n * ND; i += blockDim.x)
+    reinterpret_cast<typename W::Bits*>(z)[i] = W::kUnset;
+  cluster_sync();
+  bool late = false;
+  for (int64_t t = cluster_rank() + (int64_t)nc * (threadIdx.x >> 5); t < n; t += (int64_t)nc * kClusterWarps) {
+    const int32_t I = rows[t];
+    const int64_t pd = f_diag[I];
+    const int64_t pa = LOWER ? f_rp[I] : pd + 1;
+    const int nblk = (int)((LOWER ? pd : f_rp[I + 1]) - pa);
+    T D[ND];
+#pragma unroll
+    for (int c = 0; c < ND; ++c) D[c] = Dg[(LOWER ? pd : (int64_t)I) * BB + r * ND + c];
+    // x times the inverse of the diagonal block
+    auto solve = [&](T x) {
+      if constexpr (LOWER) {
+#pragma unroll
+        for (int c = 0; c < ND - 1; ++c) {
+          const T xc = __shfl_sync(0xffffffffu, x, c);
+          if (r > c) x = sweep_fma(-D[c], xc, x);
+        }
+      } else {
+        T rd = D[0];
+#pragma unroll
+        for (int c = 1; c < ND; ++c) rd = r == c ? D[c] : rd;
+        x *= rd;
+#pragma unroll
+        for (int c = ND - 1; c > 0; --c) {
+          const T xc = __shfl_sync(0xffffffffu, x, c);
+          if (r < c) x = sweep_fma(-D[c], xc, x);
+        }
+      }
+      return x;
+    };
+    T rhs = LOWER ? (T)vbase[off + (int64_t)I * ND + r] : y[(int64_t)I * ND + r];
+    if constexpr (kClusterScaled<T>) rhs = solve(rhs);
+    T sum = g == 0 ? -rhs : T(0), sum2 = T(0);
+    for (int k0 = 0; k0 < nblk; k0 += KB * G) {
+      int zc[KB];
+      T B[KB][ND];
+#pragma unroll
+      for (int k = 0; k < KB; ++k) {
+        const int i = k0 + k * G + g;
+        const bool on = g < G && i < nblk;
+        const int64_t p = pa + (LOWER ? i : nblk - 1 - i);
+        zc[k] = on ? f_col[p] * ND + r : -1;
+#pragma unroll
+        for (int c = 0; c < ND; ++c) B[k][c] = on ? S[p * BB + r * ND + c] : T(0);
+      }
+#pragma unroll
+      for (int k = 0; k < KB; ++k) {
+        if (k0 + k * G >= nblk) break;   // the same for every lane
+        typename W::Bits w = zc[k] >= 0 ? W::kUnset : typename W::Bits(0);
+        for (long long spin = 0; !late; ++spin) {
+          if (w == W::kUnset) w = cluster_poll<T>(z0 + (uint32_t)zc[k] * (uint32_t)sizeof(T));
+          if (!__any_sync(0xffffffffu, w == W::kUnset)) break;
+          if (spin >= kSpinMax) late = true;
+        }
+        const T zk = W::value(w);
+#pragma unroll
+        for (int c = 0; c < ND; ++c) {
+          const T x = __shfl_sync(0xffffffffu, zk, (g < G ? g : 0) * ND + c);
+          if (c & 1) sum2 = sweep_fma(B[k][c], x, sum2);
+          else sum = sweep_fma(B[k][c], x, sum);
+        }
+      }
+    }
+    sum += sum2;
+    T part[G];
+#pragma unroll
+    for (int q = 0; q < G; ++q) part[q] = __shfl_sync(0xffffffffu, sum, q * ND + r);
+#pragma unroll
+    for (int h = 1; h < G; h *= 2)
+#pragma unroll
+      for (int q = 0; q + h < G; q += 2 * h) part[q] += part[q + h];
+    T s = -part[0];
+    if constexpr (!kClusterScaled<T>) s = solve(s);
+    // lane (g, r) stores word r into the copies of the CTAs g, g + G, ...
+    if (g < G)
+      for (uint32_t c = (uint32_t)g; c < nc; c += G)
+        cluster_store<T>(z0 + (uint32_t)(I * ND + r) * (uint32_t)sizeof(T), c, s);
+    if (lane < ND) {
+      if constexpr (LOWER) y[(int64_t)I * ND + lane] = s;
+      else zoutbase[off + (int64_t)I * ND + lane] = (double)s;
+    }
+  }
+  if (late && lane == 0) atomicOr(status, (unsigned)GALES_ERR_TIMEOUT);
+  cluster_sync();   // a CTA's copy is written until every row is done
+}
+
 // y = A x (or y = b - A x) on the assembly's CSR values: warp per node row.  Lanes form
 // G = 32 / ND groups of ND, lane (g, r) takes scalar row r over the node row's blocks g,
 // g + G, ...: ND multiply-adds a block and G - 1 adds at the end.  Bound: the FP64 pipe
@@ -842,6 +1039,7 @@ struct gales_solver {
   Dev<int> d_j;
   Dev<int> d_ready;          // factorisation: ticket, then a ready flag per node row
   Dev<unsigned char> d_udiag;  // the upper sweep's scaled diagonal blocks (factor's type)
+  Dev<unsigned char> d_scaled;  // cluster sweeps in FP64: off-diagonal blocks times their inverse diagonal block
   Dev<unsigned char> d_sweep;  // substitutions: the two result vectors (factor's type), then two tickets
   Dev<unsigned int> d_status, d_count;  // error bits; CTAs of an Arnoldi pass that are done
   double* h_buf = nullptr;   // pinned: Hessenberg column and the least-squares solution
@@ -850,6 +1048,7 @@ struct gales_solver {
   int smem_optin = 0;          // opt-in shared memory per CTA
   size_t factor_smem = 0;      // dynamic shared memory of the factorisation kernel (0: level launches)
   int factor_ctas = 1;         // its resident CTAs per SM
+  int cluster = 0;             // CTAs of the sweeps' cluster (0: the sweeps through L2)
   int dot_blocks = 1;
   cudaGraphExec_t prec_graph = nullptr;
   cudaStream_t cap = nullptr;
@@ -902,6 +1101,49 @@ struct Kernels {
   }
   // The persistent factorisation where a block row and two rows' upper parts fit the shared
   // memory of an SM; rows too long for that take the level launches on global memory.
+  // A launch of one cluster of `size` CTAs.
+  struct ClusterLaunch {
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t cfg;
+    ClusterLaunch(unsigned size, size_t smem, cudaStream_t st) {
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = size;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      std::memset(&cfg, 0, sizeof(cfg));
+      cfg.gridDim = dim3(size);
+      cfg.blockDim = dim3(32 * kClusterWarps);
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = st;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+    }
+  };
+  static size_t cluster_smem(const gales_solver* s) { return (size_t)s->n_rows * sizeof(T); }
+  // Cluster size of the sweeps: the largest of 16 and 8 that the device takes, 0 where the
+  // result vector is too long for a CTA.
+  template <bool LOWER>
+  static cudaError_t prepare_cluster(gales_solver* s, int& size) {
+    const auto fn = ilu_sweep_cluster_kernel<ND, T, LOWER>;
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    for (; size > 4; size /= 2) {
+      ClusterLaunch l((unsigned)size, cluster_smem(s), nullptr);
+      int nb = 0;
+      if (cudaOccupancyMaxActiveClusters(&nb, fn, &l.cfg) == cudaSuccess && nb > 0) return cudaSuccess;
+      cudaGetLastError();
+    }
+    size = 0;
+    return cudaSuccess;
+  }
+  static int cluster_size(gales_solver* s) {
+    int size = cluster_smem(s) <= kClusterSmem && cluster_smem(s) <= (size_t)s->smem_optin ? 16 : 0;
+    if (size && (prepare_cluster<true>(s, size) != cudaSuccess || prepare_cluster<false>(s, size) != cudaSuccess)) {
+      cudaGetLastError();
+      size = 0;
+    }
+    return size;
+  }
   static cudaError_t prepare(gales_solver* s) {
     const size_t bytes = FactorSmem<ND, T>::bytes(s->max_row, s->max_u);
     s->factor_smem = 0;
@@ -941,11 +1183,31 @@ struct Kernels {
   static cudaError_t scale_diag(gales_solver* s, cudaStream_t st) {
     scale_diag_kernel<ND, T><<<(unsigned)((s->n_rows + 127) / 128), 128, 0, st>>>(
         factor_ptr<T>(s), s->d_f_diag.p, s->n_rows, reinterpret_cast<T*>(s->d_udiag.p));
+    ++s->launches;
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess || !s->cluster || !kClusterScaled<T>) return e;
+    scale_rows_kernel<ND, T><<<grid_for(s->n_nodes), 32 * kWarpsPerBlock, 0, st>>>(
+        factor_ptr<T>(s), s->d_f_rp.p, s->d_f_diag.p, reinterpret_cast<const T*>(s->d_udiag.p), s->n_nodes,
+        reinterpret_cast<T*>(s->d_scaled.p));
+    ++s->launches;
     return cudaGetLastError();
   }
   // both substitutions (result vectors and tickets set to all ones by the caller)
   static cudaError_t sweeps(gales_solver* s, const double* v, double* z, const int* j, int64_t ld, cudaStream_t st) {
     T* y = reinterpret_cast<T*>(s->d_sweep.p);
+    if (s->cluster) {
+      const ClusterLaunch l((unsigned)s->cluster, cluster_smem(s), st);
+      const T* S = kClusterScaled<T> ? reinterpret_cast<const T*>(s->d_scaled.p) : factor_ptr<T>(s);
+      const cudaError_t e = cudaLaunchKernelEx(
+          &l.cfg, ilu_sweep_cluster_kernel<ND, T, true>, S, (const int64_t*)s->d_f_rp.p, (const int32_t*)s->d_f_col.p,
+          (const int64_t*)s->d_f_diag.p, (const T*)factor_ptr<T>(s), (const int32_t*)s->d_rows_f.p, s->n_nodes, v, y,
+          (double*)nullptr, j, ld, s->d_status.p);
+      if (e != cudaSuccess) return e;
+      return cudaLaunchKernelEx(&l.cfg, ilu_sweep_cluster_kernel<ND, T, false>, S, (const int64_t*)s->d_f_rp.p,
+                                (const int32_t*)s->d_f_col.p, (const int64_t*)s->d_f_diag.p,
+                                reinterpret_cast<const T*>(s->d_udiag.p), (const int32_t*)s->d_rows_b.p, s->n_nodes,
+                                (const double*)nullptr, y, z, j, ld, s->d_status.p);
+    }
     T* x = y + s->n_rows;
     unsigned int* tk = reinterpret_cast<unsigned int*>(x + s->n_rows);
     const unsigned g = (unsigned)std::min<int64_t>((s->n_nodes + kSweepWarps - 1) / kSweepWarps, s->sms);
@@ -968,6 +1230,7 @@ struct Kernels {
 };
 
 struct Ops {
+  int (*cluster_size)(gales_solver*);
   cudaError_t (*prepare)(gales_solver*);
   cudaError_t (*to_factor)(gales_solver*, const double*, cudaStream_t);
   cudaError_t (*factor)(gales_solver*, cudaStream_t);
@@ -979,7 +1242,7 @@ struct Ops {
 template <int ND, typename T>
 Ops ops_for() {
   using K = Kernels<ND, T>;
-  return {K::prepare, K::to_factor, K::factor, K::scale_diag, K::sweeps, K::spmv};
+  return {K::cluster_size, K::prepare, K::to_factor, K::factor, K::scale_diag, K::sweeps, K::spmv};
 }
 
 template <typename T>
@@ -1009,7 +1272,7 @@ inline bool has_ilu(const gales_solver* s) {
 // z = M^-1 v for columns addressed by *j (graph) or plain pointers (j null): the two sweeps
 // after setting their result vectors and tickets to all ones (SweepWord::kUnset).
 int apply_prec(gales_solver* s, const Ops& o, const double* v, double* z, const int* j, int64_t ld, cudaStream_t st) {
-  SCK(s, cudaMemsetAsync(s->d_sweep.p, 0xff, s->d_sweep.n, st), "clear sweep vectors");
+  if (!s->cluster) SCK(s, cudaMemsetAsync(s->d_sweep.p, 0xff, s->d_sweep.n, st), "clear sweep vectors");
   SCK(s, o.sweeps(s, v, z, j, ld, st), "substitutions");
   s->launches += 2;
   return 0;
@@ -1040,7 +1303,6 @@ int factorize(gales_solver* s, const Ops& o, const double* vals, cudaStream_t st
   ++s->launches;
   SCK(s, o.factor(s, st), "factorisation");
   SCK(s, o.scale_diag(s, st), "diagonal blocks");
-  ++s->launches;
   unsigned int stat = 0;
   SCK(s, cudaMemcpyAsync(&stat, s->d_status.p, sizeof(stat), cudaMemcpyDeviceToHost, st), "status");
   SCK(s, cudaStreamSynchronize(st), "factorisation");
@@ -1184,6 +1446,11 @@ int gales_solver_create(gales_asm* h, const gales_solver_params* prm, gales_solv
     if (o.prepare(s) != cudaSuccess) {
       cudaGetLastError();
       s->factor_smem = 0;
+    }
+    s->cluster = o.cluster_size(s);
+    if (s->cluster && p.precond == GALES_PRECOND_ILU && s->d_scaled.alloc(s->f_col.size() * bb * sizeof(double))) {
+      cudaGetLastError();
+      s->cluster = 0;
     }
     rc = capture_prec_graph(s, o);
     if (rc) {
@@ -1436,6 +1703,7 @@ void gales_solver_destroy(gales_solver* s) {
   s->d_ready.release();
   s->d_sweep.release();
   s->d_udiag.release();
+  s->d_scaled.release();
   s->d_status.release();
   s->d_count.release();
   delete s;

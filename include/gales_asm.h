@@ -338,7 +338,7 @@ int gales_solver_apply(gales_solver* s, const double* v, double* z, void* stream
  * unit L strictly below the diagonal, U on and above it).  Synchronises the device. */
 int gales_solver_factor(gales_solver* s, int64_t* n_block_rows, int64_t* nnz_blocks, const int64_t** row_ptr,
                         const int32_t** col, double* vals);
-/* Number of levels of the forward and backward substitutions (launches per sweep). */
+/* Number of levels (longest dependency chains) of the forward and backward substitutions. */
 int gales_solver_levels(gales_solver* s, int32_t* n_levels_fwd, int32_t* n_levels_bwd);
 /* fluid_updater::corrector and model::dof_trimmer (fluid_updater.hpp:23-26,
  * model.hpp:176-184): I += dx on the device, then every node's dofs with index in
