@@ -7,15 +7,14 @@
 //                   flux scalars (fluid_2d.hpp:391-603), tau (fluid_2d.hpp:877-1022)
 //                   and the dc viscosity (fluid_2d.hpp:1027-1065), written as a point
 //                   record in the matrix stage's arithmetic type S.
-//   matrix_kernel - one warp per element (more for hexahedra), one lane per row of
-//                   the element block: Galerkin, least-squares and dc terms of RM_i
-//                   (fluid_2d.hpp:251-333) accumulated in registers over the points,
-//                   then the Dirichlet row replacement of scatter::execute
-//                   (scatter.hpp:62-78) and FP64 adds into the CSR values and rhs
-//                   (scatter.hpp:96-97).
-// Boundary kernel, one warp per boundary element: execute_b/RM_b
-// (fluid_2d.hpp:209-245, 341-364, 610-868) and its own scatter pass
-// (fluid_assembly.hpp:57-63), all in FP64.
+//   rows32_kernel - (gales_rows32.cuh) a warp per dof row of 32 elements: Galerkin,
+//                   least-squares and dc terms of RM_i (fluid_2d.hpp:251-333) accumulated
+//                   in registers over the points, FP64 adds into the CSR values and rhs
+//                   (scatter.hpp:96-97); rows of blocked dofs (scatter.hpp:62-78) by
+//                   dirichlet32_kernel.
+// Boundary pass, both forms: bpoint_kernel, a thread per flagged side point, then
+// boundary_kernel, a CTA per boundary element: execute_b/RM_b (fluid_2d.hpp:209-245,
+// 341-364, 610-868) and its own scatter pass (fluid_assembly.hpp:57-63).
 #pragma once
 
 #include <cuda_runtime.h>
