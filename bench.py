@@ -50,10 +50,10 @@ METRIC = "residual+Jacobian elements/s, mixed vs FP64 on 1 GB300 at <=1e-6 rel e
 BYTES_PER_ELEM_TET = 4 * 4 + 8 * 3 * 4 + 2 * 8 * 4 * 7 + 16 * (4 * 7) ** 2 + 16 * 4 * 7  # 13,552
 # DRAM bytes per element of the mixed tet interior pass (point and matrix kernels; the
 # point kernel's clear of A and b included):
-# dram__bytes_read.sum + dram__bytes_write.sum from ncu on the 163,618-tet mesh of the
-# 30^3 lattice, whose CSR bytes per element (1,002) match the 1.0M-tet mesh's (982);
-# scaled by the element count (profiles/dram_traffic_tet4_lattice30_assembly.md).
-TRAFFIC_BYTES_PER_ELEM_TET = 10502
+# dram__bytes_read.sum + dram__bytes_write.sum from ncu on a mesh of 162,000 tets, whose CSR
+# bytes per element match the 1.0M-tet mesh's; scaled by the element count
+# (profiles/interior_kernels.md).
+TRAFFIC_BYTES_PER_ELEM_TET = 7380
 LATTICE_N = 54
 
 
@@ -64,12 +64,11 @@ def peaks():
         return {}
 
 
-# Per-element instruction counts of the mixed tet pass (3 components), from ncu on the
-# 163,618-tet mesh of the 30^3 lattice (profiles/point_matrix_kernels_mixed_tet4_lattice30.md):
-# FP64 thread instructions per quadrature point of the point kernel and warp
-# instructions per element of the matrix kernel.
+# Per-element instruction counts of the mixed tet pass (3 components), from ncu on a mesh of
+# 162,000 tets (profiles/interior_kernels.md): FP64 thread instructions per quadrature point of
+# the point kernel and warp instructions per element of the row kernel.
 POINT_FP64_PER_POINT = {"dfma": 193.5, "dmul_dadd": 197.2}
-MATRIX_WARP_INST_PER_ELEM = 2758
+MATRIX_WARP_INST_PER_ELEM = 2038
 NQ_TET = 4
 
 
@@ -215,11 +214,10 @@ def cpu_oracle_rate(mesh, mat, setup, I, P, dt, row_ptr, col, colour, n_colours,
 
 BYTES_PER_ELEM_HEX = 4 * 8 + 8 * 3 * 8 + 2 * 8 * 8 * 8 + 16 * (8 * 8) ** 2 + 16 * 8 * 8  # 67,808
 # DRAM bytes per element of the mixed hex interior pass, from ncu on the 64,000-hex mesh
-# of a 40^3 grid in one chunk with a separate clear kernel, like the chunks of the
-# 160x160x156 assembly (point records far larger than L2); CSR bytes per element 14,172,
-# 1.9% above that mesh's 13,911; scaled by the element count
-# (profiles/dram_traffic_hex8_40cube_assembly.md, capture B).
-TRAFFIC_BYTES_PER_ELEM_HEX = 64817
+# of a 40^3 grid in one chunk (point records far larger than L2) less the clear of its CSR
+# values, 13,911 bytes per element, which the chunks of the 160x160x156 assembly leave to a
+# separate kernel; scaled by the element count (profiles/interior_kernels.md).
+TRAFFIC_BYTES_PER_ELEM_HEX = 60800
 
 
 def top_gas_flux_lambda(mesh, mat, I, nd):
@@ -361,7 +359,7 @@ def hex_block(args, torch, dev, with_clocks=False):
         "roofline": {"bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s",
                      "frac": ach / hbm if hbm else None, "traffic": TRAFFIC_BYTES_PER_ELEM_HEX * ne,
                      "traffic_source": "ncu DRAM bytes per element of the interior pass on 64,000 hexes x elements",
-                     "kernel": "interior pass (point_kernel + matrix_kernel, mixed form)",
+                     "kernel": "interior pass (point_kernel + rows32_kernel, mixed form)",
                      "kernel_ms": k_mx, "bytes_per_element": BYTES_PER_ELEM_HEX,
                      "peak_source": "measured (MEASURED_PEAKS.json)"},
         "objective_vjp": {"J": Jval, "ms": vjp_ms,
@@ -812,8 +810,8 @@ def main():
                                                "against the oracle on this mesh (<= 1e-12)"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                      "frac": (achieved / hbm) if hbm else None, "traffic": TRAFFIC_BYTES_PER_ELEM_TET * ne,
-                     "traffic_source": "ncu DRAM bytes per element of the interior pass on 163,618 tets x elements",
-                     "kernel": "interior pass (point_kernel + matrix_kernel, mixed form)", "kernel_ms": k_mx,
+                     "traffic_source": "ncu DRAM bytes per element of the interior pass on 162,000 tets x elements",
+                     "kernel": "interior pass (point_kernel + rows32_kernel, mixed form)", "kernel_ms": k_mx,
                      "bytes_per_element": BYTES_PER_ELEM_TET, "peak_source": "measured (MEASURED_PEAKS.json)"},
         "e2e": {"value": whole_job_rate(ne, e2e_s * 1e3, world), "unit": "elements/s",
                 "h2d_bytes_per_step": 2 * fa.n_rows * 8, "d2h_bytes_per_step": (nnz + fa.n_rows) * 8,
