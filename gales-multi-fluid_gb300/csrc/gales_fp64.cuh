@@ -1040,14 +1040,17 @@ __device__ __forceinline__ void simplex_row64(const KParams& k, const double* __
 // time: with the rows of one block side by side two thirds of the cycles waited for
 // instructions (54 ms for 998,250 tets with 7 dofs, 25 in this order; any group from 152 CTAs
 // up does).  Bound: the FP64 pipe, 83% busy with 1,757 instructions per row and 32 elements:
-// 23.3 ms for those tets, where a lane per block row that formed FPT_b took 57.
+// 23.3 ms for those tets, where a lane per block row that formed FPT_b took 57.  CTAs of
+// kRows64Warps warps; of one where the launch has fewer than 16 warps for each SM, which they
+// spread evenly (4,096 triangles with 5 dofs: 53 us against 63; 4,374 tets with 7: 151 against
+// 163; from 16 warps on no difference).
 constexpr int kRows64Warps = 4;
 constexpr int kRows64Group = 304;   // CTAs whose blocks are taken row by row (two per SM)
 
 template <int DIM, int NC>
 struct Rows64Smem {
   static constexpr int N = (DIM + 1) * Layout<DIM, NC>::ND, NS = N + 1;
-  double st[kRows64Warps][32 * NS], acc[kRows64Warps][32 * NS];
+  double st[32 * NS], acc[32 * NS];   // a warp's
 };
 
 template <int DIM, int NC>
@@ -1059,16 +1062,17 @@ __global__ void __launch_bounds__(32 * kRows64Warps)
   constexpr int ND = R::ND, N = R::N, EB = R::EB, NS = SM::NS;
   static_assert(EB == 32, "a lane per element of a block");
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  double* st = reinterpret_cast<SM*>(smem_raw)->st[threadIdx.x >> 5];
-  const int lane = threadIdx.x & 31;
-  double* acc = reinterpret_cast<SM*>(smem_raw)->acc[threadIdx.x >> 5] + lane * NS;
-  const long long nblk = (n + EB - 1) / EB, ncta = (nblk + kRows64Warps - 1) / kRows64Warps;
+  SM& sm = reinterpret_cast<SM*>(smem_raw)[threadIdx.x >> 5];
+  double* st = sm.st;
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  double* acc = sm.acc + lane * NS;
+  const long long nblk = (n + EB - 1) / EB, ncta = (nblk + warps - 1) / warps;
   // CTA order: groups of kRows64Group CTAs' blocks, all of a group's first rows, then its second
   const long long gi = (long long)blockIdx.x / ((long long)kRows64Group * ND);
   const long long c0 = gi * kRows64Group, nc = ncta - c0 < kRows64Group ? ncta - c0 : kRows64Group;
   const long long u = (long long)blockIdx.x - c0 * ND;
   const int r = (int)(u / nc);
-  const long long b0 = (c0 + u % nc) * kRows64Warps + (threadIdx.x >> 5);
+  const long long b0 = (c0 + u % nc) * warps + (threadIdx.x >> 5);
   if (b0 >= nblk) return;
   const int cnt = (int)(n - b0 * EB < EB ? n - b0 * EB : EB);
   const long long li = b0 * EB + (lane < cnt ? lane : cnt - 1);

@@ -93,7 +93,7 @@ struct Simplex64Inst {
     return nb > 0 ? nb : 1;
   }
   static cudaError_t prepare() {
-    return cudaFuncSetAttribute(rows64_kernel<DIM, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    return cudaFuncSetAttribute(rows64_kernel<DIM, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kRows64Warps * kSmem));
   }
   static LaunchResult point(const KParams& k, bool want_m, void* buf, long long first, long long n, cudaStream_t st) {
     if (n <= 0) return {cudaSuccess, 0};
@@ -111,8 +111,9 @@ struct Simplex64Inst {
       residual64_kernel<DIM, NEN, NC><<<(unsigned)((tasks + 3) / 4), 128, 0, st>>>(k, in, first, n);
       return {cudaGetLastError(), 1};
     }
-    const long long nblk = (n + R::EB - 1) / R::EB, ncta = (nblk + kRows64Warps - 1) / kRows64Warps * R::ND;
-    rows64_kernel<DIM, NC><<<(unsigned)ncta, 32 * kRows64Warps, kSmem, st>>>(k, in, first, n);
+    const int w = tasks < 16ll * k.sms ? 1 : kRows64Warps;   // see rows64_kernel
+    const long long nblk = (n + R::EB - 1) / R::EB, ncta = (nblk + w - 1) / w * R::ND;
+    rows64_kernel<DIM, NC><<<(unsigned)ncta, 32 * w, w * kSmem, st>>>(k, in, first, n);
     return dirichlet64<DIM, NEN, NC>(k, in, n, st);
   }
 };
