@@ -34,12 +34,14 @@
 // bulk copies bring them into one of two buffers in shared memory while the CTA works on the
 // other point.  CTAs of one row r of kRows32Group blocks run side by side: with all rows of a
 // block side by side the code of eight rows would not stay in the instruction cache.
-// Bound: instruction issue (2.6 of 4 per cycle, 57% of them FP32 arithmetic; ncu on 64,000
-// hexahedra with 6 dofs).  1.0M tets with 7 dofs: 2.61 ms, half a million hexahedra with 8:
-// 8.70.  A lane per (element, row), with r and b known at run time only and t_b formed in shared
-// memory by an extra pass, took 3.73 and 13.6; this mapping with the words loaded where they are
-// used, without the bulk copies, 3.26 and 10.9.  Fifth of a register file per CTA of 4 warps,
-// half for 8: 2.58 / 2.78 ms with six / four CTAs of tets, 12.3 with three of hexahedra.
+// Bound: instruction issue (2.6 of 4 per cycle, 57% of them FP32 arithmetic before its
+// multiply-adds over the columns were paired, see fma2; ncu on 64,000 hexahedra with 6 dofs).
+// Whole pass of 1.0M tets with 7 dofs: 6.11 ms, 6.21 without the pairs; of half a million
+// hexahedra with 8: 14.4 and 15.1.  The rows alone, without the pairs: 2.61 and 8.70 ms; a lane
+// per (element, row), with r and b known at run time only and t_b formed in shared memory by an
+// extra pass, took 3.73 and 13.6; this mapping with the words loaded where they are used,
+// without the bulk copies, 3.26 and 10.9.  Five CTAs of 4 warps a multiprocessor, two of 8: 2.58
+// and 2.78 ms with six and four CTAs of tets, 12.3 with three of hexahedra.
 #pragma once
 
 #include "gales_kernels.cuh"
@@ -103,6 +105,41 @@ struct KSums {
   S mu, lambda, kappa, muv[DIM], lamv[DIM], rhoD[L::NYA], rhoDH[L::NYA];
 };
 
+// Two binary32 operations in one instruction (fma.rn.f32x2 and its kin): each half rounds like
+// the single operation, and the pair takes one issue slot.
+__device__ __forceinline__ void fma2(float& x0, float& x1, float s, float y0, float y1) {   // x += s y
+  asm("{ .reg .b64 a, b, c;\n mov.b64 a, {%2, %2};\n mov.b64 b, {%3, %4};\n mov.b64 c, {%0, %1};\n"
+      " fma.rn.f32x2 c, a, b, c;\n mov.b64 {%0, %1}, c; }"
+      : "+f"(x0), "+f"(x1)
+      : "f"(s), "f"(y0), "f"(y1));
+}
+__device__ __forceinline__ void mul2(float& x0, float& x1, float s, float y0, float y1) {   // x = s y
+  asm("{ .reg .b64 a, b;\n mov.b64 a, {%2, %2};\n mov.b64 b, {%3, %4};\n mul.rn.f32x2 a, a, b;\n mov.b64 {%0, %1}, a; }"
+      : "=f"(x0), "=f"(x1)
+      : "f"(s), "f"(y0), "f"(y1));
+}
+__device__ __forceinline__ void add2(float& x0, float& x1, float y0, float y1) {   // x += y
+  asm("{ .reg .b64 a, b;\n mov.b64 a, {%0, %1};\n mov.b64 b, {%2, %3};\n add.rn.f32x2 a, a, b;\n mov.b64 {%0, %1}, a; }"
+      : "+f"(x0), "+f"(x1)
+      : "f"(y0), "f"(y1));
+}
+// x[j] += s y[j] over the columns that sel names, in the pairs (v1 v2), (v3 p), (T Y1), ... of 3D
+// or (v1 v2), (p T), (Y1 Y2), ... of 2D.
+template <int DIM, int ND, typename Sel>
+__device__ __forceinline__ void row_axpy(float (&x)[ND], float s, const float (&y)[ND], Sel sel) {
+  auto col = [](int i) { return i <= DIM ? (i + 1) % (DIM + 1) : i; };
+#pragma unroll
+  for (int i = 0; i < ND; i += 2) {
+    const int j0 = col(i), j1 = i + 1 < ND ? col(i + 1) : j0;
+    if (j1 != j0 && sel(j0) && sel(j1)) {
+      fma2(x[j0], x[j1], s, y[j0], y[j1]);
+    } else {
+      if (sel(j0)) x[j0] = fmaf(s, y[j0], x[j0]);
+      if (j1 != j0 && sel(j1)) x[j1] = fmaf(s, y[j1], x[j1]);
+    }
+  }
+}
+
 // Adds sum_kl gb_k K_kl(ROW, :) ga_l to a row of one (b, a) block (the closed form of
 // the contraction; fluid_2d.hpp:531-571):
 //   velocity row v_j: mu gb_m ga_j + lambda gb_j ga_m + mu (gb.ga) d_mj  on column v_m
@@ -133,18 +170,25 @@ __device__ __forceinline__ void viscous_row32(float (&acc)[Layout<DIM, NC>::ND],
         p2 = fmaf(gb[d], ks.lamv[d], p2);
       }
     }
-#pragma unroll
-    for (int m = 0; m < DIM; ++m) {
-      float x = fmaf(gb[m], p1, __fmul_rn(ga[m], p2));
-      if constexpr (cE) x = fmaf(ks.muv[m], gg, x);
-      if (cV && m == J) x = __fadd_rn(x, __fmul_rn(ks.mu, gg));
-      acc[1 + m] = __fadd_rn(acc[1 + m], x);
+    float x[DIM];
+    mul2(x[0], x[1], p2, ga[0], ga[1]);
+    fma2(x[0], x[1], p1, gb[0], gb[1]);
+    if constexpr (cE) fma2(x[0], x[1], gg, ks.muv[0], ks.muv[1]);
+    if constexpr (DIM == 3) {
+      x[2 % DIM] = fmaf(gb[2 % DIM], p1, __fmul_rn(ga[2 % DIM], p2));
+      if constexpr (cE) x[2 % DIM] = fmaf(ks.muv[2 % DIM], gg, x[2 % DIM]);
     }
+    if constexpr (cV) x[J] = __fadd_rn(x[J], __fmul_rn(ks.mu, gg));
+    add2(acc[1], acc[2], x[0], x[1]);
+    if constexpr (DIM == 3) acc[3] = __fadd_rn(acc[3], x[2 % DIM]);
   }
   if constexpr (cE) {
-    acc[L::iT] = fmaf(ks.kappa, gg, acc[L::iT]);
+    constexpr int ND = L::ND;
+    float y[ND];
+    y[L::iT] = ks.kappa;
 #pragma unroll
-    for (int y = 0; y < NC - 1; ++y) acc[L::iY + y] = fmaf(ks.rhoDH[y], gg, acc[L::iY + y]);
+    for (int i = 0; i < NC - 1; ++i) y[L::iY + i] = ks.rhoDH[i];
+    row_axpy<DIM, ND>(acc, gg, y, [](int j) { return j >= L::iT; });
   }
   if constexpr (cY) acc[ROW] = fmaf(ks.rhoD[IY], gg, acc[ROW]);
 }
@@ -296,10 +340,10 @@ __device__ __forceinline__ bool row32(const KParams& k, const float* __restrict_
         FD[j] = x;
         Dr[j] = dd;
       }
-      float hv[DIM];
+      float hv[ND];   // velocity columns
       const float fe = cE ? __fmul_rn(rho, __fadd_rn(F[iT], Nb)) : rF;
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) hv[d] = -fmaf(ur, gb[d], __fmul_rn(fe, k.gravity_f[d]));
+      for (int d = 0; d < DIM; ++d) hv[1 + d] = -fmaf(ur, gb[d], __fmul_rn(fe, k.gravity_f[d]));
       const float beta = fmaf(Nb, idt, -sb);
       KSums<DIM, NC, float> ks;
       float nu_j = 0.f;
@@ -334,31 +378,26 @@ __device__ __forceinline__ bool row32(const KParams& k, const float* __restrict_
         for (int d = 0; d < DIM; ++d) fk = fmaf(ga[d], F[1 + d], fk);
         const float A1 = __fmul_rn(jx, fmaf(Na, idt, sa)), A4 = __fmul_rn(jx, Na), A2 = __fmul_rn(A4, beta);
         const float f0 = (cV || cE) ? fmaf(-Na, kap, fk) : fk;
-        acc[a][0] = fmaf(A1, FD[0], fmaf(A2, Dr[0], fmaf(jx, f0, acc[a][0])));
+        acc[a][0] = fmaf(jx, f0, acc[a][0]);
+        float gv[ND];
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) {
-          float x = fmaf(A3, ga[d], fmaf(A4, hv[d], acc[a][1 + d]));
-          if (dnz(1 + d)) x = fmaf(A2, Dr[1 + d], x);
-          acc[a][1 + d] = fmaf(A1, FD[1 + d], x);
-        }
-#pragma unroll
-        for (int j = iT; j < ND; ++j) acc[a][j] = fmaf(A1, FD[j], fmaf(A2, Dr[j], acc[a][j]));
+        for (int d = 0; d < DIM; ++d) gv[1 + d] = ga[d];
+        row_axpy<DIM, ND>(acc[a], A4, hv, isV);
+        row_axpy<DIM, ND>(acc[a], A3, gv, isV);
+        row_axpy<DIM, ND>(acc[a], A2, Dr, dnz);
+        row_axpy<DIM, ND>(acc[a], A1, FD, [](int) { return true; });
         if constexpr (!AFF) {
           viscous_row32<DIM, NC, ROW>(acc[a], ks, gb, ga);
           float gg = __fmul_rn(gb[0], ga[0]);
 #pragma unroll
           for (int d = 1; d < DIM; ++d) gg = fmaf(gb[d], ga[d], gg);
           const float gn = __fmul_rn(gg, nu_j);
-#pragma unroll
-          for (int j = 0; j < ND; ++j)
-            if (dnz(j)) acc[a][j] = fmaf(gn, Dr[j], acc[a][j]);
+          row_axpy<DIM, ND>(acc[a], gn, Dr, dnz);
         }
       }
       if constexpr (AFF) {
         const float jn = __fmul_rn(jx, c(GALES_W(nu)));
-#pragma unroll
-        for (int j = 0; j < ND; ++j)
-          if (dnz(j)) Dnu[j] = fmaf(jn, Dr[j], Dnu[j]);
+        row_axpy<DIM, ND>(Dnu, jn, Dr, dnz);
         if constexpr (cV || cE) {
           const float mu = c(GALES_W(mu)), lam = c(GALES_W(lambda));
           ksum.mu = fmaf(jx, mu, ksum.mu);
@@ -395,9 +434,7 @@ __device__ __forceinline__ bool row32(const KParams& k, const float* __restrict_
       float gg = __fmul_rn(gb[0], gaf[AFF ? a : 0][0]);
 #pragma unroll
       for (int d = 1; d < DIM; ++d) gg = fmaf(gb[d], gaf[AFF ? a : 0][d], gg);
-#pragma unroll
-      for (int j = 0; j < ND; ++j)
-        if (dnz(j)) acc[a][j] = fmaf(gg, Dnu[j], acc[a][j]);
+      row_axpy<DIM, ND>(acc[a], gg, Dnu, dnz);
     }
   }
   return true;
