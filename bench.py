@@ -68,7 +68,7 @@ def peaks():
 # 162,000 tets (profiles/interior_kernels.md): FP64 thread instructions per quadrature point of
 # the point kernel and warp instructions per element of the row kernel.
 POINT_FP64_PER_POINT = {"dfma": 193.5, "dmul_dadd": 197.2}
-MATRIX_WARP_INST_PER_ELEM = 2038
+MATRIX_WARP_INST_PER_ELEM = 1932
 NQ_TET = 4
 
 
