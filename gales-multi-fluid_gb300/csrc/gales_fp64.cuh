@@ -75,25 +75,37 @@ struct Rec64 {
   }
 };
 
-// compute_h with fused operations and no divisions but the last, where the direction s1 is
-// well conditioned (|s1| > 1e-3 |dv v|: its relative error stays below ~1e-13); elsewhere
-// decided = false and the caller takes the reference's operations (compute_h_reference), whose
-// branches hang on rounding.
+// The largest |dv[i][j]|, rounded up in its last 32 bits (integer comparisons: free beside FP64).
 template <int DIM>
-__device__ __forceinline__ double compute_h64(const double (&G)[DIM][DIM], const double* v, double iv,
-                                              const double (&dv)[DIM][DIM], bool& decided) {
+__device__ __forceinline__ double max_entry(const double (&dv)[DIM][DIM]) {
+  int m = 0;
+#pragma unroll
+  for (int i = 0; i < DIM; ++i)
+#pragma unroll
+    for (int j = 0; j < DIM; ++j) m = max(m, __double2hiint(dv[i][j]) & 0x7fffffff);
+  return __hiloint2double(m, -1);
+}
+
+// compute_h with fused operations and no divisions but the last, where the direction s1 is
+// well conditioned: |s1| > 1e-3 max|dv| |v| keeps its relative error below ~1e-12.  The bound has
+// the size of the terms that dv v sums, not of the sum: a shear flow oblique to the axes has
+// dv v = 0, and what rounding leaves of it points anywhere.  Elsewhere decided = false and
+// the caller takes the reference's operations (compute_h_reference), whose branches hang on
+// rounding.  dv carries the reference's roundings; mm = max|dv|^2.
+template <int DIM>
+__device__ __forceinline__ double compute_h64(const double (&G)[DIM][DIM], const double* v, double vv, double iv,
+                                              const double (&dv)[DIM][DIM], double mm, bool& decided) {
   decided = false;
   double s0[DIM], acc[DIM], w1[DIM];
 #pragma unroll
   for (int i = 0; i < DIM; ++i) s0[i] = v[i] * iv;
-  double aa = 0.0, ip = 0.0;
+  double ip = 0.0;
 #pragma unroll
   for (int i = 0; i < DIM; ++i) {
     double t = dv[i][0] * v[0];
 #pragma unroll
     for (int j = 1; j < DIM; ++j) t = fma(dv[i][j], v[j], t);
     acc[i] = t;
-    aa = fma(t, t, aa);
     ip = fma(t, s0[i], ip);
   }
   double n1 = 0.0;
@@ -103,7 +115,7 @@ __device__ __forceinline__ double compute_h64(const double (&G)[DIM][DIM], const
     n1 = fma(w1[i], w1[i], n1);
   }
   constexpr double kMin2 = 1.0e6 * kEps * kEps;  // (1e3 DBL_EPSILON)^2
-  if (!(n1 > fmax(1.0e-6 * aa, kMin2))) return 0.0;
+  if (!(n1 > fmax(1.0e-6 * (vv * mm), kMin2))) return 0.0;
   const double A0 = qform_fma<DIM>(G, s0), A1 = qform_fma<DIM>(G, w1);
   if (A0 == 0.0 || A1 == 0.0) return 0.0;
   // h = 2 sqrt|1/A0 + n1/A1 (+ n2/A2)| = 2 sqrt|num / den|
@@ -327,6 +339,10 @@ __device__ __forceinline__ void point64(const KParams& k, long long e, int iq, d
       Iq[j] = fma(sh[i], Ie[i][j], Iq[j]);
     }
   }
+  // Gradients, summed with the reference's operations: where a field is uniform over the element
+  // what rounding leaves of its gradient decides the directions of h and, through grad rho,
+  // whether and along what the discontinuity capturing acts.  (With fused sums the blocks of such
+  // elements differed from the reference's in their leading digits.)
   double dI[DIM][ND];
   if constexpr (NEN == DIM + 1 && NQ <= 32 && (32 % NQ) == 0) {
     // a simplex's gradient is the same at its points, whose lanes are consecutive: lane iq
@@ -348,7 +364,7 @@ __device__ __forceinline__ void point64(const KParams& k, long long e, int iq, d
 #pragma unroll
         for (int j = 1; j < ND; ++j) a = (jc == j) ? Ie[i][j] : a;
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) colv[sl][d] = fma(q.ds[d][i], a, colv[sl][d]);
+        for (int d = 0; d < DIM; ++d) colv[sl][d] = add_rn(colv[sl][d], mul_rn(q.ds[d][i], a));
       }
     }
 #pragma unroll
@@ -360,9 +376,9 @@ __device__ __forceinline__ void point64(const KParams& k, long long e, int iq, d
     for (int d = 0; d < DIM; ++d)
 #pragma unroll
       for (int j = 0; j < ND; ++j) {
-        double b = q.ds[d][0] * Ie[0][j];
+        double b = mul_rn(q.ds[d][0], Ie[0][j]);
 #pragma unroll
-        for (int i = 1; i < NEN; ++i) b = fma(q.ds[d][i], Ie[i][j], b);
+        for (int i = 1; i < NEN; ++i) b = add_rn(b, mul_rn(q.ds[d][i], Ie[i][j]));
         dI[d][j] = b;
       }
   }
@@ -375,6 +391,10 @@ __device__ __forceinline__ void point64(const KParams& k, long long e, int iq, d
   double p, v[DIM], T, Y[NC], U[ND], UP[ND];
   Props<NC> pr;
   Coef<DIM, NC> c;
+  double vv, trG = 0.0;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) trG += q.G[d][d];
+  const double mdv = max_entry<DIM>(dv), mm = mdv * mdv;
   {
     double pP, vP[DIM], TP, YP[NC], rhoP, cvP;
     assign<DIM, NC>(Pq, pP, vP, TP, YP);
@@ -394,11 +414,31 @@ __device__ __forceinline__ void point64(const KParams& k, long long e, int iq, d
       // a gas has no sound speed below T = 0 (chemicals.hpp:258-264)
       if (k.has_gas && !(T >= 0.0)) pr.c = __longlong_as_double(0x7ff8000000000000ll);
     }
+    auto speed2 = [&]() {
+      double s = v[0] * v[0];
+#pragma unroll
+      for (int d = 1; d < DIM; ++d) s = fma(v[d], v[d], s);
+      return s;
+    };
+    vv = speed2();
+    // |v| below 1e-6 of its variation over the element: the reference's sums decide whether it
+    // is zero and where it points
+    if (vv * trG < 1.0e-12 * mm) {
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) {
+        double x = 0.0, y = 0.0;
+#pragma unroll
+        for (int i = 0; i < NEN; ++i) {
+          x = add_rn(x, mul_rn(sh[i], __ldg(k.I + (long long)nodes[i] * ND + 1 + d)));
+          y = add_rn(y, mul_rn(sh[i], __ldg(k.P + (long long)nodes[i] * ND + 1 + d)));
+        }
+        Iq[1 + d] = v[d] = x;
+        Pq[1 + d] = vP[d] = y;
+      }
+      vv = speed2();
+    }
     conservative<DIM, NC>(rhoP, cvP, vP, TP, YP, UP);
   }
-  double vv = v[0] * v[0];
-#pragma unroll
-  for (int d = 1; d < DIM; ++d) vv = fma(v[d], v[d], vv);
   make_coef_fast<DIM, NC>(pr, p, v, vv, T, Y, c);
   U[0] = c.rho;
 #pragma unroll
@@ -418,11 +458,8 @@ __device__ __forceinline__ void point64(const KParams& k, long long e, int iq, d
 #pragma unroll
   for (int i = 0; i < L::NYA; ++i) tb[i] = tn[i] = 0.0;
   if (v_nrm >= kEps && k.tau != GALES_TAU_NONE) {
-    double trG = 0.0;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) trG += q.G[d][d];
     bool decided;
-    double h = compute_h64<DIM>(q.G, v, iv, dv, decided);
+    double h = compute_h64<DIM>(q.G, v, vv, iv, dv, mm, decided);
     if (!decided) h = compute_h_reference<DIM, NEN, ND>(k.I, nodes, sh, q);
     double td[ND];
     const bool nondiag = tau_params<DIM, NEN, NC, EOS>(k, q, c, pr, v, v_nrm, h, trG, td);
