@@ -440,12 +440,7 @@ __device__ __forceinline__ void point64(const KParams& k, long long e, int iq, d
     conservative<DIM, NC>(rhoP, cvP, vP, TP, YP, UP);
   }
   make_coef_fast<DIM, NC>(pr, p, v, vv, T, Y, c);
-  U[0] = c.rho;
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) U[1 + d] = c.rho * v[d];
-  U[iT] = c.rho * c.E;
-#pragma unroll
-  for (int i = 0; i < NC - 1; ++i) U[iY + i] = c.rho * Y[i];
+  conservative<DIM, NC>(pr.rho, pr.cv, v, T, Y, U);
   const double iv = rsqrt(vv), v_nrm = vv > 0.0 ? vv * iv : 0.0;
   const double uE = U[iT] + p;   // energy entry of u'
   // tau (fluid_2d.hpp:877-1022): dense rows p and E, the velocity and mass-fraction rows'

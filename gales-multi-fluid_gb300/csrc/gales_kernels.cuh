@@ -633,12 +633,7 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
 #pragma unroll
   for (int d = 1; d < DIM; ++d) vv = fma(v[d], v[d], vv);
   make_coef_fast<DIM, NC>(pr, p, v, vv, T, Y, c);
-  U[0] = pr.rho;
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) U[1 + d] = pr.rho * v[d];
-  U[L::iT] = pr.rho * c.E;
-#pragma unroll
-  for (int i = 0; i < NC - 1; ++i) U[L::iY + i] = pr.rho * Y[i];
+  conservative<DIM, NC>(pr.rho, pr.cv, v, T, Y, U);
   iv = rsqrt(vv);
   v_nrm = vv > 0.0 ? vv * iv : 0.0;
   const double dt = k.dt;

@@ -88,7 +88,7 @@ GALES_MAGMA_HD double where_real(double y, double x) { return y >= 0.0 ? x : NAN
 
 // magma_mixture::properties (mixtures.hpp:163-176, submix_of_comp 187-250) of the melt
 // (Lange-Carmichael volume), dissolved H2O and CO2 (one molar volume polynomial V(p, T),
-// chemicals.hpp:155-160) and the two gases.  FULL false: rho, cv and the status bits alone.
+// chemicals.hpp:155-160) and the two gases.  FULL false: rho (and 1/rho), cv and the status bits alone.
 //
 // Bound: FP64 operations, of which a division or square root is about ten and a library power
 // over a hundred.  The constituents enter through 1/rho_c, alpha_c/rho_c, beta_c/rho_c and
@@ -129,6 +129,7 @@ GALES_MAGMA_HD void magma_props(const DevMagma& g, double p, double T, double sr
   // cv = cp - T alpha^2/(rho beta)
   const double qV = T * (VT * VT / Vp);
   o.rho = rho;
+  o.ir = g.crystal_vf == 0.0 ? ir : 1.0 / rho;
   o.cv = wf[0] * (g.melt_cp - T * g.melt_q) + wf[1] * (g.vol_cp[0] - qV * g.vol_iM[0]) +
          wf[2] * (g.vol_cp[1] - qV * g.vol_iM[1]) + wf[3] * g.gas_cv[0] + wf[4] * g.gas_cv[1];
   if (!FULL) {
@@ -137,7 +138,6 @@ GALES_MAGMA_HD void magma_props(const DevMagma& g, double p, double T, double sr
   }
   const double Rg = wf[3] * g.gas_R[0] + wf[4] * g.gas_R[1];
   const double bl = where_real(-g.melt_dVdp, m0 * -g.melt_dVdp) + where_real(Vp, m12 * Vp);
-  o.ir = g.crystal_vf == 0.0 ? ir : 1.0 / rho;
   o.alpha = rho * fma(m0, g.melt_dVdT, fma(m12, VT, Rg * ip));
   o.beta = rho * fma(m0, -g.melt_dVdp, fma(m12, Vp, Rg * (Tp * ip)));
   o.ic2 = bl + (T > 0.0 ? (wf[3] * g.gas_R[0] * g.gas_ig[0] + wf[4] * g.gas_R[1] * g.gas_ig[1]) * (Tp * ip) : NAN);
@@ -232,7 +232,7 @@ GALES_MAGMA_HD unsigned mix_point(const DevMagma* mg, int nc, double p, double T
     irho = fma(y, m.ir, irho);
     mu += y * m.mu;
     cp += y * m.cp;
-    cv += y * m.cv;
+    cv = fma(y, m.cv, cv);
     kappa += y * m.kappa;
     ss += y * m.ic2;
     alpha = fma(yr, m.alpha, alpha);
@@ -255,7 +255,8 @@ GALES_MAGMA_HD unsigned mix_point(const DevMagma* mg, int nc, double p, double T
 }
 
 // rho and cv of mix_point at shear rate 0, with its status bits (the state at the previous time
-// level, of which the assembly reads nothing else).
+// level, of which the assembly reads nothing else): its operations, so that equal states have
+// equal rho and cv.
 GALES_MAGMA_HD unsigned mix_rho_cv(const DevMagma* mg, int nc, double p, double T, const double* Y, double& rho,
                                    double& cv) {
   unsigned st = 0;
@@ -264,8 +265,8 @@ GALES_MAGMA_HD unsigned mix_rho_cv(const DevMagma* mg, int nc, double p, double 
     Props m;
     double vfg;
     sub_props<false>(mg[c], p, T, 0.0, m, vfg, st);
-    irho += Y[c] / m.rho;
-    x += Y[c] * m.cv;
+    irho = fma(Y[c], m.ir, irho);
+    x = fma(Y[c], m.cv, x);
   }
   rho = 1.0 / irho;
   cv = x;

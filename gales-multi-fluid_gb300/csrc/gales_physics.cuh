@@ -321,18 +321,23 @@ __device__ __forceinline__ double vsq(const double* v) {
   return s;
 }
 
-// U(): fluid_2d.hpp:372-385
+// U(): fluid_2d.hpp:372-385, for both time levels: the same operations, and products that no
+// later difference can absorb, so that equal states have U - U_P = 0 (the predictor starts
+// every time step from I = P).  E and |v|^2 are rounded as in make_coef_fast.
 template <int DIM, int NC>
 __device__ __forceinline__ void conservative(double rho, double cv, const double* v, double T,
                                              const double* Y, double* u) {
   using L = Layout<DIM, NC>;
-  const double E = cv * T + 0.5 * (vsq<DIM>(v));
+  double vv = v[0] * v[0];
+#pragma unroll
+  for (int k = 1; k < DIM; ++k) vv = fma(v[k], v[k], vv);
+  const double E = fma(cv, T, 0.5 * vv);
   u[0] = rho;
 #pragma unroll
-  for (int k = 0; k < DIM; ++k) u[1 + k] = rho * v[k];
-  u[L::iT] = rho * E;
+  for (int k = 0; k < DIM; ++k) u[1 + k] = __dmul_rn(rho, v[k]);
+  u[L::iT] = __dmul_rn(rho, E);
 #pragma unroll
-  for (int i = 0; i < NC - 1; ++i) u[L::iY + i] = rho * Y[i];
+  for (int i = 0; i < NC - 1; ++i) u[L::iY + i] = __dmul_rn(rho, Y[i]);
 }
 
 template <int DIM, int NC>
