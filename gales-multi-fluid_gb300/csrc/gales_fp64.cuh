@@ -410,7 +410,7 @@ __device__ __forceinline__ void point64(const KParams& k, long long e, int iq, d
 #pragma unroll
       for (int i = 0; i < NC; ++i) pr.irho_c[i] = 1.0 / pr.rho_c[i];
     } else {
-      mixture_pair_fast<NC>(k.ch, k.has_gas != 0, pP, TP, YP, p, T, Y, rhoP, cvP, pr);
+      mixture_pair_fast<NC, true>(k.ch, k.has_gas != 0, pP, TP, YP, p, T, Y, rhoP, cvP, pr);
       // a gas has no sound speed below T = 0 (chemicals.hpp:258-264)
       if (k.has_gas && !(T >= 0.0)) pr.c = __longlong_as_double(0x7ff8000000000000ll);
     }

@@ -153,7 +153,13 @@ __host__ __device__ __forceinline__ void mixture(const DevChem* ch, double p, do
 // A gas's alpha_c/rho_c = R_c/p, beta_c/rho_c = R_c T/p^2 and 1/(rho_c^2 s_c^2) =
 // (R_c/gamma_c) T/p^2, so the gas sums need 1/p alone.  A material without a gas
 // (has_gas = 0) takes rho = 1/C, rho_P = 1/C_P and never divides by p.
-template <int NC>
+// APART (the FP64 form): where the previous level has no such mixture (a program that passes
+// zeros or NaN and wants the matrix or its frozen adjoint, which do not depend on P), its D_P or
+// C_P stays out of the shared division and rho_P alone carries it.
+__device__ __forceinline__ bool far_from_one(double x) {  // not within 2^-300 .. 2^300 (no FP64 operation)
+  return (unsigned)(((__double2hiint(x) >> 20) & 0x7ff) - (1023 - 300)) > 600u;
+}
+template <int NC, bool APART = false>
 __device__ __forceinline__ void mixture_pair_fast(const DevChem* ch, bool has_gas, double pP, double TP,
                                                   const double* YP, double p, double T, const double* Y,
                                                   double& rhoP, double& cvP, Props<NC>& o) {
@@ -189,10 +195,13 @@ __device__ __forceinline__ void mixture_pair_fast(const DevChem* ch, bool has_ga
   double rho, irho, ip;
   if (has_gas) {
     const double D = fma(T, G, p * C), DP = fma(TP, GP, pP * CP);
-    const double r = 1.0 / (p * D * DP);
-    ip = D * DP * r;
-    rho = p * p * DP * r;
+    const bool apart = APART && far_from_one(DP);
+    const double DQ = apart ? 1.0 : DP;
+    const double r = 1.0 / (p * D * DQ);
+    ip = D * DQ * r;
+    rho = p * p * DQ * r;
     rhoP = pP * p * D * r;
+    if (apart) rhoP = pP / DP;
     irho = D * ip;
     const double ip2 = ip * ip;
     c2 = fma(GRg * T, ip2, c2);
@@ -200,9 +209,11 @@ __device__ __forceinline__ void mixture_pair_fast(const DevChem* ch, bool has_ga
     be = fma(G * T, ip2, be);
   } else {
     ip = 0.0;
-    const double r = 1.0 / (C * CP);
-    rho = CP * r;
-    rhoP = C * r;
+    const bool apart = APART && far_from_one(CP);
+    const double CQ = apart ? 1.0 : CP;
+    const double r = 1.0 / (C * CQ);
+    rho = CQ * r;
+    rhoP = apart ? 1.0 / CP : C * r;
     irho = C;
   }
 #pragma unroll
