@@ -62,7 +62,7 @@ struct InteriorInst {
     rows32_kernel<DIM, NEN, NC, true><<<ctas, T::THREADS, 0, st>>>(k, in, first, n);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || !any_dirichlet(k) || k.local_r) return {e, 1};
-    dirichlet32_kernel<DIM, NEN, NC><<<(unsigned)((n + 127) / 128), 128, 0, st>>>(k, in, n);
+    dirichlet32_kernel<DIM, NEN, NC><<<(unsigned)((n + RB::EB - 1) / RB::EB), 32 * NEN, 0, st>>>(k, in, n);
     return {cudaGetLastError(), 2};
   }
 };

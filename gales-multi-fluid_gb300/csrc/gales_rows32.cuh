@@ -558,10 +558,21 @@ __global__ void __launch_bounds__(32 * NEN, NEN == 8 ? 2 : 5) rows32_kernel(cons
       // one element's row per step, consecutive lanes on consecutive columns
       double* vals = k.vals + cj;
       if (k.scatter_mode != 0) {
-        for (int el = 0; el < cnt; ++el) {
-          const int64_t to = at[el * HN + ca];
-          const float x = st[el * NS + lane];
-          if (to >= 0 && x != 0.f) vals[to] += widen(x);
+        // elements of one colour share no row: their adds are independent, eight in flight
+#pragma unroll 1
+        for (int e0 = 0; e0 < 32; e0 += 8) {
+          double v[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int64_t to = at[(e0 + i) * HN + ca];
+            v[i] = to >= 0 ? vals[to] : 0.0;
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int64_t to = at[(e0 + i) * HN + ca];
+            const float x = st[(e0 + i) * NS + lane];
+            if (to >= 0 && x != 0.f) vals[to] = v[i] + widen(x);
+          }
         }
         continue;
       }
@@ -590,34 +601,47 @@ __global__ void __launch_bounds__(32 * NEN, NEN == 8 ? 2 : 5) rows32_kernel(cons
 }
 
 // Diagonal of the blocked rows (Dirichlet): avg = (1 + trace)/n of the element block
-// (scatter.hpp:62-78), from the rows' shares of the trace in row order.
+// (scatter.hpp:62-78), from the rows' shares of the trace.  A CTA takes a block of elements, a
+// lane each; its NEN warps sum a part of the shares and then write one node's rows.  Bound:
+// latency, of three trips to L2: the masks, the shares with the descriptors, the entries of a
+// coloured scatter.  A thread per element with a loop over its nodes and dofs made such a trip
+// for each of them: 10 us a launch, and a coloured assembly has one for each colour (2.10 ms for
+// 82,800 tets of one component with 32 colours; 1.68 now).
 template <int DIM, int NEN, int NC>
-__global__ void __launch_bounds__(128) dirichlet32_kernel(const KParams k, const unsigned char* __restrict__ in, long long n) {
+__global__ void __launch_bounds__(32 * NEN) dirichlet32_kernel(const KParams k, const unsigned char* __restrict__ in, long long n) {
   using RB = RecBlock<DIM, NEN, NC>;
   using S = float;
   using QPT = QP<DIM, NEN, NC, S>;
   constexpr int ND = Layout<DIM, NC>::ND, N = NEN * ND, EB = RB::EB;
-  const long long li = (long long)blockIdx.x * 128 + threadIdx.x;
-  if (li >= n) return;
-  const int l = (int)(li % EB);
-  const unsigned char* blk = in + (size_t)(li / EB) * RB::BYTES;
-  const float* rec = reinterpret_cast<const float*>(blk) + l;
-  auto d_int = [&](int b, int f) { return word_int(rec[(size_t)(b * RB::RW + f) * EB]); };
-  uint32_t any = 0u;
-#pragma unroll
-  for (int b = 0; b < NEN; ++b) any |= (uint32_t)d_int(b, GALES_W(d_blocked));
-  if (any == 0u) return;
+  __shared__ double part[NEN][EB];
+  const int b = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const unsigned char* blk = in + (size_t)blockIdx.x * RB::BYTES;
+  const float* desc = reinterpret_cast<const float*>(blk) + (size_t)b * RB::RW * EB + l;
+  const bool on = (long long)blockIdx.x * EB + l < n;
+  const uint32_t bl = on ? (uint32_t)word_int(desc[GALES_W(d_blocked) * EB]) : 0u;
+  if (!__syncthreads_or(bl != 0u)) return;
   const double* tr = reinterpret_cast<const double*>(blk + RB::TR_OFF) + l;
   double s = 0.0;
-#pragma unroll 4
-  for (int i = 0; i < N; ++i) s += tr[(size_t)i * EB];
-  const double avg = (1.0 + s) * (1.0 / N);
-  for (int b = 0; b < NEN; ++b) {
-    const uint32_t bl = (uint32_t)d_int(b, GALES_W(d_blocked));
-    for (int r = 0; r < ND; ++r)
-      if ((bl >> r) & 1u)
-        add_to(k.vals + (int64_t)d_int(b, GALES_W(d_off) + b) * ND + (int64_t)r * d_int(b, GALES_W(d_rowlen)) + r, avg,
-               k.scatter_mode);
+  if (on)
+#pragma unroll
+    for (int i = 0; i < ND; ++i) s += tr[(size_t)(b * ND + i) * EB];
+  part[b][l] = s;
+  __syncthreads();
+  if (bl == 0u) return;
+  s = 1.0;
+#pragma unroll
+  for (int a = 0; a < NEN; ++a) s += part[a][l];
+  const double avg = s * (1.0 / N);
+  double* row = k.vals + (int64_t)word_int(desc[(GALES_W(d_off) + b) * EB]) * ND;
+  const int64_t step = word_int(desc[GALES_W(d_rowlen) * EB]) + 1;
+  double v[ND];
+#pragma unroll
+  for (int r = 0; r < ND; ++r) v[r] = k.scatter_mode != 0 && ((bl >> r) & 1u) ? row[r * step] : 0.0;
+#pragma unroll
+  for (int r = 0; r < ND; ++r) {
+    if (!((bl >> r) & 1u)) continue;
+    if (k.scatter_mode != 0) row[r * step] = v[r] + avg;
+    else atomicAdd(row + r * step, avg);
   }
 }
 
