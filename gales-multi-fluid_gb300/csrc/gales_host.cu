@@ -156,7 +156,13 @@ constexpr int kVjpAux = 3 * GALES_MAX_COMP + GALES_MAX_ND;
 // into chunks that shrink toward its end, after each of which the finished CSR rows
 // are copied.
 constexpr size_t kRecordBytes = size_t(3) << 30;
-constexpr int kCopyTail = 64;    // smallest host-buffer chunk: n / kCopyTail elements
+// Smallest host-buffer chunk: n / kCopyTail elements, and enough for rows of kCopyMin bytes:
+// 0.3 ms of the host link.  A chunk costs some 40 us of launches, events and a copy call, and the
+// chunks of a small mesh are short of work: with n / kCopyTail alone (12 chunks whatever the mesh)
+// a call of 1,500 triangles took 377 us, of 82,800 tets 1.13 ms; with 1, 4 and 16 MB 100, 100, 100
+// us and 1.11, 1.00, 0.97 ms, and 1.0M tets stay at 7.89 ms.
+constexpr int kCopyTail = 64;
+constexpr double kCopyMin = 16 << 20;
 constexpr int kCopyEvents = 24;  // row copies per host-buffer assembly (at most)
 
 GeometryOps geometry_ops(int dim, int nen) {
@@ -1105,8 +1111,13 @@ int run_interior(gales_asm* h, const KParams& k, int form, bool want_m, long lon
   if (rb == 0) return fail(h, GALES_ERR_UNSUPPORTED, "no interior kernel for this element/component count");
   const long long chunk = h->chunk_elems[form];
   // host-buffer calls: chunks that shrink toward the end of the pass (a third of what
-  // remains, down to n / 64), so that the rows copied after the last chunk are few
-  const long long tail = std::max<long long>(4, (n + kCopyTail - 1) / kCopyTail / 4 * 4);
+  // remains, down to the smallest), so that the rows copied after the last chunk are few;
+  // whole blocks of point records but for the last
+  const long long blk = ops.rec_block(h->nc);
+  const double bytes_per_el = (double)h->nnz * sizeof(double) / (double)std::max<long long>(n, 1);
+  const long long least = std::max<long long>((n + kCopyTail - 1) / kCopyTail,
+                                              (long long)std::min<double>((double)n, kCopyMin / bytes_per_el));
+  const long long tail = (least + blk - 1) / blk * blk;
   void* buf = h->qpbuf.p;
   KParams kl;  // the later chunks' parameters: nothing left to clear
   const KParams* kp = &k;
@@ -1115,7 +1126,7 @@ int run_interior(gales_asm* h, const KParams& k, int form, bool want_m, long lon
     long long cnt = chunk;
     if (rc) {
       const long long rem = n - first;
-      cnt = rem <= 2 * tail ? rem : std::max(tail, (rem / 3 + 3) / 4 * 4);
+      cnt = rem <= 2 * tail ? rem : std::max(tail, (rem / 3 + blk - 1) / blk * blk);
       cnt = std::min(cnt, chunk);
     }
     cnt = std::min(cnt, n - first);
