@@ -1245,6 +1245,7 @@ Ops ops_for() {
   return {K::cluster_size, K::prepare, K::to_factor, K::factor, K::scale_diag, K::sweeps, K::spmv};
 }
 
+// nd = 2 + dim + nb_comp - 1 with one to four components (gales_asm_create)
 template <typename T>
 bool ops_t(int nd, Ops& o) {
   switch (nd) {
@@ -1253,10 +1254,6 @@ bool ops_t(int nd, Ops& o) {
     case 6: o = ops_for<6, T>(); return true;
     case 7: o = ops_for<7, T>(); return true;
     case 8: o = ops_for<8, T>(); return true;
-    case 9: o = ops_for<9, T>(); return true;
-    case 10: o = ops_for<10, T>(); return true;
-    case 11: o = ops_for<11, T>(); return true;
-    case 12: o = ops_for<12, T>(); return true;
     default: return false;
   }
 }
