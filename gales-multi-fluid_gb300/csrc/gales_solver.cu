@@ -483,6 +483,9 @@ __global__ void __launch_bounds__(kFactorThreads)
 // unknown.  Ten warps per SM keep the next levels' rows loaded (M^-1 on a 157k-node system of
 // 372 levels with 4, 8 and 10 warps: 2.57, 1.72, 1.62 ms); a block's columns spread over the groups instead of a
 // block per group, with fewer products after the last arrival, was no faster (1.67).
+template <int ND>
+constexpr int kSweepBlocks = 56 / ND < 8 ? 56 / ND : 8;   // blocks per lane held in registers
+
 template <typename T>
 struct SweepWord;
 template <>
@@ -548,8 +551,7 @@ __global__ void __launch_bounds__(32 * kSweepWarps)
                      int64_t n, const double* __restrict__ vbase, const T* __restrict__ yin, T* zw, double* zoutbase,
                      const int* __restrict__ jidx, int64_t ld, unsigned int* ticket, unsigned int* status) {
   using W = SweepWord<T>;
-  constexpr int BB = ND * ND, G = 32 / ND;
-  constexpr int KB = 56 / ND < 8 ? 56 / ND : 8;   // blocks per lane held in registers
+  constexpr int BB = ND * ND, G = 32 / ND, KB = kSweepBlocks<ND>;
   const int lane = threadIdx.x & 31;
   const int g = lane / ND, r = lane < G * ND ? lane - g * ND : 0;
   const int64_t off = jidx ? (int64_t)(*jidx) * ld : 0;
@@ -651,8 +653,21 @@ __global__ void __launch_bounds__(32 * kSweepWarps)
 // row's last arrival.  M^-1 of a 2,145-node channel (161 levels, 5 dofs): 0.23 ms with an FP64
 // factor and 0.13 with FP32, against 0.41 and 0.24 through L2.  4 or 12 warps per CTA: 0.23,
 // 0.24; a block's columns spread over the lanes, each polling its own word: 0.22 and 0.15.
-constexpr int kClusterWarps = 8;
+// A cluster has 16 of the 152 SMs, so it suits systems whose time is their levels' latency:
+// kClusterBusy bounds the register loads of blocks that a warp makes per level (a load is 1.6 us
+// FP32, 3 FP64, a level through L2 0.85 and 1.8), kClusterBytes the factor's bytes per level (16
+// SMs with a few rows in flight each read 0.2 TB/s).  M^-1 in us, cluster and L2 (loads, KB per
+// level).  Better in the cluster: 350, 572 (quads, 4 dofs, FP32; 0.22, 12), 537, 685 (hexes, 8
+// dofs, FP64; 0.20, 224), 456, 513 (the same, longer; 0.25, 283), 561, 645 (hexes, ILU(2), FP32; 0.26,
+// 167), 266, 302 (triangles, ILU(0), FP32; 0.43, 12).  Through L2: 450, 392 (hexes, FP32; 0.34, 187),
+// 1,102, 904 (the same, ILU(3); 0.27, 203), 259, 244 (tets, 5 dofs, FP32; 0.52, 82), 177, 152
+// (tets, 7 dofs, ILU(0), FP64; 0.61, 207), 225, 124 (tets, ILU(0), FP32; 1.22, 109).  An FP64 system
+// that fits was never above 283 KB a level: that line is its L2 time per level at the same rate.
+constexpr int kClusterWarps = 8, kClusterMax = 16;
 constexpr size_t kClusterSmem = 200 * 1024;
+constexpr double kClusterBusy = 0.48;
+template <typename T>
+constexpr double kClusterBytes = sizeof(T) == 8 ? 380e3 : 180e3;
 template <typename T>
 constexpr bool kClusterScaled = sizeof(T) == 8;
 
@@ -736,8 +751,7 @@ __global__ void __launch_bounds__(32 * kClusterWarps)
                              const double* __restrict__ vbase, T* __restrict__ y, double* __restrict__ zoutbase,
                              const int* __restrict__ jidx, int64_t ld, unsigned int* status) {
   using W = SweepWord<T>;
-  constexpr int BB = ND * ND, G = 32 / ND;
-  constexpr int KB = 56 / ND < 8 ? 56 / ND : 8;   // blocks per lane held in registers
+  constexpr int BB = ND * ND, G = 32 / ND, KB = kSweepBlocks<ND>;
   extern __shared__ __align__(16) unsigned char sweep_smem[];
   T* z = reinterpret_cast<T*>(sweep_smem);
   const uint32_t z0 = (uint32_t)__cvta_generic_to_shared(z);
@@ -1120,7 +1134,8 @@ struct Kernels {
   };
   static size_t cluster_smem(const gales_solver* s) { return (size_t)s->n_rows * sizeof(T); }
   // Cluster size of the sweeps: the largest of 16 and 8 that the device takes, 0 where the
-  // result vector is too long for a CTA.
+  // result vector is too long for a CTA or the work too much for a cluster's SMs (see
+  // kClusterBusy, kClusterBytes).
   template <bool LOWER>
   static cudaError_t prepare_cluster(gales_solver* s, int& size) {
     const auto fn = ilu_sweep_cluster_kernel<ND, T, LOWER>;
@@ -1137,7 +1152,18 @@ struct Kernels {
     return cudaSuccess;
   }
   static int cluster_size(gales_solver* s) {
-    int size = cluster_smem(s) <= kClusterSmem && cluster_smem(s) <= (size_t)s->smem_optin ? 16 : 0;
+    if (cluster_smem(s) > kClusterSmem || cluster_smem(s) > (size_t)s->smem_optin) return 0;
+    constexpr int64_t per = 32 / ND * kSweepBlocks<ND>;   // blocks of a row that a warp loads at once
+    int64_t loads = 0;
+    for (int64_t i = 0; i < s->n_nodes; ++i) {
+      const int64_t lower = s->f_diag[i] - s->f_rp[i], upper = s->f_rp[i + 1] - s->f_diag[i] - 1;
+      loads += std::max<int64_t>(1, (lower + per - 1) / per) + std::max<int64_t>(1, (upper + per - 1) / per);
+    }
+    const double levels = (double)(s->lev_off_f.size() - 1 + s->lev_off_b.size() - 1);
+    if ((double)loads > kClusterBusy * levels * (kClusterMax * kClusterWarps) ||
+        (double)s->f_col.size() * (ND * ND * sizeof(T)) > kClusterBytes<T> * levels)
+      return 0;
+    int size = kClusterMax;
     if (size && (prepare_cluster<true>(s, size) != cudaSuccess || prepare_cluster<false>(s, size) != cudaSuccess)) {
       cudaGetLastError();
       size = 0;
