@@ -612,8 +612,12 @@ class LinearSolver:
         self._check(self._L.gales_solver_factorize(self._h, _addr(vals), stream or None))
 
     def apply(self, v, z, stream: int = 0):
-        """z = M^-1 v with the current factor (device buffers)."""
+        """z = M^-1 v with the current factor (device buffers), enqueued; check with sync()."""
         self._check(self._L.gales_solver_apply(self._h, _addr(v), _addr(z), stream or None))
+
+    def sync(self, stream: int = 0):
+        """Wait for the stream and raise if a wait of an enqueued apply() ran out."""
+        self._check(self._L.gales_solver_sync(self._h, stream or None))
 
     def factor(self):
         """The factor as node blocks: (row_ptr, col, blocks[nnz_blocks, nd, nd])."""

@@ -198,6 +198,8 @@ def lib() -> C.CDLL:
     L.gales_solver_factorize.restype = C.c_int
     L.gales_solver_apply.argtypes = [vp, vp, vp, vp]
     L.gales_solver_apply.restype = C.c_int
+    L.gales_solver_sync.argtypes = [vp, vp]
+    L.gales_solver_sync.restype = C.c_int
     L.gales_solver_factor.argtypes = [vp, _p(i64), _p(i64), _p(_p(C.c_int64)), _p(_p(C.c_int32)), vp]
     L.gales_solver_factor.restype = C.c_int
     L.gales_solver_levels.argtypes = [vp, _p(i32), _p(i32)]
@@ -241,7 +243,7 @@ EXPORTED = [
     "gales_mesh_read", "gales_mesh_file_desc", "gales_mesh_file_free", "gales_asm_adaptive_dt", "gales_dt_update",
     "gales_asm_secondary_dofs", "gales_pressure_profile", "gales_pressure_interpolate",
     "gales_solver_default", "gales_solver_create", "gales_solver_solve", "gales_solver_factorize",
-    "gales_solver_apply", "gales_solver_factor", "gales_solver_levels", "gales_solver_correct",
+    "gales_solver_apply", "gales_solver_sync", "gales_solver_factor", "gales_solver_levels", "gales_solver_correct",
     "gales_solver_launches", "gales_solver_last_error", "gales_solver_destroy", "gales_iluk_pattern",
     "gales_magma_create", "gales_magma_properties", "gales_magma_status", "gales_magma_last_error",
     "gales_magma_destroy", "gales_asm_set_magma", "gales_asm_magma_fractions",

@@ -290,7 +290,10 @@ __global__ void ilu_factor_level_kernel(T* __restrict__ F, const int64_t* __rest
 // in level order (rows[] lists them level by level) and only ever waits on rows of earlier
 // levels, whose tickets were claimed before its own by CTAs or warps that are running, so
 // these kernels always progress; every wait is still bounded (kSpinMax polls), after which
-// GALES_ERR_TIMEOUT is set in the status word and the row goes on with what it has.
+// GALES_ERR_TIMEOUT is set in a status word and the CTA or warp waits no more: it goes through
+// its rows with what there is.  d_status[0] is the factorisation's word, which the call that runs
+// it reads; d_status[1] the substitutions', which gales_solver_apply leaves to
+// gales_solver_sync or the next factorisation or solve.
 constexpr long long kSpinMax = 1ll << 22;
 
 __device__ __forceinline__ int ld_acquire(const int* f) {
@@ -359,6 +362,7 @@ __global__ void __launch_bounds__(kFactorThreads)
   __shared__ int nm[2], s_row, s_next;
   __shared__ T ls[ND];
   const int tid = threadIdx.x;
+  bool late = false;   // thread 0: a wait ran out
   for (;;) {
     if (tid == 0) {
       const unsigned int t = atomicAdd(ticket, 1u);
@@ -391,7 +395,10 @@ __global__ void __launch_bounds__(kFactorThreads)
     for (int b = 0; b < bd; ++b) {
       const int buf = b & 1;
       if (!have) {
-        if (tid == 0 && !wait_flag(ready + RC[b])) atomicOr(status, (unsigned)GALES_ERR_TIMEOUT);
+        if (tid == 0 && !late && !wait_flag(ready + RC[b])) {
+          late = true;
+          atomicOr(status, (unsigned)GALES_ERR_TIMEOUT);
+        }
         __syncthreads();
         load(b);
       }
@@ -555,6 +562,7 @@ __global__ void __launch_bounds__(32 * kSweepWarps)
   const int lane = threadIdx.x & 31;
   const int g = lane / ND, r = lane < G * ND ? lane - g * ND : 0;
   const int64_t off = jidx ? (int64_t)(*jidx) * ld : 0;
+  bool late = false;
   for (;;) {
     unsigned int t = 0;
     if (lane == 0) t = atomicAdd(ticket, 1u) + 1u;
@@ -570,7 +578,6 @@ __global__ void __launch_bounds__(32 * kSweepWarps)
     for (int c = 0; c < ND; ++c) D[c] = LOWER ? F[pd * BB + r * ND + c] : Us[((int64_t)I * ND + r) * ND + c];
     const T rhs = LOWER ? (T)vbase[off + (int64_t)I * ND + r] : yin[(int64_t)I * ND + r];
     T sum = g == 0 ? -rhs : T(0), sum2 = T(0);
-    bool late = false;
     for (int k0 = 0; k0 < nblk; k0 += KB * G) {
       int64_t zc[KB];
       T B[KB][ND];
@@ -589,12 +596,9 @@ __global__ void __launch_bounds__(32 * kSweepWarps)
 #pragma unroll
       for (int k = 0; k < KB; ++k) {
         if (k0 + k * G >= nblk) break;   // the same for every lane
-        for (long long spin = 0; __any_sync(0xffffffffu, w[k] == W::kUnset); ++spin) {
-          if (spin >= kSpinMax) {
-            late = true;
-            break;
-          }
+        for (long long spin = 0; !late && __any_sync(0xffffffffu, w[k] == W::kUnset); ++spin) {
           if (w[k] == W::kUnset) w[k] = W::load(zw + zc[k]);
+          late = spin >= kSpinMax;
         }
         const T zk = W::value(w[k]);
 #pragma unroll
@@ -605,7 +609,6 @@ __global__ void __launch_bounds__(32 * kSweepWarps)
         }
       }
     }
-    if (late && lane == 0) atomicOr(status, (unsigned)GALES_ERR_TIMEOUT);
     // the groups' sums in a fixed order; s = rhs - sum of the blocks
     sum += sum2;
     T part[G];
@@ -638,6 +641,7 @@ __global__ void __launch_bounds__(32 * kSweepWarps)
       if constexpr (!LOWER) zoutbase[off + (int64_t)I * ND + lane] = (double)s;
     }
   }
+  if (late && lane == 0) atomicOr(status, (unsigned)GALES_ERR_TIMEOUT);
 }
 
 // Small systems: each sweep by one thread-block cluster, whose CTAs hold the whole result vector
@@ -1055,7 +1059,7 @@ struct gales_solver {
   Dev<unsigned char> d_udiag;  // the upper sweep's scaled diagonal blocks (factor's type)
   Dev<unsigned char> d_scaled;  // cluster sweeps in FP64: off-diagonal blocks times their inverse diagonal block
   Dev<unsigned char> d_sweep;  // substitutions: the two result vectors (factor's type), then two tickets
-  Dev<unsigned int> d_status, d_count;  // error bits; CTAs of an Arnoldi pass that are done
+  Dev<unsigned int> d_status, d_count;  // error bits of factorisation and substitutions; CTAs of an Arnoldi pass that are done
   double* h_buf = nullptr;   // pinned: Hessenberg column and the least-squares solution
   int m = 0;                 // Krylov vectors per cycle
   int max_row = 0, max_u = 0;  // longest factor row, longest upper part (blocks)
@@ -1227,24 +1231,24 @@ struct Kernels {
       const cudaError_t e = cudaLaunchKernelEx(
           &l.cfg, ilu_sweep_cluster_kernel<ND, T, true>, S, (const int64_t*)s->d_f_rp.p, (const int32_t*)s->d_f_col.p,
           (const int64_t*)s->d_f_diag.p, (const T*)factor_ptr<T>(s), (const int32_t*)s->d_rows_f.p, s->n_nodes, v, y,
-          (double*)nullptr, j, ld, s->d_status.p);
+          (double*)nullptr, j, ld, s->d_status.p + 1);
       if (e != cudaSuccess) return e;
       return cudaLaunchKernelEx(&l.cfg, ilu_sweep_cluster_kernel<ND, T, false>, S, (const int64_t*)s->d_f_rp.p,
                                 (const int32_t*)s->d_f_col.p, (const int64_t*)s->d_f_diag.p,
                                 reinterpret_cast<const T*>(s->d_udiag.p), (const int32_t*)s->d_rows_b.p, s->n_nodes,
-                                (const double*)nullptr, y, z, j, ld, s->d_status.p);
+                                (const double*)nullptr, y, z, j, ld, s->d_status.p + 1);
     }
     T* x = y + s->n_rows;
     unsigned int* tk = reinterpret_cast<unsigned int*>(x + s->n_rows);
     const unsigned g = (unsigned)std::min<int64_t>((s->n_nodes + kSweepWarps - 1) / kSweepWarps, s->sms);
     ilu_sweep_kernel<ND, T, true><<<g, 32 * kSweepWarps, 0, st>>>(
         factor_ptr<T>(s), s->d_f_rp.p, s->d_f_col.p, s->d_f_diag.p, nullptr, s->d_rows_f.p, s->n_nodes, v, nullptr, y,
-        nullptr, j, ld, tk, s->d_status.p);
+        nullptr, j, ld, tk, s->d_status.p + 1);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     ilu_sweep_kernel<ND, T, false><<<g, 32 * kSweepWarps, 0, st>>>(
         factor_ptr<T>(s), s->d_f_rp.p, s->d_f_col.p, s->d_f_diag.p, reinterpret_cast<const T*>(s->d_udiag.p),
-        s->d_rows_b.p, s->n_nodes, nullptr, y, x, z, j, ld, tk + 1, s->d_status.p);
+        s->d_rows_b.p, s->n_nodes, nullptr, y, x, z, j, ld, tk + 1, s->d_status.p + 1);
     return cudaGetLastError();
   }
   static cudaError_t spmv(gales_solver* s, const double* vals, const double* x, const double* b, double* y,
@@ -1316,6 +1320,15 @@ unsigned stream_grid(int64_t n, int sms) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>(b, (int64_t)sms * 8));
 }
 
+// Waits for the stream and reads both status words; the substitutions' word is cleared, so that
+// a wait that ran out is reported once.
+int read_status(gales_solver* s, cudaStream_t st, unsigned int (&w)[2]) {
+  SCK(s, cudaMemcpyAsync(w, s->d_status.p, sizeof(w), cudaMemcpyDeviceToHost, st), "status");
+  SCK(s, cudaStreamSynchronize(st), "status");
+  if (w[1]) SCK(s, cudaMemsetAsync(s->d_status.p + 1, 0, sizeof(w[1]), st), "clear status");
+  return 0;
+}
+
 int factorize(gales_solver* s, const Ops& o, const double* vals, cudaStream_t st) {
   if (s->prm.precond == GALES_PRECOND_ILU_FP32)
     SCK(s, cudaMemsetAsync(s->d_Ff.p, 0, s->d_Ff.n * sizeof(float), st), "clear factor");
@@ -1326,11 +1339,12 @@ int factorize(gales_solver* s, const Ops& o, const double* vals, cudaStream_t st
   ++s->launches;
   SCK(s, o.factor(s, st), "factorisation");
   SCK(s, o.scale_diag(s, st), "diagonal blocks");
-  unsigned int stat = 0;
-  SCK(s, cudaMemcpyAsync(&stat, s->d_status.p, sizeof(stat), cudaMemcpyDeviceToHost, st), "status");
-  SCK(s, cudaStreamSynchronize(st), "factorisation");
-  if (stat & GALES_ERR_TIMEOUT) return sfail(s, GALES_ERR_TIMEOUT, "a factorisation wait ran out");
-  if (stat) return sfail(s, GALES_ERR_SINGULAR, "zero pivot in the incomplete factorisation");
+  unsigned int w[2];
+  const int rc = read_status(s, st, w);
+  if (rc) return rc;
+  if (w[1]) return sfail(s, GALES_ERR_TIMEOUT, "a substitution wait of an earlier apply ran out");
+  if (w[0] & GALES_ERR_TIMEOUT) return sfail(s, GALES_ERR_TIMEOUT, "a factorisation wait ran out");
+  if (w[0]) return sfail(s, GALES_ERR_SINGULAR, "zero pivot in the incomplete factorisation");
   return 0;
 }
 
@@ -1456,7 +1470,7 @@ int gales_solver_create(gales_asm* h, const gales_solver_params* prm, gales_solv
                   : cudaSuccess) ||
       (has_ilu(s) ? s->d_sweep.alloc(2 * (size_t)n_rows * (p.precond == GALES_PRECOND_ILU ? sizeof(double) : sizeof(float)) +
                                      2 * sizeof(unsigned int))
-                  : cudaSuccess) || s->d_status.alloc(1) || s->d_count.upload(std::vector<unsigned int>(1, 0u))) {
+                  : cudaSuccess) || s->d_status.upload(std::vector<unsigned int>(2, 0u)) || s->d_count.upload(std::vector<unsigned int>(1, 0u))) {
     cudaGetLastError();
     return bail(GALES_ERR_NO_MEMORY);
   }
@@ -1514,6 +1528,15 @@ int gales_solver_apply(gales_solver* s, const double* v, double* z, void* stream
   Ops o;
   ops(s, o);
   return apply_prec(s, o, v, z, nullptr, 0, st);
+}
+
+int gales_solver_sync(gales_solver* s, void* stream) {
+  if (!s) return GALES_ERR_BAD_INPUT;
+  SCK(s, cudaSetDevice(s->device), "cudaSetDevice");
+  unsigned int w[2];
+  const int rc = read_status(s, (cudaStream_t)stream, w);
+  if (rc) return rc;
+  return w[1] ? sfail(s, GALES_ERR_TIMEOUT, "a substitution wait ran out") : 0;
 }
 
 int gales_solver_factor(gales_solver* s, int64_t* n_block_rows, int64_t* nnz_blocks, const int64_t** row_ptr,
@@ -1678,10 +1701,10 @@ int gales_solver_solve(gales_solver* s, const double* vals, const double* rhs, d
     SCK(s, cudaStreamSynchronize(st), "copy x");
   }
   if (prec) {  // a substitution wait that ran out (not expected on a working device)
-    unsigned int stat = 0;
-    SCK(s, cudaMemcpyAsync(&stat, s->d_status.p, sizeof(stat), cudaMemcpyDeviceToHost, st), "status");
-    SCK(s, cudaStreamSynchronize(st), "status");
-    if (stat & GALES_ERR_TIMEOUT) return sfail(s, GALES_ERR_TIMEOUT, "a substitution wait ran out");
+    unsigned int w[2];
+    rc = read_status(s, st, w);
+    if (rc) return rc;
+    if (w[1]) return sfail(s, GALES_ERR_TIMEOUT, "a substitution wait ran out");
   }
   if (res) {
     res->iterations = iters;

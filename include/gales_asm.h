@@ -330,9 +330,14 @@ int gales_solver_create(gales_asm* h, const gales_solver_params* p, gales_solver
 int gales_solver_solve(gales_solver* s, const double* vals, const double* rhs, double* x, gales_solver_result* res,
                        void* stream);
 /* The factorisation alone (synchronises), and z = M^-1 v with the current factor
- * (device arrays, enqueued on the stream). */
+ * (device arrays, enqueued on the stream).  The kernels' waits on one another are bounded;
+ * one that runs out (not expected on a working device) is GALES_ERR_TIMEOUT, of an apply
+ * from gales_solver_sync or else from the next factorize or solve. */
 int gales_solver_factorize(gales_solver* s, const double* vals, void* stream);
 int gales_solver_apply(gales_solver* s, const double* v, double* z, void* stream);
+/* Waits for the stream; GALES_ERR_TIMEOUT if a wait of an apply since the last report ran
+ * out. */
+int gales_solver_sync(gales_solver* s, void* stream);
 /* The factor as node blocks: the block pattern (host arrays owned by the solver) and,
  * when vals is not NULL, nnz_blocks * nd * nd values (block-major, row-major blocks;
  * unit L strictly below the diagonal, U on and above it).  Synchronises the device. */
