@@ -114,3 +114,33 @@ extern "C" int solver_wait_runs_out(int kernel) {
   if (cudaMemcpy(&w, s->d_status.p + 1, sizeof(w), cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
   return (int)w;
 }
+
+// The three Arnoldi passes over nv columns of n rows (V column-major): out_h = V^T w, then w,
+// out_h2 and out_h of kSubDots, then w and the norm of kSubNorm; 0 or a CUDA error.
+extern "C" int solver_arnoldi(const double* V, int64_t n, int nv, double* w, double* h, double* h1, double* h2, double* w1,
+                              double* hn) {
+  const int blocks = (int)((n + kTile - 1) / kTile);
+  double *dV, *dw, *dh, *dh2, *dn, *part;
+  unsigned int* count;
+  cudaMalloc(&dV, (size_t)n * nv * 8);
+  cudaMalloc(&dw, n * 8);
+  cudaMalloc(&dh, nv * 8);
+  cudaMalloc(&dh2, nv * 8);
+  cudaMalloc(&dn, 8);
+  cudaMalloc(&part, (size_t)blocks * nv * 8);
+  cudaMalloc(&count, sizeof(unsigned int));
+  cudaMemset(count, 0, sizeof(unsigned int));
+  cudaMemcpy(dV, V, (size_t)n * nv * 8, cudaMemcpyHostToDevice);
+  cudaMemcpy(dw, w, n * 8, cudaMemcpyHostToDevice);
+  arnoldi_kernel<kDots><<<blocks, kDotThreads>>>(dV, n, nv, dw, n, dh, dh2, nullptr, part, count);
+  cudaMemcpy(h, dh, nv * 8, cudaMemcpyDeviceToHost);
+  arnoldi_kernel<kSubDots><<<blocks, kDotThreads>>>(dV, n, nv, dw, n, dh, dh2, nullptr, part, count);
+  cudaMemcpy(h1, dh, nv * 8, cudaMemcpyDeviceToHost);
+  cudaMemcpy(h2, dh2, nv * 8, cudaMemcpyDeviceToHost);
+  cudaMemcpy(w1, dw, n * 8, cudaMemcpyDeviceToHost);
+  arnoldi_kernel<kSubNorm><<<blocks, kDotThreads>>>(dV, n, nv, dw, n, dh, dh2, dn, part, count);
+  cudaMemcpy(w, dw, n * 8, cudaMemcpyDeviceToHost);
+  cudaMemcpy(hn, dn, 8, cudaMemcpyDeviceToHost);
+  for (void* p : {(void*)dV, (void*)dw, (void*)dh, (void*)dh2, (void*)dn, (void*)part, (void*)count}) cudaFree(p);
+  return (int)cudaGetLastError();
+}
