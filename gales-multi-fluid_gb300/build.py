@@ -22,9 +22,9 @@ SOURCES = (["gales_host.cu", "gales_mesh_io.cu", "gales_solver.cu", "gales_magma
            + [f"gales_vjp_{t}.cu" for t in ("hex8", "tet4", "tri3", "quad4")]
            + [f"gales_{t}_magma_{f}.cu" for t in ("hex8", "tet4", "tri3", "quad4") for f in ("fp64", "mixed")])
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-# -fmad=false: no implicit contraction in the FP64 form's units, whose boundary fluxes, time
-# step and secondary variables perform the reference's IEEE operations (see
-# gales_physics.cuh); the mixed form's and the adjoint's units contract freely (the few steps
+# -fmad=false: no implicit contraction in the FP64 form's units, whose interpolated gradients,
+# boundary fluxes, time step and secondary variables perform the reference's IEEE operations
+# (with a mixture of chemicals; see gales_physics.cuh); the mixed form's and the adjoint's units contract freely (the few steps
 # whose rounding must match use unfused intrinsics).
 FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-fmad=false", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
          "-Xcompiler", "-ffp-contract=off"]

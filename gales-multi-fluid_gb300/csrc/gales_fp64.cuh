@@ -985,7 +985,7 @@ __device__ __forceinline__ void simplex_row64(const KParams& k, const double* __
         }
       }
       if constexpr (!total) {
-        // viscous and diffusive terms (fluid_2d.hpp:531-571; see add_viscous_row)
+        // viscous and diffusive terms (fluid_2d.hpp:531-571; the closed form beside viscous_row32)
         if constexpr (rV) {
           const double p1 = kmu * ga[J], p2 = (-2.0 / 3.0) * kmu * gb[J];
 #pragma unroll

@@ -660,9 +660,9 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
   R Ur[ND];  // U in the form's type (discontinuity capturing); U[0] = rho
 #pragma unroll
   for (int j = 0; j < ND; ++j) Ur[j] = j == 0 ? cr.rho : to_s<R>(U[j]);
-  // tau (fluid_2d.hpp:877-1022).  The branches give its diagonal parameters td; the FP64
-  // form then forms DUDY^{-1} diag(td) by LU, the mixed form in closed form, narrowed to
-  // FP32 entry by entry and only where it can be nonzero (tau_nz).
+  // tau (fluid_2d.hpp:877-1022).  The branches give its diagonal parameters td;
+  // DUDY^{-1} diag(td) follows in closed form, narrowed to FP32 entry by entry and only where
+  // it can be nonzero (tau_nz).
   R tau[ND][ND];
 #pragma unroll
   for (int r = 0; r < ND; ++r)
@@ -941,37 +941,6 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
   if (!finite_bits(JxW) || !finite_bits(pr.rho) || !isfinite(nu)) flag_error(k, GALES_ERR_NONFINITE, e);
 }
 
-// Viscous/diffusive tangent contracted with the test-function gradient gb:
-// sum_k gb_k K_kl(r, col), in closed form from the entries of K_kl
-// (fluid_2d.hpp:531-571): K_kl(1+j, v_m) = mu d_lk d_mj + mu d_lj d_mk + lambda d_kj d_lm,
-// K_kl(E, v_m) = sum_j v_j K_kl(1+j, v_m), K_kk(E, T) = kappa, K_kk(E, Y_i) = rho D_i H_i,
-// K_kk(Y_i, Y_i) = rho D_i.  gbv = gb . v.
-template <int DIM, int NC, typename S, typename C>
-__device__ __forceinline__ S kd_entry(const C& c, const S* gb, S gbv, int l, int r, int col) {
-  using L = Layout<DIM, NC>;
-  if (r == 0 || col == 0) return S(0);
-  if (r < L::iT) {
-    if (col >= L::iT) return S(0);
-    const int j = r - 1, m = col - 1;
-    S x = S(0);
-    if (m == j) x += c.mu * gb[l];
-    if (l == j) x += c.mu * gb[m];
-    if (l == m) x += c.lambda * gb[j];
-    return x;
-  }
-  if (r == L::iT) {
-    if (col < L::iT) {
-      const int m = col - 1;
-      S x = c.mu * (gb[l] * c.v[m] + c.v[l] * gb[m]);
-      if (l == m) x += c.lambda * gbv;
-      return x;
-    }
-    if (col == L::iT) return c.kappa * gb[l];
-    return c.rhoDH[col - L::iY] * gb[l];
-  }
-  return (col == r) ? c.rhoD[r - L::iY] * gb[l] : S(0);
-}
-
 // Exact widening of binary32 to binary64 with 32-bit integer operations only (see
 // narrow_rn): exponent rebias 127 -> 1023, the 23-bit significand split over the two
 // words; subnormals normalised, infinities and NaN keep their payload.
@@ -1152,7 +1121,8 @@ __global__ void __launch_bounds__(128) adaptive_dt_kernel(const KParams k, doubl
 // Secondary variables at the nodes, secondary_dofs::execute (secondary_dofs.hpp:56-101):
 // the mixture properties of every node's state at shear rate 0, written word-major:
 // out[f * n + node] for f = rho, mu, cp, cv, alpha, beta, kappa, sound speed (the
-// order of 146-153).  FP64 with the reference's operations (FP64 units).
+// order of 146-153).  FP64 with the reference's operations (FP64 units); a mixture of magmas in
+// the rearranged order of gales_magma_fast.cuh.
 template <int DIM, int NC, int EOS = kEosChemicals>
 __global__ void __launch_bounds__(128) secondary_dofs_kernel(const KParams k, double* __restrict__ out, long long n) {
   using L = Layout<DIM, NC>;

@@ -34,14 +34,6 @@ struct InteriorInst {
   // at most (n + rec_block()) rec_bytes()
   static size_t rec_bytes() { return RB::BYTES / RB::EB; }
   static int rec_block() { return RB::EB; }
-  // resident point-kernel CTAs (128 threads) per SM
-  static int point_occupancy() {
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, point_kernel<DIM, NEN, NC, NQ, S, EOS>, 128, 0) !=
-        cudaSuccess)
-      return 1;
-    return nb > 0 ? nb : 1;
-  }
   static LaunchResult point(const KParams& k, bool, void* buf, long long first, long long n, cudaStream_t st) {
     if (n <= 0) return {cudaSuccess, 0};
     const long long threads = n * NQ;
@@ -85,13 +77,6 @@ struct Simplex64Inst {
   static constexpr size_t kSmem = sizeof(Rows64Smem<DIM, NC>);
   static size_t rec_bytes() { return R::ELEM_BYTES; }
   static int rec_block() { return R::EB; }
-  static int point_occupancy() {
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, point64_kernel<DIM, NEN, NC, EOS, true>, 128, 0) !=
-        cudaSuccess)
-      return 1;
-    return nb > 0 ? nb : 1;
-  }
   static cudaError_t prepare() {
     return cudaFuncSetAttribute(rows64_kernel<DIM, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kRows64Warps * kSmem));
   }
@@ -127,13 +112,6 @@ struct Tensor64Inst {
   static constexpr size_t kSmem = sizeof(typename T::Smem);
   static size_t rec_bytes() { return R::ELEM_BYTES; }
   static int rec_block() { return R::EB; }
-  static int point_occupancy() {
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, point64_kernel<DIM, NEN, NC, EOS, true>, 128, 0) !=
-        cudaSuccess)
-      return 1;
-    return nb > 0 ? nb : 1;
-  }
   static cudaError_t prepare() {
     return cudaFuncSetAttribute(tensor64_kernel<DIM, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
   }
@@ -186,7 +164,6 @@ LaunchResult launch_boundary_nc(const KParams& k, long long n_items, cudaStream_
 // stage and matrix stage, for 1..4 components.
 struct InteriorOps {
   cudaError_t (*prepare)(int nc);
-  int (*point_occupancy)(int nc);
   size_t (*rec_bytes)(int nc);
   int (*rec_block)(int nc);
   LaunchResult (*point)(const KParams&, int nc, bool want_m, void* buf, long long first, long long n, cudaStream_t);
@@ -217,12 +194,6 @@ struct InteriorDispatch {
 #undef GALES_C
     return cudaErrorInvalidValue;
   }
-  static int point_occupancy(int nc) {
-#define GALES_C(NC) return I<NC>::point_occupancy()
-    GALES_NC_SWITCH(nc, GALES_C)
-#undef GALES_C
-    return 1;
-  }
   static size_t rec_bytes(int nc) {
 #define GALES_C(NC) return I<NC>::rec_bytes()
     GALES_NC_SWITCH(nc, GALES_C)
@@ -249,7 +220,7 @@ struct InteriorDispatch {
 #undef GALES_C
     return {cudaErrorInvalidValue, 0};
   }
-  static InteriorOps ops() { return {&prepare, &point_occupancy, &rec_bytes, &rec_block, &point, &matrix}; }
+  static InteriorOps ops() { return {&prepare, &rec_bytes, &rec_block, &point, &matrix}; }
 };
 
 // Boundary pass of one element type; S is the matrix arithmetic type of the form.

@@ -1,7 +1,8 @@
-// The mixture of sub-mixtures as the assembly's point stages take it: mix_point of
-// gales_magma.cuh rearranged for few FP64 operations (see magma_props), the same to rounding,
-// and rho and cv alone for the state at the previous time level.  The property calls and the
-// gas fractions keep gales_magma.cuh's operations, which follow the reference's one by one.
+// The mixture of sub-mixtures as the assembly takes it (interior and boundary points), the time
+// step and the secondary variables: mix_point of gales_magma.cuh rearranged for few FP64
+// operations (see magma_props), the same to rounding, and rho and cv alone for the state at the
+// previous time level.  The property calls and the gas fractions keep gales_magma.cuh's
+// operations, which follow the reference's one by one.
 // Also built for the host by the CPU tests.
 #pragma once
 

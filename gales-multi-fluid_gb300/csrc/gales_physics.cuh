@@ -19,14 +19,14 @@ namespace gales {
 
 constexpr double kEps = 2.220446049250313e-16;  // DBL_EPSILON, fluid_2d.hpp:93
 
-// The library is compiled without floating-point contraction (-fmad=false) so that
-// the point-level physics performs exactly the IEEE operations of the reference, in
+// The FP64 units are compiled without floating-point contraction (-fmad=false): what is
+// written as the reference's operations there (interpolated gradients, boundary fluxes, time
+// step, secondary variables, compute_h where it is undecided) performs its IEEE operations in
 // its order.  This matters beyond rounding: compute_h (quad.hpp:367-375) decides
 // between normalising and not normalising the cross-stream direction from a value
 // that is pure rounding noise whenever the element's velocity field is rank one
 // (e.g. every node but one on a no-slip wall), so only identical arithmetic takes
-// identical branches.  The matrix-phase loops, whose summation order is already
-// restructured, request fused multiply-adds explicitly through madd().
+// identical branches.  Everything else requests fused multiply-adds explicitly (fma, madd()).
 __device__ __forceinline__ double madd(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float madd(float a, float b, float c) { return fmaf(a, b, c); }
 

@@ -481,7 +481,9 @@ __global__ void __launch_bounds__(32 * NEN, NEN == 8 ? 2 : 5) rows32_kernel(cons
   const int r = (int)(u / nc);
   const long long b0 = c0 + u % nc;
   const int cnt = (int)(n - b0 * EB < EB ? n - b0 * EB : EB);
-  const int l = lane < cnt ? lane : cnt - 1;   // idle lanes of a last block repeat its last element
+  // Idle lanes of a last block take the scatter words of its last element; their record words
+  // are whatever the buffer holds there, and nothing that they form is stored (below cnt alone).
+  const int l = lane < cnt ? lane : cnt - 1;
   unsigned char* blk = in + (size_t)b0 * RB::BYTES;
   const float* rec = reinterpret_cast<const float*>(blk);
   if (threadIdx.x == 0) {

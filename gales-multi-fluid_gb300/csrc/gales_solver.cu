@@ -1117,8 +1117,6 @@ struct Kernels {
         vals, s->d_node_rp.p, s->d_a2f.p, s->n_nodes, factor_ptr<T>(s));
     return cudaGetLastError();
   }
-  // The persistent factorisation where a block row and two rows' upper parts fit the shared
-  // memory of an SM; rows too long for that take the level launches on global memory.
   // A launch of one cluster of `size` CTAs.
   struct ClusterLaunch {
     cudaLaunchAttribute at[1];
@@ -1174,6 +1172,8 @@ struct Kernels {
     }
     return size;
   }
+  // The persistent factorisation where a block row and two rows' upper parts fit the shared
+  // memory of an SM; rows too long for that take the level launches on global memory.
   static cudaError_t prepare(gales_solver* s) {
     const size_t bytes = FactorSmem<ND, T>::bytes(s->max_row, s->max_u);
     s->factor_smem = 0;
