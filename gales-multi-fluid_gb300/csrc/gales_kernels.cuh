@@ -634,6 +634,12 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
   for (int d = 1; d < DIM; ++d) vv = fma(v[d], v[d], vv);
   make_coef_fast<DIM, NC>(pr, p, v, vv, T, Y, c);
   conservative<DIM, NC>(pr.rho, pr.cv, v, T, Y, U);
+  // the difference at once: U_P is not needed again, and held to the record's store below it took
+  // registers whose spills cost the point stage of hexahedra with 8 dofs 14% (5.8 against 6.7 ms
+  // for 570,000)
+  R dUt[ND];
+#pragma unroll
+  for (int j = 0; j < ND; ++j) dUt[j] = narrow_rn(sub_rn(U[j], UP[j]));
   iv = rsqrt(vv);
   v_nrm = vv > 0.0 ? vv * iv : 0.0;
   const double dt = k.dt;
@@ -656,7 +662,7 @@ __device__ void point_phase(const KParams& k, long long e, int iq, const RecOut<
   SvR[L::iT] = rf * gv;
   const float idt = k.inv_dt_f;
 #pragma unroll
-  for (int j = 0; j < ND; ++j) GALES_RECA(row, j * QPT::RP) = fmaf(narrow_rn(U[j] - UP[j]), idt, -SvR[j]);
+  for (int j = 0; j < ND; ++j) GALES_RECA(row, j * QPT::RP) = fmaf(dUt[j], idt, -SvR[j]);
   R Ur[ND];  // U in the form's type (discontinuity capturing); U[0] = rho
 #pragma unroll
   for (int j = 0; j < ND; ++j) Ur[j] = j == 0 ? cr.rho : to_s<R>(U[j]);
