@@ -287,9 +287,10 @@ __device__ __forceinline__ void directions(const ElemGeo<DIM, NEN>& q, double (&
   }
 }
 
-// The point stage of one (element, point): about 1,100 FP64 operations, the FP64 pipe 84% busy
-// (7.5 ms for 4.0M points; 29 with the reference's operations one by one, among them the LU
-// inverse of DUDY, two mixtures with a division per component and 20 more divisions).  l is the element's place in its block.
+// The point stage of one (element, point): about 1,130 FP64 operations, the FP64 pipe 84% busy
+// (7.8 ms for 4.0M points, 0.3 of them the unfused gradients; 29 with the reference's operations
+// one by one, among them the LU inverse of DUDY, two mixtures with a division per component and 20
+// more divisions).  l is the element's place in its block.
 template <int DIM, int NEN, int NC, int EOS, bool WANT_M>
 __device__ __forceinline__ void point64(const KParams& k, long long e, int iq, double* __restrict__ blk, int l) {
   using L = Layout<DIM, NC>;
